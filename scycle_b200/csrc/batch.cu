@@ -67,9 +67,12 @@ __global__ void b_bc_kernel(const BatchInst* __restrict__ tab, const int* __rest
   if (I.bcR_remote) I.bcR[i] = I.vL * te * I.inv_fts + I.bcRShift[i];
 }
 
-// rhs = setRhs(bc) (+ B gVxy + C gVxz for the power law); |rhs|^2 -> sc[0]
+// rhs = setRhs(bc) (+ B gVxy + C gVxz for the power law); |rhs|^2 -> sc[0].
+// carry: w.r is the residual -rhs + A u of the instance's previous solve and
+// takes the change of the rhs, so the next solve starts from it without
+// applying the operator.
 __global__ void b_rhs_kernel(LevelDev<double> L, const BatchInst* __restrict__ tab, const int* __restrict__ mask,
-                             int in_slot, BatchWork w) {
+                             int in_slot, BatchWork w, int carry) {
   __shared__ double sh[32];
   const int k = blockIdx.z;
   if (!mask[k]) return;
@@ -80,6 +83,7 @@ __global__ void b_rhs_kernel(LevelDev<double> L, const BatchInst* __restrict__ t
   for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < w.N; node += (long)gridDim.x * blockDim.x) {
     double v = set_rhs_node(L, I.bcL, I.bcR, I.bcT, I.bcB, node);
     if (gxy) v = v + 1.0 * pl_source_node(L, gxy, gxz, node);
+    if (carry) w.r[(long)k * w.N + node] += I.rhs[node] - v;
     I.rhs[node] = v;
     acc += v * v;
   }
@@ -94,7 +98,7 @@ __global__ void b_rhs_kernel(LevelDev<double> L, const BatchInst* __restrict__ t
 // rewritten.  Frame index f < 2 * BAND * Nz: rows 0..BAND-1 and Ny-BAND..Ny-1;
 // after that, columns 0..BAND-1 and Nz-BAND..Nz-1 of the rows in between.
 __global__ void b_rhs_frame_kernel(LevelDev<double> L, const BatchInst* __restrict__ tab,
-                                   const int* __restrict__ mask, BatchWork w, int nframe) {
+                                   const int* __restrict__ mask, BatchWork w, int nframe, int carry) {
   __shared__ double sh[32];
   const int k = blockIdx.z;
   if (!mask[k]) return;
@@ -114,6 +118,7 @@ __global__ void b_rhs_frame_kernel(LevelDev<double> L, const BatchInst* __restri
     }
     const long node = (long)iy * Nz + iz;
     const double v = set_rhs_node(L, I.bcL, I.bcR, I.bcT, I.bcB, node);
+    if (carry) w.r[(long)k * w.N + node] += I.rhs[node] - v;
     I.rhs[node] = v;
     acc += v * v;
   }
@@ -429,7 +434,7 @@ __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, c
     if (MODE == 1 && first) cs[1][r0 + j][lane] = a2;
     a1 = a2 = 0.0;
   };
-  if (MODE == 0) {
+  if constexpr (MODE == 0) {
     const double* u = tab[k].u;
     const double* rhs = tab[k].rhs;
     const bool zero = sc[0] == 0.0;
@@ -439,6 +444,26 @@ __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, c
       const double v = zero ? 0.0 : -1.0 * b + Ax;
       w.r[off + node] = v;
       if (mixed) w.r32[off + node] = (float)v;
+      a1 = v * v;
+    };
+    full_apply<double, RPT>(L, ld, pre, out, row, xs);
+  } else if constexpr (MODE == 2) {
+    // defect correction with z = P r: u += z, r += A z (zero where rhs = 0);
+    // an instance whose z is not P r because a pipeline wait ran out on the
+    // way (status bit 4, the round is repeated) keeps its u and r
+    const Tz* z = zv + off;
+    double* r = w.r + off;
+    double* u = tab[k].u;
+    const bool zero = sc[0] == 0.0, lost = (w.status[k] & 4u) != 0;
+    struct UR {
+      double u, r;
+    };
+    auto ld = [&](long node, int, int) { return (double)z[node]; };
+    auto pre = [&](long node, int, int) { return UR{u[node], r[node]}; };
+    auto out = [&](long node, int, int, double Az, double zz, const UR& p) {
+      const double v = zero ? 0.0 : lost ? p.r : p.r + Az;
+      r[node] = v;
+      u[node] = zero ? 0.0 : lost ? p.u : p.u + zz;
       a1 = v * v;
     };
     full_apply<double, RPT>(L, ld, pre, out, row, xs);
@@ -510,6 +535,27 @@ static void launch_full(const BatchGroup& g, int shape, const BatchInst* tab, co
     default: SCY_FULL_LAUNCH(4, 4); break;
   }
 #undef SCY_FULL_LAUNCH
+}
+
+// End of a defect correction: sc[16 k + 1] = r.r from the instance's n
+// partials in tile order, and its test; status bit 1: residual above
+// max(rtol |rhs|, atol); bit 2: non-finite
+__global__ void b_partials_verify_kernel(const int* __restrict__ mask, BatchWork w, int n, double rtol, double atol) {
+  __shared__ double sh[32];
+  const int k = blockIdx.x;
+  if (!mask[k]) return;
+  const double* p = w.partials + (long)k * w.PB;
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += p[i];
+  acc = block_sum(acc, sh);
+  if (threadIdx.x == 0) {
+    double* sc = w.sc + 16 * k;
+    sc[1] = acc;
+    if (!isfinite(acc))
+      atomicOr(w.status + k, 2u);
+    else if (!(sqrt(acc) <= fmax(rtol * sqrt(sc[0]), atol)))
+      atomicOr(w.status + k, 1u);
+  }
 }
 
 // sc[16 k + slot] = sum of the instance's first n partials (of w.partials,
@@ -929,6 +975,7 @@ int BatchContext::create(int n_inst, const char* const* paths, const scy_solve_o
   SCY_CUDA_TRY(cudaMemset(err.p, 0, (size_t)n * 16 * sizeof(double)));
   SCY_CUDA_TRY(cudaMallocHost((void**)&err_host, (size_t)n * 16 * sizeof(double)));
   hc.assign(n, Ctl());
+  carried.assign(n, 0);
   // segment tables of the state and fault-field transfers, in the caller's
   // numbering
   {
@@ -1204,11 +1251,10 @@ int BatchContext::launch_ysolve(BatchGroup& g, int variant) {
 // banded sweeps in their three launch shapes; keeps the fastest of each.
 // The sweep's status words are cleared afterwards.
 int BatchContext::autotune(BatchGroup& g) {
-  DevBuf ones;
-  SCY_TRY(ones.alloc((size_t)g.K * sizeof(int)));
+  SCY_TRY(g.ones.alloc((size_t)g.K * sizeof(int)));
   std::vector<int> h(g.K, 1);
-  SCY_CUDA_TRY(cudaMemcpy(ones.p, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
-  const int* mask = ones.as<int>();
+  SCY_CUDA_TRY(cudaMemcpy(g.ones.p, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
+  const int* mask = g.ones.as<int>();
   cudaEvent_t e0, e1;
   SCY_CUDA_TRY(cudaEventCreate(&e0));
   SCY_CUDA_TRY(cudaEventCreate(&e1));
@@ -1265,12 +1311,26 @@ int BatchContext::autotune(BatchGroup& g) {
   // b_full_kernel); the cross form's timings stay for comparison
   g.full_shape = -1;
   if (g.L.full) {
+    // defect correction where the preconditioner is near enough to the
+    // inverse; its launch moves u, so it is timed on a table whose u is a
+    // work vector
+    g.refine = precision == SCY_PREC_FP64 && q(g.base).sbp.near_inverse() && g.fd->ybanded && !fd_dense;
+    DevBuf scratch;
+    if (g.refine) {
+      std::vector<BatchInst> t(g.K);
+      SCY_CUDA_TRY(cudaMemcpy(t.data(), g.tab.p, sizeof(BatchInst) * g.K, cudaMemcpyDeviceToHost));
+      for (int k = 0; k < g.K; ++k) t[k].u = g.w.p0 + (long)k * g.N;
+      SCY_TRY(scratch.alloc(sizeof(BatchInst) * g.K));
+      SCY_CUDA_TRY(cudaMemcpy(scratch.p, t.data(), sizeof(BatchInst) * g.K, cudaMemcpyHostToDevice));
+    }
     best_us = 1e300;
     for (int c = 0; c < kFullShapes; ++c) {
       double us = 0.0;
       int rc = timed(
           [&]() -> int {
-            if (mixed)
+            if (g.refine)
+              launch_full<2, double>(g, c, scratch.as<BatchInst>(), mask, g.w.z, 0, 0, 0, 0);
+            else if (mixed)
               launch_full<1, float>(g, c, tab, mask, g.w.z32, 1, 0, mixed, 1);
             else
               launch_full<1, double>(g, c, tab, mask, g.w.z, 1, 0, mixed, 1);
@@ -1495,6 +1555,39 @@ int BatchContext::fd_apply(BatchGroup& g) {
   return SCY_OK;
 }
 
+// its_now defect corrections of every masked instance (g.refine: the
+// preconditioner is the inverse up to rounding and the last z column, see
+// SbpContext::near_inverse): z = P r, then u += z and r += A z in one
+// launch.  carry: r already is -rhs + A u (the previous solve left it and
+// the rhs kernel added the change of the rhs); otherwise it is formed here,
+// once per accepted step, so that the rounding of the recurrence does not
+// add up over the run.  At 32 x 401 x 401 a stage solve took the residual
+// (67 us), the CG product (75), the update (46) and three partial sums (15)
+// beside the preconditioner.
+int BatchContext::solve_refine(BatchGroup& g, const int* mask, int its_now, int carry) {
+  const int shape = g.full_shape;
+  const BatchInst* tab = g.tab.as<BatchInst>();
+  const int ntiles = (int)(((g.Nz + XTZ - 1) / XTZ) * ((g.Ny + XTY - 1) / XTY));
+  const double nact = (double)active_in(g, mask);
+  cudaEvent_t pa;
+  if (!carry) {
+    SCY_TRY(prof_begin(g.stream, &pa));
+    launch_full<0, double>(g, shape, tab, mask, (const double*)nullptr, 0, 0, 0, 0);
+    SCY_LAUNCH_CHECK();
+    SCY_TRY(prof_end(g.stream, pa, PROF_RESIDUAL, nact * g.N * 24.0));
+  }
+  for (int it = 1; it <= its_now; ++it) {
+    SCY_TRY(fd_apply(g));
+    SCY_TRY(prof_begin(g.stream, &pa));
+    launch_full<2, double>(g, shape, tab, mask, g.w.z, 0, 0, 0, 0);
+    SCY_LAUNCH_CHECK();
+    SCY_TRY(prof_end(g.stream, pa, PROF_MATVEC, nact * g.N * 40.0));
+  }
+  b_partials_verify_kernel<<<g.K, 256, 0, g.stream>>>(mask, g.w, ntiles, rtol, atol);
+  SCY_LAUNCH_CHECK();
+  return SCY_OK;
+}
+
 int BatchContext::solve(BatchGroup& g, const int* mask, int its_now) {
   const int mixed = precision != SCY_PREC_FP64 ? 1 : 0;
   const int shape = g.full_shape, rpt = shape >= 0 ? kFullRpt[shape] : 0;  // rpt > 0: the separable form
@@ -1563,7 +1656,9 @@ int BatchContext::solve(BatchGroup& g, const int* mask, int its_now) {
   return SCY_OK;
 }
 
-int BatchContext::d_dt(BatchGroup& g, const int* mask, double c, int in_slot, int out_slot, int its_now) {
+int BatchContext::d_dt(BatchGroup& g, const int* mask, double c, int in_slot, int out_slot, int its_now,
+                       int fresh) {
+  const int carry = g.refine && !fresh ? 1 : 0;
   const BatchInst* tab = g.tab.as<BatchInst>();
   const dim3 fg((g.Nz + 63) / 64, 1, g.K);
   const dim3 ng(node_blocks(g.N), 1, g.K);
@@ -1572,12 +1667,15 @@ int BatchContext::d_dt(BatchGroup& g, const int* mask, double c, int in_slot, in
   if (!pl && g.Ny > 2 * BAND && g.Nz > 2 * BAND) {
     const int nframe = 2 * BAND * g.Nz + (g.Ny - 2 * BAND) * 2 * BAND;
     const dim3 rg((nframe + TB - 1) / TB < 64 ? (nframe + TB - 1) / TB : 64, 1, g.K);
-    b_rhs_frame_kernel<<<rg, TB, 0, g.stream>>>(g.L, tab, mask, g.w, nframe);
+    b_rhs_frame_kernel<<<rg, TB, 0, g.stream>>>(g.L, tab, mask, g.w, nframe, carry);
   } else {
-    b_rhs_kernel<<<ng, TB, 0, g.stream>>>(g.L, tab, mask, in_slot, g.w);
+    b_rhs_kernel<<<ng, TB, 0, g.stream>>>(g.L, tab, mask, in_slot, g.w, carry);
   }
   SCY_LAUNCH_CHECK();
-  SCY_TRY(solve(g, mask, its_now));
+  if (g.refine)
+    SCY_TRY(solve_refine(g, mask, its_now, carry));
+  else
+    SCY_TRY(solve(g, mask, its_now));
   if (pl) {
     b_pl_rates_kernel<<<ng, TB, 0, g.stream>>>(g.L, tab, mask, in_slot, out_slot, g.N);
     SCY_LAUNCH_CHECK();
@@ -1615,7 +1713,7 @@ int BatchContext::enqueue_group(BatchGroup& g, int its_now, int phases) {
   if (phases & 1) {
     b_copy_kernel<<<dim3(node_blocks(nv), 1, g.K), TB, 0, g.stream>>>(tab, mc);
     SCY_LAUNCH_CHECK();
-    SCY_TRY(d_dt(g, ma, 0.0, V_VAR, V_DVAR, its_now));
+    SCY_TRY(d_dt(g, ma, 0.0, V_VAR, V_DVAR, its_now, 1));
   }
   if (!(phases & 2)) {
     // no attempt this round: only the status words
@@ -1796,6 +1894,7 @@ int BatchContext::run(long nsteps, scy_batch_stats* st) {
     hc[i].copy = hc[i].acc = 0;
     begin_step(i);
   }
+  SCY_TRY(refresh_residuals());
   const int stages = method == SCY_RK32 ? 2 : 5;
   double* t = static_cast<double*>(ctl_host);
   double* dt = t + n;
@@ -1887,7 +1986,29 @@ int BatchContext::run(long nsteps, scy_batch_stats* st) {
       if (h.running) consume(i, c.error_from(err_host + 16 * i));
     }
   }
+  for (int i = 0; i < n; ++i) carried[i] = q(i).u_epoch;
   stats(st);
+  return SCY_OK;
+}
+
+// The carried residual of every instance whose displacement or rhs anything
+// but this batch's rounds has changed since the last run (a solve through
+// the instance's own handle, or a run that ended with an error).
+int BatchContext::refresh_residuals() {
+  for (auto& G : groups) {
+    BatchGroup& g = *G;
+    if (!g.refine) continue;
+    bool all = true;
+    for (int k = 0; k < g.K; ++k) all = all && carried[g.base + k] == q(g.base + k).u_epoch;
+    if (!all) {
+      launch_full<0, double>(g, g.full_shape, g.tab.as<BatchInst>(), g.ones.as<int>(), (const double*)nullptr, 0, 0,
+                             0, 0);
+      SCY_LAUNCH_CHECK();
+      SCY_CUDA_TRY(cudaStreamSynchronize(g.stream));
+    }
+  }
+  // until this run ends well
+  for (int i = 0; i < n; ++i) carried[i] = 0;
   return SCY_OK;
 }
 

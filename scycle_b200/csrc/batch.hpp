@@ -74,6 +74,8 @@ struct BatchGroup {
   int ys_variant = 0;  // chains per lane x warps per block of the banded sweeps (autotuned)
   int zt_pair = 0;  // z-transform products: 0 one CTA per tile, 1 two CTAs per SM, 2 persistent (autotuned)
   int zt_bf16 = 0;  // z-transform digits in bf16 (kind::f16) instead of 8-bit integers (autotuned)
+  int refine = 0;  // stage solves by defect correction with a carried residual (solve_refine) instead of CG
+  DevBuf ones;     // a mask that selects every instance
   int full_shape = -1;  // >= 0: the operator kernels in the separable form, in this launch shape (autotuned)
   // the autotuner's timings: kpb 1, 2, 4, 8; sweep variants 0..5;
   // z-transform product with 8-bit digits in the one- and two-CTAs-per-SM
@@ -135,6 +137,8 @@ struct BatchContext {
     long done_steps = 0, target = 0;
   };
   std::vector<Ctl> hc;
+  // per instance: the QDContext::u_epoch its carried residual belongs to (0: none)
+  std::vector<unsigned long long> carried;
   // the states and fault fields move between the caller's array and the
   // instances as one transfer through a staging buffer, scattered or
   // gathered by a kernel (IoSeg tables: the states, then one per field)
@@ -176,8 +180,11 @@ struct BatchContext {
   int enqueue_round(int its_now, int phases);
   int launch_round(int its_now, int phases);
   int enqueue_group(BatchGroup& g, int its_now, int phases);
-  int d_dt(BatchGroup& g, const int* mask, double c, int in_slot, int out_slot, int its_now);
+  // fresh: form the residual from the solution instead of carrying it over
+  int d_dt(BatchGroup& g, const int* mask, double c, int in_slot, int out_slot, int its_now, int fresh = 0);
   int solve(BatchGroup& g, const int* mask, int its_now);
+  int solve_refine(BatchGroup& g, const int* mask, int its_now, int carry);
+  int refresh_residuals();
   int fd_apply(BatchGroup& g);
   int combine(BatchGroup& g, const int* mask, int out_slot, std::initializer_list<int> slots,
               std::initializer_list<double> num, std::initializer_list<double> den);

@@ -118,6 +118,7 @@ __global__ void pl_axpy_kernel(double* __restrict__ x, const double* __restrict_
 // after guessTauSS only moves the first root find's starting point.
 int QDContext::pl_steady_state(const QDProblem& P, std::vector<double>& psi, std::vector<double>& slip,
                                double* gVxy, double* gVxz, int* its_out, double* err_out) {
+  ++u_epoch;
   cudaStream_t s = sbp.stream;
   const double dg = P.ss_gss_t, cap = P.pdesc.visc_cap;
   // Fault::guessSS

@@ -134,6 +134,7 @@ int qd_green_surf_launch(QDContext& q, double c, double* host_out) {
 // Body displacement for output in response mode: one full solve with the
 // boundary data of the last d_dt.
 int QDContext::full_solve_for_output() {
+  ++u_epoch;
   cudaStream_t s = sbp.stream;
   const int tb = 64, gb = (Nz + tb - 1) / tb;
   qd_bc_kernel<<<gb, tb, 0, s>>>(rk[0].as<double>() + fp.slip_off, Nz, last_t, vL, 1.0 / fts, 0, bcR_remote,
@@ -221,6 +222,7 @@ int QDContext::create(const scy_qd_desc& d, const scy_pl_desc* pld) {
     return SCY_ERR_ARG;
   }
   SCY_TRY(sbp.create(d.grid));
+  sbp.keep_rounding = pl;
   Ny = d.grid.Ny;
   Nz = d.grid.Nz;
   N = (long)Ny * Nz;
@@ -366,6 +368,7 @@ int qd_bc_launch(QDContext& q, double t, const double* var) {
 }
 
 int QDContext::d_dt(double t, const double* var, double* f) {
+  ++u_epoch;
   cudaStream_t s = sbp.stream;
   if (fp.state_law == SCY_LAW_FLASH && !fp.Tf) {
     set_error("the flash-heating law needs the heat equation's fault fields (a driver with thermalCoupling)");
@@ -419,6 +422,7 @@ int QDContext::d_dt(double t, const double* var, double* f) {
 // data: Nz solves with bcL = e_j, one with bcR = 1 and one with the current
 // fixed part of bcR (bcRShift when the right boundary is loaded, else bcR).
 int QDContext::build_green() {
+  ++u_epoch;
   cudaStream_t s = sbp.stream;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -502,6 +506,7 @@ int QDContext::build_green() {
 
 // ---------------------------------------------------------------------------
 int QDContext::steady_state_guess(std::vector<double>& psi, int keep_psi, std::vector<double>& slip) {
+  ++u_epoch;
   cudaStream_t s = sbp.stream;
   // Fault::guessSS / computePsiSS (fault.cpp:619-672)
   std::vector<double> tau(Nz), vel(Nz, vL);

@@ -44,6 +44,9 @@ struct QDContext {
   DevBuf slipVel, tauQSP, tauP, strength;  // Nz
   DevBuf bcL, bcR, bcT, bcB, bcRShift;     // boundary data
   DevBuf rhs, u, sxy;                       // N
+  // counts the operations of this driver that changed rhs or u (from 1), so
+  // that a batch notices solves made beside its own rounds
+  unsigned long long u_epoch = 1;
   DevBuf flags;                             // unsigned, fault status bits
   DevBuf fault_its;                         // unsigned long long, root iterations
   double vL = 1e-9, fts = 2.0;

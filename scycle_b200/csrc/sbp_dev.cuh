@@ -10,6 +10,8 @@
 // the product the reference assembles as a sparse matrix in
 // SbpOps_m_constGrid::constructA / SbpOps_m_varGrid::constructA.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace scy {
@@ -157,6 +159,28 @@ struct EpiCGMatvec {
     pnew[node] = p;
     q[node] = qv;
     return p * qv;
+  }
+};
+
+// Defect-correction step with the correction z: u += z, r = r - K z = r + A z
+// (r the residual the correction was made from); returns r.r.  The epilogue's
+// own operands come ahead of the operator through full_apply's pre hook.
+struct EpiCorrect {
+  double* u;
+  double* r;
+  static constexpr bool kReduce = true;
+  struct Pre {
+    double u, r;
+  };
+  __device__ __forceinline__ Pre pre(long node, int, int) const { return Pre{u[node], r[node]}; }
+  __device__ __forceinline__ double operator()(long node, int, int, double Az, double z, const Pre& p) const {
+    const double rv = p.r + Az;
+    r[node] = rv;
+    u[node] = p.u + z;
+    return rv * rv;
+  }
+  __device__ __forceinline__ double operator()(long node, int iy, int iz, double Az, double z) const {
+    return (*this)(node, iy, iz, Az, z, pre(node, iy, iz));
   }
 };
 
@@ -571,10 +595,24 @@ __device__ __forceinline__ void full_apply(const LevelDev<T>& L, const Loader& l
   }
 }
 
-// No epilogue loads to prefetch.
-struct NoPre {
-  __device__ __forceinline__ int operator()(long, int, int) const { return 0; }
-};
+// The epilogue's loads ahead of the operator: Epi::pre where it has one.
+struct NoPre {};
+template <class Epi>
+__device__ __forceinline__ auto epi_pre(const Epi& ep, long node, int iy, int iz, int)
+    -> decltype(ep.pre(node, iy, iz)) {
+  return ep.pre(node, iy, iz);
+}
+template <class Epi>
+__device__ __forceinline__ NoPre epi_pre(const Epi&, long, int, int, long) {
+  return NoPre{};
+}
+template <class Epi, typename T, class P>
+__device__ __forceinline__ double epi_out(const Epi& ep, long node, int iy, int iz, T Ax, T xv, const P& p) {
+  if constexpr (std::is_same<P, NoPre>::value)
+    return ep(node, iy, iz, Ax, xv);
+  else
+    return ep(node, iy, iz, Ax, xv, p);
+}
 
 template <typename T, int RPT, class Loader, class Epi>
 __device__ __forceinline__ void full_tile(const LevelDev<T>& L, const Loader& ld, const Epi& ep, double* partials,
@@ -582,9 +620,12 @@ __device__ __forceinline__ void full_tile(const LevelDev<T>& L, const Loader& ld
   __shared__ T xs[full_smem_values<RPT>()];
   __shared__ double red[32];
   double contrib = 0.0;
-  auto out = [&](long node, int iy, int iz, T Ax, T xv, int) { contrib += ep(node, iy, iz, Ax, xv); };
+  auto pre = [&](long node, int iy, int iz) { return epi_pre(ep, node, iy, iz, 0); };
+  auto out = [&](long node, int iy, int iz, T Ax, T xv, const auto& p) {
+    contrib += epi_out(ep, node, iy, iz, Ax, xv, p);
+  };
   auto row = [](int) {};
-  full_apply<T, RPT>(L, ld, NoPre{}, out, row, xs);
+  full_apply<T, RPT>(L, ld, pre, out, row, xs);
   if constexpr (Epi::kReduce) {
     if (partials != nullptr) {  // uniform across the grid
       double tot = block_sum(contrib, red);

@@ -920,6 +920,31 @@ int SbpContext::rebuild() {
         if (std::fabs(h.mu[i] - h.mu[0]) > tol * std::fabs(h.mu[0])) sep = false;
       }
     separable = sep ? 1 : 0;
+    // how far the operator is from the separable one the fast
+    // diagonalisation inverts (its coefficients are the line averages): only
+    // the flattened-index m3 average of the order-4 R terms differs, and
+    // those terms are part of K_sep, so the energy norm of I - K_sep^-1 K is
+    // at most the largest relative difference where their weight is not zero
+    sep_misfit = 0.0;
+    if (sep && h.order == 4) {
+      std::vector<double> az(h.Nz, 0.0);
+      for (int iy = 0; iy < h.Ny; ++iy) {
+        const double* m3 = &h.m3z[(size_t)iy * h.Nz];
+        for (int iz = 0; iz < h.Nz; ++iz) az[iz] += m3[iz];
+      }
+      for (int iz = 0; iz < h.Nz; ++iz) az[iz] = h.tz.w3[iz] != 0.0 ? h.Ny / az[iz] : 0.0;
+      for (int iy = 0; iy < h.Ny; ++iy) {
+        const double *my = &h.m3y[(size_t)iy * h.Nz], *mz = &h.m3z[(size_t)iy * h.Nz];
+        double sum = 0.0, ey = 0.0, ez = 0.0;
+        for (int iz = 0; iz < h.Nz; ++iz) sum += my[iz];
+        const double ay = h.Nz / sum;
+        for (int iz = 0; iz < h.Nz; ++iz) {
+          ey = std::max(ey, std::fabs(my[iz] * ay - 1.0));
+          if (az[iz] != 0.0) ez = std::max(ez, std::fabs(mz[iz] * az[iz] - 1.0));
+        }
+        sep_misfit = std::max(sep_misfit, h.ty.w3[iy] != 0.0 ? std::max(ey, ez) : ez);
+      }
+    }
   }
   cross.release();
   fd.reset();
@@ -1013,33 +1038,57 @@ int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts&
     pi ^= 1;
     st.iterations = it;
     if (it % check == 0 || it == o.max_its) {
-      double h[6];
-      SCY_CUDA_TRY(cudaMemcpyAsync(h, sc, 6 * sizeof(double), cudaMemcpyDeviceToHost, stream));
-      SCY_CUDA_TRY(cudaStreamSynchronize(stream));
-      if (tol < 0) {
-        st.bnorm = std::sqrt(h[0]);
-        st.rnorm0 = std::sqrt(h[5]);
-        tol = std::max(o.rtol * st.bnorm, o.atol);
-        if (h[0] == 0.0 && tol == 0.0) {
-          // zero right-hand side: the solution is zero (a warm start from
-          // an earlier solve would otherwise never reach ||r|| <= 0)
-          SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
-          st.rnorm = 0.0;
-          st.converged = 1;
-          return SCY_OK;
-        }
-      }
-      st.rnorm = std::sqrt(h[1]);
-      if (!std::isfinite(h[1])) {
-        set_error("non-finite residual in the elliptic solve");
-        return SCY_ERR_NONFINITE;
-      }
-      if (st.rnorm <= tol || st.rnorm0 <= tol) {
-        st.converged = 1;
-        break;
-      }
+      int done = 0;
+      SCY_TRY(read_convergence(o, u, tol, st, &done));
+      if (done) break;
     }
   }
+  return finish_solve(rhs, u, o, tol, st);
+}
+
+// Reads the solve's scalars back and tests convergence; sets tol at the
+// first call (tol < 0).  *done: stop iterating.
+int SbpContext::read_convergence(const scy_solve_opts& o, double* u, double& tol, scy_solve_stats& st, int* done) {
+  const size_t n = (size_t)fine->dev.Ny * fine->dev.Nz;
+  double h[6];
+  SCY_CUDA_TRY(cudaMemcpyAsync(h, scal.p, 6 * sizeof(double), cudaMemcpyDeviceToHost, stream));
+  SCY_CUDA_TRY(cudaStreamSynchronize(stream));
+  if (tol < 0) {
+    st.bnorm = std::sqrt(h[0]);
+    st.rnorm0 = std::sqrt(h[5]);
+    tol = std::max(o.rtol * st.bnorm, o.atol);
+    if (h[0] == 0.0 && tol == 0.0) {
+      // zero right-hand side: the solution is zero (a warm start from
+      // an earlier solve would otherwise never reach ||r|| <= 0)
+      SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
+      st.rnorm = 0.0;
+      st.converged = 2;  // nothing to verify
+      *done = 1;
+      return SCY_OK;
+    }
+  }
+  st.rnorm = std::sqrt(h[1]);
+  if (!std::isfinite(h[1])) {
+    set_error("non-finite residual in the elliptic solve");
+    return SCY_ERR_NONFINITE;
+  }
+  if (st.rnorm <= tol || st.rnorm0 <= tol) {
+    st.converged = 1;
+    *done = 1;
+  }
+  return SCY_OK;
+}
+
+// The optional check of the true residual, and the error of a solve that
+// did not reach its tolerance.
+int SbpContext::finish_solve(const double* rhs, double* u, const scy_solve_opts& o, double tol, scy_solve_stats& st) {
+  if (st.converged == 2) {
+    st.converged = 1;
+    return SCY_OK;
+  }
+  const LevelDev<double>& L = fine->dev;
+  double* sc = scal.as<double>();
+  double* r = cg_r.as<double>();
   if (o.verify) {
     SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{u}, EpiResidual<double, double>{rhs, r, -1.0}, &red, sc + 1,
                                    stream));
@@ -1060,6 +1109,50 @@ int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts&
   return SCY_OK;
 }
 
+// Defect correction with a preconditioner that is the inverse up to rounding
+// and the last z column (the fast diagonalisation of a separable operator):
+//   z = P r,  u += z,  r -= K z,
+// the same residual recurrence and test as pcg, without its search direction
+// and step length (both differ from z and 1 only by P's own error), so an
+// iteration is P and one operator launch instead of P and four launches.
+// Per iteration on 401 x 401 stretched (numpy): ||r|| / ||rhs|| 1.2e-9,
+// 6.4e-13, 1.1e-15 against CG's 1.2e-9, 5.7e-13, 5.1e-16.
+template <class PC>
+int SbpContext::correct(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st) {
+  const LevelDev<double>& L = fine->dev;
+  const long n = (long)L.Ny * L.Nz;
+  double* sc = scal.as<double>();
+  // sc[0]=||rhs||^2, sc[1]=r.r, sc[5]=||r0||^2
+  double* r = cg_r.as<double>();
+  dot_kernel<double, double><<<red_blocks(n), 256, 0, stream>>>(rhs, rhs, n, red.partials.as<double>(),
+                                                               red.counter.as<unsigned>(), sc + 0);
+  SCY_LAUNCH_CHECK();
+  if (!o.nonzero_guess) SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
+  SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{u}, EpiResidual<double, double>{rhs, r, -1.0}, &red, sc + 5,
+                                 stream));
+  st.iterations = 0;
+  st.converged = 0;
+  const int check = o.check_every > 0 ? o.check_every : 1;
+  double tol = -1.0;
+  int unverified = 0;
+  for (int it = 1; it <= o.max_its; ++it) {
+    double* z = nullptr;
+    SCY_TRY(pc((const double*)r, &z));
+    SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{z}, EpiCorrect{u, r}, &red, sc + 1, stream));
+    st.iterations = it;
+    if (it % check == 0 || it == o.max_its) {
+      int done = 0;
+      SCY_TRY(read_convergence(o, u, tol, st, &done));
+      if (!done) continue;
+      // a true residual above the tolerance that the recurrence met (both
+      // near rounding) is in r now: correct it, a few times at most
+      const int rc = finish_solve(rhs, u, o, tol, st);
+      if (rc != SCY_ERR_CG_NOCONV || it == o.max_its || ++unverified > 3) return rc;
+    }
+  }
+  return finish_solve(rhs, u, o, tol, st);
+}
+
 int SbpContext::ensure_fd() {
   if (fd && fd->ready) return SCY_OK;
   fd.reset(new FDPrecond());
@@ -1067,6 +1160,7 @@ int SbpContext::ensure_fd() {
 }
 
 int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st) {
+  const bool keeps = keeps_rounding(o.rtol);
   const bool use_fd = o.precond == SCY_PC_FD || (o.precond == SCY_PC_AUTO && separable);
   if (use_fd) {
     SCY_TRY(ensure_fd());
@@ -1085,7 +1179,7 @@ int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy
       *zo = z;
       return SCY_OK;
     };
-    return pcg<double>(pc, rhs, u, o, st);
+    return near_inverse() && !keeps ? correct(pc, rhs, u, o, st) : pcg<double>(pc, rhs, u, o, st);
   }
   if (o.precision == SCY_PREC_MIXED) {
     SCY_TRY(ensure_mg(mg32));

@@ -191,3 +191,28 @@ def test_solve_warm_start_converges_immediately():
     assert st2.iterations <= 1 and st2.converged
     # the extra iteration may still improve an rtol-1e-11 solution slightly
     assert np.abs(u2.cpu().numpy() - u.cpu().numpy()).max() <= 1e-9 * np.abs(u.cpu().numpy()).max()
+
+
+@pytest.mark.parametrize("ratio", (1.2, 1.0 / 1.4, 1.0 / 1.6))
+def test_solve_on_steep_geometric_stretching(ratio):
+    """Constant mu, y spacing in geometric progression: the averaged
+    coefficient of the last z column differs from the others' by
+    |1/ratio - 1| / 2 (0.08, 0.2, 0.3), and 1/4 is where the FP64 fast
+    diagonalisation's solve goes from defect correction to CG.  A residual of
+    rtol |rhs| leaves an error of at most rtol times the condition number
+    (2-norm; 3e3 to 6e5 here)."""
+    import scipy.sparse.linalg as spla
+    from scycle_b200.sbp import SbpOps
+    Ny, Nz = 25, 21
+    s = ratio ** np.arange(Ny) - 1.0
+    y = np.repeat(30.0 * s / s[-1], Nz)
+    z = np.tile(np.linspace(0.0, 24.0, Nz), Ny)
+    mu = np.full(Ny * Nz, 32.04)
+    dev = SbpOps(4, Ny, Nz, 30.0, 24.0, mu, grid="variableGridSpacing", y=y, z=z)
+    ora = OracleSbp(4, Ny, Nz, 30.0, 24.0, mu, grid="variableGridSpacing", y=y, z=z)
+    rhs = ora.set_rhs(np.linspace(0, 1, Nz) ** 2, np.full(Nz, 0.3), np.zeros(Ny), np.zeros(Ny))
+    ref = spla.spsolve(ora.A.tocsc(), rhs)
+    lam = np.linalg.eigvalsh(-0.5 * (ora.A + ora.A.T).toarray())
+    u, st = dev.solve(rhs, rtol=1e-12, max_its=60, precond="fd")
+    assert st.converged
+    assert np.linalg.norm(u.cpu().numpy() - ref) <= 1e-12 * lam[-1] / lam[0] * np.linalg.norm(ref)
