@@ -100,6 +100,9 @@ class Batch:
         S.check(S.lib().scy_batch_operator_form(self.h, int(group), C.byref(rpt), C.byref(minb)))
         shapes = ["2 chains x 2 warps (8 instances)", "1 chain x 4 warps (8)", "4 chains x 1 warp (8)",
                   "1 chain x 2 warps (4)", "2 chains x 1 warp (4)", "1 chain x 1 warp (2)"]
+        shapes += ["segments, %d instances a thread, %d groups a block" % (i, g)
+                   for i, g in ((1, 1), (2, 1), (1, 2), (2, 2), (1, 4), (2, 4))]
+        v0 = 6 if var.value >= 6 else 0
         form = "cross"
         if rpt.value:
             form = "separable, %d rows per thread, %s" % (
@@ -111,7 +114,7 @@ class Batch:
                                     "two CTAs per SM" if zt.value & 1 else "one CTA per tile",
                 "ztransform_digits": "bf16 (kind::f16)" if zt.value & 2 else "int8 (kind::i8)",
                 "operator_us_by_kpb": {k: us[i] for i, k in enumerate((1, 2, 4, 8)) if us[i] > 0},
-                "sweep_us_by_variant": {shapes[v]: us[4 + v] for v in range(6) if us[4 + v] > 0},
+                "sweep_us_by_variant": {shapes[v0 + v]: us[4 + v] for v in range(6) if us[4 + v] > 0},
                 "ztransform_us_int8_by_ctas_per_sm": {1: us[10], 2: us[11]},
                 "ztransform_us_bf16_by_ctas_per_sm": {1: us[12], 2: us[13]},
                 "ztransform_us_persistent": {"int8": us[20], "bf16": us[21]},

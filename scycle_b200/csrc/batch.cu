@@ -854,6 +854,12 @@ const int* BatchContext::d_copy(const BatchGroup& g) const {
 const int* BatchContext::d_acc(const BatchGroup& g) const { return d_copy(g) + n; }
 const int* BatchContext::d_run(const BatchGroup& g) const { return d_copy(g) + 2 * n; }
 
+// Whole chains instead of segments: one pass of whole chains takes the time of
+// one chain until they fill the GPU, segments a time that grows with the
+// instances.  Measured: 32 x 401 modes 72 us whole, 86 in segments; 3 x 301
+// 52 and 15; 7 x 97 26 and 9.
+static bool many_chains(int Nz, int K) { return (long)Nz * K >= 10000; }
+
 static bool same_operator(const SbpContext& a, const SbpContext& b) {
   const scy_grid_desc &x = a.desc, &y = b.desc;
   if (x.order != y.order || x.Ny != y.Ny || x.Nz != y.Nz || x.grid_type != y.grid_type || x.compat != y.compat)
@@ -938,7 +944,8 @@ int BatchContext::create(int n_inst, const char* const* paths, const scy_solve_o
   // members' own solves as well
   int base = 0;
   for (auto& m : members) {
-    SCY_TRY(q(base).sbp.ensure_fd());
+    SCY_TRY(q(base).sbp.ensure_fd(q(base).sbp.keeps_rounding(q(base).solve_opts.rtol) ||
+                                  many_chains(q(base).Nz, (int)m.size())));
     for (size_t k = 1; k < m.size(); ++k) q(base + (int)k).sbp.fd = q(base).sbp.fd;
     base += (int)m.size();
   }
@@ -1037,7 +1044,7 @@ int BatchContext::setup_group(int base, int K) {
   g.N = q0.N;
   // a steady-state guess changes the boundary types and back, which rebuilds
   // the members' operators: take the representative's current ones
-  SCY_TRY(q0.sbp.ensure_fd());
+  SCY_TRY(q0.sbp.ensure_fd(many_chains(g.Nz, K)));
   g.fd = q0.sbp.fd;
   g.L = q0.sbp.fine->dev;
   const long KN = (long)g.K * g.N;
@@ -1141,8 +1148,10 @@ int BatchContext::setup_group(int base, int K) {
     SCY_CUDA_TRY(cudaMemset(g.t1p.p, 0, (size_t)rowsT * Nzp * 8));
     SCY_CUDA_TRY(cudaMemset(g.t1pf.p, 0, (size_t)rowsT * Nzp * 4));
     const CUtensorMapDataType d64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64, d32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    SCY_TRY(tma_map_2d(&g.mLcol, g.fd->Lcol.p, d64, 8, g.Nz, (long)g.Ny * 9, (long)Nzp * 8, YS_C, YS_R * 9));
-    SCY_TRY(tma_map_2d(&g.mLrow, g.fd->Lrow.p, d64, 8, g.Nz, (long)(g.Ny + 8) * 9, (long)Nzp * 8, YS_C, YS_R * 9));
+    if (g.fd->Lrow.p) {
+      SCY_TRY(tma_map_2d(&g.mLcol, g.fd->Lcol.p, d64, 8, g.Nz, (long)g.Ny * 9, (long)Nzp * 8, YS_C, YS_R * 9));
+      SCY_TRY(tma_map_2d(&g.mLrow, g.fd->Lrow.p, d64, 8, g.Nz, (long)(g.Ny + 8) * 9, (long)Nzp * 8, YS_C, YS_R * 9));
+    }
     SCY_TRY(tma_map_3d(&g.mT, g.t1p.p, d64, g.Nz, g.Ny, g.K, (long)Nzp * 8, (long)g.Ny * Nzp * 8, YS_C, YS_R, YS_B));
     SCY_TRY(tma_map_2d(&g.mLcol32, g.fd->Lcol32.p, d32, 4, g.Nz, (long)g.Ny * 9, (long)Nzp * 4, YS_C, YS_R * 9));
     SCY_TRY(tma_map_2d(&g.mLrow32, g.fd->Lrow32.p, d32, 4, g.Nz, (long)(g.Ny + 8) * 9, (long)Nzp * 4, YS_C, YS_R * 9));
@@ -1206,11 +1215,14 @@ int BatchContext::setup_group(int base, int K) {
   return SCY_OK;
 }
 
-// The banded sweeps in one of their launch shapes: variant 0 two chains per
+// The banded sweeps in one of their launch shapes: variants 6 and up in
+// segments (YPart's shapes), below whole chains: variant 0 two chains per
 // lane and two warps per block, 1 one chain and four warps, 2 four chains
 // and one warp (a block serves eight instances in each)
 int BatchContext::launch_ysolve(BatchGroup& g, int variant) {
   FDPrecond& F = *g.fd;
+  if (variant >= 6)
+    return F.yp.solve(g.t1p.as<double>(), g.K, variant - 6, g.w.status, g.stream, sweep_polls, sweep_drop);
   const int Ny = g.Ny, Nz = g.Nz, K = g.K;
   const bool f32 = precision != SCY_PREC_FP64;
   const int sm = ys_smem_bytes(f32 ? 4 : 8);
@@ -1352,7 +1364,11 @@ int BatchContext::autotune(BatchGroup& g) {
   }
   if (g.fd->ybanded && !fd_dense) {
     double best_ys = 1e300;
-    for (int v = 0; v < 6; ++v) {
+    // the sweeps in segments where the operator has a plan for them (FP64)
+    // and the chains are few, else whole chains; either in six shapes
+    const int v0 = precision == SCY_PREC_FP64 && g.fd->yp.T > 0 && !many_chains(g.Nz, g.K) ? 6 : 0;
+    for (int v = v0; v < v0 + 6; ++v) {
+      if (v0 && !g.fd->yp.fits(v - v0)) continue;
       double us = 0.0;
       int rc = timed([&]() -> int { return launch_ysolve(g, v); }, &us);
       if (rc != SCY_OK) {
@@ -1360,7 +1376,7 @@ int BatchContext::autotune(BatchGroup& g) {
         cudaEventDestroy(e1);
         return rc;
       }
-      g.tune_us[4 + v] = us;
+      g.tune_us[4 + v - v0] = us;
       if (us < best_ys) {
         best_ys = us;
         g.ys_variant = v;

@@ -285,6 +285,7 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
       if (spd) {
         // padded row and column forms for the TMA-fed sweeps
         Nzp = (Nz + 3) / 4 * 4;
+        SCY_TRY(yp.build(Lbh, Ny, Nz, Nzp, s));
         std::vector<double> Lr((size_t)(Ny + bw) * 9 * Nzp, 0.0), Lc((size_t)Ny * 9 * Nzp, 0.0);
         // slot 1 holds the coupling to the row processed just before,
         // divided by L_ii: L(i+1, i) / L_ii going up (row form), L(i, i-1) /
@@ -303,8 +304,10 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
             Lc[((size_t)i * 9 + 1) * Nzp + j] = Lbh[((size_t)i * 9 + 1) * Nz + j] * Lbh[((size_t)i * 9) * Nz + j];
             for (int m = 2; m <= bw; ++m) Lc[((size_t)i * 9 + m) * Nzp + j] = Lbh[((size_t)(i + m) * 9 + m) * Nz + j];
           }
-        SCY_TRY(upload_as<double>(Lrow, Lr, s));
-        SCY_TRY(upload_as<double>(Lcol, Lc, s));
+        if (want_chains || yp.T == 0) {
+          SCY_TRY(upload_as<double>(Lrow, Lr, s));
+          SCY_TRY(upload_as<double>(Lcol, Lc, s));
+        }
         SCY_TRY(upload_as<float>(Lrow32, Lr, s));
         SCY_TRY(upload_as<float>(Lcol32, Lc, s));
         ybanded = 1;
@@ -338,13 +341,15 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
     }
     // tile maps of the TMA-fed sweeps over the one instance's transform
     const CUtensorMapDataType d64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64, d32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    SCY_TRY(tma_map_2d(&mLcol, Lcol.p, d64, 8, Nz, (long)Ny * 9, (long)Nzp * 8, YS_C, YS_R * 9));
-    SCY_TRY(tma_map_2d(&mLrow, Lrow.p, d64, 8, Nz, (long)(Ny + 8) * 9, (long)Nzp * 8, YS_C, YS_R * 9));
-    SCY_TRY(tma_map_3d(&mT, t1p.p, d64, Nz, Ny, 1, (long)Nzp * 8, (long)Ny * Nzp * 8, YS_C, YS_R, YS_B));
+    if (Lrow.p) {
+      SCY_TRY(tma_map_2d(&mLcol, Lcol.p, d64, 8, Nz, (long)Ny * 9, (long)Nzp * 8, YS_C, YS_R * 9));
+      SCY_TRY(tma_map_2d(&mLrow, Lrow.p, d64, 8, Nz, (long)(Ny + 8) * 9, (long)Nzp * 8, YS_C, YS_R * 9));
+    }
+    SCY_TRY(tma_map_3d(&mT, t1p.p, d64, Nz, Ny, 1, (long)Nzp * 8, (long)Ny * Nzp * 8, YS_C, YS_R, 2));
     SCY_TRY(tma_map_2d(&mLcol32, Lcol32.p, d32, 4, Nz, (long)Ny * 9, (long)Nzp * 4, YS_C, YS_R * 9));
     SCY_TRY(tma_map_2d(&mLrow32, Lrow32.p, d32, 4, Nz, (long)(Ny + 8) * 9, (long)Nzp * 4, YS_C, YS_R * 9));
     SCY_TRY(tma_map_3d(&mT32, t1pf.p, d32, Nz, Ny, 1, (long)Nzp * 4, (long)Ny * Nzp * 4, YS_C, YS_R, YS_B));
-    SCY_CUDA_TRY(cudaFuncSetAttribute(b_ysolve_tma_kernel<double, YS_I, YS_W>,
+    SCY_CUDA_TRY(cudaFuncSetAttribute(b_ysolve_tma_kernel<double, 1, 1>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, ys_smem_bytes(8)));
     SCY_CUDA_TRY(cudaFuncSetAttribute(b_ysolve_tma_kernel<float, YS_I, YS_W>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, ys_smem_bytes(4)));
@@ -361,14 +366,19 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
   return SCY_OK;
 }
 
-int FDPrecond::apply(const double* r, double* z, cudaStream_t s) {
+int FDPrecond::apply(const double* r, double* z, cudaStream_t s, bool chains) {
   if (ybanded) {
     double* t = t1p.as<double>();
     SCY_TRY(ozk_split(zx64, r, Nz, s));
     SCY_TRY(ozk_gemm(zx64, zw1_64, t, Nzp, Nz, s));
-    b_ysolve_tma_kernel<double, YS_I, YS_W><<<dim3((Nz + YS_C - 1) / YS_C, 1), 32 * YS_W, ys_smem_bytes(8), s>>>(
-        mLcol, mLrow, mT, t, Ny, Nz, Nzp, 1, ys_status.as<unsigned>());
-    SCY_LAUNCH_CHECK();
+    if (yp.T > 0 && !chains) {
+      SCY_TRY(yp.solve(t, 1, 0, ys_status.as<unsigned>(), s));
+    } else {
+      // one chain a lane and one warp a block: fewest instructions a row
+      b_ysolve_tma_kernel<double, 1, 1><<<dim3((Nz + YS_C - 1) / YS_C, 1), 32, ys_smem_bytes(8), s>>>(
+          mLcol, mLrow, mT, t, Ny, Nz, Nzp, 1, ys_status.as<unsigned>());
+      SCY_LAUNCH_CHECK();
+    }
     SCY_TRY(ozk_split(zx64, (const double*)t, Nzp, s));
     SCY_TRY(ozk_gemm(zx64, zw2_64, z, Nz, Nz, s));
     return SCY_OK;

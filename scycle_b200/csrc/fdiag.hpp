@@ -21,6 +21,23 @@
 
 namespace scy {
 
+// The banded solves along y in segments (ypart.cu): tables of one operator's
+// factors, laid out for the kernel.  T = 0 where it has no plan (more than
+// about 1900 rows, or off-diagonals outside its pattern); then the chains run
+// whole (ysolve.cuh).
+struct YPart {
+  int Ny = 0, Nzp = 0, T = 0, P = 0, MB = 0, base = 0, extra = 0, nb = 0;
+  DevBuf tab, wide;
+  // instances a thread x groups a block; every shape gives the same results
+  static constexpr int kShapes = 6;
+  static constexpr int kShapeI[kShapes] = {1, 2, 1, 2, 1, 2}, kShapeNG[kShapes] = {1, 1, 2, 2, 4, 4};
+  bool fits(int shape) const;
+  size_t smem_bytes(int shape) const;
+  // L: the factors, value k of row i (1 / L_ii, then L(i, i - k)) and mode j at (i * 9 + k) * Nz + j
+  int build(const std::vector<double>& L, int Ny, int Nz, int Nzp, cudaStream_t s);
+  int solve(double* t, int K, int shape, unsigned* status, cudaStream_t s, int polls = 1 << 18, int drop = 0) const;
+};
+
 struct FDPrecond {
   int Ny = 0, Nz = 0;
   int ready = 0;
@@ -42,6 +59,11 @@ struct FDPrecond {
   int ybanded = 0;
   int Nzp = 0;
   DevBuf Lrow, Lcol, Lrow32, Lcol32;
+  YPart yp;  // the FP64 sweeps in segments
+  // set before build: keep the FP64 tables of the whole chains beside the
+  // segments' (there without a plan for segments)
+  int want_chains = 0;
+  bool has_chains() const { return !ybanded || Lrow.p; }
   // With the banded form, apply / apply32 run the z transforms on the
   // integer tensor cores (digit planes: kPlanes64 for apply, kPlanes32 for apply32) and the
   // TMA-fed sweeps of the batched ensemble (one instance) on the padded
@@ -53,8 +75,8 @@ struct FDPrecond {
   CUtensorMap mLcol, mLrow, mT, mLcol32, mLrow32, mT32;
   ~FDPrecond();
   int build(const LevelHost& L, cudaStream_t s);
-  // z = K_sep^-1 r (FP64)
-  int apply(const double* r, double* z, cudaStream_t s);
+  // z = K_sep^-1 r (FP64); chains: sweep whole chains (has_chains)
+  int apply(const double* r, double* z, cudaStream_t s, bool chains = false);
   // z = K_sep^-1 r with FP32 GEMMs (z in FP32)
   int apply32(const double* r, float* z, cudaStream_t s);
 };

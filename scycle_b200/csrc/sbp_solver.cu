@@ -1153,9 +1153,10 @@ int SbpContext::correct(PC&& pc, const double* rhs, double* u, const scy_solve_o
   return finish_solve(rhs, u, o, tol, st);
 }
 
-int SbpContext::ensure_fd() {
-  if (fd && fd->ready) return SCY_OK;
+int SbpContext::ensure_fd(bool chains) {
+  if (fd && fd->ready && (!chains || fd->has_chains())) return SCY_OK;
   fd.reset(new FDPrecond());
+  fd->want_chains = chains;
   return fd->build(hosts[0], stream);
 }
 
@@ -1163,7 +1164,7 @@ int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy
   const bool keeps = keeps_rounding(o.rtol);
   const bool use_fd = o.precond == SCY_PC_FD || (o.precond == SCY_PC_AUTO && separable);
   if (use_fd) {
-    SCY_TRY(ensure_fd());
+    SCY_TRY(ensure_fd(keeps));
     if (o.precision == SCY_PREC_MIXED) {
       float* z = cg_z32.as<float>();
       auto pc = [&](const double* r, float** zo) -> int {
@@ -1175,7 +1176,7 @@ int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy
     }
     double* z = cg_z.as<double>();
     auto pc = [&](const double* r, double** zo) -> int {
-      SCY_TRY(fd->apply(r, z, stream));
+      SCY_TRY(fd->apply(r, z, stream, keeps));
       *zo = z;
       return SCY_OK;
     };

@@ -123,7 +123,7 @@ struct SbpContext {
   // the bound is 0.005 and 0.05).  Beyond it (a grid whose spacing changes by
   // half from one row to the next), and for operators that are not separable, CG.
   bool near_inverse() const { return separable && sep_misfit <= 0.25; }
-  // Solves that keep the arithmetic of plain CG: those of the
+  // Solves that keep the arithmetic of plain CG with whole sweep chains: those of the
   // power-law driver (keep_rounding: its viscous strain gVxz starts as a
   // difference of displacements that agree to rounding, so its first digits
   // are the solve's own rounding) and those asked for to near rounding, whose
@@ -152,7 +152,7 @@ struct SbpContext {
   DevBuf cross;  // cross-form planes of the fine level (built on first use)
   template <typename T>
   int ensure_mg(std::unique_ptr<Multigrid<T>>& mg);
-  int ensure_fd();
+  int ensure_fd(bool chains);  // chains: with the tables of the whole sweep chains
   template <typename Tz, class PC>
   int pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st);
   template <class PC>
