@@ -110,7 +110,8 @@ class Batch:
                 else "compiler's register count")
         return {"operator_form": form,
                 "instances_per_block": kpb.value, "sweep_variant": shapes[var.value],
-                "ztransform_shape": "persistent (one CTA per SM, two accumulator sets)" if zt.value & 4 else
+                "ztransform_shape": "persistent (one CTA per SM, resident weights, two accumulator sets)" if zt.value & 4 else
+                                    "narrow tiles" if zt.value & 8 else
                                     "two CTAs per SM" if zt.value & 1 else "one CTA per tile",
                 "ztransform_digits": "bf16 (kind::f16)" if zt.value & 2 else "int8 (kind::i8)",
                 "operator_us_by_kpb": {k: us[i] for i, k in enumerate((1, 2, 4, 8)) if us[i] > 0},

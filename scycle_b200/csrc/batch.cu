@@ -1382,15 +1382,17 @@ int BatchContext::autotune(BatchGroup& g) {
         g.ys_variant = v;
       }
     }
-    // the forward z-transform product in its three shapes (one CTA per
-    // tile, two CTAs per SM, persistent) and both digit formats (identical
-    // results)
+    // the forward z-transform product in its shapes (one CTA per tile, two
+    // CTAs per SM, persistent, narrow tiles) and both digit formats
+    // (identical results)
     {
       double zbest = 1e300;
       for (int bf = 0; bf < 2; ++bf) {
         if (bf && !g.zx16.dig.p) continue;
-        for (int pr = 0; pr < 3; ++pr) {
-          if (pr && ozk_cols_per_tile_pair(zt_planes) == 0) continue;
+        for (int pr = 0; pr < 4; ++pr) {
+          if ((pr == 1 || pr == 2) && ozk_cols_per_tile_pair(zt_planes) == 0) continue;
+          // the narrow tiles only where the rule takes them for one instance
+          if (pr == 3 && (bf || !ozk_narrow_better(zt_planes, g.K * g.Ny, g.Nz))) continue;
           const OzkOperand& X = bf ? g.zx16 : g.zx;
           const OzkOperand& W = bf ? g.zw1_16 : g.zw1;
           double us = 0.0;
@@ -1406,7 +1408,7 @@ int BatchContext::autotune(BatchGroup& g) {
             cudaEventDestroy(e1);
             return rc;
           }
-          g.tune_us[pr == 2 ? 20 + bf : 10 + 2 * bf + pr] = us;
+          if (pr < 3) g.tune_us[pr == 2 ? 20 + bf : 10 + 2 * bf + pr] = us;
           if (us < zbest) {
             zbest = us;
             g.zt_pair = pr;
@@ -2152,7 +2154,7 @@ scy_status scy_batch_tuning(scy_batch* b, int g, int* kpb, int* sweep_variant, i
   const scy::BatchGroup& G = *b->ctx.groups[g];
   if (kpb) *kpb = G.kpb;
   if (sweep_variant) *sweep_variant = G.ys_variant;
-  if (ztransform) *ztransform = (G.zt_pair == 1 ? 1 : 0) | (G.zt_bf16 << 1) | (G.zt_pair == 2 ? 4 : 0);
+  if (ztransform) *ztransform = (G.zt_pair == 1 ? 1 : 0) | (G.zt_bf16 << 1) | (G.zt_pair == 2 ? 4 : 0) | (G.zt_pair == 3 ? 8 : 0);
   if (us)
     for (int i = 0; i < 22; ++i) us[i] = G.tune_us[i];
   return SCY_OK;

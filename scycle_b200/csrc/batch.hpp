@@ -72,7 +72,7 @@ struct BatchGroup {
   DevBuf planes;  // the operator's 33 cross-stencil coefficient planes (build_cross_planes)
   int kpb = 1;    // instances per block of the operator kernels (autotuned at set-up)
   int ys_variant = 0;  // chains per lane x warps per block of the banded sweeps (autotuned)
-  int zt_pair = 0;  // z-transform products: 0 one CTA per tile, 1 two CTAs per SM, 2 persistent (autotuned)
+  int zt_pair = 0;  // z-transform products: 0 one CTA per tile, 1 two CTAs per SM, 2 persistent, 3 narrow tiles (autotuned)
   int zt_bf16 = 0;  // z-transform digits in bf16 (kind::f16) instead of 8-bit integers (autotuned)
   int refine = 0;  // stage solves by defect correction with a carried residual (solve_refine) instead of CG
   DevBuf ones;     // a mask that selects every instance

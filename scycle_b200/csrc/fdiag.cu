@@ -333,8 +333,8 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
       OzkOperand& w1 = S == kPlanes64 ? zw1_64 : zw1_32;
       OzkOperand& w2 = S == kPlanes64 ? zw2_64 : zw2_32;
       SCY_TRY(x.alloc(S, Ny, Nz, 128));
-      SCY_TRY(w1.alloc(S, Nz, Nz, ozk_cols_per_tile(S)));
-      SCY_TRY(w2.alloc(S, Nz, Nz, ozk_cols_per_tile(S)));
+      SCY_TRY(w1.alloc_weights(S, Nz, Nz));
+      SCY_TRY(w2.alloc_weights(S, Nz, Nz));
       SCY_TRY(ozk_set_host(w1, Vzh.data(), Nz, s));  // rows of Vz^T: the columns of Vz
       SCY_TRY(ozk_set_host(w2, vzt.data(), Nz, s));  // rows of Vz
       SCY_TRY(ozk_prepare(S));
@@ -369,8 +369,9 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
 int FDPrecond::apply(const double* r, double* z, cudaStream_t s, bool chains) {
   if (ybanded) {
     double* t = t1p.as<double>();
+    const int shape = ozk_narrow_better(kPlanes64, Ny, Nz) ? 3 : 0;
     SCY_TRY(ozk_split(zx64, r, Nz, s));
-    SCY_TRY(ozk_gemm(zx64, zw1_64, t, Nzp, Nz, s));
+    SCY_TRY(ozk_gemm(zx64, zw1_64, t, Nzp, Nz, s, nullptr, 1, 4u, shape));
     if (yp.T > 0 && !chains) {
       SCY_TRY(yp.solve(t, 1, 0, ys_status.as<unsigned>(), s));
     } else {
@@ -380,7 +381,7 @@ int FDPrecond::apply(const double* r, double* z, cudaStream_t s, bool chains) {
       SCY_LAUNCH_CHECK();
     }
     SCY_TRY(ozk_split(zx64, (const double*)t, Nzp, s));
-    SCY_TRY(ozk_gemm(zx64, zw2_64, z, Nz, Nz, s));
+    SCY_TRY(ozk_gemm(zx64, zw2_64, z, Nz, Nz, s, nullptr, 1, 4u, shape));
     return SCY_OK;
   }
   SCY_BLAS_TRY(cublasSetStream(blas, s));
@@ -408,13 +409,14 @@ int FDPrecond::apply(const double* r, double* z, cudaStream_t s, bool chains) {
 int FDPrecond::apply32(const double* r, float* z, cudaStream_t s) {
   if (ybanded) {
     float* t = t1pf.as<float>();
+    const int shape = ozk_narrow_better(kPlanes32, Ny, Nz) ? 3 : 0;
     SCY_TRY(ozk_split(zx32, r, Nz, s));
-    SCY_TRY(ozk_gemm(zx32, zw1_32, t, Nzp, Nz, s));
+    SCY_TRY(ozk_gemm(zx32, zw1_32, t, Nzp, Nz, s, nullptr, 1, 4u, shape));
     b_ysolve_tma_kernel<float, YS_I, YS_W><<<dim3((Nz + YS_C - 1) / YS_C, 1), 32 * YS_W, ys_smem_bytes(4), s>>>(
         mLcol32, mLrow32, mT32, t, Ny, Nz, Nzp, 1, ys_status.as<unsigned>());
     SCY_LAUNCH_CHECK();
     SCY_TRY(ozk_split(zx32, (const float*)t, Nzp, s));
-    SCY_TRY(ozk_gemm(zx32, zw2_32, z, Nz, Nz, s));
+    SCY_TRY(ozk_gemm(zx32, zw2_32, z, Nz, Nz, s, nullptr, 1, 4u, shape));
     return SCY_OK;
   }
   SCY_BLAS_TRY(cublasSetStream(blas, s));

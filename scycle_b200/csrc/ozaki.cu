@@ -24,12 +24,14 @@
 // The products are bit-identical; which is faster depends on the tensor
 // pipe's integer and bf16 rates, so callers time both.
 //
-// Three shapes: one CTA per SM per tile (all 512 tensor-memory columns, CN
+// Four shapes: one CTA per SM per tile (all 512 tensor-memory columns, CN
 // = 144 / 112 / 96 / 64 columns for S = 3 / 4 / 5 / 6-7, up to four
 // stages); for S <= 5, two CTAs per SM (256 columns each, CN = 64 / 64 / 48,
-// two stages), where one CTA's epilogue overlaps the other's products; and
-// for S <= 5 the persistent ozk_gemm_pers_kernel (one CTA per SM walking the
-// tiles of width 64 / 64 / 48 with two accumulator sets).
+// two stages), where one CTA's epilogue overlaps the other's products; for S
+// <= 5 the persistent ozk_gemm_pers_kernel (one CTA per SM, its weights' tile
+// of width 64 / 64 / 48 resident, two accumulator sets); and, for 8-bit
+// digits, tiles of 16 columns for operands of few rows, where the wide tiles
+// leave most SMs without one.
 //
 // Every mbarrier wait is bounded (2^20 polls).  A wait that runs out marks
 // the tile's rows in the caller's status words; the producer then waits
@@ -53,30 +55,38 @@ constexpr int OZK_BK = 64;   // bytes of K per stage (one 64-byte swizzle row)
 constexpr int OZK_POLLS = 1 << 20;
 constexpr int OZK_SMEM_BUDGET = 220 * 1024;
 
-// PAIR = 0: one CTA per SM; PAIR = 1: two (S <= 5)
+// PAIR = 0: one CTA per SM; PAIR = 1: two (S <= 5); PAIR = 2: narrow tiles
+// for few rows
+constexpr int OZK_NARROW = 16;
 __host__ __device__ constexpr int ozk_cn(int S, int pair = 0) {
-  return pair ? (S <= 4 ? 64 : 48) : (S <= 3 ? 144 : S == 4 ? 112 : S == 5 ? 96 : 64);
+  return pair == 2 ? OZK_NARROW : pair ? (S <= 4 ? 64 : 48) : (S <= 3 ? 144 : S == 4 ? 112 : S == 5 ? 96 : 64);
 }
-__host__ __device__ constexpr int ozk_tmem_cols(int pair) { return pair ? 256 : 512; }
+__host__ __device__ constexpr int ozk_tmem_cols(int pair) { return pair == 2 ? 128 : pair ? 256 : 512; }
 __host__ __device__ constexpr int ozk_stage_bytes(int S, int pair = 0) {
   return S * OZK_BM * OZK_BK + S * ozk_cn(S, pair) * OZK_BK;
 }
 __host__ __device__ constexpr int ozk_stages(int S, int pair = 0) {
-  return pair ? 2 : OZK_SMEM_BUDGET / ozk_stage_bytes(S) > 4 ? 4 : OZK_SMEM_BUDGET / ozk_stage_bytes(S);
+  return pair == 1 ? 2 : OZK_SMEM_BUDGET / ozk_stage_bytes(S, pair) > 4 ? 4 : OZK_SMEM_BUDGET / ozk_stage_bytes(S, pair);
 }
 // the stage ring starts on a 1024-byte (one CTA per SM) or 512-byte (two)
 // boundary: the 64-byte swizzle repeats every 512 bytes
-__host__ __device__ constexpr int ozk_align(int pair) { return pair ? 512 : 1024; }
+__host__ __device__ constexpr int ozk_align(int pair) { return pair == 1 ? 512 : 1024; }
 __host__ __device__ constexpr int ozk_smem_bytes(int S, int pair = 0) {
   return ozk_stages(S, pair) * ozk_stage_bytes(S, pair) + ozk_align(pair);
 }
 // the persistent shape (S <= 5): the two-CTAs-per-SM tile width (S * CN <=
-// 256, so two accumulator sets fit the 512 tensor-memory columns) and as
-// many stages of that width as fit one CTA's shared memory (at most four)
-__host__ __device__ constexpr int ozk_pers_stages(int S) {
-  return (227 * 1024 - 2048) / ozk_stage_bytes(S, 1) > 4 ? 4 : (227 * 1024 - 2048) / ozk_stage_bytes(S, 1);
+// 256, so two accumulator sets fit the 512 tensor-memory columns), all nkb
+// K slices of the weights' tile resident, and as many stages of X as fit
+// beside them (0: does not fit)
+__host__ __device__ constexpr int ozk_pers_x_bytes(int S) { return S * OZK_BM * OZK_BK; }
+__host__ __device__ constexpr int ozk_pers_w_bytes(int S) { return S * ozk_cn(S, 1) * OZK_BK; }
+constexpr int OZK_PERS_MAX_STAGES = 4;
+constexpr int OZK_PERS_MAX_SLICES = 16;
+inline int ozk_pers_stages(int S, int nkb) {
+  const int left = 227 * 1024 - 1024 - 1024 - nkb * ozk_pers_w_bytes(S);  // static, alignment, weights
+  const int st = left > 0 ? left / ozk_pers_x_bytes(S) : 0;
+  return nkb > OZK_PERS_MAX_SLICES || st < 2 ? 0 : st > OZK_PERS_MAX_STAGES ? OZK_PERS_MAX_STAGES : st;
 }
-__host__ __device__ constexpr int ozk_pers_smem_bytes(int S) { return ozk_pers_stages(S) * ozk_stage_bytes(S, 1) + 1024; }
 // per CTA beside the stages: the reserved kilobyte, the barriers and the
 // epilogue's exponent factors (CN + 128 doubles)
 static_assert(2 * (ozk_smem_bytes(5, 1) + 1024 + 256 + 8 * (ozk_cn(5, 1) + 128)) <= 228 * 1024,
@@ -176,7 +186,7 @@ __device__ __forceinline__ void ozk_issue_kstep(uint32_t tacc, uint32_t xa, uint
 }
 
 template <int S, typename T, int PAIR, int BF>
-__global__ void __launch_bounds__(128, PAIR ? 2 : 1)
+__global__ void __launch_bounds__(128, PAIR == 1 ? 2 : 1)
     ozk_gemm_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
                     const int* __restrict__ ex, const int* __restrict__ ew, T* __restrict__ D, long ldd, int rows,
                     int cout, int nks, unsigned* __restrict__ status, int rows_per_status, unsigned bit) {
@@ -187,7 +197,7 @@ __global__ void __launch_bounds__(128, PAIR ? 2 : 1)
   constexpr int TC = ozk_tmem_cols(PAIR);
   constexpr unsigned AL = ozk_align(PAIR);
   static_assert(S * CN <= TC, "accumulators exceed tensor memory");
-  static_assert(!PAIR || S <= 5, "two CTAs per SM only for S <= 5");
+  static_assert(PAIR != 1 || S <= 5, "two CTAs per SM only for S <= 5");
   static_assert(CN % 16 == 0 && CN >= 16 && CN <= 256, "invalid MMA N");
   extern __shared__ __align__(1024) unsigned char ozk_smem_raw[];
   __shared__ __align__(8) uint64_t full[ST], empty[ST], done;
@@ -228,7 +238,7 @@ __global__ void __launch_bounds__(128, PAIR ? 2 : 1)
   // last column tile is narrower than CN)
   const int nkb = (nks + 1) / 2;
   const int rot = (int)((blockIdx.x * 7u + blockIdx.y) % (unsigned)nkb);
-  const int nmma = max(32, min(CN, (cout - c0 + 15) / 16 * 16));
+  const int nmma = min(CN, (cout - c0 + 15) / 16 * 16);
   int issued = 0;
   if (warp >= 2) {
     // the epilogue's exponent factors, loaded while the products run
@@ -341,64 +351,84 @@ __global__ void __launch_bounds__(128, PAIR ? 2 : 1)
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TC) : "memory");
 }
 
+// four consecutive FP64 values to a 32-byte boundary in one store
+__device__ __forceinline__ void st_v4(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
 // ozk_gemm_pers_kernel<S, T, BF> (S <= 5): the same product as a persistent
-// kernel.  One CTA of 256 threads per SM walks the output tiles of 128 rows
-// x CN columns (CN of the two-CTAs-per-SM shape, S * CN <= 256), tile t =
-// blockIdx.x + k * gridDim.x (column tiles fastest), with the accumulators
-// double-buffered in tensor memory (columns 0..255 for even, 256..511 for odd
-// tiles of the CTA), so the epilogue of one tile runs while the products of
-// the next are issued.  Thread 0 of warp 0 streams the K slices of all the
-// CTA's tiles through one stage ring; thread 0 of warp 1 issues the products
-// and marks a buffer's accumulators complete (accf, by tcgen05.commit);
-// warps 4..7 (tensor-memory lanes 32 (w - 4) ..) read, combine and store
-// them and mark the buffer free (acce, one arrival per warp).  Same digit
-// formats and the same results as ozk_gemm_kernel.  Every wait is bounded;
-// a role whose wait runs out stops, the others stop at their next bounded
-// wait or at the shared flag, issued copies and products are awaited
+// kernel for many rows.  A CTA (one per SM) keeps one column tile of CN
+// columns (CN of the two-CTAs-per-SM shape, S * CN <= 256): all K slices of
+// its W digits stay in shared memory, so only X streams, through a ring of
+// nst stages, and it walks the row tiles b / ntc, + G_ct, .. of its column
+// (b = blockIdx.x, column tile b % ntc, G_ct the CTAs of that column).  The
+// S W planes of a K slice lie one behind the other, so the products of an X
+// plane with all its W planes are one MMA of N = (S + 1 - p) CN <= 240: five
+// MMAs a 32-byte K step at S = 5.  The accumulators are double-buffered in
+// tensor memory (columns 0..255 and 256..511), so the epilogue of one row
+// tile runs while the products of the next are issued.  Thread 0 of warp 0
+// loads, thread 0 of warp 1 issues the products and marks a buffer complete
+// (accf, by tcgen05.commit); warps 4..11 (tensor-memory lanes 32 (w % 4) ..,
+// the column chunks split between the two warps of a quadrant) read, combine
+// and store it and mark it free (acce, one arrival per warp).  A thread
+// stores its row's columns as whole 32-byte sectors where the row is aligned.
+// Same digit formats and the same results as ozk_gemm_kernel.  Every wait is
+// bounded; a role whose wait runs out stops, the others stop at their next
+// bounded wait or at the shared flag, issued copies and products are awaited
 // (bounded) before the tensor memory is freed, and the rows of every tile
 // of the CTA are marked in the caller's status words.
 template <int S, typename T, int BF>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(384, 1)
     ozk_gemm_pers_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
                          const int* __restrict__ ex, const int* __restrict__ ew, T* __restrict__ D, long ldd,
-                         int rows, int cout, int nks, unsigned* __restrict__ status, int rows_per_status,
+                         int rows, int cout, int nks, int nst, unsigned* __restrict__ status, int rows_per_status,
                          unsigned bit) {
   constexpr int CN = ozk_cn(S, 1);
-  constexpr int XB = S * OZK_BM * OZK_BK;
-  constexpr int WB = S * CN * OZK_BK;
-  constexpr int ST = ozk_pers_stages(S);
+  constexpr int XB = ozk_pers_x_bytes(S);
+  constexpr int WB = ozk_pers_w_bytes(S);
+  constexpr int EW = 8;  // epilogue warps
   static_assert(S <= 5 && S * CN <= 256, "two accumulator sets must fit the tensor memory");
   static_assert(CN % 16 == 0 && CN >= 32, "invalid MMA N");
   extern __shared__ __align__(1024) unsigned char ozk_smem_raw[];
-  __shared__ __align__(8) uint64_t full[ST], empty[ST], accf[2], acce[2], done;
+  __shared__ __align__(8) uint64_t full[OZK_PERS_MAX_STAGES], empty[OZK_PERS_MAX_STAGES], wbar[OZK_PERS_MAX_SLICES],
+      accf[2], acce[2], done;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int failed;
-  __shared__ int issued_q, consumed_q;
+  __shared__ int issued_q, consumed_q, issued_w;
+  __shared__ double s_sw[CN];  // 2^ew of the column tile
   unsigned char* smem = ozk_smem_raw + ((1024u - (smem_u32(ozk_smem_raw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntc = (cout + CN - 1) / CN, ntr = (rows + OZK_BM - 1) / OZK_BM, ntiles = ntc * ntr;
+  const int ntc = (cout + CN - 1) / CN, ntr = (rows + OZK_BM - 1) / OZK_BM;
+  const int ct = blockIdx.x % ntc, rt0 = blockIdx.x / ntc, rstep = ((int)gridDim.x - ct + ntc - 1) / ntc;
+  const int c0 = ct * CN;
   const int nkb = (nks + 1) / 2;
+  unsigned char* sw = smem;             // [nkb][S][CN][64 bytes]
+  unsigned char* sx = smem + nkb * WB;  // [nst][S][128][64 bytes]
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < ST; ++i) {
+    for (int i = 0; i < nst; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
+    for (int i = 0; i < nkb; ++i) mbar_init(&wbar[i], 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(&accf[b], 1);
-      mbar_init(&acce[b], 4);
+      mbar_init(&acce[b], EW);
     }
     mbar_init(&done, 1);
     fence_mbar_init();
     failed = 0;
     issued_q = 0;
     consumed_q = 0;
+    issued_w = 0;
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  if (warp == 2)
+    for (int i = lane; i < CN; i += 32) s_sw[i] = c0 + i < cout ? pow2i(ew[c0 + i]) : 0.0;
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
@@ -406,32 +436,31 @@ __global__ void __launch_bounds__(256, 1)
   if (warp == 0 && lane == 0) {
     // producer
     int q = 0;
-    for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x) {
-      const int ct = t % ntc, rt = t / ntc, c0 = ct * CN, m0 = rt * OZK_BM;
-      const int rot = (int)((ct * 7u + rt) % (unsigned)nkb);
-      bool ok = true;
+    bool ok = true;
+    for (int rt = rt0; rt < ntr && ok && !failed; rt += rstep) {
       for (int k = 0; k < nkb; ++k) {
-        const int st = q % ST, kb = (k + rot) % nkb;
-        if (q >= ST && !mbar_wait(&empty[st], ((q / ST) - 1) & 1, OZK_POLLS)) {
+        if (rt == rt0) {
+          mbar_expect_tx(&wbar[k], WB);
+          tma_load_3d(sw + k * WB, &mw, &wbar[k], k * (OZK_BK / (BF ? 2 : 1)), c0, 0);
+          issued_w = k + 1;
+        }
+        const int st = q % nst;
+        if (q >= nst && !mbar_wait(&empty[st], ((q / nst) - 1) & 1, OZK_POLLS)) {
           failed = 1;
           ok = false;
           break;
         }
-        unsigned char* sx = smem + st * (XB + WB);
-        mbar_expect_tx(&full[st], XB + WB);
-        tma_load_3d(sx, &mx, &full[st], kb * (OZK_BK / (BF ? 2 : 1)), m0, 0);
-        tma_load_3d(sx + XB, &mw, &full[st], kb * (OZK_BK / (BF ? 2 : 1)), c0, 0);
+        mbar_expect_tx(&full[st], XB);
+        tma_load_3d(sx + st * XB, &mx, &full[st], k * (OZK_BK / (BF ? 2 : 1)), rt * OZK_BM, 0);
         ++q;
       }
-      if (!ok) break;
     }
     issued_q = q;
   } else if (warp == 1 && lane == 0) {
     // MMA issuer
     int q = 0, i = 0;
-    for (int t = blockIdx.x; t < ntiles && !failed; t += gridDim.x, ++i) {
-      const int ct = t % ntc, rt = t / ntc;
-      const int rot = (int)((ct * 7u + rt) % (unsigned)nkb);
+    bool ok = true;
+    for (int rt = rt0; rt < ntr && ok && !failed; rt += rstep, ++i) {
       const int b = i & 1;
       if (i >= 2 && !mbar_wait(&acce[b], ((i >> 1) - 1) & 1, OZK_POLLS)) {
         failed = 1;
@@ -439,20 +468,19 @@ __global__ void __launch_bounds__(256, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tb = tmem + (uint32_t)(b * 256);
-      bool ok = true;
       for (int k = 0; k < nkb; ++k) {
-        const int st = q % ST, kb = (k + rot) % nkb;
-        if (!mbar_wait(&full[st], (q / ST) & 1, OZK_POLLS)) {
+        const int st = q % nst;
+        if (!mbar_wait(&wbar[k], 0, OZK_POLLS) || !mbar_wait(&full[st], (q / nst) & 1, OZK_POLLS)) {
           failed = 1;
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t xa = smem_u32(smem + st * (XB + WB));
-        const uint32_t wa = xa + XB;
+        const uint32_t xa = smem_u32(sx + st * XB);
+        const uint32_t wa = smem_u32(sw + k * WB);
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
-          if (2 * kb + ks >= nks) break;
+          if (2 * k + ks >= nks) break;
           ozk_issue_kstep<S, CN, BF>(tb, xa, wa, ks, k == 0 && ks == 0);
         }
         umma_commit(&empty[st]);
@@ -465,13 +493,13 @@ __global__ void __launch_bounds__(256, 1)
     umma_commit(&done);
   } else if (warp >= 4) {
     // epilogue
-    const int wq = warp - 4;
+    const int wq = warp & 3, half = (warp - 4) >> 2;
+    const int nc = min(CN, cout - c0);  // columns of the tile
+    const bool vec = sizeof(T) == 8 && (ldd & 3) == 0 && (reinterpret_cast<uintptr_t>(D) & 31) == 0;
     int i = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++i) {
-      const int ct = t % ntc, rt = t / ntc, c0 = ct * CN, m0 = rt * OZK_BM;
-      const int nmma = max(32, min(CN, (cout - c0 + 15) / 16 * 16));
+    for (int rt = rt0; rt < ntr; rt += rstep, ++i) {
       const int b = i & 1;
-      const int row = m0 + wq * 32 + lane;
+      const int row = rt * OZK_BM + wq * 32 + lane;
       const double xs = row < rows ? pow2i(ex[row]) : 0.0;
       const bool got = mbar_wait(&accf[b], (i >> 1) & 1, OZK_POLLS);
       if (!__all_sync(0xffffffffu, got ? 1 : 0) || failed) {
@@ -481,23 +509,39 @@ __global__ void __launch_bounds__(256, 1)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tl = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(b * 256);
 #pragma unroll 1
-      for (int cc = 0; cc < nmma; cc += 16) {
+      for (int cc = half * 16; cc < nc; cc += 32) {
         uint32_t v[S][16];
 #pragma unroll
         for (int g = 0; g < S; ++g) tmem_ld16(tl + g * CN + cc, v[g]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        double o[16];
+#pragma unroll
+        for (int q2 = 0; q2 < 16; ++q2) {
+          // the digit groups as one 64-bit integer (see ozk_gemm_kernel)
+          long long h = 0;
+#pragma unroll
+          for (int g = 0; g < S; ++g) h = (h << 7) + (long long)(BF ? (int)__uint_as_float(v[g][q2]) : (int)v[g][q2]);
+          o[q2] = (((double)h * pow2i(-7 * (S + 1))) * xs) * s_sw[cc + q2];
+        }
         if (row < rows) {
           T* drow = D + (long)row * ldd + c0 + cc;
+          if constexpr (sizeof(T) == 8) {
+            if (vec) {
 #pragma unroll
-          for (int q2 = 0; q2 < 16; ++q2) {
-            // the digit groups as one 64-bit integer (see ozk_gemm_kernel)
-            long long h = 0;
+              for (int q4 = 0; q4 < 16; q4 += 4)
+                if (cc + q4 + 3 < nc) {
+                  st_v4(drow + q4, o[q4], o[q4 + 1], o[q4 + 2], o[q4 + 3]);
+                } else {
 #pragma unroll
-            for (int g = 0; g < S; ++g)
-              h = (h << 7) + (long long)(BF ? (int)__uint_as_float(v[g][q2]) : (int)v[g][q2]);
-            const int c = c0 + cc + q2;
-            if (c < cout) drow[q2] = (T)((((double)h * pow2i(-7 * (S + 1))) * xs) * pow2i(ew[c]));
+                  for (int q2 = q4; q2 < q4 + 4; ++q2)
+                    if (cc + q2 < nc) drow[q2] = o[q2];
+                }
+              continue;
+            }
           }
+#pragma unroll
+          for (int q2 = 0; q2 < 16; ++q2)
+            if (cc + q2 < nc) drow[q2] = (T)o[q2];
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -508,12 +552,13 @@ __global__ void __launch_bounds__(256, 1)
   __syncthreads();
   if (warp == 0 && lane == 0) {
     // copies issued but never consumed (only after a wait ran out)
-    for (int q = consumed_q; q < issued_q; ++q) mbar_wait(&full[q % ST], (q / ST) & 1, OZK_POLLS);
+    for (int q = consumed_q; q < issued_q; ++q) mbar_wait(&full[q % nst], (q / nst) & 1, OZK_POLLS);
+    for (int k = 0; k < issued_w; ++k) mbar_wait(&wbar[k], 0, OZK_POLLS);
   }
   const bool okd = __syncthreads_and(mbar_wait(&done, 0, OZK_POLLS) ? 1 : 0) && !failed;
   if (!okd && threadIdx.x == 0 && status) {
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      const int m0 = (t / ntc) * OZK_BM, r1 = min(m0 + OZK_BM, rows) - 1;
+    for (int rt = rt0; rt < ntr; rt += rstep) {
+      const int m0 = rt * OZK_BM, r1 = min(m0 + OZK_BM, rows) - 1;
       for (int qq = m0 / rows_per_status; qq <= r1 / rows_per_status; ++qq) atomicOr(status + qq, bit);
     }
   }
@@ -648,7 +693,7 @@ int prepare_pers() {
   SCY_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !(attr_set >> dev & 1ull)) {
     SCY_CUDA_TRY(cudaFuncSetAttribute(ozk_gemm_pers_kernel<S, T, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      ozk_pers_smem_bytes(S)));
+                                      227 * 1024 - 1024));
     if (dev >= 0 && dev < 64) attr_set |= 1ull << dev;
   }
   return SCY_OK;
@@ -663,6 +708,10 @@ int prepare_sb() {
     if (rc == SCY_OK) rc = prepare_one<S, float, 1, BF>();
     if (rc == SCY_OK) rc = prepare_pers<S, double, BF>();
     if (rc == SCY_OK) rc = prepare_pers<S, float, BF>();
+  }
+  if constexpr (BF == 0) {
+    if (rc == SCY_OK) rc = prepare_one<S, double, 2, 0>();
+    if (rc == SCY_OK) rc = prepare_one<S, float, 2, 0>();
   }
   return rc;
 }
@@ -702,17 +751,21 @@ int launch_gemm(const OzkOperand& x, const CUtensorMap& wmap, const OzkOperand& 
   return SCY_OK;
 }
 
-// the persistent shape: one CTA per SM (at most one per tile)
+// the persistent shape: one CTA per SM (at most one per tile); *used = 0
+// where the weights' tile does not fit beside two stages
 template <int S, typename T, int BF>
 int launch_pers(const OzkOperand& x, const OzkOperand& w, T* D, long ldd, int cout, cudaStream_t s,
-                unsigned* status, int rows_per_status, unsigned bit) {
+                unsigned* status, int rows_per_status, unsigned bit, int* used) {
   constexpr int CN = ozk_cn(S, 1);
+  const int nks = x.Kp * x.esz / 32, nkb = (nks + 1) / 2, nst = ozk_pers_stages(S, nkb);
+  *used = nst > 0;
+  if (!nst) return SCY_OK;
   SCY_TRY((prepare_pers<S, T, BF>()));
   const long ntiles = (long)((cout + CN - 1) / CN) * ((x.rows + OZK_BM - 1) / OZK_BM);
   const int grid = (int)std::min<long>(ntiles, sm_count());
-  ozk_gemm_pers_kernel<S, T, BF><<<grid, 256, ozk_pers_smem_bytes(S), s>>>(
-      x.map, w.map_pair, x.expo.as<int>(), w.expo.as<int>(), D, ldd, x.rows, cout, x.Kp * x.esz / 32, status,
-      rows_per_status, bit);
+  const int smem = nkb * ozk_pers_w_bytes(S) + nst * ozk_pers_x_bytes(S) + 1024;
+  ozk_gemm_pers_kernel<S, T, BF><<<grid, 384, smem, s>>>(x.map, w.map_pair, x.expo.as<int>(), w.expo.as<int>(), D,
+                                                         ldd, x.rows, cout, nks, nst, status, rows_per_status, bit);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -721,8 +774,15 @@ template <int S, typename T, int BF>
 int launch_variant_b(const OzkOperand& x, const OzkOperand& w, T* D, long ldd, int cout, cudaStream_t s,
                      unsigned* status, int rps, unsigned bit, int pair) {
   if constexpr (S <= 5) {
-    if (pair == 2) return launch_pers<S, T, BF>(x, w, D, ldd, cout, s, status, rps, bit);
-    if (pair) return launch_gemm<S, T, 1, BF>(x, w.map_pair, w, D, ldd, cout, s, status, rps, bit);
+    if (pair == 2) {
+      int used = 0;
+      SCY_TRY((launch_pers<S, T, BF>(x, w, D, ldd, cout, s, status, rps, bit, &used)));
+      if (used) return SCY_OK;
+    }
+    if (pair == 1 || pair == 2) return launch_gemm<S, T, 1, BF>(x, w.map_pair, w, D, ldd, cout, s, status, rps, bit);
+  }
+  if constexpr (BF == 0) {
+    if (pair == 3) return launch_gemm<S, T, 2, 0>(x, w.map_narrow, w, D, ldd, cout, s, status, rps, bit);
   }
   return launch_gemm<S, T, 0, BF>(x, w.map, w, D, ldd, cout, s, status, rps, bit);
 }
@@ -737,10 +797,10 @@ int launch_variant(const OzkOperand& x, const OzkOperand& w, T* D, long ldd, int
 template <typename T>
 int gemm_any(const OzkOperand& x, const OzkOperand& w, T* D, long ldd, int cout, cudaStream_t s, unsigned* status,
              int rps, unsigned bit, int pair) {
-  pair = pair == 2 ? 2 : pair ? 1 : 0;
   if (x.S != w.S || x.Kp != w.Kp || x.K != w.K || x.esz != w.esz || cout > w.rows || cout < 1 || x.rows < 1 ||
-      w.box_rows != ozk_cn(w.S) || x.box_rows != OZK_BM || rps < 1 ||
-      (pair && (w.S > 5 || w.box_rows_pair != ozk_cn(w.S, 1)))) {
+      w.box_rows != ozk_cn(w.S) || x.box_rows != OZK_BM || rps < 1 || pair < 0 || pair > 3 ||
+      ((pair == 1 || pair == 2) && (w.S > 5 || w.box_rows_pair != ozk_cn(w.S, 1))) ||
+      (pair == 3 && (w.box_rows_narrow != OZK_NARROW || w.esz != 1))) {
     set_error("ozk_gemm: operands do not match (S %d/%d, K %d/%d, cout %d, W rows %d, shape %d)", x.S,
               w.S, x.K, w.K, cout, w.rows, pair);
     return SCY_ERR_ARG;
@@ -749,8 +809,8 @@ int gemm_any(const OzkOperand& x, const OzkOperand& w, T* D, long ldd, int cout,
     case 3: return launch_variant<3, T>(x, w, D, ldd, cout, s, status, rps, bit, pair);
     case 4: return launch_variant<4, T>(x, w, D, ldd, cout, s, status, rps, bit, pair);
     case 5: return launch_variant<5, T>(x, w, D, ldd, cout, s, status, rps, bit, pair);
-    case 6: return launch_variant<6, T>(x, w, D, ldd, cout, s, status, rps, bit, 0);
-    case 7: return launch_variant<7, T>(x, w, D, ldd, cout, s, status, rps, bit, 0);
+    case 6: return launch_variant<6, T>(x, w, D, ldd, cout, s, status, rps, bit, pair);
+    case 7: return launch_variant<7, T>(x, w, D, ldd, cout, s, status, rps, bit, pair);
     default: break;
   }
   set_error("ozk_gemm: %d digit planes (3 to 7 are built)", x.S);
@@ -782,7 +842,18 @@ int OzkOperand::alloc_weights(int S_, int rows_, int K_, int esz_) {
       tma_map_3d_sw64(&map_pair, dig.p, esz == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8,
                       Kp, rows, S, Kp * esz, plane * esz, OZK_BK / esz, box_rows_pair, S) != SCY_OK)
     return SCY_ERR_CUDA;
+  if (esz == 1) {
+    box_rows_narrow = OZK_NARROW;
+    if (tma_map_3d_sw64(&map_narrow, dig.p, CU_TENSOR_MAP_DATA_TYPE_UINT8, Kp, rows, S, Kp, plane, OZK_BK,
+                        box_rows_narrow, S) != SCY_OK)
+      return SCY_ERR_CUDA;
+  }
   return SCY_OK;
+}
+
+bool ozk_narrow_better(int S, int rows, int cols) {
+  const long wide = (long)((cols + ozk_cn(S) - 1) / ozk_cn(S)) * ((rows + OZK_BM - 1) / OZK_BM);
+  return 2 * wide <= kNumSMs;
 }
 
 bool ozk_bf16_exact(int S, int K) {

@@ -37,15 +37,15 @@ namespace scy {
 // cores read).
 struct OzkOperand {
   DevBuf dig, expo;
-  int S = 0, rows = 0, K = 0, Kp = 0, box_rows = 0, box_rows_pair = 0;
+  int S = 0, rows = 0, K = 0, Kp = 0, box_rows = 0, box_rows_pair = 0, box_rows_narrow = 0;
   int esz = 1;  // bytes of a digit: 1 (signed 8-bit) or 2 (bf16)
   long plane = 0;  // digits of one plane (rows x Kp)
-  CUtensorMap map, map_pair;
+  CUtensorMap map, map_pair, map_narrow;
   // box_rows: 128 for the row operand (X), the column tile width of S
   // (ozk_cols_per_tile) for the weights (W); Kp = K rounded up to 32 bytes
   // of digits (one MMA K step)
   int alloc(int S, int rows, int K, int box_rows, int esz = 1);
-  // the weights' operand (W) with the maps of both product shapes
+  // the weights' operand (W) with the maps of every product shape
   int alloc_weights(int S, int rows, int K, int esz = 1);
 };
 
@@ -58,6 +58,10 @@ bool ozk_bf16_exact(int S, int K);
 // (S * width <= 256; 0 for S > 5)
 int ozk_cols_per_tile(int S);
 int ozk_cols_per_tile_pair(int S);
+
+// whether the narrow tiles are the faster shape for an X of `rows` rows and
+// `cols` weight rows: while the wide tiles are at most half as many as the SMs
+bool ozk_narrow_better(int S, int rows, int cols);
 
 // sets the kernels' shared-memory limit for S planes on the current device
 // (done by the first product too; call it before capturing one in a graph)
@@ -73,8 +77,10 @@ int ozk_set_host(OzkOperand& o, const double* W, long ldw, cudaStream_t s);
 // D of row stride ldd.  x.S == w.S.  A wait inside the kernel that runs out
 // (2^20 polls) sets `bit` in status[r / rows_per_status] for the rows of its
 // tile when status is given.  pair = 1 takes the two-CTAs-per-SM shape, pair
-// = 2 the persistent shape with double-buffered accumulators (both S <= 5,
-// W made by alloc_weights); the shapes give identical results.
+// = 2 the persistent shape with resident weights and double-buffered
+// accumulators (both S <= 5; the first where the weights' tile does not fit),
+// pair = 3 narrow tiles (8-bit digits); all with W made by alloc_weights; the
+// shapes give identical results.
 int ozk_gemm(const OzkOperand& x, const OzkOperand& w, double* D, long ldd, int cout, cudaStream_t s,
              unsigned* status = nullptr, int rows_per_status = 1, unsigned bit = 4u, int pair = 0);
 int ozk_gemm(const OzkOperand& x, const OzkOperand& w, float* D, long ldd, int cout, cudaStream_t s,

@@ -141,3 +141,14 @@ def test_ozaki_bf16_digits_give_the_same_product(s, ctas):
     D8 = _matmul(X, W, s, ctas=ctas, bf16=0)
     D16 = _matmul(X, W, s, ctas=ctas, bf16=1)
     assert np.array_equal(D8, D16)
+
+
+@pytest.mark.parametrize("rows,K,cols", [(129, 500, 49), (20000, 33, 48), (300, 650, 100)])
+def test_ozaki_persistent_shape_with_few_stages(rows, K, cols):
+    """The persistent shape with two stages beside its resident weights (K =
+    500), with one K slice and many row tiles a CTA, and beyond the shared
+    memory (K = 650, another shape takes over): the one-CTA shape's product."""
+    rng = np.random.default_rng(rows + K)
+    X = rng.standard_normal((rows, K)) * np.exp(2 * rng.standard_normal((rows, 1)))
+    W = rng.standard_normal((cols, K))
+    assert np.array_equal(_matmul(X, W, 5, ctas=0), _matmul(X, W, 5, ctas=1))
