@@ -567,107 +567,56 @@ __global__ void __launch_bounds__(384, 1)
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
-// digits of one row per warp, in two coalesced passes over the row (the
-// second from L1).  The first pass (lane l reads positions 32 t + l) gives
-// the row maximum (a warp reduction) and so the row's exponent; in the
-// second lane l takes the four consecutive positions 128 t + 4 l .. + 3 and
-// writes their S digits with one store per plane (four bytes, or the four
-// bf16 patterns of the digits: the upper halves of their FP32 patterns,
-// exact for |d| <= 256).  Kp is a multiple of 4, so every store is aligned
-// and inside the row.
-template <typename Tin, int BF>
+// digits of one row per warp, the row held in registers (Kp <= 32 NT): lane l
+// takes positions 32 c + l, so the loads are coalesced whatever the row's
+// alignment and the digits of a plane leave as whole 32-byte sectors (64-byte
+// in bf16).  The row's exponent is the largest exponent field in it (an
+// integer maximum); a row with no normal value, or with an infinity or NaN,
+// takes it from the largest magnitude.  A digit is rint(t) by adding and
+// taking off 1.5 2^52 (round to nearest even; the integer stands in the sum's
+// low word), so no conversion instruction is needed.
+template <typename Tin, int BF, int NT>
 __global__ void __launch_bounds__(256) ozk_split_kernel(const Tin* __restrict__ X, long ldx, int rows, int K, int Kp,
                                                         int S, unsigned char* __restrict__ dig, long plane,
                                                         int* __restrict__ expo) {
   const int row = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
-  const Tin* x = X + (long)row * ldx;
-  double m = 0.0;
-  for (int k = lane; k < K; k += 32) m = fmax(m, fabs((double)x[k]));
-  m = warp_max(m);
-  const int e = m > 0.0 ? ilogb(m) + 2 : 0;
-  if (lane == 0) expo[row] = e;
-  for (int k0 = 4 * lane; k0 < Kp; k0 += 128) {
-    double t[4];
+  const Tin* x = X + (long)row * ldx + lane;
+  double t[NT];
+  int em = 0;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) t[u] = k0 + u < K ? ldexp((double)x[k0 + u], 7 - e) : 0.0;
-    const long at = (long)row * Kp + k0;
-    for (int i = 0; i < S; ++i) {
-      uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const double d = rint(t[u]);
-        t[u] = (t[u] - d) * 128.0;
-        if (BF) {
-          const uint32_t h = __float_as_uint((float)d) >> 16;
-          if (u < 2)
-            w0 |= h << (16 * u);
-          else
-            w1 |= h << (16 * (u - 2));
-        } else {
-          w0 |= (uint32_t)(uint8_t)(int8_t)(int)d << (8 * u);
-        }
-      }
-      if (BF)
-        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(dig) + (long)i * plane + at) = make_uint2(w0, w1);
-      else
-        *reinterpret_cast<uint32_t*>(dig + (long)i * plane + at) = w0;
-    }
+  for (int c = 0; c < NT; ++c) {
+    t[c] = 32 * c + lane < K ? (double)x[32 * c] : 0.0;
+    em = max(em, __double2hiint(t[c]) & 0x7ff00000);
   }
-}
-
-// The same digits with the row held in registers (Kp <= 128 NC): lane l
-// loads positions 128 c + 4 l .. + 3 once, takes the row maximum from them
-// and writes the digits from them (one pass over the row in memory).
-template <typename Tin, int BF, int NC>
-__global__ void __launch_bounds__(256) ozk_split_reg_kernel(const Tin* __restrict__ X, long ldx, int rows, int K,
-                                                            int Kp, int S, unsigned char* __restrict__ dig,
-                                                            long plane, int* __restrict__ expo) {
-  const int row = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const Tin* x = X + (long)row * ldx;
-  double t[NC][4];
-  double m = 0.0;
+  em = __reduce_max_sync(0xffffffffu, em) >> 20;
+  int e = em - 1023 + 2;
+  if (em == 0 || em == 0x7ff) {
+    double m = 0.0;
 #pragma unroll
-  for (int c = 0; c < NC; ++c)
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = 128 * c + 4 * lane + u;
-      t[c][u] = k < K ? (double)x[k] : 0.0;
-      m = fmax(m, fabs(t[c][u]));
-    }
-  m = warp_max(m);
-  const int e = m > 0.0 ? ilogb(m) + 2 : 0;
+    for (int c = 0; c < NT; ++c) m = fmax(m, fabs(t[c]));
+    m = warp_max(m);
+    e = m > 0.0 ? ilogb(m) + 2 : 0;
+  }
   if (lane == 0) expo[row] = e;
+  const bool fits = 7 - e >= -1022 && 7 - e <= 1023;  // 2^(7 - e) is a normal number
+  const double sc = fits ? __longlong_as_double((long long)(7 - e + 1023) << 52) : 1.0;
+  constexpr double kRint = 6755399441055744.0;  // 1.5 2^52
+  const long at = (long)row * Kp + lane;
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const int k0 = 128 * c + 4 * lane;
-    if (k0 >= Kp) break;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) t[c][u] = ldexp(t[c][u], 7 - e);
-    const long at = (long)row * Kp + k0;
+  for (int c = 0; c < NT; ++c) {
+    if (32 * c + lane >= Kp) break;
+    double v = fits ? t[c] * sc : ldexp(t[c], 7 - e);
     for (int i = 0; i < S; ++i) {
-      uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const double d = rint(t[c][u]);
-        t[c][u] = (t[c][u] - d) * 128.0;
-        if (BF) {
-          const uint32_t h = __float_as_uint((float)d) >> 16;
-          if (u < 2)
-            w0 |= h << (16 * u);
-          else
-            w1 |= h << (16 * (u - 2));
-        } else {
-          w0 |= (uint32_t)(uint8_t)(int8_t)(int)d << (8 * u);
-        }
-      }
+      const double s = __dadd_rn(v, kRint);
+      const int d = __double2loint(s);
+      v = __dmul_rn(__dsub_rn(v, __dsub_rn(s, kRint)), 128.0);
       if (BF)
-        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(dig) + (long)i * plane + at) = make_uint2(w0, w1);
+        reinterpret_cast<uint16_t*>(dig)[(long)i * plane + at + 32 * c] =
+            (uint16_t)(__float_as_uint((float)d) >> 16);  // exact for |d| <= 256
       else
-        *reinterpret_cast<uint32_t*>(dig + (long)i * plane + at) = w0;
+        dig[(long)i * plane + at + 32 * c] = (unsigned char)d;
     }
   }
 }
@@ -889,37 +838,27 @@ int OzkOperand::alloc(int S_, int rows_, int K_, int box_rows_, int esz_) {
 }
 
 template <typename Tin, int BF>
-static void launch_split_reg(OzkOperand& o, const Tin* X, long ldx, cudaStream_t s, int blocks) {
+static void launch_split(OzkOperand& o, const Tin* X, long ldx, cudaStream_t s) {
+  const int blocks = (int)(((long)o.rows * 32 + 255) / 256);
   unsigned char* d = o.dig.as<unsigned char>();
   int* ex = o.expo.as<int>();
   if (o.Kp <= 128)
-    ozk_split_reg_kernel<Tin, BF, 1><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
+    ozk_split_kernel<Tin, BF, 4><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
   else if (o.Kp <= 256)
-    ozk_split_reg_kernel<Tin, BF, 2><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
+    ozk_split_kernel<Tin, BF, 8><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
   else if (o.Kp <= 512)
-    ozk_split_reg_kernel<Tin, BF, 4><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
+    ozk_split_kernel<Tin, BF, 16><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
   else
-    ozk_split_reg_kernel<Tin, BF, 8><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
+    ozk_split_kernel<Tin, BF, 32><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
 }
 
 template <typename Tin>
 static int split_any(OzkOperand& o, const Tin* X, long ldx, cudaStream_t s) {
-  const int threads = 256;
-  const int blocks = (int)(((long)o.rows * 32 + threads - 1) / threads);
-  if (o.Kp <= 1024) {  // the row in registers
-    if (o.esz == 2)
-      launch_split_reg<Tin, 1>(o, X, ldx, s, blocks);
-    else
-      launch_split_reg<Tin, 0>(o, X, ldx, s, blocks);
-    SCY_LAUNCH_CHECK();
-    return SCY_OK;
-  }
+  // K <= 1024 (OzkOperand::alloc)
   if (o.esz == 2)
-    ozk_split_kernel<Tin, 1><<<blocks, threads, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, o.dig.as<unsigned char>(),
-                                                        o.plane, o.expo.as<int>());
+    launch_split<Tin, 1>(o, X, ldx, s);
   else
-    ozk_split_kernel<Tin, 0><<<blocks, threads, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, o.dig.as<unsigned char>(),
-                                                        o.plane, o.expo.as<int>());
+    launch_split<Tin, 0>(o, X, ldx, s);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }

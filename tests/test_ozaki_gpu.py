@@ -143,6 +143,21 @@ def test_ozaki_bf16_digits_give_the_same_product(s, ctas):
     assert np.array_equal(D8, D16)
 
 
+@pytest.mark.parametrize("K", [1, 31, 32, 33, 128, 129, 256, 480, 512, 513, 1024])
+def test_ozaki_digit_split_at_row_lengths(K):
+    """Rows at the edges of the split's register tiles (128, 256, 512, 1024
+    positions) and of its 32-position chunks, among them a zero row, a row of
+    subnormal values and one whose values span 200 decades; same arithmetic
+    as ``emulate``, so the same bar as the other products."""
+    rng = np.random.default_rng(900 + K)
+    X = rng.standard_normal((70, K)) * np.exp(3 * rng.standard_normal((70, 1)))
+    X[1] = 0.0
+    X[2] *= 1e-310
+    X[3] *= 10.0 ** rng.integers(-100, 100, K)
+    W = rng.standard_normal((40, K))
+    np.testing.assert_allclose(_matmul(X, W, 5), emulate(X, W, 5), rtol=1e-15, atol=1e-300)
+
+
 @pytest.mark.parametrize("rows,K,cols", [(129, 500, 49), (20000, 33, 48), (300, 650, 100)])
 def test_ozaki_persistent_shape_with_few_stages(rows, K, cols):
     """The persistent shape with two stages beside its resident weights (K =
