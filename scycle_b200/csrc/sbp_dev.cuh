@@ -76,6 +76,11 @@ struct LevelDev {
   // full-form tile.
   int ylo, yhi, zlo, zhi, crow, ccol, rpt;
   T cyc[BAND], czc[BAND];
+  // Levels without the full form and of at most kCrossMaxNodes nodes: the
+  // operator composed per node (cross_build_kernel), 33 planes of Ny * Nz
+  // values, offsets -8..8 along y and then -8..-1, 1..8 along z (the centre
+  // is in the y part); null elsewhere.
+  const T* cross;
 };
 
 // -------------------------------------------------------------------------
@@ -640,6 +645,127 @@ __global__ void __launch_bounds__(256) full_kernel(LevelDev<T> L, Loader ld, Epi
   full_tile<T, RPT, Loader, Epi>(L, ld, ep, partials, counter, red_out);
 }
 
+// Cross-form tile (L.cross): the operand's 8 x 32 tile and halo staged once
+// as in full_apply, then one weighted sum per node with the node's own
+// coefficients.  Away from the boundary (eight lines) only the offsets up to
+// four are not zero: 17 coefficients a node, loaded ahead of the staged tile.
+// The two-stage tile above it replaces is bound by its chain of loads, two
+// barriers and 27-term sums through six tables (12.7 us a launch at 129 x 193
+// however small the grid); this one reads 136 bytes of coefficients a node
+// instead of 48, from L2 at the sizes it is used at.
+template <typename T, class Loader, class Epi>
+__global__ void __launch_bounds__(256) cross_kernel(LevelDev<T> L, Loader ld, Epi ep, double* partials,
+                                                    unsigned int* counter, double* red_out) {
+  __shared__ T xs[full_smem_values<1>()];
+  __shared__ double red[32];
+  const int Ny = L.Ny, Nz = L.Nz;
+  const long N = (long)Ny * Nz;
+  const int y0 = blockIdx.y * TY, z0 = blockIdx.x * TZ;
+  const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int iy = y0 + ty, iz = z0 + lane;
+  const bool valid = iy < Ny && iz < Nz;
+  const long node = (long)iy * Nz + iz;
+  const T* C = L.cross + (valid ? node : 0);
+  double contrib = 0.0;
+  if (y0 >= 8 && y0 + TY - 1 <= Ny - 9 && z0 >= 8 && z0 + TZ - 1 <= Nz - 9) {
+    constexpr int H = HALF, W = TZ + 2 * H;
+    T c[17];
+#pragma unroll
+    for (int o = 0; o < 9; ++o) c[o] = C[(long)(o + 4) * N];
+#pragma unroll
+    for (int o = 0; o < 8; ++o) c[9 + o] = C[(long)(21 + o) * N];
+    const auto pv = epi_pre(ep, node, iy, iz, 0);
+    full_stage<T, TY, H, false>(ld, xs, y0, z0, Ny, Nz);
+    __syncthreads();
+    const T* xy = xs + ty * W + H + lane;        // row iy - 4
+    const T* xz = xs + (ty + H) * W + lane;      // column iz - 4
+    T s0 = T(0), s1 = T(0);
+#pragma unroll
+    for (int o = 0; o < 9; ++o) s0 += c[o] * xy[o * W];
+#pragma unroll
+    for (int o = 0; o < 4; ++o) s1 += c[9 + o] * xz[o];
+#pragma unroll
+    for (int o = 4; o < 8; ++o) s1 += c[9 + o] * xz[o + 1];
+    contrib = epi_out(ep, node, iy, iz, s0 + s1, xy[H * W], pv);
+  } else {
+    constexpr int H = 8, W = TZ + 2 * H;
+    full_stage<T, TY, H, true>(ld, xs, y0, z0, Ny, Nz);
+    __syncthreads();
+    if (valid) {
+      const auto pv = epi_pre(ep, node, iy, iz, 0);
+      const T* xy = xs + ty * W + H + lane;
+      const T* xz = xs + (ty + H) * W + lane;
+      T s0 = T(0), s1 = T(0);
+#pragma unroll
+      for (int o = 0; o < 17; ++o) s0 += C[(long)o * N] * xy[o * W];
+#pragma unroll
+      for (int o = 0; o < 8; ++o) s1 += C[(long)(17 + o) * N] * xz[o];
+#pragma unroll
+      for (int o = 8; o < 16; ++o) s1 += C[(long)(17 + o) * N] * xz[o + 1];
+      contrib = epi_out(ep, node, iy, iz, s0 + s1, xy[H * W], pv);
+    }
+  }
+  if constexpr (Epi::kReduce) {
+    if (partials != nullptr) {  // uniform across the grid
+      double tot = block_sum(contrib, red);
+      grid_reduce_finish(tot, partials, counter, red_out, red);
+    }
+  }
+}
+
+// one line's composed stencil entry: row i, column i + o of
+//   Q c D - R3^T w3 m3 R3 - R4^T w4 c R4 + SAT
+// (the product the two-stage tile applies); c(k), m3(k) the line's coefficients
+template <typename T, class C1, class M3>
+__device__ __forceinline__ double cross_line_entry(const DirDev<T>& d, int i, int o, const C1& c, const M3& m3) {
+  const int n = d.n, l = i + o;
+  if (l < 0 || l >= n) return 0.0;
+  double acc = 0.0;
+  for (int j = 0; j < BAND; ++j) {
+    const int k = i + j - HALF, b = l - k + HALF;
+    if (k < 0 || k >= n || b < 0 || b >= BAND) continue;
+    const double q = (double)d.Q[(long)i * BAND + j], r3 = (double)d.R3T[(long)i * BAND + j];
+    acc += q * c(k) * (double)d.D[(long)k * BAND + b];
+    acc -= r3 * (double)d.w3[k] * m3(k) * (double)d.R3[(long)k * BAND + b];
+    if (d.R4) acc -= (double)d.R4T[(long)i * BAND + j] * (double)d.w4[k] * c(k) * (double)d.R4[(long)k * BAND + b];
+  }
+  if (d.bc_lo == 0) {
+    if (l == 0 && i < BAND) acc += ((double)d.bs0[i] + (i == 0 ? (double)d.alphaD : 0.0)) * c(0);
+  } else if (i == 0 && o <= HALF) {
+    acc += c(0) * (double)d.D[o + HALF];
+  }
+  if (d.bc_hi == 0) {
+    if (l == n - 1 && i >= n - BAND)
+      acc += ((double)d.bsN[i - (n - BAND)] + (i == n - 1 ? (double)d.alphaD : 0.0)) * c(n - 1);
+  } else if (i == n - 1 && o >= -HALF) {
+    acc -= c(n - 1) * (double)d.D[(long)(n - 1) * BAND + o + HALF];
+  }
+  return acc;
+}
+
+template <typename T>
+__global__ void cross_build_kernel(LevelDev<T> L, T* __restrict__ C) {
+  const int Nz = L.Nz;
+  const long N = (long)L.Ny * Nz;
+  for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < N; node += (long)gridDim.x * blockDim.x) {
+    const int iy = (int)(node / Nz), iz = (int)(node - (long)iy * Nz);
+    auto cy = [&](int k) { return (double)L.cy[(long)k * Nz + iz]; };
+    auto my = [&](int k) { return (double)L.m3y[(long)k * Nz + iz]; };
+    auto cz = [&](int k) { return (double)L.cz[(long)iy * Nz + k]; };
+    auto mz = [&](int k) { return (double)L.m3z[(long)iy * Nz + k]; };
+    const double wy = (double)L.wy[node], wz = (double)L.wz[node];
+    for (int o = -8; o <= 8; ++o) {
+      const double vy = wy * cross_line_entry(L.y, iy, o, cy, my), vz = wz * cross_line_entry(L.z, iz, o, cz, mz);
+      C[(long)(o + 8) * N + node] = (T)(o == 0 ? vy + vz : vy);
+      if (o != 0) C[(long)(o < 0 ? 25 + o : 24 + o) * N + node] = (T)vz;
+    }
+  }
+}
+
+// The cross form's coefficients stay in L2 (126 MB) with the vectors up to
+// about this many nodes (17 planes in use, 36 MB).
+constexpr long kCrossMaxNodes = 1L << 18;
+
 // rhs at one node from the boundary data (SbpOps::setRhs,
 // sbpOps_m_constGrid.cpp:877-914): the SAT columns of the Dirichlet
 // boundaries and the Neumann boundary values, times the outer weights.
@@ -696,7 +822,7 @@ __global__ void __launch_bounds__(256) stencil_kernel(LevelDev<T> L, Loader ld, 
 }
 
 // Launch grid of an operator application: full-form tiles of 8*rpt x 32 when
-// L.full, else the 8 x 32 tiles of stencil_tile.
+// L.full, else the 8 x 32 tiles of cross_kernel and stencil_tile.
 template <typename T>
 inline dim3 apply_grid(const LevelDev<T>& L) {
   const int ty = L.full ? 8 * L.rpt : TY;
@@ -709,7 +835,9 @@ template <typename T, class Loader, class Epi>
 inline void launch_apply(const LevelDev<T>& L, const Loader& ld, const Epi& ep, double* partials,
                          unsigned int* counter, double* red_out, cudaStream_t s) {
   const dim3 g = apply_grid(L);
-  if (!L.full)
+  if (!L.full && L.cross)
+    cross_kernel<T, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);
+  else if (!L.full)
     stencil_kernel<T, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);
   else if (L.rpt == 4)
     full_kernel<T, 4, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);

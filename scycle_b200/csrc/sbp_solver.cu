@@ -315,6 +315,12 @@ int LevelStore<T>::init(const LevelHost& h, cudaStream_t s) {
       }
     }
   }
+  if (const long n = (long)Ny * Nz; !dev.full && n <= kCrossMaxNodes) {
+    SCY_TRY(cross.alloc((size_t)n * 33 * sizeof(T)));
+    cross_build_kernel<T><<<grid_for(n), 256, 0, s>>>(dev, cross.template as<T>());
+    SCY_LAUNCH_CHECK();
+    dev.cross = cross.template as<T>();
+  }
   return SCY_OK;
 }
 
@@ -392,6 +398,191 @@ __global__ void dense_matvec_kernel(const T* __restrict__ M, const T* __restrict
   for (int j = lane; j < n; j += 32) acc += row[j] * b[j];
   acc = warp_sum(acc);
   if (lane == 0) out[warp] = acc;
+}
+
+// The V-cycle from a level of at most kCoarseNodes nodes down, in one launch:
+// one cluster of eight blocks, a thread for each node of a block's eighth of
+// every level.  The block's coefficients (cross form), b, d and dinv stay in
+// its shared memory; the vectors the operator and the transfers read are kept
+// whole in every block, and a thread sends its new value to all eight.  A
+// phase is then one sum from shared memory and one cluster barrier.  On their
+// own the phases of these levels are launches of 6 to 14 us: with all levels
+// launched a cycle of 257 x 385 took 31 launches and 330 us; the same phases
+// in one cluster with the vectors in L2 took 7 us each, for the eight SMs'
+// share of its bandwidth.  The arithmetic per node is that of the launches it
+// replaces (Chebyshev steps, full-weighting restriction, bilinear
+// prolongation, dense inverse on the last level).
+constexpr long kCoarseNodes = 2048;
+constexpr int kCoarseLevels = 6, kCoarseBlocks = 8, kCoarseThreads = 256, kCoarseNu = 4;
+static_assert(kCoarseNodes <= kCoarseBlocks * kCoarseThreads, "one thread per node");
+
+template <typename T>
+struct CoarseLevel {
+  int Ny, Nz, chunk;
+  int oC, ox, orr, ob;  // offsets (values) in shared memory: C [33][chunk], x [2][n], r [n], b, d, dinv [chunk]
+  const T *C, *dinv;    // cross-form planes
+  // transfer to the next coarser level
+  const int *ylo, *yhi, *zlo, *zhi, *jy, *jz;
+  const T *wy0, *wy1, *wz0, *wz1;
+  T c1[kCoarseNu], c2[kCoarseNu];
+};
+template <typename T>
+struct CoarseArgs {
+  CoarseLevel<T> lev[kCoarseLevels];
+  int nlev, nu, ncoarse;
+  const T* inv;
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void st_peer(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_peer(uint32_t a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+// v to the same place in every block of the cluster
+template <typename T>
+__device__ __forceinline__ void to_all(T* p, T v) {
+  const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
+#pragma unroll
+  for (int r = 0; r < kCoarseBlocks; ++r) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(r));
+    st_peer(ra, v);
+  }
+}
+
+// (A x) at node i, the block's t-th of the level; offsets that leave the grid
+// have zero coefficients and read the node itself
+template <typename T>
+__device__ __forceinline__ T coarse_apply(const CoarseLevel<T>& L, const T* sm, const T* x, int i, int t) {
+  const int Nz = L.Nz, iy = i / Nz, iz = i - iy * Nz;
+  const T* C = sm + L.oC + t;
+  T s0 = T(0), s1 = T(0);
+#pragma unroll
+  for (int o = -8; o <= 8; ++o) s0 += C[(o + 8) * L.chunk] * x[(unsigned)(iy + o) < (unsigned)L.Ny ? i + o * Nz : i];
+#pragma unroll
+  for (int o = -8; o <= 8; ++o)
+    if (o != 0) s1 += C[(o < 0 ? 25 + o : 24 + o) * L.chunk] * x[(unsigned)(iz + o) < (unsigned)Nz ? i + o : i];
+  return s0 + s1;
+}
+
+template <typename T, typename Tin>
+__global__ void __cluster_dims__(kCoarseBlocks, 1, 1) __launch_bounds__(kCoarseThreads)
+    coarse_cycle_kernel(const __grid_constant__ CoarseArgs<T> A, const Tin* __restrict__ b_in, T* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char coarse_smem[];
+  T* const sm = reinterpret_cast<T*>(coarse_smem);
+  const int t = threadIdx.x, last = A.nlev - 1;
+  auto node = [&](const CoarseLevel<T>& L) {
+    const int i = blockIdx.x * L.chunk + t;
+    return t < L.chunk && i < L.Ny * L.Nz ? i : -1;
+  };
+  for (int l = 0; l < last; ++l) {
+    const CoarseLevel<T>& L = A.lev[l];
+    const int i = node(L);
+    if (i < 0) continue;
+    const long N = (long)L.Ny * L.Nz;
+#pragma unroll
+    for (int o = 0; o < 33; ++o) sm[L.oC + o * L.chunk + t] = L.C[o * N + i];
+    sm[L.ob + 2 * L.chunk + t] = L.dinv[i];
+  }
+  // no block's shared memory is written before every block runs
+  cluster_barrier();
+  // b of level l and the first smoothing step's x = d = c2 dinv b
+  auto start = [&](const CoarseLevel<T>& L, int i, T bv) {
+    const T dv = L.c2[0] * sm[L.ob + 2 * L.chunk + t] * bv;
+    sm[L.ob + t] = bv;
+    sm[L.ob + L.chunk + t] = dv;
+    to_all(sm + L.ox + i, dv);
+  };
+  // Chebyshev step k from buffer `from`: the new value (to the other buffer, or returned only)
+  auto step = [&](const CoarseLevel<T>& L, int i, int k, bool first, int from) {
+    const T* x = sm + L.ox + from * L.Ny * L.Nz;
+    const T res = sm[L.ob + t] + coarse_apply(L, sm, x, i, t);
+    T dv = L.c2[k] * sm[L.ob + 2 * L.chunk + t] * res;
+    if (!first && L.c1[k] != T(0)) dv += L.c1[k] * sm[L.ob + L.chunk + t];
+    sm[L.ob + L.chunk + t] = dv;
+    return x[i] + dv;
+  };
+  {
+    const int i = node(A.lev[0]);
+    if (i >= 0) start(A.lev[0], i, (T)b_in[i]);
+    cluster_barrier();
+  }
+  const int pre = (A.nu - 1) & 1;  // buffer the pre-smoothing ends in; the post-smoothing ends in buffer 1
+  for (int l = 0; l < last; ++l) {
+    const CoarseLevel<T>& L = A.lev[l];
+    const int i = node(L), n = L.Ny * L.Nz;
+    for (int k = 1; k < A.nu; ++k) {
+      const int from = (k - 1) & 1;
+      if (i >= 0) to_all(sm + L.ox + (from ^ 1) * n + i, step(L, i, k, false, from));
+      cluster_barrier();
+    }
+    if (i >= 0) to_all(sm + L.orr + i, T(1) * sm[L.ob + t] + coarse_apply(L, sm, sm + L.ox + pre * n, i, t));
+    cluster_barrier();
+    const CoarseLevel<T>& M = A.lev[l + 1];
+    const int c = node(M);
+    if (c >= 0) {
+      const int a = c / M.Nz, bb = c - a * M.Nz;
+      T acc = T(0);
+      for (int iy = L.ylo[a]; iy <= L.yhi[a]; ++iy) {
+        const T wy = (L.jy[iy] == a ? L.wy0[iy] : T(0)) + (L.jy[iy] + 1 == a ? L.wy1[iy] : T(0));
+        if (wy == T(0)) continue;
+        T accz = T(0);
+        for (int iz = L.zlo[bb]; iz <= L.zhi[bb]; ++iz) {
+          const T wz = (L.jz[iz] == bb ? L.wz0[iz] : T(0)) + (L.jz[iz] + 1 == bb ? L.wz1[iz] : T(0));
+          accz += wz * sm[L.orr + iy * L.Nz + iz];
+        }
+        acc += wy * accz;
+      }
+      if (l + 1 < last)
+        start(M, c, acc);
+      else
+        to_all(sm + M.ox + c, acc);  // the dense solve reads b whole
+    }
+    cluster_barrier();
+  }
+  // the dense inverse: one warp a row
+  {
+    const CoarseLevel<T>& L = A.lev[last];
+    const int lane = t & 31, n = A.ncoarse;
+    for (int row = (blockIdx.x * kCoarseThreads + t) >> 5; row < n; row += kCoarseBlocks * kCoarseThreads / 32) {
+      T acc = T(0);
+      for (int j = lane; j < n; j += 32) acc += A.inv[(long)row * n + j] * sm[L.ox + j];
+      acc = warp_sum(acc);
+      if (lane == 0) to_all(sm + L.ox + n + row, acc);
+    }
+    cluster_barrier();
+  }
+  for (int l = last - 1; l >= 0; --l) {
+    const CoarseLevel<T>& L = A.lev[l];
+    const CoarseLevel<T>& M = A.lev[l + 1];
+    const int i = node(L), n = L.Ny * L.Nz;
+    // x + P xc
+    if (i >= 0) {
+      const int iy = i / L.Nz, iz = i - iy * L.Nz;
+      const T* c0 = sm + M.ox + M.Ny * M.Nz + L.jy[iy] * M.Nz + L.jz[iz];
+      const T* c1 = c0 + M.Nz;
+      const T v = L.wy0[iy] * (L.wz0[iz] * c0[0] + L.wz1[iz] * c0[1]) +
+                  L.wy1[iy] * (L.wz0[iz] * c1[0] + L.wz1[iz] * c1[1]);
+      to_all(sm + L.ox + pre * n + i, sm[L.ox + pre * n + i] + v);
+    }
+    cluster_barrier();
+    for (int k = 0; k < A.nu; ++k) {
+      const int from = (pre + k) & 1;
+      const bool final = l == 0 && k == A.nu - 1;
+      if (i >= 0) {
+        const T v = step(L, i, k, k == 0, from);
+        if (final)
+          out[i] = v;
+        else
+          to_all(sm + L.ox + (from ^ 1) * n + i, v);
+      }
+      if (!final) cluster_barrier();
+    }
+  }
 }
 
 // w = dinv .* v ; returns ||w||^2 and w.v through the reducer
@@ -723,11 +914,83 @@ int Multigrid<T>::setup_smoothers(const std::vector<LevelHost>& hosts, Reducer& 
   return SCY_OK;
 }
 
+// The level from which on the cycle runs as one launch, or -1: the finest with
+// at most kCoarseNodes nodes from which on every level has the cross form and
+// all fit a block's shared memory (162 KB in FP64 where each level has a
+// quarter of the nodes of the one before).
+template <typename T>
+int Multigrid<T>::coarse_first() const {
+  int f = nlev;
+  size_t values = 0;
+  while (f > 0) {
+    const long n = (long)lev[f - 1]->Ny * lev[f - 1]->Nz;
+    values += 3 * n + 36 * ((n + kCoarseBlocks - 1) / kCoarseBlocks);
+    if (!lev[f - 1]->dev.cross || n > kCoarseNodes || values * sizeof(T) > 226 * 1024) break;
+    --f;
+  }
+  return nlev - f >= 2 && nlev - f <= kCoarseLevels && nu >= 1 && nu <= kCoarseNu ? f : -1;
+}
+
+template <typename T>
+template <typename Tin>
+int Multigrid<T>::coarse_cycle(int l, const Tin* b_in, T** x_out, cudaStream_t s) {
+  CoarseArgs<T> A{};
+  A.nlev = nlev - l;
+  A.nu = nu;
+  A.ncoarse = ncoarse;
+  A.inv = coarse_inv.template as<T>();
+  int at = 0;
+  for (int k = 0; k < A.nlev; ++k) {
+    CoarseLevel<T>& c = A.lev[k];
+    const LevelDev<T>& L = lev[l + k]->dev;
+    const int n = L.Ny * L.Nz;
+    c.Ny = L.Ny;
+    c.Nz = L.Nz;
+    c.chunk = (n + kCoarseBlocks - 1) / kCoarseBlocks;
+    c.C = L.cross;
+    c.dinv = L.dinv;
+    c.ox = at;
+    at += 2 * n;
+    if (k + 1 < A.nlev) {
+      c.oC = at;
+      at += 33 * c.chunk;
+      c.orr = at;
+      at += n;
+      c.ob = at;
+      at += 3 * c.chunk;
+      const TransferDev& t = tr[l + k];
+      c.ylo = t.ylo.template as<int>();
+      c.yhi = t.yhi.template as<int>();
+      c.zlo = t.zlo.template as<int>();
+      c.zhi = t.zhi.template as<int>();
+      c.jy = t.jy.template as<int>();
+      c.jz = t.jz.template as<int>();
+      c.wy0 = t.wy0.template as<T>();
+      c.wy1 = t.wy1.template as<T>();
+      c.wz0 = t.wz0.template as<T>();
+      c.wz1 = t.wz1.template as<T>();
+      for (int q = 0; q < nu; ++q) {
+        c.c1[q] = (T)cheb[l + k][q].c1;
+        c.c2[q] = (T)cheb[l + k][q].c2;
+      }
+    }
+  }
+  const size_t smem = (size_t)at * sizeof(T);
+  SCY_CUDA_TRY(cudaFuncSetAttribute(coarse_cycle_kernel<T, Tin>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    227 * 1024));
+  T* x = work[l].v[1].template as<T>();
+  coarse_cycle_kernel<T, Tin><<<kCoarseBlocks, kCoarseThreads, smem, s>>>(A, b_in, x);
+  SCY_LAUNCH_CHECK();
+  *x_out = x;
+  return SCY_OK;
+}
+
 // z = V-cycle(b) at level l.  b_in is the level-0 right-hand side (any
 // precision); the result is left in work[0] x buffer (returned pointer).
 template <typename T>
 template <typename Tin>
 int Multigrid<T>::vcycle(int l, const Tin* b_in, T** x_out, cudaStream_t s) {
+  if (l == coarse_first()) return coarse_cycle<Tin>(l, b_in, x_out, s);
   const LevelDev<T>& L = lev[l]->dev;
   long n = (long)L.Ny * L.Nz;
   T* xa = work[l].v[0].template as<T>();

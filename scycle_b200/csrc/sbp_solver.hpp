@@ -60,6 +60,7 @@ struct LevelStore {
   DevBuf comp[2];     // composed interior stencils Cy (Ny x 9) and CzT (9 x Nz)
   DevBuf comp17[2];   // composed whole-operator stencils Cy17 (classes x Ny x 17), CzT17 (classes x 17 x Nz)
   DevBuf cls[2];      // line classes of the full form: ycls (Nz), zcls (Ny)
+  DevBuf cross;       // the cross form's coefficient planes (LevelDev::cross)
   DevBuf fullw[2];    // the full form's outer weights wy1 (Nz), wz1 (Ny) when the interior is not separable
   LevelDev<T> dev{};
   int init(const LevelHost& h, cudaStream_t s);
@@ -94,6 +95,9 @@ struct Multigrid {
   int setup_smoothers(const std::vector<LevelHost>& hosts, Reducer& red, double* dscal, cudaStream_t s);
   template <typename Tin>
   int vcycle(int l, const Tin* b_in, T** x_out, cudaStream_t s);
+  int coarse_first() const;
+  template <typename Tin>
+  int coarse_cycle(int l, const Tin* b_in, T** x_out, cudaStream_t s);
 };
 
 int build_hierarchy(const scy_grid_desc& g, const std::vector<double>& y, const std::vector<double>& z,
