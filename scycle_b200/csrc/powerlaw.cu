@@ -3,8 +3,8 @@
 // with PowerLaw's viscous source, strains, stresses, dislocation-creep
 // viscosity and strain rates (source/powerLaw.cpp:1239-1318, :1651-1887).
 //
-// Per d_dt: boundary data, rhs = setRhs + B gVxy + C gVxz (pl_source_kernel),
-// the elliptic solve, one fused per-node kernel for the strains, stresses,
+// Per d_dt: boundary data and rhs = setRhs + B gVxy + C gVxz in one launch
+// (qd_rhs_kernel with pl_source_node), the elliptic solve, one fused per-node kernel for the strains, stresses,
 // viscosity and strain rates (pl_rates_kernel), and the fault update with
 // tau from sxy on the fault row (pl_fault_kernel).
 //
@@ -24,14 +24,6 @@
 #include "sbp_dev.cuh"
 
 namespace scy {
-
-// rhs += B gVxy + C gVxz (computeViscStrainSourceTerms, initializeMomBalMats)
-__global__ void pl_source_kernel(LevelDev<double> L, const double* __restrict__ gxy, const double* __restrict__ gxz,
-                                 double* __restrict__ rhs) {
-  const long N = (long)L.Ny * L.Nz;
-  for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < N; node += (long)gridDim.x * blockDim.x)
-    rhs[node] = rhs[node] + 1.0 * pl_source_node(L, gxy, gxz, node);
-}
 
 // computeTotalStrains, computeStresses / computeSDev, computeViscosity and
 // computeViscStrainRates (with computeViscousStrainRateSAT) per node
@@ -56,21 +48,9 @@ int pl_d_dt(QDContext& q, double t, const double* var, double* f) {
   const long N = q.N;
   const int Nz = q.Nz;
   const LevelDev<double>& L = q.sbp.fine->dev;
-  SCY_TRY(qd_bc_launch(q, t, var));
-  SCY_TRY(q.sbp.set_rhs(q.bcL.as<double>(), q.bcR.as<double>(), q.bcT.as<double>(), q.bcB.as<double>(),
-                        q.rhs.as<double>()));
   const double* gxy = var + q.key_off[SCY_KEY_GVXY];
   const double* gxz = var + q.key_off[SCY_KEY_GVXZ];
   const int gb = grid_for(N, 256, 148 * 8);
-  pl_source_kernel<<<gb, 256, 0, s>>>(L, gxy, gxz, q.rhs.as<double>());
-  SCY_LAUNCH_CHECK();
-  scy_solve_opts o = q.solve_opts;
-  o.nonzero_guess = 1;
-  scy_solve_stats st{};
-  SCY_TRY(q.sbp.solve(q.rhs.as<double>(), q.u.as<double>(), o, st));
-  q.n_solve_its += st.iterations;
-  q.n_solves += 1;
-  q.last_rnorm = st.rnorm;
   PLRatesArgs a{};
   a.L = L;
   a.u = q.u.as<double>();
@@ -88,14 +68,16 @@ int pl_d_dt(QDContext& q, double t, const double* var, double* f) {
   a.sxz = q.sxz.as<double>();
   a.sdev = q.sdev.as<double>();
   a.effVisc = q.effVisc.as<double>();
-  pl_rates_kernel<<<gb, 256, 0, s>>>(a);
-  SCY_LAUNCH_CHECK();
-  const int tb = 64, fb = (Nz + tb - 1) / tb;
-  pl_fault_kernel<<<fb, tb, 0, s>>>(q.sxy.as<double>(), q.fp, var, f, q.slipVel.as<double>(), q.tauQSP.as<double>(),
-                                    q.tauP.as<double>(), q.strength.as<double>(), q.flags.as<unsigned>(),
-                                    q.fault_its.as<unsigned long long>());
-  SCY_LAUNCH_CHECK();
-  return SCY_OK;
+  return q.solve_stage(t, var, gxy, gxz, [&]() -> int {
+    pl_rates_kernel<<<gb, 256, 0, s>>>(a);
+    SCY_LAUNCH_CHECK();
+    const int tb = 64, fb = (Nz + tb - 1) / tb;
+    pl_fault_kernel<<<fb, tb, 0, s>>>(q.sxy.as<double>(), q.fp, var, f, q.slipVel.as<double>(),
+                                      q.tauQSP.as<double>(), q.tauP.as<double>(), q.strength.as<double>(),
+                                      q.fault_flags(), q.fault_its.as<unsigned long long>());
+    SCY_LAUNCH_CHECK();
+    return SCY_OK;
+  });
 }
 
 __global__ void pl_axpy_kernel(double* __restrict__ x, const double* __restrict__ d, long n) {

@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "fault_node.cuh"
 #include "infile.hpp"
+#include "powerlaw_dev.cuh"
 #include "qd.hpp"
 #include "thermal_dev.hpp"
 
@@ -27,6 +28,49 @@ __global__ void qd_bc_kernel(const double* __restrict__ slip, int Nz, double t, 
   if (i >= Nz) return;
   if (bcL_from_slip) bcL[i] = slip[i] * inv_fts;
   if (bcR_remote) bcR[i] = vL * t * inv_fts + shift[i];
+}
+
+// Boundary data and rhs of one d_dt in one launch, with the rhs's sum of
+// squares (-> norm2) for the solve: bcL and bcR as qd_bc_kernel sets them
+// (rows iy = 0), rhs = setRhs(bc) (+ B gVxy + C gVxz for the power law), and a
+// copy of the slip velocity the root finder starts from, for a fault update
+// that has to be made again.
+__global__ void __launch_bounds__(256) qd_rhs_kernel(LevelDev<double> L, const double* __restrict__ slip, double t,
+                                                     double vL, double inv_fts, int bcL_from_slip, int bcR_remote,
+                                                     const double* __restrict__ shift, double* bcL, double* bcR,
+                                                     const double* __restrict__ bcT, const double* __restrict__ bcB,
+                                                     const double* __restrict__ gxy, const double* __restrict__ gxz,
+                                                     double* __restrict__ rhs, const double* __restrict__ V,
+                                                     double* __restrict__ V0, double* partials, unsigned* counter,
+                                                     double* norm2) {
+  __shared__ double sh[32];
+  const int Nz = L.Nz;
+  const long N = (long)L.Ny * Nz;
+  auto left = [&](int iz) { return bcL_from_slip ? slip[iz] * inv_fts : bcL[iz]; };
+  auto right = [&](int iz) { return bcR_remote ? vL * t * inv_fts + shift[iz] : bcR[iz]; };
+  auto top = [&](int iy) { return bcT[iy]; };
+  auto bottom = [&](int iy) { return bcB[iy]; };
+  double acc = 0.0;
+  for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < N; node += (long)gridDim.x * blockDim.x) {
+    double v = set_rhs_node_f(L, left, right, top, bottom, node);
+    if (gxy) v = v + 1.0 * pl_source_node(L, gxy, gxz, node);
+    rhs[node] = v;
+    acc += v * v;
+    if (node < Nz) {
+      if (bcL_from_slip) bcL[node] = slip[node] * inv_fts;
+      if (bcR_remote) bcR[node] = vL * t * inv_fts + shift[node];
+      V0[node] = V[node];
+    }
+  }
+  const double s = block_sum(acc, sh);
+  grid_reduce_finish(s, partials, counter, norm2, sh);
+}
+
+// one enqueued solve's scalars (|rhs|^2, r.r, |r0|^2) into its record
+__global__ void qd_record_kernel(const double* __restrict__ sc, double* __restrict__ rec) {
+  rec[0] = sc[0];
+  rec[1] = sc[1];
+  rec[2] = sc[5];
 }
 
 // Fault column: sxy = mu*Dy*u at iy = 0 (body2L scatter of muxDy), then the
@@ -168,10 +212,15 @@ struct KeyTable {
   long off[4], len[4];
 };
 
+// QDContext::errbuf: the error sums (12), the switch test's maximum ([12]),
+// the fault flags, and the records of an attempt's enqueued solves
+enum { RB_FLAGS = 13, RB_SOLVE = 16, RB_SIZE = RB_SOLVE + 3 * 6 };
+
 __global__ void rk_error_kernel(const double* __restrict__ lo, const double* __restrict__ hi, KeyTable kt,
-                                double* __restrict__ out) {
+                                const unsigned* __restrict__ flags, double* __restrict__ out) {
   __shared__ double sh[32];
   const int key = blockIdx.x;
+  if (key == 0 && threadIdx.x == 0) out[RB_FLAGS] = (double)(flags[0] | flags[1]);  // read back with the sums
   const long off = kt.off[key], len = kt.len[key];
   double ss = 0.0, sh2 = 0.0, mx = -INFINITY;
   for (long i = threadIdx.x; i < len; i += blockDim.x) {
@@ -338,16 +387,28 @@ int QDContext::create(const scy_qd_desc& d, const scy_pl_desc* pld) {
     SCY_TRY(b.alloc((size_t)nvar * 8));
     SCY_CUDA_TRY(cudaMemset(b.p, 0, (size_t)nvar * 8));
   }
-  SCY_TRY(errbuf.alloc(16 * 8));
+  SCY_TRY(errbuf.alloc(RB_SIZE * 8));
+  SCY_CUDA_TRY(cudaMemset(errbuf.p, 0, RB_SIZE * 8));
+  SCY_TRY(slipVel0.alloc((size_t)Nz * 8));
+  SCY_CUDA_TRY(cudaMallocHost((void**)&h_read, RB_SIZE * 8));
   return SCY_OK;
 }
 
+QDContext::~QDContext() {
+  if (h_read) cudaFreeHost(h_read);
+}
+
 int QDContext::read_flags() {
-  unsigned h = 0;
-  SCY_CUDA_TRY(cudaMemcpyAsync(&h, flags.p, sizeof(unsigned), cudaMemcpyDeviceToHost, sbp.stream));
-  SCY_CUDA_TRY(cudaStreamSynchronize(sbp.stream));
+  unsigned h = flags_read;
+  if (!flags_known) {
+    unsigned* w = reinterpret_cast<unsigned*>(h_read);
+    SCY_CUDA_TRY(cudaMemcpyAsync(w, flags.p, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, sbp.stream));
+    SCY_CUDA_TRY(cudaStreamSynchronize(sbp.stream));
+    h = w[0] | w[1];
+  }
+  flags_known = 0;
   if (h) {
-    SCY_CUDA_TRY(cudaMemsetAsync(flags.p, 0, sizeof(unsigned), sbp.stream));
+    SCY_CUDA_TRY(cudaMemsetAsync(flags.p, 0, 2 * sizeof(unsigned), sbp.stream));
     if (h & FAULT_NONFINITE) {
       set_error("non-finite value in the fault root bracket or state rate");
       return SCY_ERR_NONFINITE;
@@ -355,15 +416,6 @@ int QDContext::read_flags() {
     set_error("rootFinder BracketedNewton did not converge within %d iterations", fp.max_its);
     return SCY_ERR_ROOT_NOCONV;
   }
-  return SCY_OK;
-}
-
-int qd_bc_launch(QDContext& q, double t, const double* var) {
-  const int tb = 64, gb = (q.Nz + tb - 1) / tb;
-  qd_bc_kernel<<<gb, tb, 0, q.sbp.stream>>>(var + q.fp.slip_off, q.Nz, t, q.vL, 1.0 / q.fts, q.bcL_from_slip,
-                                            q.bcR_remote, q.bcRShift.as<double>(), q.bcL.as<double>(),
-                                            q.bcR.as<double>());
-  SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
 
@@ -393,28 +445,141 @@ int QDContext::d_dt(double t, const double* var, double* f) {
         tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), bcL.as<double>(), flags.as<unsigned>(),
         fault_its.as<unsigned long long>());
     SCY_LAUNCH_CHECK();
+    flags_known = 0;
     last_t = t;
     ++n_d_dt;
     return SCY_OK;
   }
-  const int tb = 64, gb = (Nz + tb - 1) / tb;
-  qd_bc_kernel<<<gb, tb, 0, s>>>(var + fp.slip_off, Nz, t, vL, 1.0 / fts, bcL_from_slip, bcR_remote,
-                                 bcRShift.as<double>(), bcL.as<double>(), bcR.as<double>());
+  SCY_TRY(solve_stage(t, var, nullptr, nullptr, [&]() -> int {
+    const int tb = 64, gb = (Nz + tb - 1) / tb;
+    qd_fault_kernel<<<gb, tb, 0, s>>>(sbp.fine->dev, u.as<double>(), fp, var, f, slipVel.as<double>(),
+                                      tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), fault_flags(),
+                                      fault_its.as<unsigned long long>());
+    SCY_LAUNCH_CHECK();
+    return SCY_OK;
+  }));
+  last_t = t;
+  ++n_d_dt;
+  return SCY_OK;
+}
+
+// The elliptic solve of one d_dt (boundary data and rhs from the state, the
+// viscous strains given for the power law) and what follows from its
+// displacement (after: the fault update, the viscous rates).
+//
+// Where one iteration is enough, as it is for a warm-started stage, nothing
+// is read in between: the iteration and `after` are enqueued, and the solve's
+// scalars come back with the fault's flags in one copy, or, in an attempt
+// (deferring), with the attempt's error sums.  A step of 401 x 401 waited for
+// the device six times before, about 10 us each.  A solve that turns out to
+// need more iterations goes on from its first one, and `after` is made again
+// from the same first guess (slipVel0; its flags go to a word of their own).
+int QDContext::solve_stage(double t, const double* var, const double* gxy, const double* gxz,
+                           const std::function<int()>& after) {
+  cudaStream_t s = sbp.stream;
+  flags_known = 0;
+  const int rb = grid_for(N, 256, 592);
+  qd_rhs_kernel<<<rb, 256, 0, s>>>(sbp.fine->dev, var + fp.slip_off, t, vL, 1.0 / fts, bcL_from_slip, bcR_remote,
+                                   bcRShift.as<double>(), bcL.as<double>(), bcR.as<double>(), bcT.as<double>(),
+                                   bcB.as<double>(), gxy, gxz, rhs.as<double>(), slipVel.as<double>(),
+                                   slipVel0.as<double>(), sbp.red.partials.as<double>(),
+                                   sbp.red.counter.as<unsigned>(), sbp.scal.as<double>());
   SCY_LAUNCH_CHECK();
-  SCY_TRY(sbp.set_rhs(bcL.as<double>(), bcR.as<double>(), bcT.as<double>(), bcB.as<double>(), rhs.as<double>()));
   scy_solve_opts o = solve_opts;
   o.nonzero_guess = 1;  // the previous stage's displacement is the initial guess
   scy_solve_stats st{};
-  SCY_TRY(sbp.solve(rhs.as<double>(), u.as<double>(), o, st));
+  SolvePart part;
+  part.norm_ready = 1;
+  if (!sbp.can_enqueue(o)) {
+    SCY_TRY(sbp.solve(rhs.as<double>(), u.as<double>(), o, st, part));
+    SCY_TRY(after());
+  } else {
+    part.enqueue = 1;
+    SCY_TRY(sbp.solve(rhs.as<double>(), u.as<double>(), o, st, part));
+    spec_flags = 1;
+    const int rc = after();
+    spec_flags = 0;
+    SCY_TRY(rc);
+    if (deferring) {
+      qd_record_kernel<<<1, 1, 0, s>>>(sbp.scal.as<double>(), errbuf.as<double>() + RB_SOLVE + 3 * deferred++);
+      SCY_LAUNCH_CHECK();
+      return SCY_OK;
+    }
+    SCY_CUDA_TRY(cudaMemcpyAsync(h_read, sbp.scal.p, 6 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    unsigned* hf = reinterpret_cast<unsigned*>(h_read + 6);
+    SCY_CUDA_TRY(cudaMemcpyAsync(hf, flags.p, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    SCY_CUDA_TRY(cudaStreamSynchronize(s));
+    const double tol = std::max(o.rtol * std::sqrt(h_read[0]), o.atol);
+    part.enqueue = 0;
+    part.first = h_read;
+    const bool more = !(std::sqrt(h_read[1]) <= tol || std::sqrt(h_read[5]) <= tol) || (h_read[0] == 0.0 && tol == 0.0);
+    const unsigned before = hf[0];
+    SCY_TRY(sbp.solve(rhs.as<double>(), u.as<double>(), o, st, part));
+    if (more) {
+      SCY_CUDA_TRY(cudaMemsetAsync(flags.as<unsigned>() + 1, 0, sizeof(unsigned), s));
+      SCY_CUDA_TRY(cudaMemcpyAsync(slipVel.p, slipVel0.p, (size_t)Nz * 8, cudaMemcpyDeviceToDevice, s));
+      SCY_TRY(after());
+    } else {
+      flags_known = 1;
+      flags_read = before | hf[1];
+      if (hf[1]) {
+        // final now: to the first word, so that the second holds only what
+        // the next enqueued update sets
+        hf[0] = flags_read;
+        hf[1] = 0;
+        SCY_CUDA_TRY(cudaMemcpyAsync(flags.p, hf, 2 * sizeof(unsigned), cudaMemcpyHostToDevice, s));
+        SCY_CUDA_TRY(cudaStreamSynchronize(s));
+      }
+    }
+  }
   n_solve_its += st.iterations;
   n_solves += 1;
   last_rnorm = st.rnorm;
-  qd_fault_kernel<<<gb, tb, 0, s>>>(sbp.fine->dev, u.as<double>(), fp, var, f, slipVel.as<double>(),
-                                    tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(),
-                                    flags.as<unsigned>(), fault_its.as<unsigned long long>());
-  SCY_LAUNCH_CHECK();
-  last_t = t;
-  ++n_d_dt;
+  return SCY_OK;
+}
+
+// One attempt with its solves enqueued and read back with the error sums.
+// *ok = 0: a solve needed more than one iteration; the displacement, the slip
+// velocity and the flags are again what they were before the attempt.
+int QDContext::attempt_deferred(double dt, double** lo, double** hi, double* err, int* ok) {
+  cudaStream_t s = sbp.stream;
+  const bool solves = pl || mode == SCY_QD_MODE_SOLVE;
+  if (solves) {
+    if (u_save.bytes < (size_t)N * 8) {
+      SCY_TRY(u_save.alloc((size_t)N * 8));
+      SCY_TRY(slipVel_save.alloc((size_t)Nz * 8));
+    }
+    SCY_CUDA_TRY(cudaMemcpyAsync(u_save.p, u.p, (size_t)N * 8, cudaMemcpyDeviceToDevice, s));
+    SCY_CUDA_TRY(cudaMemcpyAsync(slipVel_save.p, slipVel.p, (size_t)Nz * 8, cudaMemcpyDeviceToDevice, s));
+  }
+  const long evals = n_d_dt;
+  deferring = 1;
+  deferred = 0;
+  int rc = attempt(dt, lo, hi);
+  deferring = 0;
+  SCY_TRY(rc);
+  SCY_TRY(launch_error(*lo, *hi));
+  SCY_CUDA_TRY(cudaMemcpyAsync(h_read, errbuf.p, (RB_SOLVE + 3 * deferred) * sizeof(double), cudaMemcpyDeviceToHost, s));
+  SCY_CUDA_TRY(cudaStreamSynchronize(s));
+  *ok = 1;
+  for (int k = 0; k < deferred; ++k) {
+    const double* c = h_read + RB_SOLVE + 3 * k;
+    const double tol = std::max(solve_opts.rtol * std::sqrt(c[0]), solve_opts.atol);
+    if (!(std::sqrt(c[1]) <= tol || std::sqrt(c[2]) <= tol) || (c[0] == 0.0 && tol == 0.0)) *ok = 0;
+  }
+  if (!*ok) {
+    SCY_CUDA_TRY(cudaMemcpyAsync(u.p, u_save.p, (size_t)N * 8, cudaMemcpyDeviceToDevice, s));
+    SCY_CUDA_TRY(cudaMemcpyAsync(slipVel.p, slipVel_save.p, (size_t)Nz * 8, cudaMemcpyDeviceToDevice, s));
+    SCY_CUDA_TRY(cudaMemsetAsync(flags.p, 0, 2 * sizeof(unsigned), s));
+    n_d_dt = evals;
+    return SCY_OK;
+  }
+  n_solves += deferred;
+  n_solve_its += deferred;
+  if (deferred) last_rnorm = std::sqrt(h_read[RB_SOLVE + 3 * (deferred - 1) + 1]);
+  flags_known = 1;
+  flags_read = (unsigned)h_read[RB_FLAGS];
+  *err = error_from(h_read);
   return SCY_OK;
 }
 
@@ -591,19 +756,26 @@ double QDContext::compute_step_size(double totErr) {
   return dt;
 }
 
-int QDContext::compute_error(const double* lo, const double* hi, double* err) {
+int QDContext::launch_error(const double* lo, const double* hi) {
   cudaStream_t s = sbp.stream;
   KeyTable kt;
   for (int k = 0; k < 4; ++k) {
     kt.off[k] = key_off[k];
     kt.len[k] = key_len[k];
   }
-  rk_error_kernel<<<pl ? 4 : 2, 1024, 0, s>>>(lo, hi, kt, errbuf.as<double>());
+  rk_error_kernel<<<pl ? 4 : 2, 1024, 0, s>>>(lo, hi, kt, flags.as<unsigned>(), errbuf.as<double>());
   SCY_LAUNCH_CHECK();
-  double h[12];
-  SCY_CUDA_TRY(cudaMemcpyAsync(h, errbuf.p, (pl ? 12 : 6) * sizeof(double), cudaMemcpyDeviceToHost, s));
+  return SCY_OK;
+}
+
+int QDContext::compute_error(const double* lo, const double* hi, double* err) {
+  cudaStream_t s = sbp.stream;
+  SCY_TRY(launch_error(lo, hi));
+  SCY_CUDA_TRY(cudaMemcpyAsync(h_read, errbuf.p, RB_SOLVE * sizeof(double), cudaMemcpyDeviceToHost, s));
   SCY_CUDA_TRY(cudaStreamSynchronize(s));
-  *err = error_from(h);
+  *err = error_from(h_read);
+  flags_known = 1;
+  flags_read = (unsigned)h_read[RB_FLAGS];
   return SCY_OK;
 }
 
@@ -798,9 +970,18 @@ int QDContext::integrate_steps(long nsteps, scy_ode_stats* st) {
         forced_accept = forced_acc[forced_pos];
         ++forced_pos;
       }
-      SCY_TRY(attempt(deltaT, &lo, &hi));
+      // response mode has no solves to miss; after a miss the next attempts
+      // test every solve as they go
+      int ok = 0;
+      const bool defer = !th && defer_pause == 0 && (mode == SCY_QD_MODE_RESPONSE || sbp.can_enqueue(solve_opts));
+      if (defer) SCY_TRY(attempt_deferred(deltaT, &lo, &hi, &totErr, &ok));
+      if (defer_pause > 0) --defer_pause;
+      if (!ok) {
+        if (defer) defer_pause = 16;
+        SCY_TRY(attempt(deltaT, &lo, &hi));
+        SCY_TRY(compute_error(lo, hi, &totErr));
+      }
       used_dt = deltaT;
-      SCY_TRY(compute_error(lo, hi, &totErr));
       SCY_TRY(read_flags());
       bool acc = (ode.method == SCY_RK32 && !imex) ? (totErr <= totTol) : (totErr < totTol);
       if (forced) acc = forced_accept != 0;
@@ -823,7 +1004,10 @@ int QDContext::integrate_steps(long nsteps, scy_ode_stats* st) {
     // one backward-Euler heat step with the new slip velocity and tauP
     if (th && th->coupled) SCY_TRY(th->set_fault_temperature());
     SCY_TRY(d_dt(currT, var, dvar));
-    SCY_TRY(read_flags());
+    // response mode launches one kernel: its flags come with the next attempt's
+    // error sums, or at the end of this call
+    const bool later = mode == SCY_QD_MODE_RESPONSE && !pl && !th && !out && !monitor && ckpt <= 0;
+    if (!later) SCY_TRY(read_flags());
     if (th) SCY_TRY(th->step(*this, deltaT));
     if (totErr != 0.0) newDeltaT = compute_step_size(totErr);
     errA[1] = errA[0];
@@ -849,6 +1033,7 @@ int QDContext::integrate_steps(long nsteps, scy_ode_stats* st) {
     }
     deltaT = newDeltaT;
   }
+  if (done_steps > 0 && mode == SCY_QD_MODE_RESPONSE) SCY_TRY(read_flags());
   if (st) {
     st->t = currT;
     st->dt = last_dt;

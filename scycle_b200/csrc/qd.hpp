@@ -47,7 +47,17 @@ struct QDContext {
   // counts the operations of this driver that changed rhs or u (from 1), so
   // that a batch notices solves made beside its own rounds
   unsigned long long u_epoch = 1;
-  DevBuf flags;                             // unsigned, fault status bits
+  DevBuf flags;                             // two words of fault status bits: updates of finished / of enqueued solves
+  DevBuf slipVel0, u_save, slipVel_save;    // what an enqueued fault update or attempt started from
+  double* h_read = nullptr;                 // pinned, for read-backs
+  int flags_known = 0;                      // flags_read holds the flags as of the last launch
+  unsigned flags_read = 0;
+  int spec_flags = 0, deferring = 0, deferred = 0, defer_pause = 0;
+  unsigned* fault_flags() const { return flags.as<unsigned>() + (spec_flags ? 1 : 0); }
+  QDContext() = default;
+  QDContext(const QDContext&) = delete;
+  QDContext& operator=(const QDContext&) = delete;
+  ~QDContext();
   DevBuf fault_its;                         // unsigned long long, root iterations
   double vL = 1e-9, fts = 2.0;
   int bcL_from_slip = 1, bcR_remote = 1;
@@ -59,7 +69,7 @@ struct QDContext {
   scy_ode_opts ode{};
   int ode_ready = 0;
   DevBuf rk[16];  // var, dvar, k/f stage vectors, lo/hi
-  DevBuf errbuf;  // 8 doubles
+  DevBuf errbuf;  // what an attempt reads back (RB_* in qd.cu)
   double currT = 0, deltaT = 0, newDeltaT = 0, totTol = 1e-9, last_dt = 0;
   long stepCount = 0, numRejected = 0, numMin = 0, numMax = 0;
   double errA[2] = {0, 0};
@@ -143,6 +153,10 @@ struct QDContext {
   int phase_stopped = 0;
   double compute_step_size(double totErr);
   int compute_error(const double* lo, const double* hi, double* err);
+  int launch_error(const double* lo, const double* hi);
+  int attempt_deferred(double dt, double** lo, double** hi, double* err, int* ok);
+  int solve_stage(double t, const double* var, const double* gxy, const double* gxz,
+                  const std::function<int()>& after);
   // computeError from the per-key sums (sum d^2, sum hi^2, max |d/hi|) at h[3*key]
   double error_from(const double* h) const;
   int attempt(double dt, double** lo, double** hi);
@@ -150,8 +164,6 @@ struct QDContext {
 };
 
 int qd_green_surf_launch(QDContext& q, double c, double* host_out);
-// bcL = slip/faultTypeScale, bcR = vL t/faultTypeScale + bcRShift from the state var
-int qd_bc_launch(QDContext& q, double t, const double* var);
 // StrikeSlip_PowerLaw_qd::d_dt (powerlaw.cu)
 int pl_d_dt(QDContext& q, double t, const double* var, double* f);
 

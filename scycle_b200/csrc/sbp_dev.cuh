@@ -768,36 +768,45 @@ constexpr long kCrossMaxNodes = 1L << 18;
 
 // rhs at one node from the boundary data (SbpOps::setRhs,
 // sbpOps_m_constGrid.cpp:877-914): the SAT columns of the Dirichlet
-// boundaries and the Neumann boundary values, times the outer weights.
-__device__ __forceinline__ double set_rhs_node(const LevelDev<double>& L, const double* __restrict__ bcL,
-                                               const double* __restrict__ bcR, const double* __restrict__ bcT,
-                                               const double* __restrict__ bcB, long node) {
+// boundaries and the Neumann boundary values, times the outer weights.  The
+// boundary values come as bcL(iz), bcR(iz), bcT(iy), bcB(iy).
+template <class FL, class FR, class FT, class FB>
+__device__ __forceinline__ double set_rhs_node_f(const LevelDev<double>& L, const FL& bcL, const FR& bcR,
+                                                 const FT& bcT, const FB& bcB, long node) {
   const int Ny = L.Ny, Nz = L.Nz;
   const int iy = (int)(node / Nz), iz = (int)(node % Nz);
   double sy = 0.0, sz = 0.0;
   if (L.y.bc_lo == 0) {
-    if (iy < BAND) sy += (L.y.bs0[iy] + (iy == 0 ? L.y.alphaD : 0.0)) * L.cy[iz] * bcL[iz];
+    if (iy < BAND) sy += (L.y.bs0[iy] + (iy == 0 ? L.y.alphaD : 0.0)) * L.cy[iz] * bcL(iz);
   } else if (iy == 0) {
-    sy += bcL[iz];
+    sy += bcL(iz);
   }
   if (L.y.bc_hi == 0) {
     if (iy >= Ny - BAND)
-      sy += (L.y.bsN[iy - (Ny - BAND)] + (iy == Ny - 1 ? L.y.alphaD : 0.0)) * L.cy[(long)(Ny - 1) * Nz + iz] * bcR[iz];
+      sy += (L.y.bsN[iy - (Ny - BAND)] + (iy == Ny - 1 ? L.y.alphaD : 0.0)) * L.cy[(long)(Ny - 1) * Nz + iz] * bcR(iz);
   } else if (iy == Ny - 1) {
-    sy -= bcR[iz];
+    sy -= bcR(iz);
   }
   if (L.z.bc_lo == 0) {
-    if (iz < BAND) sz += (L.z.bs0[iz] + (iz == 0 ? L.z.alphaD : 0.0)) * L.cz[(long)iy * Nz] * bcT[iy];
+    if (iz < BAND) sz += (L.z.bs0[iz] + (iz == 0 ? L.z.alphaD : 0.0)) * L.cz[(long)iy * Nz] * bcT(iy);
   } else if (iz == 0) {
-    sz += bcT[iy];
+    sz += bcT(iy);
   }
   if (L.z.bc_hi == 0) {
     if (iz >= Nz - BAND)
-      sz += (L.z.bsN[iz - (Nz - BAND)] + (iz == Nz - 1 ? L.z.alphaD : 0.0)) * L.cz[(long)iy * Nz + Nz - 1] * bcB[iy];
+      sz += (L.z.bsN[iz - (Nz - BAND)] + (iz == Nz - 1 ? L.z.alphaD : 0.0)) * L.cz[(long)iy * Nz + Nz - 1] * bcB(iy);
   } else if (iz == Nz - 1) {
-    sz -= bcB[iy];
+    sz -= bcB(iy);
   }
   return L.wy[node] * sy + L.wz[node] * sz;
+}
+
+__device__ __forceinline__ double set_rhs_node(const LevelDev<double>& L, const double* __restrict__ bcL,
+                                               const double* __restrict__ bcR, const double* __restrict__ bcT,
+                                               const double* __restrict__ bcB, long node) {
+  return set_rhs_node_f(
+      L, [&](int i) { return bcL[i]; }, [&](int i) { return bcR[i]; }, [&](int i) { return bcT[i]; },
+      [&](int i) { return bcB[i]; }, node);
 }
 
 // Shear stress mu * Dy u on the fault row iy = 0 at column iz (muxDy of

@@ -1259,7 +1259,8 @@ int SbpContext::set_rhs(const double* bcL, const double* bcR, const double* bcT,
 }
 
 template <typename Tz, class PC>
-int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st) {
+int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st,
+                    const SolvePart& part) {
   const LevelDev<double>& L = fine->dev;
   const long n = (long)L.Ny * L.Nz;
   double* sc = scal.as<double>();
@@ -1269,21 +1270,32 @@ int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts&
   double* r = cg_r.as<double>();
   double* q = cg_q.as<double>();
   const int rb = red_blocks(n);
-  dot_kernel<double, double><<<rb, 256, 0, stream>>>(rhs, rhs, n, parts, cnt, sc + 0);
-  SCY_LAUNCH_CHECK();
-  if (!o.nonzero_guess) SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
-  // r = f - K u with f = -rhs, K = -A  ->  r = -rhs + A u
-  SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{u}, EpiResidual<double, double>{rhs, r, -1.0}, &red, sc + 5,
-                                 stream));
   st.iterations = 0;
   st.converged = 0;
   const int check = o.check_every > 0 ? o.check_every : 1;
   double tol = -1.0;
-  int pi = 0;
+  int pi = 0, it0 = 1;
+  if (part.first) {
+    // resumed after its first iteration, whose scalars the caller has read
+    int done = 0;
+    SCY_TRY(test_convergence(part.first, o, u, tol, st, &done));
+    st.iterations = pi = 1;
+    if (done) return finish_solve(rhs, u, o, tol, st);
+    it0 = 2;
+  } else {
+    if (!part.norm_ready) {
+      dot_kernel<double, double><<<rb, 256, 0, stream>>>(rhs, rhs, n, parts, cnt, sc + 0);
+      SCY_LAUNCH_CHECK();
+    }
+    if (!o.nonzero_guess) SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
+    // r = f - K u with f = -rhs, K = -A  ->  r = -rhs + A u
+    SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{u}, EpiResidual<double, double>{rhs, r, -1.0}, &red, sc + 5,
+                                   stream));
+  }
   // The first read-back happens after the first batch of `check` iterations
   // (a warm-started stage solve is never converged on entry); iterations
   // past convergence are harmless no-ops (alpha = 0).
-  for (int it = 1; it <= o.max_its; ++it) {
+  for (int it = it0; it <= o.max_its; ++it) {
     Tz* z = nullptr;
     SCY_TRY(pc((const double*)r, &z));
     if (it > 1) {
@@ -1300,6 +1312,7 @@ int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts&
     SCY_LAUNCH_CHECK();
     pi ^= 1;
     st.iterations = it;
+    if (part.enqueue) return SCY_OK;
     if (it % check == 0 || it == o.max_its) {
       int done = 0;
       SCY_TRY(read_convergence(o, u, tol, st, &done));
@@ -1312,10 +1325,15 @@ int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts&
 // Reads the solve's scalars back and tests convergence; sets tol at the
 // first call (tol < 0).  *done: stop iterating.
 int SbpContext::read_convergence(const scy_solve_opts& o, double* u, double& tol, scy_solve_stats& st, int* done) {
-  const size_t n = (size_t)fine->dev.Ny * fine->dev.Nz;
   double h[6];
   SCY_CUDA_TRY(cudaMemcpyAsync(h, scal.p, 6 * sizeof(double), cudaMemcpyDeviceToHost, stream));
   SCY_CUDA_TRY(cudaStreamSynchronize(stream));
+  return test_convergence(h, o, u, tol, st, done);
+}
+
+int SbpContext::test_convergence(const double* h, const scy_solve_opts& o, double* u, double& tol,
+                                 scy_solve_stats& st, int* done) {
+  const size_t n = (size_t)fine->dev.Ny * fine->dev.Nz;
   if (tol < 0) {
     st.bnorm = std::sqrt(h[0]);
     st.rnorm0 = std::sqrt(h[5]);
@@ -1381,28 +1399,41 @@ int SbpContext::finish_solve(const double* rhs, double* u, const scy_solve_opts&
 // Per iteration on 401 x 401 stretched (numpy): ||r|| / ||rhs|| 1.2e-9,
 // 6.4e-13, 1.1e-15 against CG's 1.2e-9, 5.7e-13, 5.1e-16.
 template <class PC>
-int SbpContext::correct(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st) {
+int SbpContext::correct(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st,
+                        const SolvePart& part) {
   const LevelDev<double>& L = fine->dev;
   const long n = (long)L.Ny * L.Nz;
   double* sc = scal.as<double>();
   // sc[0]=||rhs||^2, sc[1]=r.r, sc[5]=||r0||^2
   double* r = cg_r.as<double>();
-  dot_kernel<double, double><<<red_blocks(n), 256, 0, stream>>>(rhs, rhs, n, red.partials.as<double>(),
-                                                               red.counter.as<unsigned>(), sc + 0);
-  SCY_LAUNCH_CHECK();
-  if (!o.nonzero_guess) SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
-  SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{u}, EpiResidual<double, double>{rhs, r, -1.0}, &red, sc + 5,
-                                 stream));
   st.iterations = 0;
   st.converged = 0;
   const int check = o.check_every > 0 ? o.check_every : 1;
   double tol = -1.0;
-  int unverified = 0;
-  for (int it = 1; it <= o.max_its; ++it) {
+  int unverified = 0, it0 = 1;
+  if (part.first) {
+    // resumed after its first iteration (never with a true-residual check)
+    int done = 0;
+    SCY_TRY(test_convergence(part.first, o, u, tol, st, &done));
+    st.iterations = 1;
+    if (done) return finish_solve(rhs, u, o, tol, st);
+    it0 = 2;
+  } else {
+    if (!part.norm_ready) {
+      dot_kernel<double, double><<<red_blocks(n), 256, 0, stream>>>(rhs, rhs, n, red.partials.as<double>(),
+                                                                   red.counter.as<unsigned>(), sc + 0);
+      SCY_LAUNCH_CHECK();
+    }
+    if (!o.nonzero_guess) SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
+    SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{u}, EpiResidual<double, double>{rhs, r, -1.0}, &red, sc + 5,
+                                   stream));
+  }
+  for (int it = it0; it <= o.max_its; ++it) {
     double* z = nullptr;
     SCY_TRY(pc((const double*)r, &z));
     SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{z}, EpiCorrect{u, r}, &red, sc + 1, stream));
     st.iterations = it;
+    if (part.enqueue) return SCY_OK;
     if (it % check == 0 || it == o.max_its) {
       int done = 0;
       SCY_TRY(read_convergence(o, u, tol, st, &done));
@@ -1423,7 +1454,13 @@ int SbpContext::ensure_fd(bool chains) {
   return fd->build(hosts[0], stream);
 }
 
-int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st) {
+bool SbpContext::can_enqueue(const scy_solve_opts& o) const {
+  return (o.precond == SCY_PC_FD || (o.precond == SCY_PC_AUTO && separable)) && o.precision == SCY_PREC_FP64 &&
+         !o.verify && o.check_every <= 1 && o.max_its >= 1;
+}
+
+int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st,
+                      const SolvePart& part) {
   const bool keeps = keeps_rounding(o.rtol);
   const bool use_fd = o.precond == SCY_PC_FD || (o.precond == SCY_PC_AUTO && separable);
   if (use_fd) {
@@ -1435,7 +1472,7 @@ int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy
         *zo = z;
         return SCY_OK;
       };
-      return pcg<float>(pc, rhs, u, o, st);
+      return pcg<float>(pc, rhs, u, o, st, part);
     }
     double* z = cg_z.as<double>();
     auto pc = [&](const double* r, double** zo) -> int {
@@ -1443,16 +1480,16 @@ int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy
       *zo = z;
       return SCY_OK;
     };
-    return near_inverse() && !keeps ? correct(pc, rhs, u, o, st) : pcg<double>(pc, rhs, u, o, st);
+    return near_inverse() && !keeps ? correct(pc, rhs, u, o, st, part) : pcg<double>(pc, rhs, u, o, st, part);
   }
   if (o.precision == SCY_PREC_MIXED) {
     SCY_TRY(ensure_mg(mg32));
     auto pc = [&](const double* r, float** zo) -> int { return mg32->vcycle(0, r, zo, stream); };
-    return pcg<float>(pc, rhs, u, o, st);
+    return pcg<float>(pc, rhs, u, o, st, part);
   }
   SCY_TRY(ensure_mg(mg64));
   auto pc = [&](const double* r, double** zo) -> int { return mg64->vcycle(0, r, zo, stream); };
-  return pcg<double>(pc, rhs, u, o, st);
+  return pcg<double>(pc, rhs, u, o, st, part);
 }
 
 int SbpContext::residual_dd(const double* rhs, const double* u, double* r, double* rnorm2_host) {

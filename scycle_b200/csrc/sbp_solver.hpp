@@ -106,6 +106,16 @@ int build_hierarchy(const scy_grid_desc& g, const std::vector<double>& y, const 
 
 struct FDPrecond;
 
+// How much of a solve a call does.  norm_ready: scal[0] already holds (in
+// stream order) the sum of squares of the rhs.  enqueue: launch the residual
+// and the first iteration and return without reading anything; the scalars
+// scal[0], [1], [5] then say whether that was enough.  first: resume such a
+// solve, with its scal[0..5] as read.
+struct SolvePart {
+  int norm_ready = 0, enqueue = 0;
+  const double* first = nullptr;
+};
+
 struct SbpContext {
   SbpContext();
   ~SbpContext();
@@ -144,7 +154,11 @@ struct SbpContext {
   int rebuild();
   int apply(int op, const double* in, double* out);
   int set_rhs(const double* bcL, const double* bcR, const double* bcT, const double* bcB, double* rhs);
-  int solve(const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st);
+  int solve(const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st,
+            const SolvePart& part = SolvePart());
+  // whether a solve with these options can be enqueued (the fast
+  // diagonalisation in FP64, tested every iteration by the recurrence)
+  bool can_enqueue(const scy_solve_opts& o) const;
   int solve_noalloc(const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st);
   int change_bc(int R, int T, int L, int B);
   // r = rhs - A u with A u summed in double-double arithmetic (error-free
@@ -158,9 +172,12 @@ struct SbpContext {
   int ensure_mg(std::unique_ptr<Multigrid<T>>& mg);
   int ensure_fd(bool chains);  // chains: with the tables of the whole sweep chains
   template <typename Tz, class PC>
-  int pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st);
+  int pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st, const SolvePart& part);
   template <class PC>
-  int correct(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st);
+  int correct(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st,
+              const SolvePart& part);
+  int test_convergence(const double* h, const scy_solve_opts& o, double* u, double& tol, scy_solve_stats& st,
+                       int* done);
   int read_convergence(const scy_solve_opts& o, double* u, double& tol, scy_solve_stats& st, int* done);
   int finish_solve(const double* rhs, double* u, const scy_solve_opts& o, double tol, scy_solve_stats& st);
 };
