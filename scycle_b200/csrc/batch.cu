@@ -642,7 +642,7 @@ __global__ void b_fault_kernel(LevelDev<double> L, const BatchInst* __restrict__
   const int k = blockIdx.z;
   if (!mask[k]) return;
   const BatchInst& I = tab[k];
-  const int iz = blockIdx.x * blockDim.x + threadIdx.x;
+  const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= I.fp.Nz) return;
   const double sxy = I.c1 ? I.sxy[iz] : fault_row_sxy(L, I.u, iz);
   fault_node_update(iz, sxy, I.fp, I.rk[in_slot], I.rk[out_slot], I.slipVel, I.tauQSP, I.tauP, I.strength, I.flags,
@@ -1698,7 +1698,7 @@ int BatchContext::d_dt(BatchGroup& g, const int* mask, double c, int in_slot, in
     b_pl_rates_kernel<<<ng, TB, 0, g.stream>>>(g.L, tab, mask, in_slot, out_slot, g.N);
     SCY_LAUNCH_CHECK();
   }
-  b_fault_kernel<<<fg, 64, 0, g.stream>>>(g.L, tab, mask, in_slot, out_slot);
+  b_fault_kernel<<<dim3((4 * g.Nz + 63) / 64, 1, g.K), 64, 0, g.stream>>>(g.L, tab, mask, in_slot, out_slot);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }

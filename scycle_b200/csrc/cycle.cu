@@ -112,7 +112,8 @@ struct FDFaultArgs {
 
 constexpr int kFaultBlock = 128;
 
-// Fault_fd::d_dt for fault node iz (fault.cpp:1436-1575), the fault-row
+// Fault_fd::d_dt for fault node iz by its four lanes together (fault_dev.cuh;
+// lane 0 stores) (fault.cpp:1436-1575), the fault-row
 // stress of uNext + u0, tauQS and tauP; returns eta V / tauQS.  d2u is the
 // node's Hinv Jinv A u; un(k) returns uNext at body row k (k = 1..4).
 template <class Rows>
@@ -132,6 +133,9 @@ __device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, int iz, do
   const double Phi = 2.0 / dt * (u - uPrev) + dt * an / rho;
   const double fricPen = dt / alphay / rho;
   const double psi = A.psi[iz];
+  const bool out = (threadIdx.x & 3) == 0;
+  const double V0 = fabs(A.slipVel[iz]), E = exp(psi / a);
+  __syncwarp(node_lanes());  // every lane has V0 before lane 0 overwrites it
   // ComputeVel_fd::computeVel (fault.cpp:1594-1644)
   double V;
   const double lk = fp.locked[iz];
@@ -148,23 +152,22 @@ __device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, int iz, do
     } else if (fabs(0.0 - right) < 1e-14) {
       V = 0.0;
     } else {
-      const ResidVelFD R1{right, fricPen, sN, psi, a, fp.v0, exp(psi / a)};
+      const ResidVelFD R1{right, fricPen, sN, psi, a, fp.v0, E};
       int its = 0;
       bool ok = true;
-      V = bracketed_newton_f(R1, 0.0, right, fabs(A.slipVel[iz]), fp.root_tol, fp.max_its, &its, &ok);
-      atomicAdd(&st->its, (unsigned long long)its);
+      V = bracketed_newton_f(R1, 0.0, right, V0, fp.root_tol, fp.max_its, &its, &ok);
+      if (out) atomicAdd(&st->its, (unsigned long long)its);
       if (!ok) bad |= FAULT_ROOT_NOCONV;
     }
   }
   // velocity and displacement update (fault.cpp:1481-1496)
   if (!(V < 1e-14)) {
-    const double fric = strength_psi(sN, psi, V, a, fp.v0);
+    const double fric = a * sN * asinh((0.5 * V / fp.v0) * E);  // strength_psi
     const double alpha = 1.0 / (rho * alphay) * fric / V;
     const double Ad = 1.0 + alpha * dt;
     V = Phi / (1. + dt * alpha);
     u = (2. * u + (an * dt * dt / rho) + (dt * alpha - 1.) * uPrev) / Ad;
   }
-  A.slipVel[iz] = V;
   // ComputeAging_fd / ComputeSlipLaw_fd (fault.cpp:1702-1745, :1802-1846)
   const double psiPrev = A.psiPrev[iz];
   double psiN;
@@ -178,13 +181,16 @@ __device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, int iz, do
       const ResidSlipFD R2{psiPrev, V, a, fp.b[iz], fp.f0, fp.v0, fp.Dc[iz], dt};
       psiN = bracketed_newton_f(R2, -2.0, 2.0, psi, fp.root_tol, fp.max_its, &its, &ok);
     }
-    atomicAdd(&st->its, (unsigned long long)its);
+    if (out) atomicAdd(&st->its, (unsigned long long)its);
     if (!ok) bad |= FAULT_ROOT_NOCONV;
   }
-  A.psiNext[iz] = psiN;
-  A.slipNext[iz] = A.fts * u + slip0;
-  A.strength[iz] = strength_psi(sN, psiN, V, a, fp.v0);
-  A.uNext[iz] = u;  // body row 0 takes the fault displacement
+  if (out) {
+    A.slipVel[iz] = V;
+    A.psiNext[iz] = psiN;
+    A.slipNext[iz] = A.fts * u + slip0;
+    A.uNext[iz] = u;  // body row 0 takes the fault displacement
+    A.strength[iz] = strength_psi(sN, psiN, V, a, fp.v0);
+  }
   // sxy = mu * Dy (uNext + u0) at the fault (LinearElastic::computeStresses)
   double d = 0.0;
 #pragma unroll
@@ -197,8 +203,10 @@ __device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, int iz, do
   }
   if (A.var_grid) d *= A.qy0[iz];
   const double tq = A.mu0[iz] * d + 1.0 * fp.prestress[iz];
-  A.tauQSP[iz] = tq;
-  A.tauP[iz] = -1.0 * (eta * V) + tq;
+  if (out) {
+    A.tauQSP[iz] = tq;
+    A.tauP[iz] = -1.0 * (eta * V) + tq;
+  }
   if (!isfinite(V) || !isfinite(psiN)) bad |= FAULT_NONFINITE;
   *bad_out = bad;
   return eta * V / tq;
@@ -237,13 +245,13 @@ __global__ void __launch_bounds__(kFaultBlock) fd_fault_kernel(FDFaultArgs A) {
   CycleDevState* st = A.st;
   if (st->stop) return;
   const int Nz = A.fp.Nz;
-  const int iz = blockIdx.x * blockDim.x + threadIdx.x;
+  const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   double R = -INFINITY;
   if (iz < Nz) {
     unsigned bad = 0;
     auto rows = [&](int k) { return A.uNext[(long)k * Nz + iz]; };
     R = fd_fault_node(A, iz, A.d2u[iz], rows, &bad);
-    if (bad) atomicOr(&st->flags, bad);
+    if (bad && (threadIdx.x & 3) == 0) atomicOr(&st->flags, bad);
   }
   __shared__ double sh[32];
   double m = warp_max(R);
@@ -272,18 +280,22 @@ __global__ void __launch_bounds__(256) fd_step_kernel(LevelDev<double> L, LoadPl
   wave_tile<RPT>(L, ld, e);
   if (!fault_tile) return;
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  double R = -INFINITY;
-  if (threadIdx.x < 32) {
-    const int iz = blockIdx.x * TZ + lane;
+  __shared__ double s_max[4];
+  if (threadIdx.x < 4 * TZ) {
+    const int col = threadIdx.x >> 2, iz = blockIdx.x * TZ + col;
+    double R = -INFINITY;
     if (iz < A.fp.Nz) {
       unsigned bad = 0;
-      auto rows = [&](int k) { return s_rows[k * TZ + lane]; };
-      R = fd_fault_node(A, iz, s_d2u[lane], rows, &bad);
-      if (bad) atomicOr(&st->flags, bad);
+      auto rows = [&](int k) { return s_rows[k * TZ + col]; };
+      R = fd_fault_node(A, iz, s_d2u[col], rows, &bad);
+      if (bad && (threadIdx.x & 3) == 0) atomicOr(&st->flags, bad);
     }
     R = warp_max(R);
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = R;
   }
+  __syncthreads();
+  double R = s_max[0];
+  for (int w = 1; w < 4; ++w) R = s_max[w] > R ? s_max[w] : R;
   fd_switch_test(A, R);
 }
 
@@ -449,7 +461,7 @@ int CycleContext::create(const scy_qd_desc& qd, const scy_cycle_desc& cd) {
   SCY_TRY(tau0.alloc(Nz * 8));
   // block maxima of the switch test: one per fault-row tile (fused step) or
   // per fault block (two-launch step)
-  SCY_TRY(dstate.alloc(sizeof(CycleDevState) + 8 * (size_t)((Nz + TZ - 1) / TZ + (Nz + kFaultBlock - 1) / kFaultBlock + 2)));
+  SCY_TRY(dstate.alloc(sizeof(CycleDevState) + 8 * (size_t)((Nz + TZ - 1) / TZ + (4 * Nz + kFaultBlock - 1) / kFaultBlock + 2)));
   SCY_CUDA_TRY(cudaMemsetAsync(dstate.p, 0, dstate.bytes, s));
   SCY_CUDA_TRY(cudaMallocHost((void**)&h_state, sizeof(CycleDevState)));
   std::memset(h_state, 0, sizeof(CycleDevState));
@@ -677,7 +689,7 @@ int CycleContext::fd_launch_step(int r, cudaStream_t s, int part) {
     SCY_LAUNCH_CHECK();
   }
   if (part & FD_FAULT) {
-    fd_fault_kernel<<<(Nz + kFaultBlock - 1) / kFaultBlock, kFaultBlock, 0, s>>>(A);
+    fd_fault_kernel<<<(4 * Nz + kFaultBlock - 1) / kFaultBlock, kFaultBlock, 0, s>>>(A);
     SCY_LAUNCH_CHECK();
   }
   return SCY_OK;

@@ -1,4 +1,12 @@
-// Rate-and-state fault on the device: one thread per fault node.
+// Rate-and-state fault on the device: four lanes per fault node.
+//
+// A node's update is one chain of root-find evaluations (asinh, exp, divides:
+// some 600 cycles each), and a fault has far fewer nodes than the GPU has
+// lanes.  The four lanes of a node hold the same data and take the same
+// branches; where the chain forks they evaluate its ends at the same time
+// (bracket_eval: the start and both ends of the bracket), so a root takes 1 +
+// its iterations instead of 4 + its iterations evaluations.  The values are
+// those of one thread evaluating them in turn.
 //
 // Follows Fault_qd::d_dt / ComputeVel_qd::computeVel (reference
 // source/fault.cpp:861-1059), BracketedNewton::findRoot
@@ -68,19 +76,35 @@ __device__ __forceinline__ void resid_qd(double V, double tauQS, double eta, dou
   J = (exact ? A * B / s : A * V / s) + eta;
 }
 
+// the mask of the calling lane's group of four
+__device__ __forceinline__ unsigned node_lanes() { return 0xfu << (threadIdx.x & 28); }
+
+// f and f' at x0, f at left and at right, one lane each (lane 3 repeats x0)
+template <class Resid>
+__device__ __forceinline__ void bracket_eval(const Resid& R, double left, double right, double x0, double& f,
+                                             double& fp, double& fl, double& fr) {
+  const int q = threadIdx.x & 3;
+  double v, d;
+  R(q == 1 ? left : q == 2 ? right : x0, v, d);
+  const unsigned m = node_lanes();
+  f = __shfl_sync(m, v, 0, 4);
+  fp = __shfl_sync(m, d, 0, 4);
+  fl = __shfl_sync(m, v, 1, 4);
+  fr = __shfl_sync(m, v, 2, 4);
+}
+
 // Safeguarded Newton on [left, right] starting from x0 for the residual
 // R(x, f, f'), following BracketedNewton::findRoot (rootFinder.cpp:174-257).
 // Returns the root; sets *its and *ok.  Every loop is bounded by max_its.
+// Called by the four lanes of a node together.
 template <class Resid>
 __device__ __forceinline__ double bracketed_newton_f(const Resid& R, double left, double right, double x0,
                                                      double atol, int max_its, int* its, bool* ok) {
-  double f, fp, fl, fr, dum;
+  double f, fp, fl, fr;
   *its = 0;
   *ok = true;
-  R(x0, f, fp);
+  bracket_eval(R, left, right, x0, f, fp, fl, fr);
   if (fabs(f) <= atol) return x0;
-  R(left, fl, dum);
-  R(right, fr, dum);
   if (!isfinite(fl) || !isfinite(fr)) {
     *ok = false;
     return x0;
@@ -94,7 +118,6 @@ __device__ __forceinline__ double bracketed_newton_f(const Resid& R, double left
   }
   double x = x0;
   double dxold = fabs(right - left), dx = dxold;
-  R(x, f, fp);
   int n = 0;
   while (n <= max_its && fabs(f) >= atol) {
     if (((x - right) * fp - f) * ((x - left) * fp - f) > 0.0 || fabs(2.0 * f) > fabs(dxold * fp)) {
@@ -128,26 +151,25 @@ struct ResidQD {
   }
 };
 
-__device__ __forceinline__ double bracketed_newton(double left, double right, double x0, double atol, int max_its,
-                                                   double tauQS, double eta, double sN, double psi, double a,
-                                                   double v0, int exact, int* its, bool* ok) {
-  const ResidQD R{tauQS, eta, sN, exp(psi / a), a, v0, exact};
-  return bracketed_newton_f(R, left, right, x0, atol, max_its, its, ok);
-}
-
 __device__ __forceinline__ double aging_law_psi(double psi, double V, double b, double f0, double v0, double Dc) {
   double A = exp((f0 - psi) / b);
   if (!isinf(A) && b > 1e-3) return (b * v0 / Dc) * (A - V / v0);
   return 0.0;
 }
 
-__device__ __forceinline__ double slip_law_psi(double psi, double V, double a, double b, double f0, double v0,
-                                               double Dc) {
+// S = asinh((|V| / (2 v0)) exp(psi / a))
+__device__ __forceinline__ double slip_law_of_asinh(double S, double V, double a, double b, double f0, double v0,
+                                                    double Dc) {
   if (V == 0.0) return 0.0;
   double absV = fabs(V);
   double fss = f0 + (a - b) * log(absV / v0);
-  double f = a * asinh((absV / 2.0 / v0) * exp(psi / a));
+  double f = a * S;
   return -absV / Dc * (f - fss);
+}
+
+__device__ __forceinline__ double slip_law_psi(double psi, double V, double a, double b, double f0, double v0,
+                                               double Dc) {
+  return slip_law_of_asinh(asinh((fabs(V) / 2.0 / v0) * exp(psi / a)), V, a, b, f0, v0, Dc);
 }
 
 }  // namespace scy

@@ -1,5 +1,6 @@
-// Fault_qd::d_dt for one fault node (one thread per node), shared by the
-// linear-elastic, response-mode and power-law drivers.
+// Fault_qd::d_dt for one fault node (its four lanes together, see
+// fault_dev.cuh), shared by the linear-elastic, response-mode and power-law
+// drivers.
 #pragma once
 #include "fault_dev.cuh"
 
@@ -7,16 +8,18 @@ namespace scy {
 
 // Fault_qd::d_dt for one node given its quasi-static shear stress from the
 // body (fault.cpp:861-918): prestress, bracketed Newton, state law, tauP,
-// strength.
+// strength.  Lane 0 of the four stores.
 __device__ __forceinline__ void fault_node_update(int iz, double tau_body, const FaultParams& fp,
                                                   const double* __restrict__ var, double* __restrict__ f,
                                                   double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                                   double* __restrict__ tauP, double* __restrict__ strength,
                                                   unsigned* flags, unsigned long long* its_total) {
+  const bool out = (threadIdx.x & 3) == 0;
   const double tq = tau_body + fp.prestress[iz];
-  tauQSP[iz] = tq;
   const double psi = var[fp.psi_off + iz];
   const double a = fp.a[iz], sN = fp.sN[iz], eta = fp.eta[iz];
+  const double E = exp(psi / a), V0 = slipVel[iz];
+  __syncwarp(node_lanes());  // every lane has V0 before lane 0 overwrites it
   double V;
   const double lk = fp.locked[iz];
   if (lk > 0.5) {
@@ -26,37 +29,42 @@ __device__ __forceinline__ void fault_node_update(int iz, double tau_body, const
   } else {
     double left = 0.0, right = tq / eta;
     if (isnan(right)) {
-      atomicOr(flags, (unsigned)FAULT_NONFINITE);
-      V = slipVel[iz];
+      if (out) atomicOr(flags, (unsigned)FAULT_NONFINITE);
+      V = V0;
     } else if (fabs(left - right) < 1e-14) {
       V = left;
     } else {
       int its = 0;
       bool ok = true;
-      V = bracketed_newton(left, right, slipVel[iz], fp.root_tol, fp.max_its, tq, eta, sN, psi, a, fp.v0,
-                           fp.jacobian, &its, &ok);
-      atomicAdd(its_total, (unsigned long long)its);
-      if (!ok) atomicOr(flags, (unsigned)FAULT_ROOT_NOCONV);
+      const ResidQD R{tq, eta, sN, E, a, fp.v0, fp.jacobian};
+      V = bracketed_newton_f(R, left, right, V0, fp.root_tol, fp.max_its, &its, &ok);
+      if (out) {
+        atomicAdd(its_total, (unsigned long long)its);
+        if (!ok) atomicOr(flags, (unsigned)FAULT_ROOT_NOCONV);
+      }
     }
   }
-  slipVel[iz] = V;
+  const double S = asinh((0.5 * V / fp.v0) * E);  // of the strength and, in magnitude, of the slip law
   double dpsi;
   if (fp.state_law == 0)
     dpsi = aging_law_psi(psi, V, fp.b[iz], fp.f0, fp.v0, fp.Dc[iz]);
   else if (fp.state_law == 1)
-    dpsi = slip_law_psi(psi, V, a, fp.b[iz], fp.f0, fp.v0, fp.Dc[iz]);
+    dpsi = slip_law_of_asinh(fabs(S), V, a, fp.b[iz], fp.f0, fp.v0, fp.Dc[iz]);
   else if (fp.state_law == 3) {
     // flashHeating_psi_Vec (fault.cpp:2199-2243): Vw from the fault's temperature
     const double vw = flash_heating_vw(fp.Tf[iz], fp.rc_f[iz], fp.k_f[iz], fp.fl_D, fp.Tw[iz], fp.fl_tau_c);
-    fp.Vw[iz] = vw;
+    if (out) fp.Vw[iz] = vw;
     dpsi = flash_heating_psi(psi, V, vw, fp.fl_fw, fp.Dc[iz], a, fp.b[iz], fp.f0, fp.v0);
   } else
     dpsi = 0.0;
+  if (!out) return;
   if (!isfinite(dpsi) || !isfinite(V)) atomicOr(flags, (unsigned)FAULT_NONFINITE);
+  tauQSP[iz] = tq;
+  slipVel[iz] = V;
   f[fp.psi_off + iz] = dpsi;
   f[fp.slip_off + iz] = V;
   tauP[iz] = tq - eta * V;
-  strength[iz] = strength_psi(sN, psi, V, a, fp.v0);
+  strength[iz] = a * sN * S;
 }
 
 }  // namespace scy

@@ -38,7 +38,7 @@ __global__ void pl_fault_kernel(const double* __restrict__ sxy, FaultParams fp, 
                                 double* __restrict__ f, double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                 double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                 unsigned long long* its_total) {
-  const int iz = blockIdx.x * blockDim.x + threadIdx.x;
+  const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
   fault_node_update(iz, sxy[iz], fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
 }
@@ -71,7 +71,7 @@ int pl_d_dt(QDContext& q, double t, const double* var, double* f) {
   return q.solve_stage(t, var, gxy, gxz, [&]() -> int {
     pl_rates_kernel<<<gb, 256, 0, s>>>(a);
     SCY_LAUNCH_CHECK();
-    const int tb = 64, fb = (Nz + tb - 1) / tb;
+    const int tb = 64, fb = (4 * Nz + tb - 1) / tb;
     pl_fault_kernel<<<fb, tb, 0, s>>>(q.sxy.as<double>(), q.fp, var, f, q.slipVel.as<double>(),
                                       q.tauQSP.as<double>(), q.tauP.as<double>(), q.strength.as<double>(),
                                       q.fault_flags(), q.fault_its.as<unsigned long long>());

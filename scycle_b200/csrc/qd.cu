@@ -80,7 +80,7 @@ __global__ void qd_fault_kernel(LevelDev<double> L, const double* __restrict__ u
                                 double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                 double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                 unsigned long long* its_total) {
-  int iz = blockIdx.x * blockDim.x + threadIdx.x;
+  const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
   const double sxy = fault_row_sxy(L, u, iz);
   fault_node_update(iz, sxy, fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
@@ -93,13 +93,13 @@ __global__ void qd_fault_given_tau_kernel(const double* __restrict__ tau_body, F
                                           double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                           double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                           unsigned long long* its_total) {
-  int iz = blockIdx.x * blockDim.x + threadIdx.x;
+  const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
   fault_node_update(iz, tau_body[iz], fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
 }
 
 int QDContext::fault_d_dt(const double* var, const double* tau_body, double* f) {
-  const int tb = 64, gb = (Nz + tb - 1) / tb;
+  const int tb = 64, gb = (4 * Nz + tb - 1) / tb;
   qd_fault_given_tau_kernel<<<gb, tb, 0, sbp.stream>>>(tau_body, fp, var, f, slipVel.as<double>(),
                                                        tauQSP.as<double>(), tauP.as<double>(),
                                                        strength.as<double>(), flags.as<unsigned>(),
@@ -128,8 +128,8 @@ __global__ void qd_response_column_kernel(LevelDev<double> L, const double* __re
 }
 
 // Fault-response d_dt: one warp per fault node forms
-// tau = GL[iz,:] . (slip/faultTypeScale) + c g1[iz] + gs[iz], lane 0 then
-// runs the fault update.
+// tau = GL[iz,:] . (slip/faultTypeScale) + c g1[iz] + gs[iz], its first four
+// lanes then run the fault update.
 __global__ void qd_green_kernel(const double* __restrict__ GL, const double* __restrict__ g1,
                                 const double* __restrict__ gs, double c, double inv_fts, FaultParams fp,
                                 const double* __restrict__ var, double* __restrict__ f, double* __restrict__ slipVel,
@@ -143,8 +143,8 @@ __global__ void qd_green_kernel(const double* __restrict__ GL, const double* __r
   double acc = 0.0;
   for (int j = lane; j < Nz; j += 32) acc += row[j] * (slip[j] * inv_fts);
   acc = warp_sum(acc);
-  if (lane == 0) {
-    bcL[warp] = slip[warp] * inv_fts;  // kept for output fields
+  if (lane < 4) {
+    if (lane == 0) bcL[warp] = slip[warp] * inv_fts;  // kept for output fields
     const double tau = acc + (c * g1[warp] + gs[warp]);
     fault_node_update(warp, tau, fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
   }
@@ -451,7 +451,7 @@ int QDContext::d_dt(double t, const double* var, double* f) {
     return SCY_OK;
   }
   SCY_TRY(solve_stage(t, var, nullptr, nullptr, [&]() -> int {
-    const int tb = 64, gb = (Nz + tb - 1) / tb;
+    const int tb = 64, gb = (4 * Nz + tb - 1) / tb;
     qd_fault_kernel<<<gb, tb, 0, s>>>(sbp.fine->dev, u.as<double>(), fp, var, f, slipVel.as<double>(),
                                       tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), fault_flags(),
                                       fault_its.as<unsigned long long>());
