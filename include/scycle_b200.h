@@ -683,8 +683,8 @@ scy_status scy_batch_set_sweep_test(scy_batch* b, int polls, int drop_first_copy
  * set-up every group times, on its own buffers, the CG operator kernel in
  * the cross form (33 coefficient planes) with 1, 2, 4 and 8 instances per
  * block and, when the operator is separable over every node, in the
- * separable form (1D coefficient tables) with 1, 2 and 4 rows per thread,
- * the banded sweeps in six launch shapes (chains per lane x warps per block:
+ * separable form (1D coefficient tables) with 1, 2, 16 and 32 rows per thread,
+ * the banded sweeps in six launch shapes (whole chains; chains per lane x warps per block:
  * 2 x 2, 1 x 4, 4 x 1 serving 8 instances per block, 1 x 2 and 2 x 1
  * serving 4, 1 x 1 serving 2) and the z-transform product in three shapes
  * (one CTA per tile, two CTAs per SM, persistent: one CTA per SM with two
@@ -695,14 +695,15 @@ scy_status scy_batch_set_sweep_test(scy_batch* b, int polls, int drop_first_copy
  * doubles, may be NULL) the timings in microseconds per launch (cross form
  * at kpb 1, 2, 4, 8; sweep shapes 0-5; product with 8-bit digits, one and
  * two CTAs per SM; with bf16 digits, one and two CTAs per SM; separable form
- * at 1, 2, 4 rows per thread with the compiler's register count, then with
- * registers fitted to four blocks per SM; persistent product with 8-bit and
+ * at 1 and 2 rows per thread with the compiler's register count, then with
+ * registers fitted to four blocks per SM, then at 16 and 32 rows per thread,
+ * where warps walk down 32 columns; persistent product with 8-bit and
  * with bf16 digits; 0 where not tried).  The separable form is used
  * whenever the operator has it (its results do not depend on its launch
  * shape; they differ from the cross form's by rounding). */
 scy_status scy_batch_tuning(scy_batch* b, int g, int* kpb, int* sweep_variant, int* ztransform, double* us);
 /* The operator kernels group g runs: *rows_per_thread = 0 for the cross
- * form, else the separable form's rows per thread (1, 2 or 4), and
+ * form, else the separable form's rows per thread (1, 2, 16 or 32), and
  * *min_blocks_per_sm (may be NULL) the blocks per SM its registers are
  * fitted to (1: the compiler's choice; 0 for the cross form). */
 scy_status scy_batch_operator_form(scy_batch* b, int g, int* rows_per_thread, int* min_blocks_per_sm);

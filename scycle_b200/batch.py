@@ -92,7 +92,7 @@ class Batch:
     def tuning(self, group=0):
         """The autotuner's choices for a group: the operator kernels' form
         (cross form with instances per block, or separable form with rows
-        per thread), the sweep launch shape, the z-transform product's shape
+        per thread: 1 or 2 in tiles, 16 or 32 in walks by warps), the sweep launch shape, the z-transform product's shape
         and digits, and the timings (us)."""
         kpb, var, zt, rpt, minb = C.c_int(), C.c_int(), C.c_int(), C.c_int(), C.c_int()
         us = (C.c_double * 22)()
@@ -119,10 +119,10 @@ class Batch:
                 "ztransform_us_int8_by_ctas_per_sm": {1: us[10], 2: us[11]},
                 "ztransform_us_bf16_by_ctas_per_sm": {1: us[12], 2: us[13]},
                 "ztransform_us_persistent": {"int8": us[20], "bf16": us[21]},
-                "operator_us_separable_by_rows_per_thread": {r: us[14 + i] for i, r in enumerate((1, 2, 4))
-                                                             if us[14 + i] > 0},
+                "operator_us_separable_by_rows_per_thread": {r: us[i] for i, r in ((14, 1), (15, 2), (18, 16), (19, 32))
+                                                             if us[i] > 0},
                 "operator_us_separable_4_blocks_per_sm_by_rows_per_thread": {
-                    r: us[17 + i] for i, r in enumerate((1, 2, 4)) if us[17 + i] > 0}}
+                    r: us[i] for i, r in ((16, 1), (17, 2)) if us[i] > 0}}
 
     def profile_clear(self):
         S.check(S.lib().scy_batch_profile_clear(self.h))

@@ -409,30 +409,70 @@ __global__ void __launch_bounds__(XT) b_cross_kernel(const double* __restrict__ 
 
 // The same two products when the group's operator is separable over every
 // node (L.full: one 17-point stencil per row and per column from 1D tables
-// shared by the group, L1/L2-resident): one instance per block
-// (blockIdx.z), its 8*RPT x 32 tile staged once and applied by full_apply
-// (register window along y, 9-point interior), so per node only the
-// instance's own fields move.  The partial sums do not depend on RPT: the
-// contributions go to shared memory by node, then for every band of 8 rows
-// (a tile of the 8 x 32 layout, index blockIdx.x + gridDim.x * band) each
-// column adds its 8 rows in order and one warp sum adds the 32 columns.
+// shared by the group, L1/L2-resident), and the defect correction: one
+// instance per blockIdx.z, so per node only the instance's own fields move.
+// RPT > 0: an 8 * RPT x 32 tile per block (full_apply); RPT = 0: walks by
+// warps (march_part), the shorter way where the warps fill the GPU several
+// times over.  Both give the same results, and the same partial sums, one per
+// 8 x 32 tile (index tile column + columns * band): each column adds its 8
+// rows in order, then one warp sum adds the 32 columns.
+// At 32 x 401 x 401 the defect correction takes 85 us in tiles and 64 in
+// walks (206 MB, 31 us at the copy rate: the shared-memory pipe is 57 % busy,
+// and 14 warps per SM leave part of the loads' latency open); at 7 x 129 x
+// 97, all edge, the tiles are 4 % of a step the faster.
 template <int MODE, typename Tz, int RPT, int MINB>
 __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, const BatchInst* __restrict__ tab,
                                                      const int* __restrict__ mask, BatchWork w,
                                                      const Tz* __restrict__ zv, int first, int pi, int mixed,
-                                                     int store_p) {
-  __shared__ double xs[full_smem_values<RPT>()];
-  __shared__ double cs[2][8 * RPT][TZ];  // contributions by node of the tile
+                                                     int store_p, MarchPlan p) {
+  __shared__ double xs[RPT > 0 ? full_smem_values<RPT>() : kMarchWarps * kMarchSmem];
+  __shared__ double cs[2][8 * RPT + 1][TZ];  // contributions by node of the tile
   const int k = blockIdx.z;
   if (!mask[k]) return;
-  const int tid = threadIdx.x, lane = tid & 31, r0 = (tid >> 5) * RPT;
+  const int tid = threadIdx.x, lane = tid & 31, wv = tid >> 5, r0 = wv * RPT;
   const long off = (long)k * w.N;
   const double* sc = w.sc + 16 * k;
-  double a1 = 0.0, a2 = 0.0;  // the current row's contributions
-  auto row = [&](int j) {
-    cs[0][r0 + j][lane] = a1;
-    if (MODE == 1 && first) cs[1][r0 + j][lane] = a2;
-    a1 = a2 = 0.0;
+  double a1 = 0.0, a2 = 0.0;  // the column's contributions, of the rows of a band so far
+  // the operator with these hooks on the block's part of the grid
+  auto apply = [&](const auto& ld, const auto& pre, auto& out) {
+    if constexpr (RPT > 0) {
+      auto row = [&](int j) {
+        cs[0][r0 + j][lane] = a1;
+        if (MODE == 1 && first) cs[1][r0 + j][lane] = a2;
+        a1 = a2 = 0.0;
+      };
+      full_apply<double, RPT>(L, ld, pre, out, row, xs, blockIdx.y * 8 * RPT, blockIdx.x * TZ);
+      __syncthreads();
+      const int band = blockIdx.y * RPT + wv;
+      if (wv < RPT && band * 8 < L.Ny) {
+        const long slot = (long)k * w.PB + blockIdx.x + (long)gridDim.x * band;
+        double t = 0.0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) t += cs[0][wv * 8 + r][lane];
+        t = warp_sum(t);
+        if (lane == 0) w.partials[slot] = t;
+        if (MODE == 1 && first) {
+          t = 0.0;
+#pragma unroll
+          for (int r = 0; r < 8; ++r) t += cs[1][wv * 8 + r][lane];
+          t = warp_sum(t);
+          if (lane == 0) w.partials2[slot] = t;
+        }
+      }
+    } else {
+      auto chunk = [&](int y, int tx) {
+        if ((y & 7) == 0) return;  // a band's second half ends it
+        const long slot = (long)k * w.PB + tx + (long)p.nx * (y >> 3);
+        double t = warp_sum(a1);
+        if (lane == 0) w.partials[slot] = t;
+        if (MODE == 1 && first) {
+          t = warp_sum(a2);
+          if (lane == 0) w.partials2[slot] = t;
+        }
+        a1 = a2 = 0.0;
+      };
+      march_part<double>(L, p, blockIdx.x, wv, ld, pre, out, chunk, xs + wv * kMarchSmem);
+    }
   };
   if constexpr (MODE == 0) {
     const double* u = tab[k].u;
@@ -444,9 +484,9 @@ __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, c
       const double v = zero ? 0.0 : -1.0 * b + Ax;
       w.r[off + node] = v;
       if (mixed) w.r32[off + node] = (float)v;
-      a1 = v * v;
+      a1 += __dmul_rn(v, v);
     };
-    full_apply<double, RPT>(L, ld, pre, out, row, xs);
+    apply(ld, pre, out);
   } else if constexpr (MODE == 2) {
     // defect correction with z = P r: u += z, r += A z (zero where rhs = 0);
     // an instance whose z is not P r because a pipeline wait ran out on the
@@ -464,9 +504,9 @@ __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, c
       const double v = zero ? 0.0 : lost ? p.r : p.r + Az;
       r[node] = v;
       u[node] = zero ? 0.0 : lost ? p.u : p.u + zz;
-      a1 = v * v;
+      a1 += __dmul_rn(v, v);
     };
-    full_apply<double, RPT>(L, ld, pre, out, row, xs);
+    apply(ld, pre, out);
   } else {
     double beta = 0.0;
     if (!first) {
@@ -486,53 +526,34 @@ __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, c
       const double qv = -Ax;
       if (store_p) pnew[node] = p;
       q[node] = qv;
-      a1 = p * qv;
-      if (first) a2 = rv * p;
+      a1 += __dmul_rn(p, qv);
+      if (first) a2 += __dmul_rn(rv, p);
     };
-    full_apply<double, RPT>(L, ld, pre, out, row, xs);
-  }
-  __syncthreads();
-  const int wv = tid >> 5, band = blockIdx.y * RPT + wv;
-  if (wv < RPT && band * 8 < L.Ny) {
-    const long slot = (long)k * w.PB + blockIdx.x + (long)gridDim.x * band;
-    double t = 0.0;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) t += cs[0][wv * 8 + r][lane];
-    t = warp_sum(t);
-    if (lane == 0) w.partials[slot] = t;
-    if (MODE == 1 && first) {
-      t = 0.0;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) t += cs[1][wv * 8 + r][lane];
-      t = warp_sum(t);
-      if (lane == 0) w.partials2[slot] = t;
-    }
+    apply(ld, pre, out);
   }
 }
 
-// grid of b_full_kernel: column tiles, row tiles of 8*rpt, instances
-static dim3 full_grid(const BatchGroup& g, int rpt) {
-  return dim3((g.Nz + TZ - 1) / TZ, (g.Ny + 8 * rpt - 1) / (8 * rpt), g.K);
-}
-
-// the separable form's launch shapes: rows per thread x minimum blocks per
-// SM the compiler fits its registers to (1: its own choice)
+// the separable form's launch shapes: tiles of 8 * rpt rows or walks of 4 *
+// chunks rows, and the blocks per SM the compiler fits its registers to (1:
+// its own choice)
 constexpr int kFullShapes = 6;
-constexpr int kFullRpt[kFullShapes] = {1, 2, 4, 1, 2, 4}, kFullMinb[kFullShapes] = {1, 1, 1, 4, 4, 4};
+constexpr int kFullRpt[kFullShapes] = {1, 2, 1, 2, 0, 0}, kFullMinb[kFullShapes] = {1, 1, 4, 4, 2, 2},
+              kFullChunks[kFullShapes] = {0, 0, 0, 0, 4, 8};
 
 template <int MODE, typename Tz>
 static void launch_full(const BatchGroup& g, int shape, const BatchInst* tab, const int* mask, const Tz* zv,
                         int first, int pi, int mixed, int store_p) {
-  const dim3 grid = full_grid(g, kFullRpt[shape]);
+  const int rpt = kFullRpt[shape];
+  const MarchPlan p = march_plan(g.L, kFullChunks[shape]);
+  const dim3 grid = rpt ? dim3((g.Nz + TZ - 1) / TZ, (g.Ny + 8 * rpt - 1) / (8 * rpt), g.K) : dim3(p.blocks, 1, g.K);
 #define SCY_FULL_LAUNCH(R, M) \
-  b_full_kernel<MODE, Tz, R, M><<<grid, 256, 0, g.stream>>>(g.L, tab, mask, g.w, zv, first, pi, mixed, store_p)
+  b_full_kernel<MODE, Tz, R, M><<<grid, 256, 0, g.stream>>>(g.L, tab, mask, g.w, zv, first, pi, mixed, store_p, p)
   switch (shape) {
     case 0: SCY_FULL_LAUNCH(1, 1); break;
     case 1: SCY_FULL_LAUNCH(2, 1); break;
-    case 2: SCY_FULL_LAUNCH(4, 1); break;
-    case 3: SCY_FULL_LAUNCH(1, 4); break;
-    case 4: SCY_FULL_LAUNCH(2, 4); break;
-    default: SCY_FULL_LAUNCH(4, 4); break;
+    case 2: SCY_FULL_LAUNCH(1, 4); break;
+    case 3: SCY_FULL_LAUNCH(2, 4); break;
+    default: SCY_FULL_LAUNCH(0, 2); break;
   }
 #undef SCY_FULL_LAUNCH
 }
@@ -1316,10 +1337,10 @@ int BatchContext::autotune(BatchGroup& g) {
     }
   }
   g.kpb = best;
-  // the separable form (when the operator is separable over every node) at
-  // 1, 2 and 4 rows per thread: used whenever it exists, so that a group's
+  // the separable form (when the operator is separable over every node) in
+  // six launch shapes: used whenever it exists, so that a group's
   // results do not depend on timings (its arithmetic differs from the cross
-  // form's by rounding; its rows per thread change nothing, see
+  // form's by rounding; its launch shape changes nothing, see
   // b_full_kernel); the cross form's timings stay for comparison
   g.full_shape = -1;
   if (g.L.full) {
@@ -1608,9 +1629,9 @@ int BatchContext::solve_refine(BatchGroup& g, const int* mask, int its_now, int 
 
 int BatchContext::solve(BatchGroup& g, const int* mask, int its_now) {
   const int mixed = precision != SCY_PREC_FP64 ? 1 : 0;
-  const int shape = g.full_shape, rpt = shape >= 0 ? kFullRpt[shape] : 0;  // rpt > 0: the separable form
-  const dim3 tg = rpt ? full_grid(g, rpt)
-                      : dim3((g.Nz + XTZ - 1) / XTZ, (g.Ny + XTY - 1) / XTY, (g.K + g.kpb - 1) / g.kpb);
+  const int shape = g.full_shape;
+  const bool sep = shape >= 0;  // the separable form
+  const dim3 tg((g.Nz + XTZ - 1) / XTZ, (g.Ny + XTY - 1) / XTY, (g.K + g.kpb - 1) / g.kpb);
   const dim3 ng(node_blocks(g.N), 1, g.K);
   const BatchInst* tab = g.tab.as<BatchInst>();
   const double* C = g.planes.as<double>();
@@ -1619,10 +1640,10 @@ int BatchContext::solve(BatchGroup& g, const int* mask, int its_now) {
   // node and active instance the operand, rhs and result (residual) or z,
   // p_old, p and q
   const double nact = (double)active_in(g, mask);
-  const double coef_b = rpt ? 0.0 : 33.0 * 8 * g.N;
+  const double coef_b = sep ? 0.0 : 33.0 * 8 * g.N;
   cudaEvent_t pa;
   SCY_TRY(prof_begin(g.stream, &pa));
-  if (rpt)
+  if (sep)
     launch_full<0, double>(g, shape, tab, mask, (const double*)nullptr, 0, 0, mixed, 0);
   else
     b_cross_kernel<0, double><<<tg, XT, xs_smem_bytes(0, 8), g.stream>>>(C, g.Ny, g.Nz, tab, mask, g.w, nullptr, 0,
@@ -1645,9 +1666,9 @@ int BatchContext::solve(BatchGroup& g, const int* mask, int its_now) {
       SCY_LAUNCH_CHECK();
     }
     SCY_TRY(prof_begin(g.stream, &pa));
-    if (rpt && mixed)
+    if (sep && mixed)
       launch_full<1, float>(g, shape, tab, mask, g.w.z32, first, pi, mixed, store_p);
-    else if (rpt)
+    else if (sep)
       launch_full<1, double>(g, shape, tab, mask, g.w.z, first, pi, mixed, store_p);
     else if (mixed)
       b_cross_kernel<1, float><<<tg, XT, xs_smem_bytes(1, 4), g.stream>>>(C, g.Ny, g.Nz, tab, mask, g.w, g.w.z32, first,
@@ -2163,7 +2184,7 @@ scy_status scy_batch_tuning(scy_batch* b, int g, int* kpb, int* sweep_variant, i
 scy_status scy_batch_operator_form(scy_batch* b, int g, int* rows_per_thread, int* min_blocks_per_sm) {
   if (!b || !rows_per_thread || g < 0 || g >= (int)b->ctx.groups.size()) return SCY_ERR_ARG;
   const int shape = b->ctx.groups[g]->full_shape;
-  *rows_per_thread = shape >= 0 ? scy::kFullRpt[shape] : 0;
+  *rows_per_thread = shape >= 0 ? scy::kFullRpt[shape] + scy::kFullChunks[shape] * scy::kChunk : 0;
   if (min_blocks_per_sm) *min_blocks_per_sm = shape >= 0 ? scy::kFullMinb[shape] : 0;
   return SCY_OK;
 }

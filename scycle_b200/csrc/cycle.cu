@@ -71,27 +71,11 @@ struct EpiWave {
   }
 };
 
-// RPT = 0: the two-stage tile (stencil_tile); 1, 2, 4: the full-form tile
-// with that many rows per thread (full_tile).
-template <int RPT>
-__device__ __forceinline__ void wave_tile(const LevelDev<double>& L, const LoadPlain<double>& ld, const EpiWave& ep) {
-  if constexpr (RPT == 0) {
-    stencil_tile<double, LoadPlain<double>, EpiWave>(L, ld, ep, nullptr, nullptr, nullptr);
-  } else {
-    __shared__ double xs[full_smem_values<RPT>()];
-    const double* __restrict__ up = ep.uPrev;
-    auto pre = [&](long node, int, int) { return up[node]; };
-    auto out = [&](long node, int iy, int iz, double Ax, double u, double upv) { ep.apply(node, iy, iz, Ax, u, upv); };
-    auto row = [](int) {};
-    full_apply<double, RPT>(L, ld, pre, out, row, xs);
-  }
-}
-
-template <int RPT>
+// The wave update where the operator has no full form: the two-stage tile.
 __global__ void __launch_bounds__(256) fd_wave_kernel(LevelDev<double> L, LoadPlain<double> ld, EpiWave ep,
                                                       const CycleDevState* st) {
   if (st->stop) return;
-  wave_tile<RPT>(L, ld, ep);
+  stencil_tile<double, LoadPlain<double>, EpiWave>(L, ld, ep, nullptr, nullptr, nullptr);
 }
 
 struct FDFaultArgs {
@@ -212,25 +196,32 @@ __device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, int iz, do
   return eta * V / tq;
 }
 
-// The last of the gridDim.x participating blocks finishes max(eta V / tauQS)
+// The last of the nblocks participating blocks (blockIdx.x 0 .. nblocks - 1) finishes max(eta V / tauQS)
 // and runs checkSwitchRegime for the fully dynamic phase.
-__device__ __forceinline__ void fd_switch_test(const FDFaultArgs& A, double block_max) {
+__device__ __forceinline__ void fd_switch_test(const FDFaultArgs& A, double block_max, unsigned nblocks) {
   CycleDevState* st = A.st;
   __shared__ bool am_last;
   if (threadIdx.x == 0) {
     A.partials[blockIdx.x] = block_max;
     __threadfence();
     const unsigned prev = atomicAdd(&st->counter, 1u);
-    am_last = prev == gridDim.x - 1;
+    am_last = prev == nblocks - 1;
   }
   __syncthreads();
-  if (am_last && threadIdx.x == 0) {
-    __threadfence();
+  if (!am_last || threadIdx.x >= 32) return;
+  // one warp reads the maxima, each lane its own in order (not one after the
+  // other: a read takes half a microsecond); a NaN counts only in the first,
+  // as in mx = v > mx ? v : mx from block 0 on
+  __threadfence();
+  double m = -INFINITY;
+  for (unsigned b = 1 + threadIdx.x; b < nblocks; b += 32) {
+    const double v = ((volatile double*)A.partials)[b];
+    m = v > m ? v : m;
+  }
+  m = warp_max(m);
+  if (threadIdx.x == 0) {
     double mx = ((volatile double*)A.partials)[0];
-    for (unsigned b = 1; b < gridDim.x; ++b) {
-      const double v = ((volatile double*)A.partials)[b];
-      mx = v > mx ? v : mx;
-    }
+    mx = m > mx ? m : mx;
     st->maxR = mx;
     if (!st->allowed && mx > A.limit_fd) st->allowed = 1;
     if (st->allowed && mx < A.trigger_fd2qd) st->stop = 1;
@@ -259,14 +250,37 @@ __global__ void __launch_bounds__(kFaultBlock) fd_fault_kernel(FDFaultArgs A) {
   __syncthreads();
   double b = sh[0];
   for (int w = 1; w < (int)(blockDim.x >> 5); ++w) b = sh[w] > b ? sh[w] : b;
-  fd_switch_test(A, b);
+  fd_switch_test(A, b, gridDim.x);
+}
+
+// The fault update of a fault tile's 32 columns (z0 on) from the rows it just
+// computed, and the switch test
+__device__ __forceinline__ void fd_fault_tile(const FDFaultArgs& A, int z0, const double* s_rows, const double* s_d2u,
+                                              unsigned nblocks) {
+  __shared__ double s_max[4];
+  __syncthreads();
+  if (threadIdx.x < 4 * TZ) {
+    const int col = threadIdx.x >> 2, iz = z0 + col;
+    double R = -INFINITY;
+    if (iz < A.fp.Nz) {
+      unsigned bad = 0;
+      auto rows = [&](int k) { return s_rows[k * TZ + col]; };
+      R = fd_fault_node(A, iz, s_d2u[col], rows, &bad);
+      if (bad && (threadIdx.x & 3) == 0) atomicOr(&A.st->flags, bad);
+    }
+    R = warp_max(R);
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = R;
+  }
+  __syncthreads();
+  double R = s_max[0];
+  for (int w = 1; w < 4; ++w) R = s_max[w] > R ? s_max[w] : R;
+  fd_switch_test(A, R, nblocks);
 }
 
 // One fully dynamic step in one launch: every tile applies the wave update;
 // the tiles of the fault row (blockIdx.y == 0, rows 0 .. 7 or more) then run
 // the fault update of their 32 columns from the rows they just computed,
 // while the rest of the grid is still stepping the body.
-template <int RPT>
 __global__ void __launch_bounds__(256) fd_step_kernel(LevelDev<double> L, LoadPlain<double> ld, EpiWave ep,
                                                       FDFaultArgs A) {
   CycleDevState* st = A.st;
@@ -277,26 +291,43 @@ __global__ void __launch_bounds__(256) fd_step_kernel(LevelDev<double> L, LoadPl
   EpiWave e = ep;
   e.s_rows = fault_tile ? s_rows : nullptr;
   e.s_d2u = fault_tile ? s_d2u : nullptr;
-  wave_tile<RPT>(L, ld, e);
+  stencil_tile<double, LoadPlain<double>, EpiWave>(L, ld, e, nullptr, nullptr, nullptr);
   if (!fault_tile) return;
-  __syncthreads();
-  __shared__ double s_max[4];
-  if (threadIdx.x < 4 * TZ) {
-    const int col = threadIdx.x >> 2, iz = blockIdx.x * TZ + col;
-    double R = -INFINITY;
-    if (iz < A.fp.Nz) {
-      unsigned bad = 0;
-      auto rows = [&](int k) { return s_rows[k * TZ + col]; };
-      R = fd_fault_node(A, iz, s_d2u[col], rows, &bad);
-      if (bad && (threadIdx.x & 3) == 0) atomicOr(&st->flags, bad);
+  fd_fault_tile(A, blockIdx.x * TZ, s_rows, s_d2u, gridDim.x);
+}
+
+// The same with the operator in the full form: one block per 8 x 32 tile of
+// rows 0 .. 7 first (FAULT: with the fault update), the rest of the body in
+// walks by warps (march_part).  Bound by the fault tiles' chain of dependent
+// FP64 roots: a step of 61 x 61 takes 13.0 us, one of 801 x 801 15.4 (17.0
+// with the body in block-staged tiles and 18.2 with, besides, the tiles'
+// maxima read one after the other).
+template <bool FAULT>
+__global__ void __launch_bounds__(32 * kMarchWarps, 2) fd_march_kernel(LevelDev<double> L, LoadPlain<double> ld,
+                                                                       EpiWave ep, FDFaultArgs A, MarchPlan p) {
+  if (A.st->stop) return;
+  constexpr int NS = kMarchWarps * kMarchSmem > full_smem_values<1>() ? kMarchWarps * kMarchSmem : full_smem_values<1>();
+  __shared__ double sm[NS];
+  __shared__ double s_rows[5 * TZ];
+  __shared__ double s_d2u[TZ];
+  const int nx = p.nx, wv = threadIdx.x >> 5;
+  EpiWave e = ep;
+  e.s_rows = e.s_d2u = nullptr;
+  const double* __restrict__ up = ep.uPrev;
+  auto pre = [&](long node, int, int) { return up[node]; };
+  auto out = [&](long node, int iy, int iz, double Ax, double u, double upv) { e.apply(node, iy, iz, Ax, u, upv); };
+  if ((int)blockIdx.x < nx) {
+    if (FAULT) {
+      e.s_rows = s_rows;
+      e.s_d2u = s_d2u;
     }
-    R = warp_max(R);
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = R;
+    auto row = [](int) {};
+    full_apply<double, 1>(L, ld, pre, out, row, sm, 0, blockIdx.x * TZ);
+    if (FAULT) fd_fault_tile(A, blockIdx.x * TZ, s_rows, s_d2u, nx);
+  } else {
+    auto none = [](int, int) {};
+    march_part<double>(L, p, blockIdx.x - nx, wv, ld, pre, out, none, sm + wv * kMarchSmem);
   }
-  __syncthreads();
-  double R = s_max[0];
-  for (int w = 1; w < 4; ++w) R = s_max[w] > R ? s_max[w] : R;
-  fd_switch_test(A, R);
 }
 
 // max over the fault of eta V / tauQS (the quasi-dynamic phase's test)
@@ -665,27 +696,20 @@ int CycleContext::fd_launch_step(int r, cudaStream_t s, int part) {
   A.st = st;
   const LoadPlain<double> ld{u3[cur].as<double>()};
   const dim3 g = apply_grid(L);
-  const int rpt = L.full ? L.rpt : 0;
+  const MarchPlan mp = L.full ? march_plan(L, march_chunks(L), 1) : MarchPlan{};
+  const int mg = mp.nx + mp.blocks;
   if (part & FD_FUSED) {
-    if (rpt == 4)
-      fd_step_kernel<4><<<g, 256, 0, s>>>(L, ld, ep, A);
-    else if (rpt == 2)
-      fd_step_kernel<2><<<g, 256, 0, s>>>(L, ld, ep, A);
-    else if (rpt == 1)
-      fd_step_kernel<1><<<g, 256, 0, s>>>(L, ld, ep, A);
+    if (L.full)
+      fd_march_kernel<true><<<mg, 32 * kMarchWarps, 0, s>>>(L, ld, ep, A, mp);
     else
-      fd_step_kernel<0><<<g, 256, 0, s>>>(L, ld, ep, A);
+      fd_step_kernel<<<g, 256, 0, s>>>(L, ld, ep, A);
     SCY_LAUNCH_CHECK();
   }
   if (part & FD_WAVE) {
-    if (rpt == 4)
-      fd_wave_kernel<4><<<g, 256, 0, s>>>(L, ld, ep, st);
-    else if (rpt == 2)
-      fd_wave_kernel<2><<<g, 256, 0, s>>>(L, ld, ep, st);
-    else if (rpt == 1)
-      fd_wave_kernel<1><<<g, 256, 0, s>>>(L, ld, ep, st);
+    if (L.full)
+      fd_march_kernel<false><<<mg, 32 * kMarchWarps, 0, s>>>(L, ld, ep, A, mp);
     else
-      fd_wave_kernel<0><<<g, 256, 0, s>>>(L, ld, ep, st);
+      fd_wave_kernel<<<g, 256, 0, s>>>(L, ld, ep, st);
     SCY_LAUNCH_CHECK();
   }
   if (part & FD_FAULT) {

@@ -76,6 +76,7 @@ struct LevelDev {
   // full-form tile.
   int ylo, yhi, zlo, zhi, crow, ccol, rpt;
   T cyc[BAND], czc[BAND];
+  const T* Cy10;  // the 9 middle entries of class 0's rows, ten values a row (the last zero)
   // Levels without the full form and of at most kCrossMaxNodes nodes: the
   // operator composed per node (cross_build_kernel), 33 planes of Ny * Nz
   // values, offsets -8..8 along y and then -8..-1, 1..8 along z (the centre
@@ -134,6 +135,7 @@ struct EpiStore {
   T* out;
   T scale;
   static constexpr bool kReduce = false;
+  static constexpr bool kMarch = true;
   __device__ __forceinline__ double operator()(long node, int, int, T Ax, T) const {
     out[node] = scale * Ax;
     return 0.0;
@@ -494,7 +496,7 @@ __device__ __forceinline__ void full_stage(const Loader& ld, T* xs, int y0, int 
     if (at[a] >= 0) xs[at[a]] = v[a];
 }
 
-// The tile of block (blockIdx.x, blockIdx.y): stages the operand through
+// The 8 * RPT x 32 tile from (y0, z0) on: stages the operand through
 // ld(node, iy, iz) into xs; then pre(node, iy, iz) is called for each of
 // the thread's output nodes (the epilogue's own loads, issued before the
 // operator is applied so their latency is hidden; default value where the
@@ -506,11 +508,10 @@ __device__ __forceinline__ void full_stage(const Loader& ld, T* xs, int y0, int 
 // differ from row to row.
 template <typename T, int RPT, class Loader, class Pre, class Out, class Row>
 __device__ __forceinline__ void full_apply(const LevelDev<T>& L, const Loader& ld, const Pre& pre, Out& out, Row& row,
-                                           T* xs) {
+                                           T* xs, int y0, int z0) {
   constexpr int TYB = 8 * RPT;
   using P = decltype(pre(0L, 0, 0));
   const int Ny = L.Ny, Nz = L.Nz;
-  const int y0 = blockIdx.y * TYB, z0 = blockIdx.x * TZ;
   const int tid = threadIdx.x, lane = tid & 31, r0 = (tid >> 5) * RPT;
   const int iz = z0 + lane;
   const bool inner = y0 >= L.ylo && y0 + TYB - 1 <= L.yhi && z0 >= L.zlo && z0 + TZ - 1 <= L.zhi;
@@ -619,6 +620,312 @@ __device__ __forceinline__ double epi_out(const Epi& ep, long node, int iy, int 
     return ep(node, iy, iz, Ax, xv, p);
 }
 
+// -------------------------------------------------------------------------
+// The full form by warps, on the grid's interior: a warp walks down 32 columns
+// in chunks of 4 rows, a lane per column.  The values along y stay in a
+// register window (a row is loaded once), a chunk's rows with their halo along
+// z go through the warp's own part of shared memory, and the next chunk's
+// rows, halo and epilogue operands are loaded while this one is computed: a
+// row costs 9 + 9 multiply-adds, 8 shared reads and one global read per lane,
+// and no warp waits for another.  The row's y coefficients are a broadcast
+// (Cy10: class 0's nine middle entries, ten to a row), the column's z
+// coefficients stay in registers.  Sums run in the order of full_apply: the
+// results are the same to the bit.  Chunks at the grid's edges go to warps of
+// their own (march_edge).
+//
+// The block-staged tile spends 200 to 240 warp instructions per 32 outputs,
+// mostly on staging through index arithmetic, and its warps wait at the
+// barrier for half of their time; a walk spends 85.  At 2049 x 1537 the
+// operator takes 27 us here and 31 there (floor 7.7 us): 24 warps' registers
+// would fit an SM only with spills, and with 16 the loads' latency is partly
+// open; the shared-memory pipe is 59 % busy.
+constexpr int kMarchWarps = 8;
+constexpr int kChunk = 4;                            // rows of a chunk
+constexpr int kMarchRows = kChunk * (TZ + 2 * HALF);  // shared values of an interior chunk's rows
+constexpr int kEdgeRows = kChunk * (TZ + 16);         // and of an edge chunk's
+constexpr int kMarchSmem = kEdgeRows + 2 * kChunk * 17;  // of one warp: the rows, then their y coefficients
+
+template <typename T>
+struct Vec2;
+template <>
+struct Vec2<double> {
+  using type = double2;
+};
+template <>
+struct Vec2<float> {
+  using type = float2;
+};
+
+// The walk over rows y0 .. yend - 1 (whole chunks inside the interior box) of
+// columns z0 .. z0 + 31.  ld, pre, out as for full_apply; chunk(y, tx) after the
+// chunk from row y of tile column tx, warp-uniform.
+template <typename T, class Loader, class Pre, class Out, class Chunk>
+__device__ __forceinline__ void march(const LevelDev<T>& L, const Loader& ld, const Pre& pre, Out& out, Chunk& chunk,
+                                      T* sm, int y0, int yend, int z0, int tx) {
+  constexpr int R = kChunk, H = HALF, W = TZ + 2 * H;
+  using P = decltype(pre(0L, 0, 0));
+  using T2 = typename Vec2<T>::type;
+  if (y0 >= yend) return;
+  const int Nz = L.Nz, lane = threadIdx.x & 31, iz = z0 + lane;
+  const int hr = lane >> 3, hk = lane & 7, hc = hk < H ? z0 - H + hk : z0 + TZ + hk - H;  // the lane's halo value
+  const int hs = hr * W + (hk < H ? hk : TZ + hk);
+  // the chunk's y coefficients: lane l < 20 moves two of the 40 values
+  const T2* cyp = reinterpret_cast<const T2*>(L.Cy10) + (long)y0 * 5 + min(lane, 5 * R - 1);
+  T2* cys = reinterpret_cast<T2*>(sm + kMarchRows);
+  const bool cyl = !L.crow && lane < 5 * R;
+  T w[R + 2 * H], hv, cz[BAND];
+  P pv[R];
+  T2 cv = __ldg(cyp);
+  long n0 = (long)y0 * Nz + iz, nh = (long)(y0 + hr) * Nz + hc;
+#pragma unroll
+  for (int k = 0; k < R + 2 * H; ++k) w[k] = ld(n0 + (long)(k - H) * Nz, y0 + k - H, iz);
+  hv = ld(nh, y0 + hr, hc);
+#pragma unroll
+  for (int r = 0; r < R; ++r) pv[r] = pre(n0 + (long)r * Nz, y0 + r, iz);
+#pragma unroll
+  for (int o = 0; o < BAND; ++o) cz[o] = L.ccol ? L.czc[o] : __ldg(L.CzT17 + (long)(o + 8 - HALF) * Nz + iz);
+  const T wyv = __ldg(L.wy1 + iz);
+  for (;;) {
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; ++r) sm[r * W + H + lane] = w[r + H];
+    sm[hs] = hv;
+    if (cyl) cys[lane] = cv;
+    __syncwarp();
+    // the next chunk's (at the end of the walk this chunk's again, not used)
+    const int st = y0 + R < yend ? R : 0;
+    const long nn = n0 + (long)st * Nz;
+    T nx[R];
+    P pn[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) nx[k] = ld(nn + (long)(k + H) * Nz, y0 + st + k + H, iz);
+    nh += (long)st * Nz;
+    hv = ld(nh, y0 + st + hr, hc);
+    cyp += st * 5;
+    if (cyl) cv = __ldg(cyp);
+#pragma unroll
+    for (int r = 0; r < R; ++r) pn[r] = pre(nn + (long)r * Nz, y0 + st + r, iz);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int iy = y0 + r;
+      const T* cy = sm + kMarchRows + r * 10;
+      const T* xr = sm + r * W + lane;
+      T sy = T(0), sz = T(0);
+#pragma unroll
+      for (int o = 0; o < BAND; ++o) {
+        sy += (L.crow ? L.cyc[o] : cy[o]) * w[r + o];
+        sz += cz[o] * (o == HALF ? w[r + HALF] : xr[o]);
+      }
+      out(n0 + (long)r * Nz, iy, iz, wyv * sy + __ldg(L.wz1 + iy) * sz, w[r + HALF], pv[r]);
+    }
+    chunk(y0, tx);
+    if (st == 0) break;
+    y0 += R;
+    n0 = nn;
+#pragma unroll
+    for (int k = 0; k < 2 * H; ++k) w[k] = w[k + R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      w[k + 2 * H] = nx[k];
+      pv[k] = pn[k];
+    }
+  }
+}
+
+// One chunk at the grid's edges, by a warp: rows y0 .. y0 + 3 of 32 columns,
+// zeros outside the grid; the four outer offsets of either side only where
+// the line's stencil has them, classes by column and row as in full_apply.
+// All loads come first; the rows' y coefficients of class 0 and of one
+// exceptional class go through shared memory.
+template <typename T, class Loader, class Pre, class Out>
+__device__ __forceinline__ void march_edge(const LevelDev<T>& L, const Loader& ld, const Pre& pre, Out& out, T* sm,
+                                           int y0, int z0) {
+  constexpr int R = kChunk, H = 8, W = TZ + 2 * H, NC = R * 17;
+  using P = decltype(pre(0L, 0, 0));
+  const int Ny = L.Ny, Nz = L.Nz, lane = threadIdx.x & 31, iz = z0 + lane;
+  const long n0 = (long)y0 * Nz + iz;
+  const bool col = iz < Nz;
+  T* cys = sm + kEdgeRows;
+  const int yc = col ? __ldg(L.ycls + iz) : 0;
+  int zc[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) zc[r] = y0 + r < Ny ? __ldg(L.zcls + y0 + r) : 0;  // the same for the whole warp
+  T w[R + 2 * H], hv[2], cv[3];
+#pragma unroll
+  for (int k = 0; k < R + 2 * H; ++k) {
+    const int iy = y0 + k - H;
+    w[k] = col && iy >= 0 && iy < Ny ? ld(n0 + (long)(k - H) * Nz, iy, iz) : T(0);
+  }
+  const int hk = lane & 15, hc = hk < H ? z0 - H + hk : z0 + TZ + hk - H;  // halo column, rows lane / 16 + 2 j
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int iy = y0 + (lane >> 4) + 2 * j;
+    hv[j] = hc >= 0 && hc < Nz && iy < Ny ? ld((long)iy * Nz + hc, iy, hc) : T(0);
+  }
+  const int nc = min(NC, (Ny - y0) * 17);
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    cv[j] = lane + 32 * j < nc ? __ldg(L.Cy17 + (long)y0 * 17 + lane + 32 * j) : T(0);
+  P pv[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) pv[r] = col && y0 + r < Ny ? pre(n0 + (long)r * Nz, y0 + r, iz) : P{};
+  const T wyv = col ? __ldg(L.wy1 + iz) : T(0);
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < R; ++r) sm[r * W + H + lane] = w[r + H];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) sm[((lane >> 4) + 2 * j) * W + (hk < H ? hk : TZ + hk)] = hv[j];
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+    if (lane + 32 * j < NC) cys[lane + 32 * j] = cv[j];
+  const unsigned exc = __ballot_sync(0xffffffffu, yc != 0);
+  int yx = 0;  // the exceptional class in shared memory
+  if (exc != 0) {
+    yx = __shfl_sync(0xffffffffu, yc, __ffs(exc) - 1);
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (lane + 32 * j < nc) cys[NC + lane + 32 * j] = __ldg(L.Cy17 + ((long)yx * Ny + y0) * 17 + lane + 32 * j);
+  }
+  __syncwarp();
+  const bool far_z = iz < L.zlo || iz > L.zhi, own = yc != 0 && yc != yx;
+  T sz[R] = {};
+  if (zc[0] == 0 || zc[1] == 0 || zc[2] == 0 || zc[3] == 0) {
+    const T* cz = L.CzT17 + (col ? iz : 0);
+#pragma unroll
+    for (int o = 0; o < 17; ++o) {
+      if (far_z || (o >= H - HALF && o <= H + HALF)) {
+        const T c = __ldg(cz + (long)o * Nz);
+#pragma unroll
+        for (int r = 0; r < R; ++r) sz[r] += c * sm[r * W + lane + o];
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int iy = y0 + r;
+    if (!col || iy >= Ny) continue;
+    if (zc[r] != 0) {
+      const T* cc = L.CzT17 + (long)zc[r] * 17 * Nz + iz;
+      sz[r] = T(0);
+#pragma unroll
+      for (int o = 0; o < 17; ++o) sz[r] += __ldg(cc + (long)o * Nz) * sm[r * W + lane + o];
+    }
+    T sy = T(0);
+    if (!own) {
+      const T* cy = cys + (yc != 0 ? NC : 0) + r * 17;
+      const bool fy = yc != 0 || iy < L.ylo || iy > L.yhi;
+      if (fy) {
+#pragma unroll
+        for (int o = 0; o < H - HALF; ++o) sy += cy[o] * w[r + o];
+      }
+#pragma unroll
+      for (int o = H - HALF; o <= H + HALF; ++o) sy += cy[o] * w[r + o];
+      if (fy) {
+#pragma unroll
+        for (int o = H + HALF + 1; o < 17; ++o) sy += cy[o] * w[r + o];
+      }
+    } else {
+      const T* cy = L.Cy17 + ((long)yc * Ny + iy) * 17;
+#pragma unroll
+      for (int o = 0; o < 17; ++o) sy += __ldg(cy + o) * w[r + o];
+    }
+    out(n0 + (long)r * Nz, iy, iz, wyv * sy + __ldg(L.wz1 + iy) * sz[r], w[r + H], pv[r]);
+  }
+}
+
+// Warps of a launch: ech chunks of one 8 x 32 tile outside the interior box
+// (tiles [tx0, tx1) x [ty0, ty1)) each, in whole blocks, the first t0 tiles
+// left out; then the box, a walk of nch chunks each.
+struct MarchPlan {
+  int nx, ny, tx0, tx1, ty0, ty1, nch, ech, t0, edge, blocks;
+};
+template <typename T>
+inline MarchPlan march_plan(const LevelDev<T>& L, int nch, int skip_bands = 0) {
+  MarchPlan p;
+  p.nx = (L.Nz + TZ - 1) / TZ;
+  p.ny = (L.Ny + 7) / 8;
+  p.tx0 = (L.zlo + TZ - 1) / TZ;
+  p.tx1 = (L.zhi + 1) / TZ;
+  p.ty0 = (L.ylo + 7) / 8;
+  p.ty1 = (L.yhi + 1) / 8;
+  if (p.tx1 <= p.tx0 || p.ty1 <= p.ty0) p.tx0 = p.tx1 = p.ty0 = p.ty1 = 0;
+  const int chunks = 2 * (p.ty1 - p.ty0), cols = p.tx1 - p.tx0;
+  p.nch = nch > 0 ? nch : 1;
+  p.ech = p.nch > 1 ? 2 : 1;
+  p.t0 = skip_bands * p.nx;
+  p.edge = ((p.nx * p.ny - cols * (p.ty1 - p.ty0) - p.t0) * (2 / p.ech) + kMarchWarps - 1) / kMarchWarps;
+  p.blocks = p.edge + cols * ((chunks + kMarchWarps * p.nch - 1) / (kMarchWarps * p.nch));
+  return p;
+}
+
+// The part of warp wv of block b: pre, out, chunk as for march.
+template <typename T, class Loader, class Pre, class Out, class Chunk>
+__device__ __forceinline__ void march_part(const LevelDev<T>& L, const MarchPlan& p, int b, int wv, const Loader& ld,
+                                           const Pre& pre, Out& out, Chunk& chunk, T* sm) {
+  const int cols = p.tx1 - p.tx0;
+  if (b < p.edge) {
+    const int tb = (p.ty0 + p.ny - p.ty1) * p.nx;  // tiles of the bands outside the box
+    const int nt = p.ech == 2 ? 1 : 2;
+    int t = b * kMarchWarps + wv, half = 0, tx, ty;
+    if (nt == 2) {
+      half = t & 1;
+      t >>= 1;
+    }
+    t += p.t0;
+    if (t < tb) {
+      ty = t / p.nx;
+      tx = t - ty * p.nx;
+      if (ty >= p.ty0) ty += p.ty1 - p.ty0;
+    } else {
+      t -= tb;
+      const int nc = p.nx - cols;
+      if (nc == 0) return;
+      ty = t / nc;
+      tx = t - ty * nc;
+      ty += p.ty0;
+      if (ty >= p.ty1) return;
+      if (tx >= p.tx0) tx += cols;
+    }
+#pragma unroll 1
+    for (int c = half; c < half + p.ech; ++c) {
+      const int y0 = ty * 8 + c * kChunk;
+      if (y0 < L.Ny) march_edge<T>(L, ld, pre, out, sm, y0, tx * TZ);
+      chunk(y0, tx);
+    }
+  } else {
+    b -= p.edge;
+    const int seg = b / cols, tx = p.tx0 + b - seg * cols, y0 = 8 * p.ty0 + (seg * kMarchWarps + wv) * p.nch * kChunk;
+    march<T>(L, ld, pre, out, chunk, sm, y0, min(8 * p.ty1, y0 + p.nch * kChunk), tx * TZ, tx);
+  }
+}
+
+template <typename T, class Loader, class Epi>
+__global__ void __launch_bounds__(32 * kMarchWarps, 2) march_kernel(LevelDev<T> L, Loader ld, Epi ep, MarchPlan p) {
+  static_assert(!Epi::kReduce, "the warp form has no grid sum");
+  __shared__ T sm[kMarchWarps * kMarchSmem];
+  auto pre = [&](long node, int iy, int iz) { return epi_pre(ep, node, iy, iz, 0); };
+  auto out = [&](long node, int iy, int iz, T Ax, T xv, const auto& q) { epi_out(ep, node, iy, iz, Ax, xv, q); };
+  auto none = [](int, int) {};
+  const int wv = threadIdx.x >> 5;
+  march_part<T>(L, p, blockIdx.x, wv, ld, pre, out, none, sm + wv * kMarchSmem);
+}
+
+// Chunks per walk of a launch: as many as leave about 16 warps per SM, since
+// a walk's first window costs 8 rows more.
+template <typename T>
+inline int march_chunks(const LevelDev<T>& L) {
+  const long chunks = (long)(L.Nz / TZ) * (L.Ny / kChunk), slots = 16L * kNumSMs;
+  return (int)((chunks + slots - 1) / slots);
+}
+
+// Epilogues that take the warp form (march_kernel): those without a sum.  The
+// others keep the tile, whose sums their results depend on (CG's scalars), or
+// which is as fast at the sizes they run at (EpiCorrect at 401 x 401).
+template <class Epi, class = void>
+struct TakesMarch : std::false_type {};
+template <class Epi>
+struct TakesMarch<Epi, std::enable_if_t<Epi::kMarch>> : std::true_type {};
+
 template <typename T, int RPT, class Loader, class Epi>
 __device__ __forceinline__ void full_tile(const LevelDev<T>& L, const Loader& ld, const Epi& ep, double* partials,
                                           unsigned int* counter, double* red_out) {
@@ -630,7 +937,7 @@ __device__ __forceinline__ void full_tile(const LevelDev<T>& L, const Loader& ld
     contrib += epi_out(ep, node, iy, iz, Ax, xv, p);
   };
   auto row = [](int) {};
-  full_apply<T, RPT>(L, ld, pre, out, row, xs);
+  full_apply<T, RPT>(L, ld, pre, out, row, xs, blockIdx.y * 8 * RPT, blockIdx.x * TZ);
   if constexpr (Epi::kReduce) {
     if (partials != nullptr) {  // uniform across the grid
       double tot = block_sum(contrib, red);
@@ -844,6 +1151,17 @@ template <typename T, class Loader, class Epi>
 inline void launch_apply(const LevelDev<T>& L, const Loader& ld, const Epi& ep, double* partials,
                          unsigned int* counter, double* red_out, cudaStream_t s) {
   const dim3 g = apply_grid(L);
+  if constexpr (TakesMarch<Epi>::value) {
+    // below, nearly all of the grid is edge, and the tiles are as fast or
+    // faster (a call at 61 x 61: 20.5 us in tiles, 21.5 in walks; 257 x 129:
+    // 21.2 and 21.6; 401 x 401: 23.6 and 22.8; 1201 x 1201: 34.7 and 31.9;
+    // 2049 x 1537: 45.0 and 40.9; 4097 x 3073: 107.8 and 94.1)
+    if (L.full && (long)L.Ny * L.Nz >= 65536) {
+      const MarchPlan p = march_plan(L, march_chunks(L));
+      march_kernel<T, Loader, Epi><<<p.blocks, 32 * kMarchWarps, 0, s>>>(L, ld, ep, p);
+      return;
+    }
+  }
   if (!L.full && L.cross)
     cross_kernel<T, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);
   else if (!L.full)

@@ -269,6 +269,11 @@ int LevelStore<T>::init(const LevelHost& h, cudaStream_t s) {
     // are the separable interior's where that exists
     FullForm F;
     if (build_full_form(h, F)) {
+      std::vector<double> cy10((size_t)Ny * 10, 0.0);
+      for (int i = 0; i < Ny; ++i)
+        for (int o = 0; o < BAND; ++o) cy10[(size_t)i * 10 + o] = F.Cy17[(size_t)i * 17 + 8 - HALF + o];
+      SCY_TRY(upload<T>(comp10, cy10, s));
+      dev.Cy10 = comp10.template as<T>();
       SCY_TRY(upload<T>(comp17[0], F.Cy17, s));
       SCY_TRY(upload<T>(comp17[1], F.CzT17, s));
       SCY_TRY(upload_ints<T>(cls[0], F.ycls, s));

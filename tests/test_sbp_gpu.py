@@ -132,6 +132,33 @@ def test_full_form_every_rows_per_thread(monkeypatch, rpt, grid, mu_kind):
     assert _rel(u.cpu().numpy(), ref) <= 1e-9
 
 
+@pytest.mark.parametrize("Ny,Nz,grid,mu_kind", [
+    (256, 256, "constantGridSpacing", "constant"), (257, 263, "variableGridSpacing", "constant"),
+    (383, 177, "constantGridSpacing", "one_column"), (1100, 61, "variableGridSpacing", "constant"),
+    (33, 2001, "variableGridSpacing", "one_column"), (801, 353, "constantGridSpacing", "constant")])
+def test_apply_A_in_walks(Ny, Nz, grid, mu_kind):
+    """A x by warps that walk down 32 columns (grids of 65536 nodes or more
+    whose operator is separable over every node): interior boxes that end
+    inside tiles, no interior box at all (one exceptional column near one
+    side, few rows), walks of one and of several chunks, partial last tiles.
+    Both sides sum at most 34 products per node in FP64 from the same 1D
+    operators; the composed coefficients' rounding leaves about 1e-14."""
+    Ly, Lz = 30.0, 24.0
+    q = np.repeat(np.arange(Ny) / (Ny - 1), Nz)
+    r = np.tile(np.arange(Nz) / (Nz - 1), Ny)
+    var = grid == "variableGridSpacing"
+    y = Ly * np.sinh(2 * q) / np.sinh(2) if var else None
+    z = Lz * (r + 0.2 * r * r) / 1.2 if var else None
+    mu = np.full(Ny * Nz, 32.04)
+    if mu_kind == "one_column":
+        mu.reshape(Ny, Nz)[:, Nz // 3] = 27.5
+    from scycle_b200.sbp import SbpOps
+    dev = SbpOps(4, Ny, Nz, Ly, Lz, mu, grid=grid, y=y, z=z)
+    ora = OracleSbp(4, Ny, Nz, Ly, Lz, mu, grid=grid, y=y, z=z)
+    x = np.random.default_rng(Ny).standard_normal(Ny * Nz)
+    assert _rel(dev.apply("A", x).cpu().numpy(), ora.A @ x) <= 1e-13
+
+
 @pytest.mark.parametrize("precision", ("fp64", "mixed"))
 def test_fast_diagonalisation_on_separable_stretched_grid(precision):
     """Constant mu, y(iy) and z(iz) stretched independently: the separable part
