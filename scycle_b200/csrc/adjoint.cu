@@ -20,6 +20,7 @@ struct AxCombo {
 };
 
 __global__ void adj_combine_kernel(double* __restrict__ out, const double* __restrict__ y, AxCombo cb, long n) {
+  chain_enter();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   double v = cb.c[0] * cb.f[0][i] + y[i];
@@ -29,12 +30,14 @@ __global__ void adj_combine_kernel(double* __restrict__ out, const double* __res
 
 // y += a x over n entries
 __global__ void adj_axpy_kernel(double* __restrict__ y, const double* __restrict__ x, double a, long n) {
+  chain_enter();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i < n) y[i] += a * x[i];
 }
 
 // y = a x over n entries
 __global__ void adj_scale_kernel(double* __restrict__ y, const double* __restrict__ x, double a, long n) {
+  chain_enter();
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i < n) y[i] = a * x[i];
 }
@@ -44,6 +47,7 @@ __global__ void adj_scale_kernel(double* __restrict__ y, const double* __restric
 __global__ void adj_capture_kernel(const double* __restrict__ y, long psi_off, const double* __restrict__ V,
                                    const double* __restrict__ tq, const double* __restrict__ u, int Ny, int Nz,
                                    double* __restrict__ ev, double* __restrict__ evs) {
+  chain_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < Nz) {
     ev[i] = y[psi_off + i];
@@ -57,6 +61,7 @@ __global__ void adj_capture_kernel(const double* __restrict__ y, long psi_off, c
 __global__ void adj_misfit_kernel(const double* __restrict__ V, const double* __restrict__ u, int Ny, int Nz,
                                   const double* __restrict__ ts, const double* __restrict__ tv, double ws, double wv,
                                   double* __restrict__ obs_s, double* __restrict__ obs_v, double* __restrict__ Jn) {
+  chain_enter();
   __shared__ double sh[32];
   double acc = 0.0;
   for (int i = threadIdx.x; i < Ny; i += blockDim.x) {
@@ -84,6 +89,7 @@ __global__ void adj_misfit_kernel(const double* __restrict__ V, const double* __
 __global__ void adj_fault_kernel(const double* __restrict__ ev, FaultParams fp, const double* __restrict__ lf,
                                  const double* __restrict__ tv, double wv, double* __restrict__ ly,
                                  double* __restrict__ ltau, double* __restrict__ grad) {
+  chain_enter();
   const int iz = blockIdx.x * blockDim.x + threadIdx.x;
   const int Nz = fp.Nz;
   if (iz >= Nz) return;
@@ -139,6 +145,7 @@ __global__ void adj_fault_kernel(const double* __restrict__ ev, FaultParams fp, 
 
 // lu = d tau / d u ^T ltau: tau(iz) = mu(iz) [qy(iz)] sum_k D0[k] u(k, iz), k = 0..4
 __global__ void adj_tau_scatter_kernel(LevelDev<double> L, const double* __restrict__ ltau, double* __restrict__ lu) {
+  chain_enter();
   const int iz = blockIdx.x * blockDim.x + threadIdx.x;
   const int Nz = L.Nz;
   if (iz >= Nz) return;
@@ -154,6 +161,7 @@ __global__ void adj_tau_scatter_kernel(LevelDev<double> L, const double* __restr
 // lu(iy, 0) += 2 ws (surfDisp(iy) - target(iy))
 __global__ void adj_surf_kernel(const double* __restrict__ us, const double* __restrict__ ts, double ws, int Ny,
                                 int Nz, double* __restrict__ lu) {
+  chain_enter();
   const int iy = blockIdx.x * blockDim.x + threadIdx.x;
   if (iy < Ny) lu[(long)iy * Nz] += 2.0 * ws * (us[iy] - ts[iy]);
 }
@@ -161,6 +169,7 @@ __global__ void adj_surf_kernel(const double* __restrict__ us, const double* __r
 // ly[slip] += (M_L^T w) / faultTypeScale: the setRhs column of bcL
 __global__ void adj_bcl_kernel(LevelDev<double> L, const double* __restrict__ w, double inv_fts, long slip_off,
                                double* __restrict__ ly) {
+  chain_enter();
   const int iz = blockIdx.x * blockDim.x + threadIdx.x;
   const int Ny = L.Ny, Nz = L.Nz;
   if (iz >= Nz) return;
@@ -265,7 +274,7 @@ int AdjointContext::stage_combine(double* out, const double* y,
     ++j;
   }
   cb.nf = j;
-  adj_combine_kernel<<<blocks(q->nvar, 256), 256, 0, q->sbp.stream>>>(out, y, cb, q->nvar);
+  chain_launch(adj_combine_kernel, blocks(q->nvar, 256), 256, 0, q->sbp.stream, out, y, cb, q->nvar);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -278,8 +287,8 @@ int AdjointContext::eval(double t, const double* y, double* f, long slot, int e,
     const int Nz = q->Nz, Ny = q->Ny;
     double* evp = ev.as<double>() + ((size_t)slot * 3 + e) * 3 * Nz;
     double* evsp = e == 0 ? evs.as<double>() + (size_t)slot * Ny : nullptr;
-    adj_capture_kernel<<<blocks(std::max(Nz, Ny), 128), 128, 0, q->sbp.stream>>>(
-        y, q->fp.psi_off, q->slipVel.as<double>(), q->tauQSP.as<double>(), q->u.as<double>(), Ny, Nz, evp, evsp);
+    chain_launch(adj_capture_kernel, blocks(std::max(Nz, Ny), 128), 128, 0, q->sbp.stream, y, q->fp.psi_off,
+                 q->slipVel.as<double>(), q->tauQSP.as<double>(), q->u.as<double>(), Ny, Nz, evp, evsp);
     SCY_LAUNCH_CHECK();
   }
   return SCY_OK;
@@ -315,11 +324,10 @@ int AdjointContext::forward(double* J, int keep_checkpoints) {
     SCY_CUDA_TRY(cudaMemcpyAsync(var, hi, nv * 8, cudaMemcpyDeviceToDevice, s));
     t = t + dt;
     SCY_TRY(eval(t, var, f0, 0, 0, 0));
-    adj_misfit_kernel<<<1, 256, 0, s>>>(q->slipVel.as<double>(), q->u.as<double>(), Ny, Nz,
-                                        have_targets ? tgt_s.as<double>() + (size_t)n * Ny : nullptr,
-                                        have_targets ? tgt_v.as<double>() + (size_t)n * Nz : nullptr, w_s, w_v,
-                                        obs_s.as<double>() + (size_t)n * Ny, obs_v.as<double>() + (size_t)n * Nz,
-                                        Jn.as<double>() + n);
+    chain_launch(adj_misfit_kernel, 1, 256, 0, s, q->slipVel.as<double>(), q->u.as<double>(), Ny, Nz,
+                 have_targets ? tgt_s.as<double>() + (size_t)n * Ny : nullptr,
+                 have_targets ? tgt_v.as<double>() + (size_t)n * Nz : nullptr, w_s, w_v,
+                 obs_s.as<double>() + (size_t)n * Ny, obs_v.as<double>() + (size_t)n * Nz, Jn.as<double>() + n);
     SCY_LAUNCH_CHECK();
   }
   SCY_TRY(q->read_flags());
@@ -370,16 +378,16 @@ int AdjointContext::vjp(long slot, int e, const double* lam_f, double* lam_y, in
   const LevelDev<double>& L = q->sbp.fine->dev;
   const double* evp = ev.as<double>() + ((size_t)slot * 3 + e) * 3 * Nz;
   const bool mf = with_misfit && have_targets;
-  adj_fault_kernel<<<blocks(Nz, 128), 128, 0, s>>>(evp, q->fp, lam_f,
-                                                   mf ? tgt_v.as<double>() + (size_t)step * Nz : nullptr, w_v, lam_y,
-                                                   ltau.as<double>(), grad.as<double>());
+  chain_launch(adj_fault_kernel, blocks(Nz, 128), 128, 0, s, evp, q->fp, lam_f,
+               mf ? tgt_v.as<double>() + (size_t)step * Nz : nullptr, w_v, lam_y, ltau.as<double>(),
+               grad.as<double>());
   SCY_LAUNCH_CHECK();
   SCY_CUDA_TRY(cudaMemsetAsync(lu.p, 0, N * 8, s));
-  adj_tau_scatter_kernel<<<blocks(Nz, 128), 128, 0, s>>>(L, ltau.as<double>(), lu.as<double>());
+  chain_launch(adj_tau_scatter_kernel, blocks(Nz, 128), 128, 0, s, L, ltau.as<double>(), lu.as<double>());
   SCY_LAUNCH_CHECK();
   if (mf) {
-    adj_surf_kernel<<<blocks(Ny, 128), 128, 0, s>>>(evs.as<double>() + (size_t)slot * Ny,
-                                                    tgt_s.as<double>() + (size_t)step * Ny, w_s, Ny, Nz, lu.as<double>());
+    chain_launch(adj_surf_kernel, blocks(Ny, 128), 128, 0, s, evs.as<double>() + (size_t)slot * Ny,
+                 tgt_s.as<double>() + (size_t)step * Ny, w_s, Ny, Nz, lu.as<double>());
     SCY_LAUNCH_CHECK();
   }
   // A w = lu (A is symmetric: the adjoint solve is a forward solve)
@@ -391,7 +399,7 @@ int AdjointContext::vjp(long slot, int e, const double* lam_f, double* lam_y, in
   q->n_solves += 1;
   q->n_solve_its += st.iterations;
   if (q->bcL_from_slip) {
-    adj_bcl_kernel<<<blocks(Nz, 128), 128, 0, s>>>(L, w.as<double>(), 1.0 / q->fts, q->fp.slip_off, lam_y);
+    chain_launch(adj_bcl_kernel, blocks(Nz, 128), 128, 0, s, L, w.as<double>(), 1.0 / q->fts, q->fp.slip_off, lam_y);
     SCY_LAUNCH_CHECK();
   }
   return SCY_OK;
@@ -421,22 +429,22 @@ int AdjointContext::gradient(double* J, double* ga, double* gb, double* gDc) {
       // n+1 (lF0) and its fields the misfit of state n+1
       SCY_TRY(vjp(j + 1, 0, lF0.as<double>(), ly.as<double>(), 1, n));
       // y_{n+1} = y_n + dt/6 f0 + 2dt/3 f1 + dt/6 f2
-      adj_scale_kernel<<<gbk, tb, 0, s>>>(lf0.as<double>(), ly.as<double>(), dt / 6.0, nv);
-      adj_scale_kernel<<<gbk, tb, 0, s>>>(lf1.as<double>(), ly.as<double>(), 2 * dt / 3.0, nv);
-      adj_scale_kernel<<<gbk, tb, 0, s>>>(lf2.as<double>(), ly.as<double>(), dt / 6.0, nv);
+      chain_launch(adj_scale_kernel, gbk, tb, 0, s, lf0.as<double>(), ly.as<double>(), dt / 6.0, nv);
+      chain_launch(adj_scale_kernel, gbk, tb, 0, s, lf1.as<double>(), ly.as<double>(), 2 * dt / 3.0, nv);
+      chain_launch(adj_scale_kernel, gbk, tb, 0, s, lf2.as<double>(), ly.as<double>(), dt / 6.0, nv);
       SCY_LAUNCH_CHECK();
       // f2 = d_dt(k2), k2 = y - dt f0 + 2 dt f1
       SCY_CUDA_TRY(cudaMemsetAsync(lk.p, 0, nv * 8, s));
       SCY_TRY(vjp(j, 2, lf2.as<double>(), lk.as<double>(), 0, 0));
-      adj_axpy_kernel<<<gbk, tb, 0, s>>>(ly.as<double>(), lk.as<double>(), 1.0, nv);
-      adj_axpy_kernel<<<gbk, tb, 0, s>>>(lf0.as<double>(), lk.as<double>(), -dt, nv);
-      adj_axpy_kernel<<<gbk, tb, 0, s>>>(lf1.as<double>(), lk.as<double>(), 2 * dt, nv);
+      chain_launch(adj_axpy_kernel, gbk, tb, 0, s, ly.as<double>(), lk.as<double>(), 1.0, nv);
+      chain_launch(adj_axpy_kernel, gbk, tb, 0, s, lf0.as<double>(), lk.as<double>(), -dt, nv);
+      chain_launch(adj_axpy_kernel, gbk, tb, 0, s, lf1.as<double>(), lk.as<double>(), 2 * dt, nv);
       SCY_LAUNCH_CHECK();
       // f1 = d_dt(k1), k1 = y + dt/2 f0
       SCY_CUDA_TRY(cudaMemsetAsync(lk.p, 0, nv * 8, s));
       SCY_TRY(vjp(j, 1, lf1.as<double>(), lk.as<double>(), 0, 0));
-      adj_axpy_kernel<<<gbk, tb, 0, s>>>(ly.as<double>(), lk.as<double>(), 1.0, nv);
-      adj_axpy_kernel<<<gbk, tb, 0, s>>>(lf0.as<double>(), lk.as<double>(), 0.5 * dt, nv);
+      chain_launch(adj_axpy_kernel, gbk, tb, 0, s, ly.as<double>(), lk.as<double>(), 1.0, nv);
+      chain_launch(adj_axpy_kernel, gbk, tb, 0, s, lf0.as<double>(), lk.as<double>(), 0.5 * dt, nv);
       SCY_LAUNCH_CHECK();
       SCY_CUDA_TRY(cudaMemcpyAsync(lF0.p, lf0.p, nv * 8, cudaMemcpyDeviceToDevice, s));
     }

@@ -57,6 +57,7 @@ __device__ __forceinline__ double stage_time(const double* t, const double* dt, 
 __global__ void b_bc_kernel(const BatchInst* __restrict__ tab, const int* __restrict__ mask,
                             const double* __restrict__ t, const double* __restrict__ dt, int base, double c,
                             int in_slot) {
+  chain_enter();
   const int k = blockIdx.z;
   if (!mask[k]) return;
   const BatchInst& I = tab[k];
@@ -73,6 +74,7 @@ __global__ void b_bc_kernel(const BatchInst* __restrict__ tab, const int* __rest
 // applying the operator.
 __global__ void b_rhs_kernel(LevelDev<double> L, const BatchInst* __restrict__ tab, const int* __restrict__ mask,
                              int in_slot, BatchWork w, int carry) {
+  chain_enter();
   __shared__ double sh[32];
   const int k = blockIdx.z;
   if (!mask[k]) return;
@@ -99,6 +101,7 @@ __global__ void b_rhs_kernel(LevelDev<double> L, const BatchInst* __restrict__ t
 // after that, columns 0..BAND-1 and Nz-BAND..Nz-1 of the rows in between.
 __global__ void b_rhs_frame_kernel(LevelDev<double> L, const BatchInst* __restrict__ tab,
                                    const int* __restrict__ mask, BatchWork w, int nframe, int carry) {
+  chain_enter();
   __shared__ double sh[32];
   const int k = blockIdx.z;
   if (!mask[k]) return;
@@ -129,6 +132,7 @@ __global__ void b_rhs_frame_kernel(LevelDev<double> L, const BatchInst* __restri
 // rz = r.z -> sc[2] (the previous value moves to sc[3])
 template <typename Tz>
 __global__ void b_dot_rz_kernel(const int* __restrict__ mask, BatchWork w, const Tz* __restrict__ z) {
+  chain_enter();
   __shared__ double sh[32];
   const int k = blockIdx.z;
   if (!mask[k]) return;
@@ -202,6 +206,7 @@ __global__ void __launch_bounds__(XT) b_cross_kernel(const double* __restrict__ 
                                                       const BatchInst* __restrict__ tab, const int* __restrict__ mask,
                                                       BatchWork w, const Tz* __restrict__ zv, int first, int pi,
                                                       int mixed, int kpb, int store_p = 1) {
+  chain_enter();
   constexpr int NV = (XNS + XT - 1) / XT;  // staged values per thread
   extern __shared__ __align__(16) unsigned char xsm[];
   __shared__ double red[XKPB][XW];  // warp sums by instance
@@ -425,6 +430,7 @@ __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, c
                                                      const int* __restrict__ mask, BatchWork w,
                                                      const Tz* __restrict__ zv, int first, int pi, int mixed,
                                                      int store_p, MarchPlan p) {
+  chain_enter();
   __shared__ double xs[RPT > 0 ? full_smem_values<RPT>() : kMarchWarps * kMarchSmem];
   __shared__ double cs[2][8 * RPT + 1][TZ];  // contributions by node of the tile
   const int k = blockIdx.z;
@@ -547,7 +553,8 @@ static void launch_full(const BatchGroup& g, int shape, const BatchInst* tab, co
   const MarchPlan p = march_plan(g.L, kFullChunks[shape]);
   const dim3 grid = rpt ? dim3((g.Nz + TZ - 1) / TZ, (g.Ny + 8 * rpt - 1) / (8 * rpt), g.K) : dim3(p.blocks, 1, g.K);
 #define SCY_FULL_LAUNCH(R, M) \
-  b_full_kernel<MODE, Tz, R, M><<<grid, 256, 0, g.stream>>>(g.L, tab, mask, g.w, zv, first, pi, mixed, store_p, p)
+  launch(g.chain, b_full_kernel<MODE, Tz, R, M>, grid, 256, 0, g.stream, g.L, tab, mask, g.w, zv, first, pi, mixed,  \
+         store_p, p)
   switch (shape) {
     case 0: SCY_FULL_LAUNCH(1, 1); break;
     case 1: SCY_FULL_LAUNCH(2, 1); break;
@@ -562,6 +569,7 @@ static void launch_full(const BatchGroup& g, int shape, const BatchInst* tab, co
 // partials in tile order, and its test; status bit 1: residual above
 // max(rtol |rhs|, atol); bit 2: non-finite
 __global__ void b_partials_verify_kernel(const int* __restrict__ mask, BatchWork w, int n, double rtol, double atol) {
+  chain_enter();
   __shared__ double sh[32];
   const int k = blockIdx.x;
   if (!mask[k]) return;
@@ -582,6 +590,7 @@ __global__ void b_partials_verify_kernel(const int* __restrict__ mask, BatchWork
 // sc[16 k + slot] = sum of the instance's first n partials (of w.partials,
 // or of w.partials2 when second is set), in tile order
 __global__ void b_partials_kernel(const int* __restrict__ mask, BatchWork w, int n, int slot, int second = 0) {
+  chain_enter();
   __shared__ double sh[32];
   const int k = blockIdx.x;
   if (!mask[k]) return;
@@ -596,6 +605,7 @@ __global__ void b_partials_kernel(const int* __restrict__ mask, BatchWork w, int
 // was not stored and is z (the first iteration); last: r is only summed
 __global__ void b_update_kernel(const BatchInst* __restrict__ tab, const int* __restrict__ mask, BatchWork w, int pi,
                                 int mixed, int pz, int last) {
+  chain_enter();
   __shared__ double sh[32];
   const int k = blockIdx.z;
   if (!mask[k]) return;
@@ -627,6 +637,7 @@ __global__ void b_update_kernel(const BatchInst* __restrict__ tab, const int* __
 
 // status bit 1: residual above max(rtol |rhs|, atol); bit 2: non-finite
 __global__ void b_verify_kernel(const int* __restrict__ mask, BatchWork w, double rtol, double atol) {
+  chain_enter();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= w.K || !mask[k]) return;
   const double* sc = w.sc + 16 * k;
@@ -638,6 +649,7 @@ __global__ void b_verify_kernel(const int* __restrict__ mask, BatchWork w, doubl
 
 template <typename T>
 __global__ void b_scale_kernel(T* __restrict__ x, const T* __restrict__ s, long N) {
+  chain_enter();
   const long off = (long)blockIdx.z * N;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N; i += (long)gridDim.x * blockDim.x)
     x[off + i] *= s[i];
@@ -646,6 +658,7 @@ __global__ void b_scale_kernel(T* __restrict__ x, const T* __restrict__ s, long 
 // the caller's array <-> the instances' vectors, one segment per instance
 // (blockIdx.y): scatter into the instances, or gather from them
 __global__ void b_io_kernel(const IoSeg* __restrict__ seg, double* __restrict__ stage, int gather) {
+  chain_enter();
   const IoSeg g = seg[blockIdx.y];
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < g.n; i += (long)gridDim.x * blockDim.x) {
     if (gather)
@@ -660,6 +673,7 @@ __global__ void b_io_kernel(const IoSeg* __restrict__ seg, double* __restrict__ 
 // the material's sxy there (power law)
 __global__ void b_fault_kernel(LevelDev<double> L, const BatchInst* __restrict__ tab, const int* __restrict__ mask,
                                int in_slot, int out_slot) {
+  chain_enter();
   const int k = blockIdx.z;
   if (!mask[k]) return;
   const BatchInst& I = tab[k];
@@ -673,6 +687,7 @@ __global__ void b_fault_kernel(LevelDev<double> L, const BatchInst* __restrict__
 // power law: strains, stresses, viscosity and viscous strain rates per node
 __global__ void b_pl_rates_kernel(LevelDev<double> L, const BatchInst* __restrict__ tab, const int* __restrict__ mask,
                                   int in_slot, int out_slot, long N) {
+  chain_enter();
   const int k = blockIdx.z;
   if (!mask[k]) return;
   const BatchInst& I = tab[k];
@@ -706,6 +721,7 @@ struct BCombo {
 
 __global__ void b_combine_kernel(const BatchInst* __restrict__ tab, const int* __restrict__ mask,
                                  const double* __restrict__ dt, int base, int out_slot, BCombo cb) {
+  chain_enter();
   const int k = blockIdx.z;
   if (!mask[k]) return;
   const BatchInst& I = tab[k];
@@ -730,6 +746,7 @@ __global__ void b_combine_kernel(const BatchInst* __restrict__ tab, const int* _
 }
 
 __global__ void b_copy_kernel(const BatchInst* __restrict__ tab, const int* __restrict__ mask) {
+  chain_enter();
   const int k = blockIdx.z;
   if (!mask[k]) return;
   const BatchInst& I = tab[k];
@@ -740,6 +757,7 @@ __global__ void b_copy_kernel(const BatchInst* __restrict__ tab, const int* __re
 // per (key, instance): sum (lo-hi)^2, sum hi^2, max |lo-hi|/hi -> err[16 g + 3 key ..]
 __global__ void b_error_kernel(const BatchInst* __restrict__ tab, const int* __restrict__ mask, int base,
                                double* __restrict__ err) {
+  chain_enter();
   __shared__ double sh[32];
   const int k = blockIdx.z, key = blockIdx.x;
   if (!mask[k]) return;
@@ -777,6 +795,7 @@ __global__ void b_error_kernel(const BatchInst* __restrict__ tab, const int* __r
 
 // fault flags and solve status of every instance of the group -> err[16 g + 14, 15], cleared
 __global__ void b_status_kernel(const BatchInst* __restrict__ tab, BatchWork w, int base, double* __restrict__ err) {
+  chain_enter();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= w.K) return;
   err[16L * (base + k) + 14] = (double)atomicExch(tab[k].flags, 0u);
@@ -1034,7 +1053,7 @@ int BatchContext::create(int n_inst, const char* const* paths, const scy_solve_o
 int BatchContext::set_states(const double* host) {
   SCY_CUDA_TRY(cudaMemcpyAsync(io.p, host, (size_t)io_states * sizeof(double), cudaMemcpyHostToDevice, stream));
   const dim3 gr((unsigned)std::min((io_maxn + 255) / 256, 64L), (unsigned)n);
-  b_io_kernel<<<gr, 256, 0, stream>>>(io_seg.as<IoSeg>(), io.as<double>(), 0);
+  launch(false, b_io_kernel, gr, 256, 0, stream, io_seg.as<IoSeg>(), io.as<double>(), 0);
   SCY_LAUNCH_CHECK();
   SCY_CUDA_TRY(cudaStreamSynchronize(stream));
   return SCY_OK;
@@ -1047,7 +1066,7 @@ int BatchContext::get_fault_field(int field, double* host) {
     return SCY_ERR_ARG;
   }
   const dim3 gr((unsigned)std::min((io_maxn + 255) / 256, 64L), (unsigned)n);
-  b_io_kernel<<<gr, 256, 0, stream>>>(io_seg.as<IoSeg>() + (size_t)(1 + field) * n, io.as<double>(), 1);
+  launch(false, b_io_kernel, gr, 256, 0, stream, io_seg.as<IoSeg>() + (size_t)(1 + field) * n, io.as<double>(), 1);
   SCY_LAUNCH_CHECK();
   SCY_CUDA_TRY(cudaMemcpyAsync(host, io.p, (size_t)io_fault * sizeof(double), cudaMemcpyDeviceToHost, stream));
   SCY_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -1069,6 +1088,10 @@ int BatchContext::setup_group(int base, int K) {
   g.fd = q0.sbp.fd;
   g.L = q0.sbp.fine->dev;
   const long KN = (long)g.K * g.N;
+  // one group (one stream) of few nodes: a step of 7 x 129 x 97 takes 266 us
+  // chained and 282 not, 8 x 201 x 201 337 and 341, 32 x 129 x 129 413 and
+  // 413, 16 x 201 x 201 403 and 396, 4 x 401 x 401 402 and 391
+  g.chain = K == n && KN <= 400000;
   for (auto& v : g.vec) {
     SCY_TRY(v.alloc((size_t)KN * 8));
     SCY_CUDA_TRY(cudaMemset(v.p, 0, (size_t)KN * 8));
@@ -1188,6 +1211,7 @@ int BatchContext::setup_group(int base, int K) {
     {
       const int S = zt_planes, Nz = g.Nz;
       SCY_TRY(g.zx.alloc(S, (int)rowsT, Nz, 128));
+      g.zx.chain = g.zx16.chain = g.chain;
       SCY_TRY(g.zw1.alloc_weights(S, Nz, Nz));
       SCY_TRY(g.zw2.alloc_weights(S, Nz, Nz));
       std::vector<double> vz((size_t)Nz * Nz), vzt((size_t)Nz * Nz);
@@ -1243,7 +1267,7 @@ int BatchContext::setup_group(int base, int K) {
 int BatchContext::launch_ysolve(BatchGroup& g, int variant) {
   FDPrecond& F = *g.fd;
   if (variant >= 6)
-    return F.yp.solve(g.t1p.as<double>(), g.K, variant - 6, g.w.status, g.stream, sweep_polls, sweep_drop);
+    return F.yp.solve(g.t1p.as<double>(), g.K, variant - 6, g.w.status, g.stream, g.chain, sweep_polls, sweep_drop);
   const int Ny = g.Ny, Nz = g.Nz, K = g.K;
   const bool f32 = precision != SCY_PREC_FP64;
   const int sm = ys_smem_bytes(f32 ? 4 : 8);
@@ -1252,14 +1276,12 @@ int BatchContext::launch_ysolve(BatchGroup& g, int variant) {
   do {                                                                                                              \
     constexpr int B = 2 * (I) * (W);                                                                                \
     const dim3 grid((Nz + YS_C - 1) / YS_C, (K + B - 1) / B);                                                      \
-    if (f32)                                                                                                        \
-      b_ysolve_tma_kernel<float, I, W><<<grid, 32 * W, sm, g.stream>>>(g.mLcol32, g.mLrow32, M32,                  \
-                                                                       g.t1pf.as<float>(), Ny, Nz, F.Nzp, K,        \
-                                                                       g.w.status, sweep_polls, sweep_drop);        \
-    else                                                                                                            \
-      b_ysolve_tma_kernel<double, I, W><<<grid, 32 * W, sm, g.stream>>>(g.mLcol, g.mLrow, M64, g.t1p.as<double>(),  \
-                                                                        Ny, Nz, F.Nzp, K, g.w.status, sweep_polls,  \
-                                                                        sweep_drop);                                \
+    if (f32)                                                                                                      \
+      launch(g.chain, b_ysolve_tma_kernel<float, I, W>, grid, 32 * W, sm, g.stream, g.mLcol32, g.mLrow32, M32,    \
+             g.t1pf.as<float>(), Ny, Nz, F.Nzp, K, g.w.status, sweep_polls, sweep_drop);                          \
+    else                                                                                                          \
+      launch(g.chain, b_ysolve_tma_kernel<double, I, W>, grid, 32 * W, sm, g.stream, g.mLcol, g.mLrow, M64,       \
+             g.t1p.as<double>(), Ny, Nz, F.Nzp, K, g.w.status, sweep_polls, sweep_drop);                          \
   } while (0)
   static_assert(2 * 2 * 2 == YS_B && 2 * 4 * 1 == YS_B && 2 * 1 * 4 == YS_B, "sweep variants 0-2 serve YS_B instances");
   if (variant == 1)
@@ -1316,11 +1338,11 @@ int BatchContext::autotune(BatchGroup& g) {
     int rc = timed(
         [&]() -> int {
           if (mixed)
-            b_cross_kernel<1, float><<<tg, XT, xs_smem_bytes(1, 4), g.stream>>>(C, g.Ny, g.Nz, tab, mask, g.w, g.w.z32,
-                                                                                1, 0, mixed, kpb, 1);
+            launch(g.chain, b_cross_kernel<1, float>, tg, XT, xs_smem_bytes(1, 4), g.stream, C, g.Ny, g.Nz, tab, mask,
+                   g.w, g.w.z32, 1, 0, mixed, kpb, 1);
           else
-            b_cross_kernel<1, double><<<tg, XT, xs_smem_bytes(1, 8), g.stream>>>(C, g.Ny, g.Nz, tab, mask, g.w, g.w.z,
-                                                                                 1, 0, mixed, kpb, 1);
+            launch(g.chain, b_cross_kernel<1, double>, tg, XT, xs_smem_bytes(1, 8), g.stream, C, g.Ny, g.Nz, tab,
+                   mask, g.w, g.w.z, 1, 0, mixed, kpb, 1);
           SCY_LAUNCH_CHECK();
           return SCY_OK;
         },
@@ -1443,6 +1465,7 @@ int BatchContext::autotune(BatchGroup& g) {
         g.zw2 = std::move(g.zw2_16);
       } else {
         g.zx16 = OzkOperand();
+        g.zx.chain = g.chain;
         g.zw1_16 = OzkOperand();
         g.zw2_16 = OzkOperand();
       }
@@ -1568,7 +1591,7 @@ int BatchContext::fd_apply(BatchGroup& g) {
                              g.w.t1f, Nz));
     SCY_BLAS_TRY(cublasSgemmStridedBatched(g.blas, CUBLAS_OP_N, CUBLAS_OP_N, Nz, Ny, Ny, &one, g.w.t1f, Nz, N, vy,
                                            Ny, 0, &zero, g.w.t2f, Nz, N, K));
-    b_scale_kernel<float><<<sg, TB, 0, g.stream>>>(g.w.t2f, F.inv_lam32.as<float>(), N);
+    launch(g.chain, b_scale_kernel<float>, sg, TB, 0, g.stream, g.w.t2f, F.inv_lam32.as<float>(), N);
     SCY_LAUNCH_CHECK();
     SCY_BLAS_TRY(cublasSgemmStridedBatched(g.blas, CUBLAS_OP_N, CUBLAS_OP_T, Nz, Ny, Ny, &one, g.w.t2f, Nz, N, vy,
                                            Ny, 0, &zero, g.w.t1f, Nz, N, K));
@@ -1583,7 +1606,7 @@ int BatchContext::fd_apply(BatchGroup& g) {
                              g.w.t1, Nz));
     SCY_BLAS_TRY(cublasDgemmStridedBatched(g.blas, CUBLAS_OP_N, CUBLAS_OP_N, Nz, Ny, Ny, &one, g.w.t1, Nz, N, vy, Ny,
                                            0, &zero, g.w.t2, Nz, N, K));
-    b_scale_kernel<double><<<sg, TB, 0, g.stream>>>(g.w.t2, F.inv_lam.as<double>(), N);
+    launch(g.chain, b_scale_kernel<double>, sg, TB, 0, g.stream, g.w.t2, F.inv_lam.as<double>(), N);
     SCY_LAUNCH_CHECK();
     SCY_BLAS_TRY(cublasDgemmStridedBatched(g.blas, CUBLAS_OP_N, CUBLAS_OP_T, Nz, Ny, Ny, &one, g.w.t2, Nz, N, vy, Ny,
                                            0, &zero, g.w.t1, Nz, N, K));
@@ -1622,7 +1645,7 @@ int BatchContext::solve_refine(BatchGroup& g, const int* mask, int its_now, int 
     SCY_LAUNCH_CHECK();
     SCY_TRY(prof_end(g.stream, pa, PROF_MATVEC, nact * g.N * 40.0));
   }
-  b_partials_verify_kernel<<<g.K, 256, 0, g.stream>>>(mask, g.w, ntiles, rtol, atol);
+  launch(g.chain, b_partials_verify_kernel, g.K, 256, 0, g.stream, mask, g.w, ntiles, rtol, atol);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -1646,11 +1669,11 @@ int BatchContext::solve(BatchGroup& g, const int* mask, int its_now) {
   if (sep)
     launch_full<0, double>(g, shape, tab, mask, (const double*)nullptr, 0, 0, mixed, 0);
   else
-    b_cross_kernel<0, double><<<tg, XT, xs_smem_bytes(0, 8), g.stream>>>(C, g.Ny, g.Nz, tab, mask, g.w, nullptr, 0,
-                                                                         0, mixed, g.kpb);
+    launch(g.chain, b_cross_kernel<0, double>, tg, XT, xs_smem_bytes(0, 8), g.stream, C, g.Ny, g.Nz, tab, mask, g.w,
+           nullptr, 0, 0, mixed, g.kpb, 1);
   SCY_LAUNCH_CHECK();
   SCY_TRY(prof_end(g.stream, pa, PROF_RESIDUAL, coef_b + nact * g.N * (24.0 + (mixed ? 4 : 0))));
-  b_partials_kernel<<<g.K, 256, 0, g.stream>>>(mask, g.w, ntiles, 5);
+  launch(g.chain, b_partials_kernel, g.K, 256, 0, g.stream, mask, g.w, ntiles, 5, 0);
   SCY_LAUNCH_CHECK();
   int pi = 0;
   for (int it = 1; it <= its_now; ++it) {
@@ -1660,9 +1683,9 @@ int BatchContext::solve(BatchGroup& g, const int* mask, int its_now) {
     SCY_TRY(fd_apply(g));
     if (!first) {
       if (mixed)
-        b_dot_rz_kernel<float><<<ng, TB, 0, g.stream>>>(mask, g.w, g.w.z32);
+        launch(g.chain, b_dot_rz_kernel<float>, ng, TB, 0, g.stream, mask, g.w, g.w.z32);
       else
-        b_dot_rz_kernel<double><<<ng, TB, 0, g.stream>>>(mask, g.w, g.w.z);
+        launch(g.chain, b_dot_rz_kernel<double>, ng, TB, 0, g.stream, mask, g.w, g.w.z);
       SCY_LAUNCH_CHECK();
     }
     SCY_TRY(prof_begin(g.stream, &pa));
@@ -1671,26 +1694,26 @@ int BatchContext::solve(BatchGroup& g, const int* mask, int its_now) {
     else if (sep)
       launch_full<1, double>(g, shape, tab, mask, g.w.z, first, pi, mixed, store_p);
     else if (mixed)
-      b_cross_kernel<1, float><<<tg, XT, xs_smem_bytes(1, 4), g.stream>>>(C, g.Ny, g.Nz, tab, mask, g.w, g.w.z32, first,
-                                                                           pi, mixed, g.kpb, store_p);
+      launch(g.chain, b_cross_kernel<1, float>, tg, XT, xs_smem_bytes(1, 4), g.stream, C, g.Ny, g.Nz, tab, mask, g.w,
+             g.w.z32, first, pi, mixed, g.kpb, store_p);
     else
-      b_cross_kernel<1, double><<<tg, XT, xs_smem_bytes(1, 8), g.stream>>>(C, g.Ny, g.Nz, tab, mask, g.w, g.w.z, first,
-                                                                            pi, mixed, g.kpb, store_p);
+      launch(g.chain, b_cross_kernel<1, double>, tg, XT, xs_smem_bytes(1, 8), g.stream, C, g.Ny, g.Nz, tab, mask, g.w,
+             g.w.z, first, pi, mixed, g.kpb, store_p);
     SCY_LAUNCH_CHECK();
     // z, q, p when stored, and r (first iteration) or p_old (later ones)
     SCY_TRY(prof_end(g.stream, pa, PROF_MATVEC,
                      coef_b + nact * g.N * ((mixed ? 4.0 : 8.0) + 8.0 + (store_p ? 8.0 : 0.0) + 8.0)));
-    b_partials_kernel<<<g.K, 256, 0, g.stream>>>(mask, g.w, ntiles, 4);
+    launch(g.chain, b_partials_kernel, g.K, 256, 0, g.stream, mask, g.w, ntiles, 4, 0);
     SCY_LAUNCH_CHECK();
     if (first) {
-      b_partials_kernel<<<g.K, 256, 0, g.stream>>>(mask, g.w, ntiles, 2, 1);
+      launch(g.chain, b_partials_kernel, g.K, 256, 0, g.stream, mask, g.w, ntiles, 2, 1);
       SCY_LAUNCH_CHECK();
     }
-    b_update_kernel<<<ng, TB, 0, g.stream>>>(tab, mask, g.w, pi, mixed, store_p ? 0 : 1, last);
+    launch(g.chain, b_update_kernel, ng, TB, 0, g.stream, tab, mask, g.w, pi, mixed, store_p ? 0 : 1, last);
     SCY_LAUNCH_CHECK();
     pi ^= 1;
   }
-  b_verify_kernel<<<(g.K + 127) / 128, 128, 0, g.stream>>>(mask, g.w, rtol, atol);
+  launch(g.chain, b_verify_kernel, (g.K + 127) / 128, 128, 0, g.stream, mask, g.w, rtol, atol);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -1701,14 +1724,14 @@ int BatchContext::d_dt(BatchGroup& g, const int* mask, double c, int in_slot, in
   const BatchInst* tab = g.tab.as<BatchInst>();
   const dim3 fg((g.Nz + 63) / 64, 1, g.K);
   const dim3 ng(node_blocks(g.N), 1, g.K);
-  b_bc_kernel<<<fg, 64, 0, g.stream>>>(tab, mask, d_t(), d_dt_(), g.base, c, in_slot);
+  launch(g.chain, b_bc_kernel, fg, 64, 0, g.stream, tab, mask, d_t(), d_dt_(), g.base, c, in_slot);
   SCY_LAUNCH_CHECK();
   if (!pl && g.Ny > 2 * BAND && g.Nz > 2 * BAND) {
     const int nframe = 2 * BAND * g.Nz + (g.Ny - 2 * BAND) * 2 * BAND;
     const dim3 rg((nframe + TB - 1) / TB < 64 ? (nframe + TB - 1) / TB : 64, 1, g.K);
-    b_rhs_frame_kernel<<<rg, TB, 0, g.stream>>>(g.L, tab, mask, g.w, nframe, carry);
+    launch(g.chain, b_rhs_frame_kernel, rg, TB, 0, g.stream, g.L, tab, mask, g.w, nframe, carry);
   } else {
-    b_rhs_kernel<<<ng, TB, 0, g.stream>>>(g.L, tab, mask, in_slot, g.w, carry);
+    launch(g.chain, b_rhs_kernel, ng, TB, 0, g.stream, g.L, tab, mask, in_slot, g.w, carry);
   }
   SCY_LAUNCH_CHECK();
   if (g.refine)
@@ -1716,10 +1739,11 @@ int BatchContext::d_dt(BatchGroup& g, const int* mask, double c, int in_slot, in
   else
     SCY_TRY(solve(g, mask, its_now));
   if (pl) {
-    b_pl_rates_kernel<<<ng, TB, 0, g.stream>>>(g.L, tab, mask, in_slot, out_slot, g.N);
+    launch(g.chain, b_pl_rates_kernel, ng, TB, 0, g.stream, g.L, tab, mask, in_slot, out_slot, g.N);
     SCY_LAUNCH_CHECK();
   }
-  b_fault_kernel<<<dim3((4 * g.Nz + 63) / 64, 1, g.K), 64, 0, g.stream>>>(g.L, tab, mask, in_slot, out_slot);
+  launch(g.chain, b_fault_kernel, dim3((4 * g.Nz + 63) / 64, 1, g.K), 64, 0, g.stream, g.L, tab, mask, in_slot,
+         out_slot);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -1736,7 +1760,7 @@ int BatchContext::combine(BatchGroup& g, const int* mask, int out_slot, std::ini
   for (double v : den) cb.den[j++] = v;
   long nv = q(g.base).nvar;
   const dim3 gr(node_blocks(nv), 1, g.K);
-  b_combine_kernel<<<gr, TB, 0, g.stream>>>(g.tab.as<BatchInst>(), mask, d_dt_(), g.base, out_slot, cb);
+  launch(g.chain, b_combine_kernel, gr, TB, 0, g.stream, g.tab.as<BatchInst>(), mask, d_dt_(), g.base, out_slot, cb);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -1750,7 +1774,7 @@ int BatchContext::enqueue_group(BatchGroup& g, int its_now, int phases) {
   const int* mr = d_run(g);
   const long nv = q(g.base).nvar;
   if (phases & 1) {
-    b_copy_kernel<<<dim3(node_blocks(nv), 1, g.K), TB, 0, g.stream>>>(tab, mc);
+    launch(g.chain, b_copy_kernel, dim3(node_blocks(nv), 1, g.K), TB, 0, g.stream, tab, mc);
     SCY_LAUNCH_CHECK();
     SCY_TRY(d_dt(g, ma, 0.0, V_VAR, V_DVAR, its_now, 1));
   }
@@ -1781,10 +1805,10 @@ int BatchContext::enqueue_group(BatchGroup& g, int its_now, int phases) {
     SCY_TRY(combine(g, mr, V_HI, {V_DVAR, V_F3, V_F4, V_F5, V_F6}, {b1, b3, b4, b5, b6}, {1.0, 1.0, 1.0, 1.0, 1.0}));
   }
   if (phases & 2) {
-    b_error_kernel<<<dim3(4, 1, g.K), 1024, 0, g.stream>>>(tab, mr, g.base, err.as<double>());
+    launch(g.chain, b_error_kernel, dim3(4, 1, g.K), 1024, 0, g.stream, tab, mr, g.base, err.as<double>());
     SCY_LAUNCH_CHECK();
   }
-  b_status_kernel<<<(g.K + 127) / 128, 128, 0, g.stream>>>(tab, g.w, g.base, err.as<double>());
+  launch(g.chain, b_status_kernel, (g.K + 127) / 128, 128, 0, g.stream, tab, g.w, g.base, err.as<double>());
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }

@@ -71,6 +71,7 @@ struct BatchGroup {
   CUtensorMap mT4, mT2, mT4_32, mT2_32;                 // the transform for 4 and 2 instances per block
   DevBuf planes;  // the operator's 33 cross-stencil coefficient planes (build_cross_planes)
   int kpb = 1;    // instances per block of the operator kernels (autotuned at set-up)
+  bool chain = false;  // launches chained (launch() in common.cuh)
   int ys_variant = 0;  // chains per lane x warps per block of the banded sweeps (autotuned)
   int zt_pair = 0;  // z-transform products: 0 one CTA per tile, 1 two CTAs per SM, 2 persistent, 3 narrow tiles (autotuned)
   int zt_bf16 = 0;  // z-transform digits in bf16 (kind::f16) instead of 8-bit integers (autotuned)

@@ -43,6 +43,47 @@ void count_launches(long long n);  // n kernels launched at once (a CUDA graph r
     if (s_ != SCY_OK) return s_;                                               \
   } while (0)
 
+// Launches of a chain of short kernels: the next kernel's blocks are placed on
+// the SMs as soon as every block of the running one has started
+// (programmatic stream serialisation), and wait there in chain_enter() until
+// all of its work is done and visible, so that neither its launch nor the
+// ramp of its blocks adds to the chain.  Every kernel that is launched this
+// way calls chain_enter() before it touches memory that an earlier kernel
+// reads or writes, in every thread; so each kernel's completion implies that
+// of all before it.  After an ordinary launch chain_enter() does nothing.
+//
+// A stage of the quasi-dynamic step is 10 launches of 2 to 12 us with 1 to 3
+// us between them: four steps at 101 x 101 take 848 us chained and 1079 not,
+// at 401 x 401 1262 and 1440, a multigrid solve at 257 x 385 (302 launches)
+// 1804 and 2278.  chain = false where it does not pay: kernels that fill the
+// GPU several times over (at 32 x 401 x 401 the waiting blocks take places on
+// some SMs first and the next kernel starts uneven: 1275 us a step chained,
+// 1204 not) and launches on several streams at once (three groups of a
+// power-law batch: 1200 and 1145), where they take the other streams' places.
+__device__ __forceinline__ void chain_enter() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline void launch(bool chain, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = chain ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);  // an error stays for SCY_LAUNCH_CHECK
+}
+template <typename... P, typename... A>
+inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  launch(true, kernel, grid, block, smem, s, static_cast<A&&>(args)...);
+}
+
 constexpr int kBlock = 256;
 constexpr int kNumSMs = 148;
 

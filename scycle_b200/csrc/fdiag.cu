@@ -134,10 +134,12 @@ int gen_eig(std::vector<double>& negL, const std::vector<double>& M, int n, std:
 
 template <typename T>
 __global__ void scale_by_kernel(T* __restrict__ x, const T* __restrict__ s, long n) {
+  chain_enter();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) x[i] *= s[i];
 }
 
 __global__ void to_f32_kernel(const double* __restrict__ a, float* __restrict__ b, long n) {
+  chain_enter();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
     b[i] = (float)a[i];
 }
@@ -373,11 +375,11 @@ int FDPrecond::apply(const double* r, double* z, cudaStream_t s, bool chains) {
     SCY_TRY(ozk_split(zx64, r, Nz, s));
     SCY_TRY(ozk_gemm(zx64, zw1_64, t, Nzp, Nz, s, nullptr, 1, 4u, shape));
     if (yp.T > 0 && !chains) {
-      SCY_TRY(yp.solve(t, 1, 0, ys_status.as<unsigned>(), s));
+      SCY_TRY(yp.solve(t, 1, 0, ys_status.as<unsigned>(), s, true));
     } else {
       // one chain a lane and one warp a block: fewest instructions a row
-      b_ysolve_tma_kernel<double, 1, 1><<<dim3((Nz + YS_C - 1) / YS_C, 1), 32, ys_smem_bytes(8), s>>>(
-          mLcol, mLrow, mT, t, Ny, Nz, Nzp, 1, ys_status.as<unsigned>());
+      chain_launch(b_ysolve_tma_kernel<double, 1, 1>, dim3((Nz + YS_C - 1) / YS_C, 1), 32, ys_smem_bytes(8), s, mLcol,
+                   mLrow, mT, t, Ny, Nz, Nzp, 1, ys_status.as<unsigned>(), 1 << 18, 0);
       SCY_LAUNCH_CHECK();
     }
     SCY_TRY(ozk_split(zx64, (const double*)t, Nzp, s));
@@ -397,7 +399,7 @@ int FDPrecond::apply(const double* r, double* z, cudaStream_t s, bool chains) {
   count_launch();
   count_launch();
   long n = (long)Ny * Nz;
-  scale_by_kernel<double><<<grid_for(n), 256, 0, s>>>(b, inv_lam.as<double>(), n);
+  chain_launch(scale_by_kernel<double>, grid_for(n), 256, 0, s, b, inv_lam.as<double>(), n);
   SCY_LAUNCH_CHECK();
   SCY_BLAS_TRY(cublasDgemm(blas, CUBLAS_OP_N, CUBLAS_OP_T, Nz, Ny, Ny, &one, b, Nz, vy, Ny, &zero, a, Nz));
   SCY_BLAS_TRY(cublasDgemm(blas, CUBLAS_OP_N, CUBLAS_OP_N, Nz, Ny, Nz, &one, vz, Nz, a, Nz, &zero, z, Nz));
@@ -412,8 +414,8 @@ int FDPrecond::apply32(const double* r, float* z, cudaStream_t s) {
     const int shape = ozk_narrow_better(kPlanes32, Ny, Nz) ? 3 : 0;
     SCY_TRY(ozk_split(zx32, r, Nz, s));
     SCY_TRY(ozk_gemm(zx32, zw1_32, t, Nzp, Nz, s, nullptr, 1, 4u, shape));
-    b_ysolve_tma_kernel<float, YS_I, YS_W><<<dim3((Nz + YS_C - 1) / YS_C, 1), 32 * YS_W, ys_smem_bytes(4), s>>>(
-        mLcol32, mLrow32, mT32, t, Ny, Nz, Nzp, 1, ys_status.as<unsigned>());
+    chain_launch(b_ysolve_tma_kernel<float, YS_I, YS_W>, dim3((Nz + YS_C - 1) / YS_C, 1), 32 * YS_W, ys_smem_bytes(4),
+                 s, mLcol32, mLrow32, mT32, t, Ny, Nz, Nzp, 1, ys_status.as<unsigned>(), 1 << 18, 0);
     SCY_LAUNCH_CHECK();
     SCY_TRY(ozk_split(zx32, (const float*)t, Nzp, s));
     SCY_TRY(ozk_gemm(zx32, zw2_32, z, Nz, Nz, s, nullptr, 1, 4u, shape));
@@ -426,7 +428,7 @@ int FDPrecond::apply32(const double* r, float* z, cudaStream_t s) {
   const float one = 1.0f, zero = 0.0f;
   long n = (long)Ny * Nz;
   float* rf = r32.as<float>();
-  to_f32_kernel<<<grid_for(n), 256, 0, s>>>(r, rf, n);
+  chain_launch(to_f32_kernel, grid_for(n), 256, 0, s, r, rf, n);
   SCY_LAUNCH_CHECK();
   float* a = t1f.as<float>();
   float* b = t2f.as<float>();
@@ -436,7 +438,7 @@ int FDPrecond::apply32(const double* r, float* z, cudaStream_t s) {
   SCY_BLAS_TRY(cublasSgemm(blas, CUBLAS_OP_N, CUBLAS_OP_N, Nz, Ny, Ny, &one, a, Nz, vy, Ny, &zero, b, Nz));
   count_launch();
   count_launch();
-  scale_by_kernel<float><<<grid_for(n), 256, 0, s>>>(b, inv_lam32.as<float>(), n);
+  chain_launch(scale_by_kernel<float>, grid_for(n), 256, 0, s, b, inv_lam32.as<float>(), n);
   SCY_LAUNCH_CHECK();
   SCY_BLAS_TRY(cublasSgemm(blas, CUBLAS_OP_N, CUBLAS_OP_T, Nz, Ny, Ny, &one, b, Nz, vy, Ny, &zero, a, Nz));
   SCY_BLAS_TRY(cublasSgemm(blas, CUBLAS_OP_N, CUBLAS_OP_N, Nz, Ny, Nz, &one, vz, Nz, a, Nz, &zero, z, Nz));

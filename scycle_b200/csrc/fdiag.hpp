@@ -35,7 +35,7 @@ struct YPart {
   size_t smem_bytes(int shape) const;
   // L: the factors, value k of row i (1 / L_ii, then L(i, i - k)) and mode j at (i * 9 + k) * Nz + j
   int build(const std::vector<double>& L, int Ny, int Nz, int Nzp, cudaStream_t s);
-  int solve(double* t, int K, int shape, unsigned* status, cudaStream_t s, int polls = 1 << 18, int drop = 0) const;
+  int solve(double* t, int K, int shape, unsigned* status, cudaStream_t s, bool chain, int polls = 1 << 18, int drop = 0) const;
 };
 
 struct FDPrecond {

@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(128, PAIR == 1 ? 2 : 1)
     ozk_gemm_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
                     const int* __restrict__ ex, const int* __restrict__ ew, T* __restrict__ D, long ldd, int rows,
                     int cout, int nks, unsigned* __restrict__ status, int rows_per_status, unsigned bit) {
+  chain_enter();
   constexpr int CN = ozk_cn(S, PAIR);
   constexpr int XB = S * OZK_BM * OZK_BK;
   constexpr int WB = S * CN * OZK_BK;
@@ -383,6 +384,7 @@ __global__ void __launch_bounds__(384, 1)
                          const int* __restrict__ ex, const int* __restrict__ ew, T* __restrict__ D, long ldd,
                          int rows, int cout, int nks, int nst, unsigned* __restrict__ status, int rows_per_status,
                          unsigned bit) {
+  chain_enter();
   constexpr int CN = ozk_cn(S, 1);
   constexpr int XB = ozk_pers_x_bytes(S);
   constexpr int WB = ozk_pers_w_bytes(S);
@@ -579,6 +581,7 @@ template <typename Tin, int BF, int NT>
 __global__ void __launch_bounds__(256) ozk_split_kernel(const Tin* __restrict__ X, long ldx, int rows, int K, int Kp,
                                                         int S, unsigned char* __restrict__ dig, long plane,
                                                         int* __restrict__ expo) {
+  chain_enter();
   const int row = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
@@ -693,9 +696,8 @@ int launch_gemm(const OzkOperand& x, const CUtensorMap& wmap, const OzkOperand& 
     if (rc != SCY_OK) return rc;
   }
   const dim3 grid((cout + CN - 1) / CN, (x.rows + OZK_BM - 1) / OZK_BM);
-  ozk_gemm_kernel<S, T, PAIR, BF><<<grid, 128, ozk_smem_bytes(S, PAIR), s>>>(
-      x.map, wmap, x.expo.as<int>(), w.expo.as<int>(), D, ldd, x.rows, cout, x.Kp * x.esz / 32, status,
-      rows_per_status, bit);
+  launch(x.chain, ozk_gemm_kernel<S, T, PAIR, BF>, grid, 128, ozk_smem_bytes(S, PAIR), s, x.map, wmap,
+         x.expo.as<int>(), w.expo.as<int>(), D, ldd, x.rows, cout, x.Kp * x.esz / 32, status, rows_per_status, bit);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -713,8 +715,8 @@ int launch_pers(const OzkOperand& x, const OzkOperand& w, T* D, long ldd, int co
   const long ntiles = (long)((cout + CN - 1) / CN) * ((x.rows + OZK_BM - 1) / OZK_BM);
   const int grid = (int)std::min<long>(ntiles, sm_count());
   const int smem = nkb * ozk_pers_w_bytes(S) + nst * ozk_pers_x_bytes(S) + 1024;
-  ozk_gemm_pers_kernel<S, T, BF><<<grid, 384, smem, s>>>(x.map, w.map_pair, x.expo.as<int>(), w.expo.as<int>(), D,
-                                                         ldd, x.rows, cout, nks, nst, status, rows_per_status, bit);
+  launch(x.chain, ozk_gemm_pers_kernel<S, T, BF>, grid, 384, smem, s, x.map, w.map_pair, x.expo.as<int>(),
+         w.expo.as<int>(), D, ldd, x.rows, cout, nks, nst, status, rows_per_status, bit);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -843,13 +845,13 @@ static void launch_split(OzkOperand& o, const Tin* X, long ldx, cudaStream_t s) 
   unsigned char* d = o.dig.as<unsigned char>();
   int* ex = o.expo.as<int>();
   if (o.Kp <= 128)
-    ozk_split_kernel<Tin, BF, 4><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
+    launch(o.chain, ozk_split_kernel<Tin, BF, 4>, blocks, 256, 0, s, X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
   else if (o.Kp <= 256)
-    ozk_split_kernel<Tin, BF, 8><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
+    launch(o.chain, ozk_split_kernel<Tin, BF, 8>, blocks, 256, 0, s, X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
   else if (o.Kp <= 512)
-    ozk_split_kernel<Tin, BF, 16><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
+    launch(o.chain, ozk_split_kernel<Tin, BF, 16>, blocks, 256, 0, s, X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
   else
-    ozk_split_kernel<Tin, BF, 32><<<blocks, 256, 0, s>>>(X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
+    launch(o.chain, ozk_split_kernel<Tin, BF, 32>, blocks, 256, 0, s, X, ldx, o.rows, o.K, o.Kp, o.S, d, o.plane, ex);
 }
 
 template <typename Tin>

@@ -40,6 +40,7 @@ struct OzkOperand {
   int S = 0, rows = 0, K = 0, Kp = 0, box_rows = 0, box_rows_pair = 0, box_rows_narrow = 0;
   int esz = 1;  // bytes of a digit: 1 (signed 8-bit) or 2 (bf16)
   long plane = 0;  // digits of one plane (rows x Kp)
+  bool chain = true;  // the launches on this row operand are chained (launch() in common.cuh)
   CUtensorMap map, map_pair, map_narrow;
   // box_rows: 128 for the row operand (X), the column tile width of S
   // (ozk_cols_per_tile) for the weights (W); Kp = K rounded up to 32 bytes

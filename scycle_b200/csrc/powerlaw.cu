@@ -28,6 +28,7 @@ namespace scy {
 // computeTotalStrains, computeStresses / computeSDev, computeViscosity and
 // computeViscStrainRates (with computeViscousStrainRateSAT) per node
 __global__ void pl_rates_kernel(PLRatesArgs a) {
+  chain_enter();
   const long N = (long)a.L.Ny * a.L.Nz;
   for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < N; node += (long)gridDim.x * blockDim.x)
     pl_rates_node(a.L, a, node);
@@ -38,6 +39,7 @@ __global__ void pl_fault_kernel(const double* __restrict__ sxy, FaultParams fp, 
                                 double* __restrict__ f, double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                 double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                 unsigned long long* its_total) {
+  chain_enter();
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
   fault_node_update(iz, sxy[iz], fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
@@ -69,18 +71,19 @@ int pl_d_dt(QDContext& q, double t, const double* var, double* f) {
   a.sdev = q.sdev.as<double>();
   a.effVisc = q.effVisc.as<double>();
   return q.solve_stage(t, var, gxy, gxz, [&]() -> int {
-    pl_rates_kernel<<<gb, 256, 0, s>>>(a);
+    chain_launch(pl_rates_kernel, gb, 256, 0, s, a);
     SCY_LAUNCH_CHECK();
     const int tb = 64, fb = (4 * Nz + tb - 1) / tb;
-    pl_fault_kernel<<<fb, tb, 0, s>>>(q.sxy.as<double>(), q.fp, var, f, q.slipVel.as<double>(),
-                                      q.tauQSP.as<double>(), q.tauP.as<double>(), q.strength.as<double>(),
-                                      q.fault_flags(), q.fault_its.as<unsigned long long>());
+    chain_launch(pl_fault_kernel, fb, tb, 0, s, q.sxy.as<double>(), q.fp, var, f, q.slipVel.as<double>(),
+                 q.tauQSP.as<double>(), q.tauP.as<double>(), q.strength.as<double>(), q.fault_flags(),
+                 q.fault_its.as<unsigned long long>());
     SCY_LAUNCH_CHECK();
     return SCY_OK;
   });
 }
 
 __global__ void pl_axpy_kernel(double* __restrict__ x, const double* __restrict__ d, long n) {
+  chain_enter();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) x[i] += d[i];
 }
 
@@ -223,7 +226,7 @@ int QDContext::pl_steady_state(const QDProblem& P, std::vector<double>& psi, std
       }
       ++steps;
       SCY_CUDA_TRY(cudaMemcpyAsync(dkeep.p, dv.p, N * 8, cudaMemcpyDeviceToDevice, s));
-      pl_axpy_kernel<<<grid_for(N), kBlock, 0, s>>>(dv.as<double>(), dcor.as<double>(), N);
+      chain_launch(pl_axpy_kernel, grid_for(N), kBlock, 0, s, dv.as<double>(), dcor.as<double>(), N);
       SCY_LAUNCH_CHECK();
     }
     SCY_TRY(eta.apply(SCY_OP_DY, dv.as<double>(), dgxy.as<double>()));

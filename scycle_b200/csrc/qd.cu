@@ -24,6 +24,7 @@ namespace scy {
 __global__ void qd_bc_kernel(const double* __restrict__ slip, int Nz, double t, double vL, double inv_fts,
                              int bcL_from_slip, int bcR_remote, const double* __restrict__ shift,
                              double* __restrict__ bcL, double* __restrict__ bcR) {
+  chain_enter();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Nz) return;
   if (bcL_from_slip) bcL[i] = slip[i] * inv_fts;
@@ -43,6 +44,7 @@ __global__ void __launch_bounds__(256) qd_rhs_kernel(LevelDev<double> L, const d
                                                      double* __restrict__ rhs, const double* __restrict__ V,
                                                      double* __restrict__ V0, double* partials, unsigned* counter,
                                                      double* norm2) {
+  chain_enter();
   __shared__ double sh[32];
   const int Nz = L.Nz;
   const long N = (long)L.Ny * Nz;
@@ -68,6 +70,7 @@ __global__ void __launch_bounds__(256) qd_rhs_kernel(LevelDev<double> L, const d
 
 // one enqueued solve's scalars (|rhs|^2, r.r, |r0|^2) into its record
 __global__ void qd_record_kernel(const double* __restrict__ sc, double* __restrict__ rec) {
+  chain_enter();
   rec[0] = sc[0];
   rec[1] = sc[1];
   rec[2] = sc[5];
@@ -80,6 +83,7 @@ __global__ void qd_fault_kernel(LevelDev<double> L, const double* __restrict__ u
                                 double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                 double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                 unsigned long long* its_total) {
+  chain_enter();
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
   const double sxy = fault_row_sxy(L, u, iz);
@@ -93,6 +97,7 @@ __global__ void qd_fault_given_tau_kernel(const double* __restrict__ tau_body, F
                                           double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                           double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                           unsigned long long* its_total) {
+  chain_enter();
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
   fault_node_update(iz, tau_body[iz], fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
@@ -100,10 +105,9 @@ __global__ void qd_fault_given_tau_kernel(const double* __restrict__ tau_body, F
 
 int QDContext::fault_d_dt(const double* var, const double* tau_body, double* f) {
   const int tb = 64, gb = (4 * Nz + tb - 1) / tb;
-  qd_fault_given_tau_kernel<<<gb, tb, 0, sbp.stream>>>(tau_body, fp, var, f, slipVel.as<double>(),
-                                                       tauQSP.as<double>(), tauP.as<double>(),
-                                                       strength.as<double>(), flags.as<unsigned>(),
-                                                       fault_its.as<unsigned long long>());
+  chain_launch(qd_fault_given_tau_kernel, gb, tb, 0, sbp.stream, tau_body, fp, var, f, slipVel.as<double>(),
+               tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), flags.as<unsigned>(),
+               fault_its.as<unsigned long long>());
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -112,6 +116,7 @@ int QDContext::fault_d_dt(const double* var, const double* tau_body, double* f) 
 // matrices: out[iz * ld + col] = mu * Dy u at (0, iz); surf[iy * ld + col] = u(iy, 0).
 __global__ void qd_response_column_kernel(LevelDev<double> L, const double* __restrict__ u, double* __restrict__ out,
                                           double* __restrict__ surf, int ld, int col) {
+  chain_enter();
   const int Ny = L.Ny, Nz = L.Nz;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < Nz) {
@@ -135,6 +140,7 @@ __global__ void qd_green_kernel(const double* __restrict__ GL, const double* __r
                                 const double* __restrict__ var, double* __restrict__ f, double* __restrict__ slipVel,
                                 double* __restrict__ tauQSP, double* __restrict__ tauP, double* __restrict__ strength,
                                 double* __restrict__ bcL, unsigned* flags, unsigned long long* its_total) {
+  chain_enter();
   const int Nz = fp.Nz;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= Nz) return;
@@ -154,6 +160,7 @@ __global__ void qd_green_kernel(const double* __restrict__ GL, const double* __r
 __global__ void qd_green_surf_kernel(const double* __restrict__ SL, const double* __restrict__ s1,
                                      const double* __restrict__ ss, double c, int Ny, int Nz,
                                      const double* __restrict__ bcL, double* __restrict__ out) {
+  chain_enter();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= Ny) return;
   const double* row = SL + (long)warp * Nz;
@@ -166,9 +173,8 @@ __global__ void qd_green_surf_kernel(const double* __restrict__ SL, const double
 int qd_green_surf_launch(QDContext& q, double c, double* host_out) {
   cudaStream_t s = q.sbp.stream;
   const int wpb = 4;
-  qd_green_surf_kernel<<<(q.Ny + wpb - 1) / wpb, 32 * wpb, 0, s>>>(q.SL.as<double>(), q.s1.as<double>(),
-                                                                   q.ss.as<double>(), c, q.Ny, q.Nz,
-                                                                   q.bcL.as<double>(), q.sxy.as<double>());
+  chain_launch(qd_green_surf_kernel, (q.Ny + wpb - 1) / wpb, 32 * wpb, 0, s, q.SL.as<double>(), q.s1.as<double>(),
+               q.ss.as<double>(), c, q.Ny, q.Nz, q.bcL.as<double>(), q.sxy.as<double>());
   SCY_LAUNCH_CHECK();
   SCY_CUDA_TRY(cudaMemcpyAsync(host_out, q.sxy.p, (size_t)q.Ny * 8, cudaMemcpyDeviceToHost, s));
   SCY_CUDA_TRY(cudaStreamSynchronize(s));
@@ -181,8 +187,8 @@ int QDContext::full_solve_for_output() {
   ++u_epoch;
   cudaStream_t s = sbp.stream;
   const int tb = 64, gb = (Nz + tb - 1) / tb;
-  qd_bc_kernel<<<gb, tb, 0, s>>>(rk[0].as<double>() + fp.slip_off, Nz, last_t, vL, 1.0 / fts, 0, bcR_remote,
-                                 bcRShift.as<double>(), bcL.as<double>(), bcR.as<double>());
+  chain_launch(qd_bc_kernel, gb, tb, 0, s, rk[0].as<double>() + fp.slip_off, Nz, last_t, vL, 1.0 / fts, 0, bcR_remote,
+               bcRShift.as<double>(), bcL.as<double>(), bcR.as<double>());
   SCY_LAUNCH_CHECK();
   SCY_TRY(sbp.set_rhs(bcL.as<double>(), bcR.as<double>(), bcT.as<double>(), bcB.as<double>(), rhs.as<double>()));
   scy_solve_opts o = solve_opts;
@@ -199,6 +205,7 @@ struct Combo {
 };
 
 __global__ void rk_combine_kernel(double* __restrict__ out, const double* __restrict__ var, Combo cb, long n) {
+  chain_enter();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   double v = cb.c[0] * cb.f[0][i] + var[i];
@@ -218,6 +225,7 @@ enum { RB_FLAGS = 13, RB_SOLVE = 16, RB_SIZE = RB_SOLVE + 3 * 6 };
 
 __global__ void rk_error_kernel(const double* __restrict__ lo, const double* __restrict__ hi, KeyTable kt,
                                 const unsigned* __restrict__ flags, double* __restrict__ out) {
+  chain_enter();
   __shared__ double sh[32];
   const int key = blockIdx.x;
   if (key == 0 && threadIdx.x == 0) out[RB_FLAGS] = (double)(flags[0] | flags[1]);  // read back with the sums
@@ -440,10 +448,10 @@ int QDContext::d_dt(double t, const double* var, double* f) {
     if (!green_ready) SCY_TRY(build_green());
     const double c = bcR_remote ? vL * t * (1.0 / fts) : 0.0;
     const int wpb = 4;
-    qd_green_kernel<<<(Nz + wpb - 1) / wpb, 32 * wpb, 0, s>>>(
-        GL.as<double>(), g1.as<double>(), gs.as<double>(), c, 1.0 / fts, fp, var, f, slipVel.as<double>(),
-        tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), bcL.as<double>(), flags.as<unsigned>(),
-        fault_its.as<unsigned long long>());
+    chain_launch(qd_green_kernel, (Nz + wpb - 1) / wpb, 32 * wpb, 0, s, GL.as<double>(), g1.as<double>(),
+                 gs.as<double>(), c, 1.0 / fts, fp, var, f, slipVel.as<double>(), tauQSP.as<double>(),
+                 tauP.as<double>(), strength.as<double>(), bcL.as<double>(), flags.as<unsigned>(),
+                 fault_its.as<unsigned long long>());
     SCY_LAUNCH_CHECK();
     flags_known = 0;
     last_t = t;
@@ -452,9 +460,9 @@ int QDContext::d_dt(double t, const double* var, double* f) {
   }
   SCY_TRY(solve_stage(t, var, nullptr, nullptr, [&]() -> int {
     const int tb = 64, gb = (4 * Nz + tb - 1) / tb;
-    qd_fault_kernel<<<gb, tb, 0, s>>>(sbp.fine->dev, u.as<double>(), fp, var, f, slipVel.as<double>(),
-                                      tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), fault_flags(),
-                                      fault_its.as<unsigned long long>());
+    chain_launch(qd_fault_kernel, gb, tb, 0, s, sbp.fine->dev, u.as<double>(), fp, var, f, slipVel.as<double>(),
+                 tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), fault_flags(),
+                 fault_its.as<unsigned long long>());
     SCY_LAUNCH_CHECK();
     return SCY_OK;
   }));
@@ -479,11 +487,10 @@ int QDContext::solve_stage(double t, const double* var, const double* gxy, const
   cudaStream_t s = sbp.stream;
   flags_known = 0;
   const int rb = grid_for(N, 256, 592);
-  qd_rhs_kernel<<<rb, 256, 0, s>>>(sbp.fine->dev, var + fp.slip_off, t, vL, 1.0 / fts, bcL_from_slip, bcR_remote,
-                                   bcRShift.as<double>(), bcL.as<double>(), bcR.as<double>(), bcT.as<double>(),
-                                   bcB.as<double>(), gxy, gxz, rhs.as<double>(), slipVel.as<double>(),
-                                   slipVel0.as<double>(), sbp.red.partials.as<double>(),
-                                   sbp.red.counter.as<unsigned>(), sbp.scal.as<double>());
+  chain_launch(qd_rhs_kernel, rb, 256, 0, s, sbp.fine->dev, var + fp.slip_off, t, vL, 1.0 / fts, bcL_from_slip,
+               bcR_remote, bcRShift.as<double>(), bcL.as<double>(), bcR.as<double>(), bcT.as<double>(),
+               bcB.as<double>(), gxy, gxz, rhs.as<double>(), slipVel.as<double>(), slipVel0.as<double>(),
+               sbp.red.partials.as<double>(), sbp.red.counter.as<unsigned>(), sbp.scal.as<double>());
   SCY_LAUNCH_CHECK();
   scy_solve_opts o = solve_opts;
   o.nonzero_guess = 1;  // the previous stage's displacement is the initial guess
@@ -501,7 +508,8 @@ int QDContext::solve_stage(double t, const double* var, const double* gxy, const
     spec_flags = 0;
     SCY_TRY(rc);
     if (deferring) {
-      qd_record_kernel<<<1, 1, 0, s>>>(sbp.scal.as<double>(), errbuf.as<double>() + RB_SOLVE + 3 * deferred++);
+      chain_launch(qd_record_kernel, 1, 1, 0, s, sbp.scal.as<double>(),
+                   errbuf.as<double>() + RB_SOLVE + 3 * deferred++);
       SCY_LAUNCH_CHECK();
       return SCY_OK;
     }
@@ -621,7 +629,8 @@ int QDContext::build_green() {
     SCY_TRY(sbp.set_rhs(bL.as<double>(), bR.as<double>(), bcT.as<double>(), bcB.as<double>(), rhs.as<double>()));
     scy_solve_stats st{};
     SCY_TRY(sbp.solve(rhs.as<double>(), uu.as<double>(), o, st));
-    qd_response_column_kernel<<<gb, tb, 0, s>>>(L, uu.as<double>(), GL.as<double>(), SL.as<double>(), Nz, j);
+    chain_launch(qd_response_column_kernel, gb, tb, 0, s, L, uu.as<double>(), GL.as<double>(), SL.as<double>(), Nz,
+                 j);
     SCY_LAUNCH_CHECK();
   }
   // bcR = 1 and the fixed part of bcR
@@ -638,7 +647,8 @@ int QDContext::build_green() {
     SCY_TRY(sbp.set_rhs(bL.as<double>(), bR.as<double>(), bcT.as<double>(), bcB.as<double>(), rhs.as<double>()));
     scy_solve_stats st{};
     SCY_TRY(sbp.solve(rhs.as<double>(), uu.as<double>(), o, st));
-    qd_response_column_kernel<<<gb, tb, 0, s>>>(L, uu.as<double>(), cols.as<double>(), scol.as<double>(), 2, k);
+    chain_launch(qd_response_column_kernel, gb, tb, 0, s, L, uu.as<double>(), cols.as<double>(), scol.as<double>(), 2,
+                 k);
     SCY_LAUNCH_CHECK();
   }
   // split the two columns into g1/gs and s1/ss
@@ -763,7 +773,7 @@ int QDContext::launch_error(const double* lo, const double* hi) {
     kt.off[k] = key_off[k];
     kt.len[k] = key_len[k];
   }
-  rk_error_kernel<<<pl ? 4 : 2, 1024, 0, s>>>(lo, hi, kt, flags.as<unsigned>(), errbuf.as<double>());
+  chain_launch(rk_error_kernel, pl ? 4 : 2, 1024, 0, s, lo, hi, kt, flags.as<unsigned>(), errbuf.as<double>());
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -822,15 +832,16 @@ int QDContext::attempt(double dt, double** lo, double** hi) {
   if (ode.method == SCY_RK32) {
     double* fa = rk[V_F1].as<double>();
     double* fb = rk[V_F2].as<double>();
-    rk_combine_kernel<<<gb, tb, 0, s>>>(k, var, combo({{f0, 0.5 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, 0.5 * dt}}), n);
     SCY_LAUNCH_CHECK();
     SCY_TRY(d_dt(t + 0.5 * dt, k, fa));
-    rk_combine_kernel<<<gb, tb, 0, s>>>(k, var, combo({{f0, -dt}, {fa, 2 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, -dt}, {fa, 2 * dt}}), n);
     SCY_LAUNCH_CHECK();
     SCY_TRY(d_dt(t + dt, k, fb));
-    rk_combine_kernel<<<gb, tb, 0, s>>>(L, var, combo({{f0, 0.5 * dt}, {fb, 0.5 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, L, var, combo({{f0, 0.5 * dt}, {fb, 0.5 * dt}}), n);
     SCY_LAUNCH_CHECK();
-    rk_combine_kernel<<<gb, tb, 0, s>>>(H, var, combo({{f0, dt / 6.0}, {fa, 2 * dt / 3.0}, {fb, dt / 6.0}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, H, var, combo({{f0, dt / 6.0}, {fa, 2 * dt / 3.0}, {fb, dt / 6.0}}),
+                 n);
     SCY_LAUNCH_CHECK();
   } else {
     using namespace rk43;
@@ -839,28 +850,28 @@ int QDContext::attempt(double dt, double** lo, double** hi) {
     double* f4 = rk[V_F4].as<double>();
     double* f5 = rk[V_F5].as<double>();
     double* f6 = rk[V_F6].as<double>();
-    rk_combine_kernel<<<gb, tb, 0, s>>>(k, var, combo({{f0, a21 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a21 * dt}}), n);
     SCY_LAUNCH_CHECK();
     SCY_TRY(d_dt(t + c2 * dt, k, f2));
-    rk_combine_kernel<<<gb, tb, 0, s>>>(k, var, combo({{f0, a31 * dt}, {f2, a32 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a31 * dt}, {f2, a32 * dt}}), n);
     SCY_LAUNCH_CHECK();
     SCY_TRY(d_dt(t + c3 * dt, k, f3));
-    rk_combine_kernel<<<gb, tb, 0, s>>>(k, var, combo({{f0, a41 * dt}, {f2, a42 * dt}, {f3, a43 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a41 * dt}, {f2, a42 * dt}, {f3, a43 * dt}}), n);
     SCY_LAUNCH_CHECK();
     SCY_TRY(d_dt(t + c4 * dt, k, f4));
-    rk_combine_kernel<<<gb, tb, 0, s>>>(k, var,
-                                        combo({{f0, a51 * dt}, {f2, a52 * dt}, {f3, a53 * dt}, {f4, a54 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a51 * dt}, {f2, a52 * dt}, {f3, a53 * dt}, {f4,
+                 a54 * dt}}), n);
     SCY_LAUNCH_CHECK();
     SCY_TRY(d_dt(t + c5 * dt, k, f5));
-    rk_combine_kernel<<<gb, tb, 0, s>>>(
-        k, var, combo({{f0, a61 * dt}, {f2, a62 * dt}, {f3, a63 * dt}, {f4, a64 * dt}, {f5, a65 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a61 * dt}, {f2, a62 * dt}, {f3, a63 * dt}, {f4,
+                 a64 * dt}, {f5, a65 * dt}}), n);
     SCY_LAUNCH_CHECK();
     SCY_TRY(d_dt(t + c6 * dt, k, f6));
-    rk_combine_kernel<<<gb, tb, 0, s>>>(
-        L, var, combo({{f0, hb1 * dt}, {f3, hb3 * dt}, {f4, hb4 * dt}, {f5, hb5 * dt}, {f6, hb6 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, L, var, combo({{f0, hb1 * dt}, {f3, hb3 * dt}, {f4, hb4 * dt}, {f5,
+                 hb5 * dt}, {f6, hb6 * dt}}), n);
     SCY_LAUNCH_CHECK();
-    rk_combine_kernel<<<gb, tb, 0, s>>>(
-        H, var, combo({{f0, b1 * dt}, {f3, b3 * dt}, {f4, b4 * dt}, {f5, b5 * dt}, {f6, b6 * dt}}), n);
+    chain_launch(rk_combine_kernel, gb, tb, 0, s, H, var, combo({{f0, b1 * dt}, {f3, b3 * dt}, {f4, b4 * dt}, {f5,
+                 b5 * dt}, {f6, b6 * dt}}), n);
     SCY_LAUNCH_CHECK();
   }
   *lo = L;

@@ -901,6 +901,7 @@ __device__ __forceinline__ void march_part(const LevelDev<T>& L, const MarchPlan
 
 template <typename T, class Loader, class Epi>
 __global__ void __launch_bounds__(32 * kMarchWarps, 2) march_kernel(LevelDev<T> L, Loader ld, Epi ep, MarchPlan p) {
+  chain_enter();
   static_assert(!Epi::kReduce, "the warp form has no grid sum");
   __shared__ T sm[kMarchWarps * kMarchSmem];
   auto pre = [&](long node, int iy, int iz) { return epi_pre(ep, node, iy, iz, 0); };
@@ -949,6 +950,7 @@ __device__ __forceinline__ void full_tile(const LevelDev<T>& L, const Loader& ld
 template <typename T, int RPT, class Loader, class Epi>
 __global__ void __launch_bounds__(256) full_kernel(LevelDev<T> L, Loader ld, Epi ep, double* partials,
                                                    unsigned int* counter, double* red_out) {
+  chain_enter();
   full_tile<T, RPT, Loader, Epi>(L, ld, ep, partials, counter, red_out);
 }
 
@@ -963,6 +965,7 @@ __global__ void __launch_bounds__(256) full_kernel(LevelDev<T> L, Loader ld, Epi
 template <typename T, class Loader, class Epi>
 __global__ void __launch_bounds__(256) cross_kernel(LevelDev<T> L, Loader ld, Epi ep, double* partials,
                                                     unsigned int* counter, double* red_out) {
+  chain_enter();
   __shared__ T xs[full_smem_values<1>()];
   __shared__ double red[32];
   const int Ny = L.Ny, Nz = L.Nz;
@@ -1052,6 +1055,7 @@ __device__ __forceinline__ double cross_line_entry(const DirDev<T>& d, int i, in
 
 template <typename T>
 __global__ void cross_build_kernel(LevelDev<T> L, T* __restrict__ C) {
+  chain_enter();
   const int Nz = L.Nz;
   const long N = (long)L.Ny * Nz;
   for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < N; node += (long)gridDim.x * blockDim.x) {
@@ -1134,6 +1138,7 @@ __device__ __forceinline__ double fault_row_sxy(const LevelDev<double>& L, const
 template <typename T, class Loader, class Epi>
 __global__ void __launch_bounds__(256) stencil_kernel(LevelDev<T> L, Loader ld, Epi ep, double* partials,
                                                       unsigned int* counter, double* red_out) {
+  chain_enter();
   stencil_tile<T, Loader, Epi>(L, ld, ep, partials, counter, red_out);
 }
 
@@ -1158,20 +1163,20 @@ inline void launch_apply(const LevelDev<T>& L, const Loader& ld, const Epi& ep, 
     // 2049 x 1537: 45.0 and 40.9; 4097 x 3073: 107.8 and 94.1)
     if (L.full && (long)L.Ny * L.Nz >= 65536) {
       const MarchPlan p = march_plan(L, march_chunks(L));
-      march_kernel<T, Loader, Epi><<<p.blocks, 32 * kMarchWarps, 0, s>>>(L, ld, ep, p);
+      chain_launch(march_kernel<T, Loader, Epi>, p.blocks, 32 * kMarchWarps, 0, s, L, ld, ep, p);
       return;
     }
   }
   if (!L.full && L.cross)
-    cross_kernel<T, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);
+    chain_launch(cross_kernel<T, Loader, Epi>, g, 256, 0, s, L, ld, ep, partials, counter, red_out);
   else if (!L.full)
-    stencil_kernel<T, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);
+    chain_launch(stencil_kernel<T, Loader, Epi>, g, 256, 0, s, L, ld, ep, partials, counter, red_out);
   else if (L.rpt == 4)
-    full_kernel<T, 4, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);
+    chain_launch(full_kernel<T, 4, Loader, Epi>, g, 256, 0, s, L, ld, ep, partials, counter, red_out);
   else if (L.rpt == 2)
-    full_kernel<T, 2, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);
+    chain_launch(full_kernel<T, 2, Loader, Epi>, g, 256, 0, s, L, ld, ep, partials, counter, red_out);
   else
-    full_kernel<T, 1, Loader, Epi><<<g, 256, 0, s>>>(L, ld, ep, partials, counter, red_out);
+    chain_launch(full_kernel<T, 1, Loader, Epi>, g, 256, 0, s, L, ld, ep, partials, counter, red_out);
 }
 
 }  // namespace scy

@@ -322,7 +322,7 @@ int LevelStore<T>::init(const LevelHost& h, cudaStream_t s) {
   }
   if (const long n = (long)Ny * Nz; !dev.full && n <= kCrossMaxNodes) {
     SCY_TRY(cross.alloc((size_t)n * 33 * sizeof(T)));
-    cross_build_kernel<T><<<grid_for(n), 256, 0, s>>>(dev, cross.template as<T>());
+    chain_launch(cross_build_kernel<T>, grid_for(n), 256, 0, s, dev, cross.template as<T>());
     SCY_LAUNCH_CHECK();
     dev.cross = cross.template as<T>();
   }
@@ -360,6 +360,7 @@ static int launch_stencil(const LevelDev<T>& L, Ld ld, Ep ep, Reducer* red, doub
 template <typename T, typename Tin>
 __global__ void cheb_first_kernel(const Tin* __restrict__ b_in, T* __restrict__ b_keep, const T* __restrict__ dinv,
                                   T* __restrict__ d, T* __restrict__ x, T c2, long n) {
+  chain_enter();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     T bv = (T)b_in[i];
     if (b_keep) b_keep[i] = bv;
@@ -375,6 +376,7 @@ __global__ void restrict_kernel(const T* __restrict__ rf, T* __restrict__ bc, in
                                 const int* __restrict__ zlo, const int* __restrict__ zhi,
                                 const int* __restrict__ jy, const T* __restrict__ wy0, const T* __restrict__ wy1,
                                 const int* __restrict__ jz, const T* __restrict__ wz0, const T* __restrict__ wz1) {
+  chain_enter();
   long n = (long)Ncy * Ncz;
   for (long c = blockIdx.x * (long)blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x) {
     int a = (int)(c / Ncz), bb = (int)(c % Ncz);
@@ -396,6 +398,7 @@ __global__ void restrict_kernel(const T* __restrict__ rf, T* __restrict__ bc, in
 // out = M b with a dense n x n matrix; one warp per row.
 template <typename T>
 __global__ void dense_matvec_kernel(const T* __restrict__ M, const T* __restrict__ b, T* __restrict__ out, int n) {
+  chain_enter();
   int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= n) return;
   const T* row = M + (long)warp * n;
@@ -477,6 +480,7 @@ __device__ __forceinline__ T coarse_apply(const CoarseLevel<T>& L, const T* sm, 
 template <typename T, typename Tin>
 __global__ void __cluster_dims__(kCoarseBlocks, 1, 1) __launch_bounds__(kCoarseThreads)
     coarse_cycle_kernel(const __grid_constant__ CoarseArgs<T> A, const Tin* __restrict__ b_in, T* __restrict__ out) {
+  chain_enter();
   extern __shared__ __align__(16) unsigned char coarse_smem[];
   T* const sm = reinterpret_cast<T*>(coarse_smem);
   const int t = threadIdx.x, last = A.nlev - 1;
@@ -594,6 +598,7 @@ __global__ void __cluster_dims__(kCoarseBlocks, 1, 1) __launch_bounds__(kCoarseT
 template <typename T>
 __global__ void power_step_kernel(const T* __restrict__ Kv, const T* __restrict__ dinv, T* __restrict__ w, long n,
                                   double* partials, unsigned* counter, double* out) {
+  chain_enter();
   __shared__ double sh[32];
   double acc = 0.0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
@@ -607,6 +612,7 @@ __global__ void power_step_kernel(const T* __restrict__ Kv, const T* __restrict_
 
 template <typename T>
 __global__ void scale_kernel(T* __restrict__ v, const double* __restrict__ nrm2, long n) {
+  chain_enter();
   double s = 1.0 / sqrt(*nrm2);
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) v[i] = (T)(v[i] * s);
 }
@@ -615,6 +621,7 @@ __global__ void scale_kernel(T* __restrict__ v, const double* __restrict__ nrm2,
 template <typename Ta, typename Tb>
 __global__ void dot_kernel(const Ta* __restrict__ a, const Tb* __restrict__ b, long n, double* partials,
                            unsigned* counter, double* out) {
+  chain_enter();
   __shared__ double sh[32];
   double acc = 0.0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
@@ -638,6 +645,7 @@ __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e
 // does not enter r.
 __global__ void residual_dd_kernel(const double* __restrict__ C, const double* __restrict__ x,
                                    const double* __restrict__ rhs, double* __restrict__ r, int Ny, int Nz) {
+  chain_enter();
   const long N = (long)Ny * Nz;
   for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < N; node += (long)gridDim.x * blockDim.x) {
     const int iy = (int)(node / Nz), iz = (int)(node % Nz);
@@ -669,6 +677,7 @@ __global__ void cg_update_kernel(double* __restrict__ x, double* __restrict__ r,
                                  const double* __restrict__ q, const double* __restrict__ rz,
                                  const double* __restrict__ pq, long n, double* partials, unsigned* counter,
                                  double* out) {
+  chain_enter();
   __shared__ double sh[32];
   const double pqv = *pq;
   const double alpha = pqv != 0.0 ? *rz / pqv : 0.0;  // zero search direction: nothing to add
@@ -683,7 +692,9 @@ __global__ void cg_update_kernel(double* __restrict__ x, double* __restrict__ r,
   grid_reduce_finish(t, partials, counter, out, sh);
 }
 
-__global__ void copy_scalar_kernel(double* dst, const double* src) { *dst = *src; }
+__global__ void copy_scalar_kernel(double* dst, const double* src) {
+  chain_enter();
+  *dst = *src; }
 
 // ------------------------------------------------------------------------
 int Reducer::init(int max_blocks) {
@@ -883,15 +894,14 @@ int Multigrid<T>::setup_smoothers(const std::vector<LevelHost>& hosts, Reducer& 
     double lam = 0.0;
     for (int it = 0; it < 20; ++it) {
       SCY_TRY(launch_stencil<T>(lev[l]->dev, LoadPlain<T>{v}, EpiStore<T>{Kv, T(-1)}, nullptr, nullptr, s));
-      power_step_kernel<T><<<red_blocks(n), 256, 0, s>>>(Kv, lev[l]->dev.dinv, v, n,
-                                                          red.partials.template as<double>(),
-                                                          red.counter.template as<unsigned>(), dscal);
+      chain_launch(power_step_kernel<T>, red_blocks(n), 256, 0, s, Kv, lev[l]->dev.dinv, v, n,
+                   red.partials.template as<double>(), red.counter.template as<unsigned>(), dscal);
       SCY_LAUNCH_CHECK();
       double nrm2 = 0.0;
       SCY_CUDA_TRY(cudaMemcpyAsync(&nrm2, dscal, sizeof(double), cudaMemcpyDeviceToHost, s));
       SCY_CUDA_TRY(cudaStreamSynchronize(s));
       lam = std::sqrt(nrm2);  // v had unit norm after the first normalisation
-      scale_kernel<T><<<red_blocks(n), 256, 0, s>>>(v, dscal, n);
+      chain_launch(scale_kernel<T>, red_blocks(n), 256, 0, s, v, dscal, n);
       SCY_LAUNCH_CHECK();
       if (it == 0) lam = 0.0;
     }
@@ -984,7 +994,7 @@ int Multigrid<T>::coarse_cycle(int l, const Tin* b_in, T** x_out, cudaStream_t s
   SCY_CUDA_TRY(cudaFuncSetAttribute(coarse_cycle_kernel<T, Tin>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
   T* x = work[l].v[1].template as<T>();
-  coarse_cycle_kernel<T, Tin><<<kCoarseBlocks, kCoarseThreads, smem, s>>>(A, b_in, x);
+  chain_launch(coarse_cycle_kernel<T, Tin>, kCoarseBlocks, kCoarseThreads, smem, s, A, b_in, x);
   SCY_LAUNCH_CHECK();
   *x_out = x;
   return SCY_OK;
@@ -1006,21 +1016,21 @@ int Multigrid<T>::vcycle(int l, const Tin* b_in, T** x_out, cudaStream_t s) {
   if (l == nlev - 1) {
     const T* bb = (const T*)b_in;
     if (!std::is_same<Tin, T>::value) {
-      cheb_first_kernel<T, Tin><<<grid_for(n), 256, 0, s>>>(b_in, b, L.dinv, d, xa, T(0), n);
+      chain_launch(cheb_first_kernel<T, Tin>, grid_for(n), 256, 0, s, b_in, b, L.dinv, d, xa, T(0), n);
       SCY_LAUNCH_CHECK();
       bb = b;
     }
     int warps_per_block = 8;
-    dense_matvec_kernel<T><<<(ncoarse + warps_per_block - 1) / warps_per_block, 256, 0, s>>>(
-        coarse_inv.template as<T>(), bb, xa, ncoarse);
+    chain_launch(dense_matvec_kernel<T>, (ncoarse + warps_per_block - 1) / warps_per_block, 256, 0, s,
+                 coarse_inv.template as<T>(), bb, xa, ncoarse);
     SCY_LAUNCH_CHECK();
     *x_out = xa;
     return SCY_OK;
   }
   // pre-smoothing (x starts at zero)
   const T* bl = std::is_same<Tin, T>::value ? (const T*)b_in : b;
-  cheb_first_kernel<T, Tin><<<grid_for(n), 256, 0, s>>>(b_in, std::is_same<Tin, T>::value ? nullptr : b, L.dinv,
-                                                       d, xa, (T)cheb[l][0].c2, n);
+  chain_launch(cheb_first_kernel<T, Tin>, grid_for(n), 256, 0, s, b_in, std::is_same<Tin, T>::value ? nullptr : b,
+               L.dinv, d, xa, (T)cheb[l][0].c2, n);
   SCY_LAUNCH_CHECK();
   T* x = xa;
   T* xo = xb;
@@ -1035,12 +1045,10 @@ int Multigrid<T>::vcycle(int l, const Tin* b_in, T** x_out, cudaStream_t s) {
   long nc = (long)C.Ny * C.Nz;
   T* bcoarse = work[l + 1].v[3].template as<T>();
   const TransferDev& t = tr[l];
-  restrict_kernel<T><<<grid_for(nc), 256, 0, s>>>(r, bcoarse, L.Nz, C.Ny, C.Nz, t.ylo.template as<int>(),
-                                                  t.yhi.template as<int>(), t.zlo.template as<int>(),
-                                                  t.zhi.template as<int>(), t.jy.template as<int>(),
-                                                  t.wy0.template as<T>(), t.wy1.template as<T>(),
-                                                  t.jz.template as<int>(), t.wz0.template as<T>(),
-                                                  t.wz1.template as<T>());
+  chain_launch(restrict_kernel<T>, grid_for(nc), 256, 0, s, r, bcoarse, L.Nz, C.Ny, C.Nz, t.ylo.template as<int>(),
+               t.yhi.template as<int>(), t.zlo.template as<int>(), t.zhi.template as<int>(), t.jy.template as<int>(),
+               t.wy0.template as<T>(), t.wy1.template as<T>(), t.jz.template as<int>(), t.wz0.template as<T>(),
+               t.wz1.template as<T>());
   SCY_LAUNCH_CHECK();
   T* xc = nullptr;
   SCY_TRY(vcycle<T>(l + 1, bcoarse, &xc, s));
@@ -1067,6 +1075,7 @@ enum class Dir { Y, Z };
 
 template <Dir d, int kind>  // kind 0: D, 1: mu*D, 2: D*mu
 __global__ void deriv_kernel(LevelDev<double> L, const double* __restrict__ in, double* __restrict__ out) {
+  chain_enter();
   const int Ny = L.Ny, Nz = L.Nz;
   long n = (long)Ny * Nz;
   for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < n; node += (long)gridDim.x * blockDim.x) {
@@ -1105,6 +1114,7 @@ __global__ void deriv_kernel(LevelDev<double> L, const double* __restrict__ in, 
 }
 
 __global__ void hmul_kernel(LevelDev<double> L, const double* __restrict__ in, double* __restrict__ out, int inv) {
+  chain_enter();
   const int Nz = L.Nz;
   long n = (long)L.Ny * Nz;
   for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < n; node += (long)gridDim.x * blockDim.x) {
@@ -1118,6 +1128,7 @@ __global__ void hmul_kernel(LevelDev<double> L, const double* __restrict__ in, d
 __global__ void set_rhs_kernel(LevelDev<double> L, const double* __restrict__ bcL, const double* __restrict__ bcR,
                                const double* __restrict__ bcT, const double* __restrict__ bcB,
                                double* __restrict__ rhs) {
+  chain_enter();
   long n = (long)L.Ny * L.Nz;
   for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < n; node += (long)gridDim.x * blockDim.x)
     rhs[node] = set_rhs_node(L, bcL, bcR, bcT, bcB, node);
@@ -1239,14 +1250,14 @@ int SbpContext::apply(int op, const double* in, double* out) {
   switch (op) {
     case SCY_OP_A:
       return launch_stencil<double>(L, LoadPlain<double>{in}, EpiStore<double>{out, 1.0}, nullptr, nullptr, stream);
-    case SCY_OP_DY: deriv_kernel<Dir::Y, 0><<<g, 256, 0, stream>>>(L, in, out); break;
-    case SCY_OP_DZ: deriv_kernel<Dir::Z, 0><<<g, 256, 0, stream>>>(L, in, out); break;
-    case SCY_OP_MUXDY: deriv_kernel<Dir::Y, 1><<<g, 256, 0, stream>>>(L, in, out); break;
-    case SCY_OP_MUXDZ: deriv_kernel<Dir::Z, 1><<<g, 256, 0, stream>>>(L, in, out); break;
-    case SCY_OP_DYXMU: deriv_kernel<Dir::Y, 2><<<g, 256, 0, stream>>>(L, in, out); break;
-    case SCY_OP_DZXMU: deriv_kernel<Dir::Z, 2><<<g, 256, 0, stream>>>(L, in, out); break;
-    case SCY_OP_H: hmul_kernel<<<g, 256, 0, stream>>>(L, in, out, 0); break;
-    case SCY_OP_HINV: hmul_kernel<<<g, 256, 0, stream>>>(L, in, out, 1); break;
+    case SCY_OP_DY: chain_launch(deriv_kernel<Dir::Y, 0>, g, 256, 0, stream, L, in, out); break;
+    case SCY_OP_DZ: chain_launch(deriv_kernel<Dir::Z, 0>, g, 256, 0, stream, L, in, out); break;
+    case SCY_OP_MUXDY: chain_launch(deriv_kernel<Dir::Y, 1>, g, 256, 0, stream, L, in, out); break;
+    case SCY_OP_MUXDZ: chain_launch(deriv_kernel<Dir::Z, 1>, g, 256, 0, stream, L, in, out); break;
+    case SCY_OP_DYXMU: chain_launch(deriv_kernel<Dir::Y, 2>, g, 256, 0, stream, L, in, out); break;
+    case SCY_OP_DZXMU: chain_launch(deriv_kernel<Dir::Z, 2>, g, 256, 0, stream, L, in, out); break;
+    case SCY_OP_H: chain_launch(hmul_kernel, g, 256, 0, stream, L, in, out, 0); break;
+    case SCY_OP_HINV: chain_launch(hmul_kernel, g, 256, 0, stream, L, in, out, 1); break;
     default:
       set_error("unknown operator %d", op);
       return SCY_ERR_ARG;
@@ -1258,7 +1269,7 @@ int SbpContext::apply(int op, const double* in, double* out) {
 int SbpContext::set_rhs(const double* bcL, const double* bcR, const double* bcT, const double* bcB, double* rhs) {
   const LevelDev<double>& L = fine->dev;
   long n = (long)L.Ny * L.Nz;
-  set_rhs_kernel<<<grid_for(n), 256, 0, stream>>>(L, bcL, bcR, bcT, bcB, rhs);
+  chain_launch(set_rhs_kernel, grid_for(n), 256, 0, stream, L, bcL, bcR, bcT, bcB, rhs);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -1289,7 +1300,7 @@ int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts&
     it0 = 2;
   } else {
     if (!part.norm_ready) {
-      dot_kernel<double, double><<<rb, 256, 0, stream>>>(rhs, rhs, n, parts, cnt, sc + 0);
+      chain_launch(dot_kernel<double, double>, rb, 256, 0, stream, rhs, rhs, n, parts, cnt, sc + 0);
       SCY_LAUNCH_CHECK();
     }
     if (!o.nonzero_guess) SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
@@ -1304,16 +1315,16 @@ int SbpContext::pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts&
     Tz* z = nullptr;
     SCY_TRY(pc((const double*)r, &z));
     if (it > 1) {
-      copy_scalar_kernel<<<1, 1, 0, stream>>>(sc + 3, sc + 2);
+      chain_launch(copy_scalar_kernel, 1, 1, 0, stream, sc + 3, sc + 2);
       SCY_LAUNCH_CHECK();
     }
-    dot_kernel<double, Tz><<<rb, 256, 0, stream>>>(r, z, n, parts, cnt, sc + 2);
+    chain_launch(dot_kernel<double, Tz>, rb, 256, 0, stream, r, z, n, parts, cnt, sc + 2);
     SCY_LAUNCH_CHECK();
     double* pold = cg_p[pi].as<double>();
     double* pnew = cg_p[pi ^ 1].as<double>();
     LoadPUpdate<Tz> lp{z, pold, sc + 2, sc + 3, it == 1 ? 1 : 0};
     SCY_TRY(launch_stencil<double>(L, lp, EpiCGMatvec{pnew, q}, &red, sc + 4, stream));
-    cg_update_kernel<<<rb, 256, 0, stream>>>(u, r, pnew, q, sc + 2, sc + 4, n, parts, cnt, sc + 1);
+    chain_launch(cg_update_kernel, rb, 256, 0, stream, u, r, pnew, q, sc + 2, sc + 4, n, parts, cnt, sc + 1);
     SCY_LAUNCH_CHECK();
     pi ^= 1;
     st.iterations = it;
@@ -1425,8 +1436,8 @@ int SbpContext::correct(PC&& pc, const double* rhs, double* u, const scy_solve_o
     it0 = 2;
   } else {
     if (!part.norm_ready) {
-      dot_kernel<double, double><<<red_blocks(n), 256, 0, stream>>>(rhs, rhs, n, red.partials.as<double>(),
-                                                                   red.counter.as<unsigned>(), sc + 0);
+      chain_launch(dot_kernel<double, double>, red_blocks(n), 256, 0, stream, rhs, rhs, n, red.partials.as<double>(),
+                   red.counter.as<unsigned>(), sc + 0);
       SCY_LAUNCH_CHECK();
     }
     if (!o.nonzero_guess) SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
@@ -1508,12 +1519,12 @@ int SbpContext::residual_dd(const double* rhs, const double* u, double* r, doubl
                                  stream));
     SCY_CUDA_TRY(cudaStreamSynchronize(stream));
   }
-  residual_dd_kernel<<<grid_for(n, 256, 4096), 256, 0, stream>>>(cross.as<double>(), u, rhs, r, h.Ny, h.Nz);
+  chain_launch(residual_dd_kernel, grid_for(n, 256, 4096), 256, 0, stream, cross.as<double>(), u, rhs, r, h.Ny, h.Nz);
   SCY_LAUNCH_CHECK();
   if (rnorm2_host) {
     double* sc = scal.as<double>();
-    dot_kernel<double, double><<<red_blocks(n), 256, 0, stream>>>(r, r, n, red.partials.as<double>(),
-                                                                 red.counter.as<unsigned>(), sc + 6);
+    chain_launch(dot_kernel<double, double>, red_blocks(n), 256, 0, stream, r, r, n, red.partials.as<double>(),
+                 red.counter.as<unsigned>(), sc + 6);
     SCY_LAUNCH_CHECK();
     SCY_CUDA_TRY(cudaMemcpyAsync(rnorm2_host, sc + 6, sizeof(double), cudaMemcpyDeviceToHost, stream));
     SCY_CUDA_TRY(cudaStreamSynchronize(stream));

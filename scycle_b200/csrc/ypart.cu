@@ -60,6 +60,7 @@ constexpr int kRow = 14, kMaxPad = 7;
 
 template <int T, int I>
 __global__ void __launch_bounds__(384) ypart_kernel(const YPartArgs A) {
+  chain_enter();
   constexpr int S = T * kRow + 2;
   extern __shared__ __align__(128) unsigned char yp_smem[];
   __shared__ __align__(8) uint64_t bar;
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(384) ypart_kernel(const YPartArgs A) {
 int dev_smem_limit() { return 225 * 1024; }  // beside the static kilobyte
 
 template <int T, int I>
-int launch_one(const YPartArgs& A, size_t smem, int nb, int NG, cudaStream_t s) {
+int launch_one(const YPartArgs& A, size_t smem, int nb, int NG, cudaStream_t s, bool chain) {
   const int TP = (A.P * A.MB + 31) / 32 * 32;
   SCY_CUDA_TRY(cudaFuncSetAttribute(ypart_kernel<T, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     dev_smem_limit()));
@@ -264,7 +265,7 @@ int launch_one(const YPartArgs& A, size_t smem, int nb, int NG, cudaStream_t s) 
   // as many blocks a mode block as are resident at once: each takes its
   // instances in turn with the tables it has loaded
   const int want = (A.K + NG * I - 1) / (NG * I), fit = std::max(1, per_sm * kNumSMs / nb);
-  ypart_kernel<T, I><<<dim3(nb, std::min(want, fit)), dim3(TP, NG), smem, s>>>(A);
+  launch(chain, ypart_kernel<T, I>, dim3(nb, std::min(want, fit)), dim3(TP, NG), smem, s, A);
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -379,13 +380,13 @@ int YPart::build(const std::vector<double>& L, int Ny_, int Nz, int Nzp_, cudaSt
   return SCY_OK;
 }
 
-int YPart::solve(double* t, int K, int shape, unsigned* status, cudaStream_t s, int polls, int drop) const {
+int YPart::solve(double* t, int K, int shape, unsigned* status, cudaStream_t s, bool chain, int polls, int drop) const {
   const YPartArgs A{tab.as<double>(), wide.as<double>(), t, Ny, Nzp, K, P, MB, base, extra, status, polls, drop};
   const int I = kShapeI[shape], NG = kShapeNG[shape];
   const size_t smem = smem_bytes(shape);
   switch (T) {
 #define SCY_YP(TV) \
-  case TV: return I == 1 ? launch_one<TV, 1>(A, smem, nb, NG, s) : launch_one<TV, 2>(A, smem, nb, NG, s)
+  case TV: return I == 1 ? launch_one<TV, 1>(A, smem, nb, NG, s, chain) : launch_one<TV, 2>(A, smem, nb, NG, s, chain)
     SCY_YP(8);
     SCY_YP(12);
     SCY_YP(16);

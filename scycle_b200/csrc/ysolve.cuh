@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(32 * W) b_ysolve_tma_kernel(const __grid_const
                                                               T* __restrict__ t, int Ny, int Nz, int Nzp, int K,
                                                               unsigned* __restrict__ status,
                                                               int first_polls = 1 << 18, int drop_first = 0) {
+  chain_enter();
   constexpr int B = 2 * W * I;
   extern __shared__ __align__(128) unsigned char ys_smem[];
   constexpr int CT = YS_R * 9 * YS_C, DT = B * YS_R * YS_C;  // elements per tile

@@ -159,6 +159,45 @@ def test_apply_A_in_walks(Ny, Nz, grid, mu_kind):
     assert _rel(dev.apply("A", x).cpu().numpy(), ora.A @ x) <= 1e-13
 
 
+@pytest.mark.parametrize("Ny,Nz,mu_var", [(17, 17, False), (41, 33, True), (129, 97, False), (260, 256, False)])
+def test_chained_launches_keep_stream_order(Ny, Nz, mu_var):
+    """Launches whose blocks are placed before the kernel ahead of them has
+    finished: chains A (A (... x)) of small and larger grids and of several
+    blocks per SM, without a wait in between and between ordinary launches
+    and copies of another library, on two streams at once, give bitwise what
+    the same applications give one at a time."""
+    import ctypes as C
+    import torch
+    from scycle_b200 import _lib as S
+    from scycle_b200.sbp import SbpOps
+    rng = np.random.default_rng(Ny)
+    mu = 32.04 + (2 * rng.random(Ny * Nz) if mu_var else np.zeros(Ny * Nz))
+    devs = [SbpOps(4, Ny, Nz, 30.0, 24.0, mu) for _ in range(2)]
+    streams = [torch.cuda.Stream() for _ in devs]
+    x = torch.from_numpy(rng.standard_normal(Ny * Nz)).cuda()
+    scale, n = 1e-6, 12
+    ref = x
+    for _ in range(n):
+        ref = devs[0].apply("A", ref) * scale
+    out = []
+    torch.cuda.synchronize()
+    for d, st in zip(devs, streams):
+        S.check(S.lib().scy_sbp_set_stream(d.h, C.c_void_p(st.cuda_stream)))
+        with torch.cuda.stream(st):
+            a, b, keep = x.clone(), torch.empty_like(x), torch.empty_like(x)
+            for _ in range(n):
+                S.check(S.lib().scy_sbp_apply(d.h, S.OPS["A"], C.c_void_p(a.data_ptr()), C.c_void_p(b.data_ptr())))
+                # twice more into a buffer that the next round overwrites
+                S.check(S.lib().scy_sbp_apply(d.h, S.OPS["A"], C.c_void_p(b.data_ptr()), C.c_void_p(keep.data_ptr())))
+                torch.mul(b, scale, out=a)
+            out.append((a, b, keep))
+    torch.cuda.synchronize()
+    for a, _, _ in out:
+        assert torch.equal(a, ref)
+    for d in devs:
+        S.check(S.lib().scy_sbp_set_stream(d.h, C.c_void_p(0)))
+
+
 @pytest.mark.parametrize("precision", ("fp64", "mixed"))
 def test_fast_diagonalisation_on_separable_stretched_grid(precision):
     """Constant mu, y(iy) and z(iz) stretched independently: the separable part
