@@ -157,6 +157,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr));
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[16]) { tmem_ld16(taddr, v); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&v)[8]) { tmem_ld8(taddr, v); }
+
 // The digit products of one 32-byte K step: X plane p times the stack of W
 // planes 1 .. S+1-p.  Their products belong to the consecutive groups
 // p-1 .. S-1, whose accumulators are consecutive in tensor memory, and the
@@ -185,16 +193,20 @@ __device__ __forceinline__ void ozk_issue_kstep(uint32_t tacc, uint32_t xa, uint
   }
 }
 
+// Threads of a tile: four warps, or eight for the narrow tiles, where the
+// epilogue (S FP64 conversions and sums an output) is a third of the kernel.
+__host__ __device__ constexpr int ozk_threads(int pair) { return pair == 2 ? 256 : 128; }
+
 template <int S, typename T, int PAIR, int BF>
-__global__ void __launch_bounds__(128, PAIR == 1 ? 2 : 1)
+__global__ void __launch_bounds__(ozk_threads(PAIR), PAIR == 1 ? 2 : 1)
     ozk_gemm_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mw,
                     const int* __restrict__ ex, const int* __restrict__ ew, T* __restrict__ D, long ldd, int rows,
                     int cout, int nks, unsigned* __restrict__ status, int rows_per_status, unsigned bit) {
-  chain_enter();
   constexpr int CN = ozk_cn(S, PAIR);
   constexpr int XB = S * OZK_BM * OZK_BK;
   constexpr int WB = S * CN * OZK_BK;
   constexpr int ST = ozk_stages(S, PAIR);
+  constexpr int NT = ozk_threads(PAIR), EC = PAIR == 2 ? 8 : 16;  // columns a warp combines at a time
   constexpr int TC = ozk_tmem_cols(PAIR);
   constexpr unsigned AL = ozk_align(PAIR);
   static_assert(S * CN <= TC, "accumulators exceed tensor memory");
@@ -241,9 +253,21 @@ __global__ void __launch_bounds__(128, PAIR == 1 ? 2 : 1)
   const int rot = (int)((blockIdx.x * 7u + blockIdx.y) % (unsigned)nkb);
   const int nmma = min(CN, (cout - c0 + 15) / 16 * 16);
   int issued = 0;
+  if (warp == 0 && lane == 0) {
+    // the weights (laid out at set-up) of the first stages ahead of the wait
+    // for the kernel that makes X: with this and the sweeps' tables loaded
+    // likewise, four chained steps take 1208 us at 401 x 401 and 813 at 101 x
+    // 101 (1262 and 848 with the wait first)
+    for (int q = 0; q < min(ST, nkb); ++q) {
+      mbar_expect_tx(&full[q], XB + WB);
+      tma_load_3d(smem + q * (XB + WB) + XB, &mw, &full[q], (q + rot) % nkb * (OZK_BK / (BF ? 2 : 1)), c0, 0);
+    }
+  }
+  __syncwarp();
+  chain_enter();
   if (warp >= 2) {
     // the epilogue's exponent factors, loaded while the products run
-    for (int i = threadIdx.x - 64; i < CN + OZK_BM; i += 64) {
+    for (int i = threadIdx.x - 64; i < CN + OZK_BM; i += NT - 64) {
       if (i < CN)
         s_sw[i] = c0 + i < cout ? pow2i(ew[c0 + i]) : 0.0;
       else
@@ -259,10 +283,10 @@ __global__ void __launch_bounds__(128, PAIR == 1 ? 2 : 1)
         break;
       }
       unsigned char* sx = smem + st * (XB + WB);
-      mbar_expect_tx(&full[st], XB + WB);
+      if (q >= ST) mbar_expect_tx(&full[st], XB + WB);
       // x coordinate in digits: 64 bytes of K per stage
       tma_load_3d(sx, &mx, &full[st], kb * (OZK_BK / (BF ? 2 : 1)), m0, 0);
-      tma_load_3d(sx + XB, &mw, &full[st], kb * (OZK_BK / (BF ? 2 : 1)), c0, 0);
+      if (q >= ST) tma_load_3d(sx + XB, &mw, &full[st], kb * (OZK_BK / (BF ? 2 : 1)), c0, 0);
       ++issued;
     }
   } else if (warp == 1 && lane == 0) {
@@ -302,47 +326,56 @@ __global__ void __launch_bounds__(128, PAIR == 1 ? 2 : 1)
       for (int q = m0 / rows_per_status; q <= r1 / rows_per_status; ++q) atomicOr(status + q, bit);
     }
   } else {
-    // epilogue: warp w owns tensor-memory lanes 32 w .. 32 w + 31 (rows);
-    // a thread combines its row's groups, 16 columns at a time, applies the
-    // exponent factors (exact powers of two, loaded during the products)
-    // and stores the 16 values of its row segment
-    const int rl = warp * 32 + lane, row = m0 + rl;
+    // epilogue: warp w owns tensor-memory lanes 32 (w % 4) .. + 31 (rows);
+    // a thread combines its row's groups, EC columns at a time (of eight
+    // warps, every second EC columns), applies the exponent factors (exact
+    // powers of two, loaded during the products) and stores the values of
+    // its row segment
+    const int rl = (warp & 3) * 32 + lane, row = m0 + rl;
     const double xs = s_xs[rl];
-    const uint32_t tl = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll 1
-    for (int cc = 0; cc < nmma; cc += 16) {
-      uint32_t v[S][16];
+    for (int cc = (warp >> 2) * EC; cc < nmma; cc += NT / 128 * EC) {
+      uint32_t v[S][EC];
 #pragma unroll
-      for (int g = 0; g < S; ++g) tmem_ld16(tl + g * CN + cc, v[g]);
+      for (int g = 0; g < S; ++g) tmem_ld(tl + g * CN + cc, v[g]);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      double acc[16];
+      double acc[EC];
       if constexpr (S <= 5) {
         // sum_g P_g 2^(-7 (g+2)) as one 64-bit integer (|P_g| < 2^24, so
         // the Horner sum stays below 2^52) times 2^(-7 (S+1)): exact, the
         // same value as the FP64 sum below, with one conversion per output
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
+        for (int q = 0; q < EC; ++q) {
           long long h = 0;
 #pragma unroll
           for (int g = 0; g < S; ++g) h = (h << 7) + (long long)(BF ? (int)__uint_as_float(v[g][q]) : (int)v[g][q]);
           acc[q] = (double)h * pow2i(-7 * (S + 1));
         }
       } else {
+        // smallest weights first; the five smallest as one 64-bit integer
+        // (below 2^53 while |P_g| < 2^24, as their FP64 sum, so the same
+        // value: one conversion instead of five)
 #pragma unroll
-        for (int q = 0; q < 16; ++q) acc[q] = 0.0;
+        for (int q = 0; q < EC; ++q) {
+          long long h = 0;
 #pragma unroll
-        for (int g = S - 1; g >= 0; --g) {
-          // smallest weights first
+          for (int g = S - 5; g < S; ++g)
+            h = (h << 7) + (long long)(BF ? (int)__uint_as_float(v[g][q]) : (int)v[g][q]);
+          acc[q] = (double)h * pow2i(-7 * (S + 1));
+        }
+#pragma unroll
+        for (int g = S - 6; g >= 0; --g) {
           const double wgt = pow2i(-7 * (g + 2));
 #pragma unroll
-          for (int q = 0; q < 16; ++q)
+          for (int q = 0; q < EC; ++q)
             acc[q] += (BF ? (double)__uint_as_float(v[g][q]) : (double)(int)v[g][q]) * wgt;
         }
       }
       if (row < rows) {
         T* drow = D + (long)row * ldd + c0 + cc;
 #pragma unroll
-        for (int q = 0; q < 16; ++q)
+        for (int q = 0; q < EC; ++q)
           if (c0 + cc + q < cout) drow[q] = (T)((acc[q] * xs) * s_sw[cc + q]);
       }
     }
@@ -696,7 +729,7 @@ int launch_gemm(const OzkOperand& x, const CUtensorMap& wmap, const OzkOperand& 
     if (rc != SCY_OK) return rc;
   }
   const dim3 grid((cout + CN - 1) / CN, (x.rows + OZK_BM - 1) / OZK_BM);
-  launch(x.chain, ozk_gemm_kernel<S, T, PAIR, BF>, grid, 128, ozk_smem_bytes(S, PAIR), s, x.map, wmap,
+  launch(x.chain, ozk_gemm_kernel<S, T, PAIR, BF>, grid, ozk_threads(PAIR), ozk_smem_bytes(S, PAIR), s, x.map, wmap,
          x.expo.as<int>(), w.expo.as<int>(), D, ldd, x.rows, cout, x.Kp * x.esz / 32, status, rows_per_status, bit);
   SCY_LAUNCH_CHECK();
   return SCY_OK;

@@ -60,7 +60,6 @@ constexpr int kRow = 14, kMaxPad = 7;
 
 template <int T, int I>
 __global__ void __launch_bounds__(384) ypart_kernel(const YPartArgs A) {
-  chain_enter();
   constexpr int S = T * kRow + 2;
   extern __shared__ __align__(128) unsigned char yp_smem[];
   __shared__ __align__(8) uint64_t bar;
@@ -89,6 +88,9 @@ __global__ void __launch_bounds__(384) ypart_kernel(const YPartArgs A) {
                      : "memory");
     }
   }
+  // (the tables, laid out at set-up, ahead of the wait for the kernel that
+  // makes t)
+  chain_enter();
   __syncthreads();
   const bool act = q < PM;
   const int seg = act ? q / MB : 0, mode = act ? q % MB : 0;
