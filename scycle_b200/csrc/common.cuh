@@ -161,4 +161,35 @@ __device__ __forceinline__ void grid_reduce_finish(double block_total, double* p
   }
 }
 
+// The same for two sums at once (partials: 2 * blocks).
+__device__ __forceinline__ void grid_reduce_finish2(double tot0, double tot1, double* partials, unsigned int* counter,
+                                                    double* out0, double* out1, double* sh) {
+  __shared__ bool am_last;
+  const unsigned int nblocks = gridDim.x * gridDim.y;
+  const unsigned int bid = blockIdx.x + gridDim.x * blockIdx.y;
+  if (threadIdx.x == 0) {
+    partials[bid] = tot0;
+    partials[nblocks + bid] = tot1;
+    __threadfence();
+    unsigned int prev = atomicAdd(counter, 1u);
+    am_last = (prev == nblocks - 1);
+  }
+  __syncthreads();
+  if (am_last) {
+    __threadfence();
+    double s0 = 0.0, s1 = 0.0;
+    for (int i = threadIdx.x; i < (int)nblocks; i += blockDim.x) {
+      s0 += ((volatile double*)partials)[i];
+      s1 += ((volatile double*)partials)[nblocks + i];
+    }
+    s0 = block_sum(s0, sh);
+    s1 = block_sum(s1, sh);
+    if (threadIdx.x == 0) {
+      *out0 = s0;
+      *out1 = s1;
+      *counter = 0u;
+    }
+  }
+}
+
 }  // namespace scy

@@ -36,36 +36,87 @@ __global__ void qd_bc_kernel(const double* __restrict__ slip, int Nz, double t, 
 // (rows iy = 0), rhs = setRhs(bc) (+ B gVxy + C gVxz for the power law), and a
 // copy of the slip velocity the root finder starts from, for a fault update
 // that has to be made again.
-__global__ void __launch_bounds__(256) qd_rhs_kernel(LevelDev<double> L, const double* __restrict__ slip, double t,
-                                                     double vL, double inv_fts, int bcL_from_slip, int bcR_remote,
-                                                     const double* __restrict__ shift, double* bcL, double* bcR,
-                                                     const double* __restrict__ bcT, const double* __restrict__ bcB,
-                                                     const double* __restrict__ gxy, const double* __restrict__ gxz,
-                                                     double* __restrict__ rhs, const double* __restrict__ V,
-                                                     double* __restrict__ V0, double* partials, unsigned* counter,
-                                                     double* norm2) {
+struct QDRhs {
+  const double* slip;
+  double t, vL, inv_fts;
+  int bcL_from_slip, bcR_remote;
+  const double* shift;
+  double *bcL, *bcR;
+  const double *bcT, *bcB;
+  double* rhs;
+  const double* V;
+  double* V0;
+  __device__ __forceinline__ double left(int iz) const { return bcL_from_slip ? slip[iz] * inv_fts : bcL[iz]; }
+  __device__ __forceinline__ double right(int iz) const {
+    return bcR_remote ? vL * t * inv_fts + shift[iz] : bcR[iz];
+  }
+  // column iz's boundary data and first guess
+  __device__ __forceinline__ void column(int iz) const {
+    if (bcL_from_slip) bcL[iz] = slip[iz] * inv_fts;
+    if (bcR_remote) bcR[iz] = vL * t * inv_fts + shift[iz];
+    V0[iz] = V[iz];
+  }
+};
+
+__global__ void __launch_bounds__(256) qd_rhs_kernel(LevelDev<double> L, QDRhs q, const double* __restrict__ gxy,
+                                                     const double* __restrict__ gxz, double* partials,
+                                                     unsigned* counter, double* norm2) {
   chain_enter();
   __shared__ double sh[32];
   const int Nz = L.Nz;
   const long N = (long)L.Ny * Nz;
-  auto left = [&](int iz) { return bcL_from_slip ? slip[iz] * inv_fts : bcL[iz]; };
-  auto right = [&](int iz) { return bcR_remote ? vL * t * inv_fts + shift[iz] : bcR[iz]; };
-  auto top = [&](int iy) { return bcT[iy]; };
-  auto bottom = [&](int iy) { return bcB[iy]; };
+  auto left = [&](int iz) { return q.left(iz); };
+  auto right = [&](int iz) { return q.right(iz); };
+  auto top = [&](int iy) { return q.bcT[iy]; };
+  auto bottom = [&](int iy) { return q.bcB[iy]; };
   double acc = 0.0;
   for (long node = blockIdx.x * (long)blockDim.x + threadIdx.x; node < N; node += (long)gridDim.x * blockDim.x) {
     double v = set_rhs_node_f(L, left, right, top, bottom, node);
     if (gxy) v = v + 1.0 * pl_source_node(L, gxy, gxz, node);
-    rhs[node] = v;
+    q.rhs[node] = v;
     acc += v * v;
-    if (node < Nz) {
-      if (bcL_from_slip) bcL[node] = slip[node] * inv_fts;
-      if (bcR_remote) bcR[node] = vL * t * inv_fts + shift[node];
-      V0[node] = V[node];
-    }
+    if (node < Nz) q.column((int)node);
   }
   const double s = block_sum(acc, sh);
   grid_reduce_finish(s, partials, counter, norm2, sh);
+}
+
+// The rhs together with the residual that a defect correction starts from, r =
+// A u - rhs, and both sums of squares, where the operator has its full form:
+// one launch and one pass over the grid instead of two (no source terms).
+// Bound by latency as the operator's other launches; at 401 x 401 the two
+// kernels took 6.9 + 9.3 us, this one 10.8, and four steps 1234 and 1177; at
+// 61 x 61 5.2 + 6.2 and 7.6.
+template <int RPT>
+__global__ void __launch_bounds__(256) qd_rhs_residual_kernel(LevelDev<double> L, QDRhs q,
+                                                              const double* __restrict__ u, double* __restrict__ r,
+                                                              double* partials, unsigned* counter, double* norm2,
+                                                              double* r2) {
+  chain_enter();
+  __shared__ double xs[full_smem_values<RPT>()];
+  __shared__ double sh[32];
+  double ab = 0.0, ar = 0.0;
+  auto left = [&](int iz) { return q.left(iz); };
+  auto right = [&](int iz) { return q.right(iz); };
+  auto top = [&](int iy) { return q.bcT[iy]; };
+  auto bottom = [&](int iy) { return q.bcB[iy]; };
+  auto ld = [&](long node, int, int) { return u[node]; };
+  auto pre = [&](long, int iy, int iz) {
+    return set_rhs_at(L, left, right, top, bottom, iy, iz, L.wy1[iz], L.wz1[iy]);
+  };
+  auto out = [&](long node, int iy, int iz, double Au, double, double b) {
+    const double v = -1.0 * b + Au;
+    q.rhs[node] = b;
+    r[node] = v;
+    ab += b * b;
+    ar += v * v;
+    if (iy == 0) q.column(iz);
+  };
+  auto row = [](int) {};
+  full_apply<double, RPT>(L, ld, pre, out, row, xs, blockIdx.y * 8 * RPT, blockIdx.x * TZ);
+  ab = block_sum(ab, sh);
+  ar = block_sum(ar, sh);
+  grid_reduce_finish2(ab, ar, partials, counter, norm2, r2, sh);
 }
 
 // one enqueued solve's scalars (|rhs|^2, r.r, |r0|^2) into its record
@@ -486,17 +537,27 @@ int QDContext::solve_stage(double t, const double* var, const double* gxy, const
                            const std::function<int()>& after) {
   cudaStream_t s = sbp.stream;
   flags_known = 0;
-  const int rb = grid_for(N, 256, 592);
-  chain_launch(qd_rhs_kernel, rb, 256, 0, s, sbp.fine->dev, var + fp.slip_off, t, vL, 1.0 / fts, bcL_from_slip,
-               bcR_remote, bcRShift.as<double>(), bcL.as<double>(), bcR.as<double>(), bcT.as<double>(),
-               bcB.as<double>(), gxy, gxz, rhs.as<double>(), slipVel.as<double>(), slipVel0.as<double>(),
-               sbp.red.partials.as<double>(), sbp.red.counter.as<unsigned>(), sbp.scal.as<double>());
-  SCY_LAUNCH_CHECK();
   scy_solve_opts o = solve_opts;
   o.nonzero_guess = 1;  // the previous stage's displacement is the initial guess
   scy_solve_stats st{};
   SolvePart part;
   part.norm_ready = 1;
+  const LevelDev<double>& L = sbp.fine->dev;
+  const QDRhs q{var + fp.slip_off,      t, vL, 1.0 / fts, bcL_from_slip, bcR_remote, bcRShift.as<double>(),
+                bcL.as<double>(),       bcR.as<double>(), bcT.as<double>(), bcB.as<double>(), rhs.as<double>(),
+                slipVel.as<double>(),   slipVel0.as<double>()};
+  double *parts = sbp.red.partials.as<double>(), *sc = sbp.scal.as<double>();
+  unsigned* counter = sbp.red.counter.as<unsigned>();
+  if (L.full && !gxy && sbp.corrects(o)) {
+    part.resid_ready = 1;
+    const dim3 g = apply_grid(L);
+    const auto k = L.rpt == 4 ? qd_rhs_residual_kernel<4>
+                   : L.rpt == 2 ? qd_rhs_residual_kernel<2> : qd_rhs_residual_kernel<1>;
+    chain_launch(k, g, 256, 0, s, L, q, u.as<double>(), sbp.cg_r.as<double>(), parts, counter, sc, sc + 5);
+  } else {
+    chain_launch(qd_rhs_kernel, grid_for(N, 256, 592), 256, 0, s, L, q, gxy, gxz, parts, counter, sc);
+  }
+  SCY_LAUNCH_CHECK();
   if (!sbp.can_enqueue(o)) {
     SCY_TRY(sbp.solve(rhs.as<double>(), u.as<double>(), o, st, part));
     SCY_TRY(after());

@@ -465,9 +465,10 @@ constexpr int full_smem_values() {
 // columns z0-H .. z0-1, z0+32 .. z0+31+H of rows y0 .. y0+TYB-1 at
 // (r + H, c) of xs (pitch 32 + 2H) through ld(node, iy, iz), zeros outside
 // the grid when CHECK (else every node is inside).  256 threads; a thread
-// issues all its loads before its stores, so they are in flight together.
-template <typename T, int TYB, int H, bool CHECK, class Loader>
-__device__ __forceinline__ void full_stage(const Loader& ld, T* xs, int y0, int z0, int Ny, int Nz) {
+// issues all its loads before its stores, so they are in flight together;
+// mid() comes between the two, so that its loads are in flight with them.
+template <typename T, int TYB, int H, bool CHECK, class Loader, class Mid>
+__device__ __forceinline__ void full_stage(const Loader& ld, T* xs, int y0, int z0, int Ny, int Nz, const Mid& mid) {
   constexpr int W = TZ + 2 * H, NM = (TYB + 2 * H) * TZ, NT = NM + TYB * 2 * H, NV = (NT + 255) / 256;
   const int tid = threadIdx.x;
   T v[NV];
@@ -491,6 +492,7 @@ __device__ __forceinline__ void full_stage(const Loader& ld, T* xs, int y0, int 
     v[a] = T(0);
     if (i < NT && (!CHECK || (iy >= 0 && iy < Ny && iz >= 0 && iz < Nz))) v[a] = ld((long)iy * Nz + iz, iy, iz);
   }
+  mid();
 #pragma unroll
   for (int a = 0; a < NV; ++a)
     if (at[a] >= 0) xs[at[a]] = v[a];
@@ -527,12 +529,13 @@ __device__ __forceinline__ void full_apply(const LevelDev<T>& L, const Loader& l
       const int i = tid + 256 * a;
       cyv[a] = (rows_differ && i < TYB * BAND) ? L.Cy17[(long)(y0 + i / BAND) * 17 + (8 - HALF) + i % BAND] : T(0);
     }
-    full_stage<T, TYB, H, false>(ld, xs, y0, z0, Ny, Nz);  // all inside the grid
+    full_stage<T, TYB, H, false>(ld, xs, y0, z0, Ny, Nz, [&]() {  // all inside the grid
 #pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-      const int iy = y0 + r0 + j;
-      pv[j] = pre((long)iy * Nz + iz, iy, iz);
-    }
+      for (int j = 0; j < RPT; ++j) {
+        const int iy = y0 + r0 + j;
+        pv[j] = pre((long)iy * Nz + iz, iy, iz);
+      }
+    });
 #pragma unroll
     for (int a = 0; a < NC; ++a)
       if (rows_differ && tid + 256 * a < TYB * BAND) cys[tid + 256 * a] = cyv[a];
@@ -561,12 +564,13 @@ __device__ __forceinline__ void full_apply(const LevelDev<T>& L, const Loader& l
     }
   } else {
     constexpr int H = 8, W = TZ + 2 * H;
-    full_stage<T, TYB, H, true>(ld, xs, y0, z0, Ny, Nz);
+    full_stage<T, TYB, H, true>(ld, xs, y0, z0, Ny, Nz, [&]() {
 #pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-      const int iy = y0 + r0 + j;
-      pv[j] = (iz < Nz && iy < Ny) ? pre((long)iy * Nz + iz, iy, iz) : P{};
-    }
+      for (int j = 0; j < RPT; ++j) {
+        const int iy = y0 + r0 + j;
+        pv[j] = (iz < Nz && iy < Ny) ? pre((long)iy * Nz + iz, iy, iz) : P{};
+      }
+    });
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < RPT; ++j) {
@@ -985,7 +989,7 @@ __global__ void __launch_bounds__(256) cross_kernel(LevelDev<T> L, Loader ld, Ep
 #pragma unroll
     for (int o = 0; o < 8; ++o) c[9 + o] = C[(long)(21 + o) * N];
     const auto pv = epi_pre(ep, node, iy, iz, 0);
-    full_stage<T, TY, H, false>(ld, xs, y0, z0, Ny, Nz);
+    full_stage<T, TY, H, false>(ld, xs, y0, z0, Ny, Nz, []() {});
     __syncthreads();
     const T* xy = xs + ty * W + H + lane;        // row iy - 4
     const T* xz = xs + (ty + H) * W + lane;      // column iz - 4
@@ -999,7 +1003,7 @@ __global__ void __launch_bounds__(256) cross_kernel(LevelDev<T> L, Loader ld, Ep
     contrib = epi_out(ep, node, iy, iz, s0 + s1, xy[H * W], pv);
   } else {
     constexpr int H = 8, W = TZ + 2 * H;
-    full_stage<T, TY, H, true>(ld, xs, y0, z0, Ny, Nz);
+    full_stage<T, TY, H, true>(ld, xs, y0, z0, Ny, Nz, []() {});
     __syncthreads();
     if (valid) {
       const auto pv = epi_pre(ep, node, iy, iz, 0);
@@ -1082,10 +1086,20 @@ constexpr long kCrossMaxNodes = 1L << 18;
 // boundaries and the Neumann boundary values, times the outer weights.  The
 // boundary values come as bcL(iz), bcR(iz), bcT(iy), bcB(iy).
 template <class FL, class FR, class FT, class FB>
+__device__ __forceinline__ double set_rhs_at(const LevelDev<double>& L, const FL& bcL, const FR& bcR, const FT& bcT,
+                                             const FB& bcB, int iy, int iz, double wy, double wz);
+
+template <class FL, class FR, class FT, class FB>
 __device__ __forceinline__ double set_rhs_node_f(const LevelDev<double>& L, const FL& bcL, const FR& bcR,
                                                  const FT& bcT, const FB& bcB, long node) {
+  const int iy = (int)(node / L.Nz), iz = (int)(node % L.Nz);
+  return set_rhs_at(L, bcL, bcR, bcT, bcB, iy, iz, L.wy[node], L.wz[node]);
+}
+
+template <class FL, class FR, class FT, class FB>
+__device__ __forceinline__ double set_rhs_at(const LevelDev<double>& L, const FL& bcL, const FR& bcR, const FT& bcT,
+                                             const FB& bcB, int iy, int iz, double wy, double wz) {
   const int Ny = L.Ny, Nz = L.Nz;
-  const int iy = (int)(node / Nz), iz = (int)(node % Nz);
   double sy = 0.0, sz = 0.0;
   if (L.y.bc_lo == 0) {
     if (iy < BAND) sy += (L.y.bs0[iy] + (iy == 0 ? L.y.alphaD : 0.0)) * L.cy[iz] * bcL(iz);
@@ -1109,7 +1123,7 @@ __device__ __forceinline__ double set_rhs_node_f(const LevelDev<double>& L, cons
   } else if (iz == Nz - 1) {
     sz -= bcB(iy);
   }
-  return L.wy[node] * sy + L.wz[node] * sz;
+  return wy * sy + wz * sz;
 }
 
 __device__ __forceinline__ double set_rhs_node(const LevelDev<double>& L, const double* __restrict__ bcL,

@@ -1169,7 +1169,7 @@ int SbpContext::create(const scy_grid_desc& g) {
       return SCY_ERR_ARG;
     }
   const int tiles = ((g.Nz + TZ - 1) / TZ) * ((g.Ny + TY - 1) / TY);
-  SCY_TRY(red.init(1024 + tiles));
+  SCY_TRY(red.init(1024 + 2 * tiles));
   SCY_TRY(scal.alloc(sizeof(double) * 16));
   SCY_CUDA_TRY(cudaMemset(scal.p, 0, sizeof(double) * 16));
   long n = N;
@@ -1441,8 +1441,9 @@ int SbpContext::correct(PC&& pc, const double* rhs, double* u, const scy_solve_o
       SCY_LAUNCH_CHECK();
     }
     if (!o.nonzero_guess) SCY_CUDA_TRY(cudaMemsetAsync(u, 0, n * sizeof(double), stream));
-    SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{u}, EpiResidual<double, double>{rhs, r, -1.0}, &red, sc + 5,
-                                   stream));
+    if (!part.resid_ready)
+      SCY_TRY(launch_stencil<double>(L, LoadPlain<double>{u}, EpiResidual<double, double>{rhs, r, -1.0}, &red, sc + 5,
+                                     stream));
   }
   for (int it = it0; it <= o.max_its; ++it) {
     double* z = nullptr;
@@ -1471,15 +1472,14 @@ int SbpContext::ensure_fd(bool chains) {
 }
 
 bool SbpContext::can_enqueue(const scy_solve_opts& o) const {
-  return (o.precond == SCY_PC_FD || (o.precond == SCY_PC_AUTO && separable)) && o.precision == SCY_PREC_FP64 &&
+  return uses_fd(o) && o.precision == SCY_PREC_FP64 &&
          !o.verify && o.check_every <= 1 && o.max_its >= 1;
 }
 
 int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st,
                       const SolvePart& part) {
   const bool keeps = keeps_rounding(o.rtol);
-  const bool use_fd = o.precond == SCY_PC_FD || (o.precond == SCY_PC_AUTO && separable);
-  if (use_fd) {
+  if (uses_fd(o)) {
     SCY_TRY(ensure_fd(keeps));
     if (o.precision == SCY_PREC_MIXED) {
       float* z = cg_z32.as<float>();
@@ -1496,7 +1496,7 @@ int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy
       *zo = z;
       return SCY_OK;
     };
-    return near_inverse() && !keeps ? correct(pc, rhs, u, o, st, part) : pcg<double>(pc, rhs, u, o, st, part);
+    return corrects(o) ? correct(pc, rhs, u, o, st, part) : pcg<double>(pc, rhs, u, o, st, part);
   }
   if (o.precision == SCY_PREC_MIXED) {
     SCY_TRY(ensure_mg(mg32));

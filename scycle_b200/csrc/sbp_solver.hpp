@@ -108,12 +108,13 @@ int build_hierarchy(const scy_grid_desc& g, const std::vector<double>& y, const 
 struct FDPrecond;
 
 // How much of a solve a call does.  norm_ready: scal[0] already holds (in
-// stream order) the sum of squares of the rhs.  enqueue: launch the residual
+// stream order) the sum of squares of the rhs.  resid_ready (where corrects()):
+// cg_r and scal[5] the residual of u and its sum of squares besides.  enqueue: launch the residual
 // and the first iteration and return without reading anything; the scalars
 // scal[0], [1], [5] then say whether that was enough.  first: resume such a
 // solve, with its scal[0..5] as read.
 struct SolvePart {
-  int norm_ready = 0, enqueue = 0;
+  int norm_ready = 0, resid_ready = 0, enqueue = 0;
   const double* first = nullptr;
 };
 
@@ -137,6 +138,13 @@ struct SbpContext {
   // (measured: 1e-3 at 401 and 1e-2 at 33 rows of the stretched grids, where
   // the bound is 0.005 and 0.05).  Beyond it (a grid whose spacing changes by
   // half from one row to the next), and for operators that are not separable, CG.
+  bool uses_fd(const scy_solve_opts& o) const {
+    return o.precond == SCY_PC_FD || (o.precond == SCY_PC_AUTO && separable);
+  }
+  // a solve by defect correction (correct())
+  bool corrects(const scy_solve_opts& o) const {
+    return uses_fd(o) && o.precision == SCY_PREC_FP64 && near_inverse() && !keeps_rounding(o.rtol);
+  }
   bool near_inverse() const { return separable && sep_misfit <= 0.25; }
   // Solves that keep the arithmetic of plain CG with whole sweep chains: those of the
   // power-law driver (keep_rounding: its viscous strain gVxz starts as a

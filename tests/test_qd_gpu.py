@@ -64,6 +64,30 @@ def test_d_dt_matches_oracle(tmp_path, law, grid, prestress, exact):
         assert _nrel(dev.field("surfDisp"), ora.u[::P["Nz"]]) <= REL
 
 
+@pytest.mark.parametrize("n,grid,rpt", [(17, "constantGridSpacing", 1), (33, "variableGridSpacing", 1),
+                                        (61, "constantGridSpacing", 2), (61, "variableGridSpacing", 4),
+                                        (130, "constantGridSpacing", 4), (137, "variableGridSpacing", 2)])
+def test_d_dt_with_rhs_and_residual_in_one_launch(tmp_path, monkeypatch, n, grid, rpt):
+    """Solves by defect correction (tolerance 1e-12) start from the rhs and
+    residual that one launch makes, here in tiles of 8, 16 and 32 rows, on
+    grids of one partial tile up to ones with interior tiles.  The solve's
+    1e-12 grows by about 10 in the stress and by tau / (a sN), about 40, in
+    the velocity: 4e-10, within the tolerance of 1e-9."""
+    from scycle_b200.qd import QD
+    monkeypatch.setenv("SCY_FULL_RPT", str(rpt))
+    P = _problem(tmp_path, n=n, grid=grid, prestress=26.5)
+    ora = QDLinearElastic(P, keep_history=False)
+    dev = QD(P, solve_rtol=1e-12, exact_jacobian=True)
+    rng = np.random.default_rng(n)
+    for t in (0.0, 3.0e7, 1.1e9):
+        psi = P["psi"] + 1e-3 * rng.standard_normal(P["Nz"])
+        slip = 0.05 * rng.random(P["Nz"])
+        fo = ora.d_dt(t, {"psi": psi, "slip": slip})
+        fd = dev.d_dt(t, psi, slip)
+        assert _rel(fd["slip"], fo["slip"], 1e-30) <= REL
+        assert _nrel(fd["psi"], fo["psi"]) <= REL
+
+
 @pytest.mark.parametrize("law,exact", [("agingLaw", False), ("slipLaw", True)])
 def test_fault_d_dt_alone_matches_oracle(tmp_path, law, exact):
     """Fault_qd::d_dt on its own (scy_qd_fault_d_dt): given the body's shear
