@@ -10,8 +10,9 @@
 // take alone.
 //
 // A stage d_dt of a group: boundary data and rhs (with its norm), the
-// residual of the warm start, `its` preconditioned CG iterations, the
-// device convergence test, and the fault update (linear elastic) or the
+// residual of the warm start (carried over from the stage before where the
+// solves are defect corrections), `its` defect corrections or preconditioned
+// CG iterations, the device convergence test, and the fault update (linear elastic) or the
 // viscous rates and fault update (power law), following
 // StrikeSlip_LinearElastic_qd::d_dt (strikeSlip_linearElastic_qd.cpp:756-798)
 // and StrikeSlip_PowerLaw_qd::d_dt (strikeSlip_powerLaw_qd.cpp:633-690).
@@ -680,7 +681,7 @@ __global__ void b_fault_kernel(LevelDev<double> L, const BatchInst* __restrict__
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= I.fp.Nz) return;
   const double sxy = I.c1 ? I.sxy[iz] : fault_row_sxy(L, I.u, iz);
-  fault_node_update(iz, sxy, I.fp, I.rk[in_slot], I.rk[out_slot], I.slipVel, I.tauQSP, I.tauP, I.strength, I.flags,
+  fault_node_update(iz, sxy, I.fp, I.rk[in_slot][I.fp.psi_off + iz], I.rk[out_slot], I.slipVel, I.tauQSP, I.tauP, I.strength, I.flags,
                     I.fault_its);
 }
 

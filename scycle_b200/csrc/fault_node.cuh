@@ -7,16 +7,15 @@
 namespace scy {
 
 // Fault_qd::d_dt for one node given its quasi-static shear stress from the
-// body (fault.cpp:861-918): prestress, bracketed Newton, state law, tauP,
+// body and its state psi (fault.cpp:861-918): prestress, bracketed Newton, state law, tauP,
 // strength.  Lane 0 of the four stores.
 __device__ __forceinline__ void fault_node_update(int iz, double tau_body, const FaultParams& fp,
-                                                  const double* __restrict__ var, double* __restrict__ f,
+                                                  double psi, double* __restrict__ f,
                                                   double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                                   double* __restrict__ tauP, double* __restrict__ strength,
                                                   unsigned* flags, unsigned long long* its_total) {
   const bool out = (threadIdx.x & 3) == 0;
   const double tq = tau_body + fp.prestress[iz];
-  const double psi = var[fp.psi_off + iz];
   const double a = fp.a[iz], sN = fp.sN[iz], eta = fp.eta[iz];
   const double E = exp(psi / a), V0 = slipVel[iz];
   __syncwarp(node_lanes());  // every lane has V0 before lane 0 overwrites it

@@ -1,7 +1,7 @@
 // FP64-accurate products on the integer tensor cores (see ozaki.hpp).
 //
-// ozk_gemm_kernel<S, T>: one CTA of 128 threads per output tile of 128 rows
-// x CN columns.  Thread 0 of warp 0 streams 64-byte K slices of the S digit
+// ozk_gemm_kernel<S, T>: one CTA of 128 threads (256 for the narrow tiles) per
+// output tile of 128 rows x CN columns.  Thread 0 of warp 0 streams 64-byte K slices of the S digit
 // planes of both operands into a ring of shared-memory stages by TMA
 // (cp.async.bulk.tensor, 64-byte swizzle, completion on an mbarrier per
 // stage); thread 0 of warp 1 issues, per stage and per 32-byte K step, the
@@ -11,7 +11,7 @@
 // (the products of one X plane with a stack of W planes as one MMA of N up
 // to 256, see ozk_issue_kstep), and frees each stage with tcgen05.commit on
 // its "empty" mbarrier.  After
-// the last stage all four warps read their 32 rows of the accumulators
+// the last stage all warps read their 32 rows of the accumulators
 // (tcgen05.ld 32x32b), combine the groups with their powers of two, apply
 // the row and column exponents (loaded by warps 2 and 3 while the products
 // run) and store their row segments.

@@ -42,7 +42,7 @@ __global__ void pl_fault_kernel(const double* __restrict__ sxy, FaultParams fp, 
   chain_enter();
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
-  fault_node_update(iz, sxy[iz], fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
+  fault_node_update(iz, sxy[iz], fp, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags, its_total);
 }
 
 int pl_d_dt(QDContext& q, double t, const double* var, double* f) {

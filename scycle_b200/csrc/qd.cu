@@ -138,7 +138,7 @@ __global__ void qd_fault_kernel(LevelDev<double> L, const double* __restrict__ u
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
   const double sxy = fault_row_sxy(L, u, iz);
-  fault_node_update(iz, sxy, fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
+  fault_node_update(iz, sxy, fp, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags, its_total);
 }
 
 // Fault_qd::d_dt with the body's shear stress on the fault given by the
@@ -151,7 +151,7 @@ __global__ void qd_fault_given_tau_kernel(const double* __restrict__ tau_body, F
   chain_enter();
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= fp.Nz) return;
-  fault_node_update(iz, tau_body[iz], fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
+  fault_node_update(iz, tau_body[iz], fp, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags, its_total);
 }
 
 int QDContext::fault_d_dt(const double* var, const double* tau_body, double* f) {
@@ -183,27 +183,77 @@ __global__ void qd_response_column_kernel(LevelDev<double> L, const double* __re
   if (i < Ny && surf) surf[(long)i * ld + col] = u[(long)i * Nz];
 }
 
+// A stage's state: var + sum_j c_j f_j (var itself with no terms)
+struct Combo {
+  const double* f[5];
+  double c[5];
+  int nf;
+};
+__device__ __forceinline__ double combine(const double* __restrict__ var, const Combo& cb, long i) {
+  double v = var[i], x[5];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) x[j] = j < cb.nf ? cb.f[j][i] : 0.0;  // all in flight together
+#pragma unroll
+  for (int j = 0; j < 5; ++j)
+    if (j < cb.nf) v = cb.c[j] * x[j] + v;
+  return v;
+}
+
 // Fault-response d_dt: one warp per fault node forms
 // tau = GL[iz,:] . (slip/faultTypeScale) + c g1[iz] + gs[iz], its first four
-// lanes then run the fault update.
-__global__ void qd_green_kernel(const double* __restrict__ GL, const double* __restrict__ g1,
-                                const double* __restrict__ gs, double c, double inv_fts, FaultParams fp,
-                                const double* __restrict__ var, double* __restrict__ f, double* __restrict__ slipVel,
-                                double* __restrict__ tauQSP, double* __restrict__ tauP, double* __restrict__ strength,
-                                double* __restrict__ bcL, unsigned* flags, unsigned long long* its_total) {
+// lanes then run the fault update.  The stage's state is combined here (and
+// kept in k where it has terms): the block puts the slip of all nodes in
+// shared memory, kGreenCols at a time, so a stage is one launch.  GL is laid
+// out before any step: its first kGreenPre entries per lane are requested
+// ahead of the wait for the kernel before.  Bound by latency (the state's
+// loads, the dot product, the root): at 401 nodes 8 steps of RK43 took 659 us
+// with a launch for each combination and the error sums, 616 so (625 with
+// four warps a block).
+constexpr int kGreenWarps = 8, kGreenCols = 1024, kGreenPre = 16;
+__global__ void __launch_bounds__(32 * kGreenWarps)
+    qd_green_kernel(const double* __restrict__ GL, const double* __restrict__ g1, const double* __restrict__ gs,
+                    double c, double inv_fts, FaultParams fp, const double* __restrict__ var, Combo cb,
+                    double* __restrict__ k, double* __restrict__ f, double* __restrict__ slipVel,
+                    double* __restrict__ tauQSP, double* __restrict__ tauP, double* __restrict__ strength,
+                    double* __restrict__ bcL, unsigned* flags, unsigned long long* its_total) {
+  __shared__ double sm[kGreenCols];
+  const int Nz = fp.Nz, lane = threadIdx.x & 31;
+  const int iz = blockIdx.x * kGreenWarps + (threadIdx.x >> 5);
+  const double* row = GL + (long)(iz < Nz ? iz : 0) * Nz;
+  double gl[kGreenPre];
+#pragma unroll
+  for (int m = 0; m < kGreenPre; ++m) gl[m] = lane + 32 * m < Nz ? row[lane + 32 * m] : 0.0;
   chain_enter();
-  const int Nz = fp.Nz;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= Nz) return;
-  const double* row = GL + (long)warp * Nz;
-  const double* slip = var + fp.slip_off;
+  const int own = iz < Nz ? iz : 0;
+  const double slip = combine(var, cb, fp.slip_off + own), psi = combine(var, cb, fp.psi_off + own);
+  const double tau0 = c * g1[own] + gs[own];
   double acc = 0.0;
-  for (int j = lane; j < Nz; j += 32) acc += row[j] * (slip[j] * inv_fts);
+  for (int j0 = 0; j0 < Nz; j0 += kGreenCols) {
+    const int n = min(kGreenCols, Nz - j0);
+    if (j0 > 0) __syncthreads();
+#pragma unroll 2
+    for (int j = threadIdx.x; j < n; j += 32 * kGreenWarps) sm[j] = combine(var, cb, fp.slip_off + j0 + j);
+    __syncthreads();
+    int j = lane;
+    if (j0 == 0) {
+#pragma unroll
+      for (int m = 0; m < kGreenPre; ++m, j += 32)
+        if (j < n) acc += gl[m] * (sm[j] * inv_fts);
+    }
+    for (; j < n; j += 32) acc += row[j0 + j] * (sm[j] * inv_fts);
+  }
+  if (iz >= Nz) return;
   acc = warp_sum(acc);
   if (lane < 4) {
-    if (lane == 0) bcL[warp] = slip[warp] * inv_fts;  // kept for output fields
-    const double tau = acc + (c * g1[warp] + gs[warp]);
-    fault_node_update(warp, tau, fp, var, f, slipVel, tauQSP, tauP, strength, flags, its_total);
+    if (lane == 0) {
+      bcL[iz] = slip * inv_fts;  // kept for output fields
+      if (cb.nf > 0) {
+        k[fp.slip_off + iz] = slip;
+        k[fp.psi_off + iz] = psi;
+      }
+    }
+    const double tau = acc + tau0;
+    fault_node_update(iz, tau, fp, psi, f, slipVel, tauQSP, tauP, strength, flags, its_total);
   }
 }
 
@@ -249,19 +299,11 @@ int QDContext::full_solve_for_output() {
 }
 
 // out = ((var + c0 f0) + c1 f1) + ... in the reference's WAXPY/AXPY order
-struct Combo {
-  const double* f[5];
-  double c[5];
-  int nf;
-};
-
 __global__ void rk_combine_kernel(double* __restrict__ out, const double* __restrict__ var, Combo cb, long n) {
   chain_enter();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double v = cb.c[0] * cb.f[0][i] + var[i];
-  for (int j = 1; j < cb.nf; ++j) v = v + cb.c[j] * cb.f[j][i];
-  out[i] = v;
+  out[i] = combine(var, cb, i);
 }
 
 // Per integrated field (block b handles SCY_KEY b at [off[b], off[b]+len[b])):
@@ -274,17 +316,19 @@ struct KeyTable {
 // the fault flags, and the records of an attempt's enqueued solves
 enum { RB_FLAGS = 13, RB_SOLVE = 16, RB_SIZE = RB_SOLVE + 3 * 6 };
 
-__global__ void rk_error_kernel(const double* __restrict__ lo, const double* __restrict__ hi, KeyTable kt,
-                                const unsigned* __restrict__ flags, double* __restrict__ out) {
-  chain_enter();
+// Block b's field with at(i, lo, hi) giving the two solutions at index i
+template <class At>
+__device__ __forceinline__ void error_sums(const KeyTable& kt, const unsigned* __restrict__ flags,
+                                           double* __restrict__ out, const At& at) {
   __shared__ double sh[32];
   const int key = blockIdx.x;
   if (key == 0 && threadIdx.x == 0) out[RB_FLAGS] = (double)(flags[0] | flags[1]);  // read back with the sums
   const long off = kt.off[key], len = kt.len[key];
   double ss = 0.0, sh2 = 0.0, mx = -INFINITY;
   for (long i = threadIdx.x; i < len; i += blockDim.x) {
-    double h = hi[off + i];
-    double d = lo[off + i] - h;
+    double l, h;
+    at(off + i, l, h);
+    double d = l - h;
     ss += d * d;
     sh2 += h * h;
     double r = fabs(d) / h;
@@ -305,6 +349,26 @@ __global__ void rk_error_kernel(const double* __restrict__ lo, const double* __r
       out[key * 3 + 2] = t;
     }
   }
+}
+
+__global__ void rk_error_kernel(const double* __restrict__ lo, const double* __restrict__ hi, KeyTable kt,
+                                const unsigned* __restrict__ flags, double* __restrict__ out) {
+  chain_enter();
+  error_sums(kt, flags, out, [&](long i, double& l, double& h) {
+    l = lo[i];
+    h = hi[i];
+  });
+}
+
+__global__ void __launch_bounds__(1024) rk_finish_kernel(double* __restrict__ lo, double* __restrict__ hi,
+                                                         const double* __restrict__ var, Combo cl, Combo ch,
+                                                         KeyTable kt, const unsigned* __restrict__ flags,
+                                                         double* __restrict__ out) {
+  chain_enter();
+  error_sums(kt, flags, out, [&](long i, double& l, double& h) {
+    lo[i] = l = combine(var, cl, i);
+    hi[i] = h = combine(var, ch, i);
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -497,16 +561,7 @@ int QDContext::d_dt(double t, const double* var, double* f) {
   }
   if (mode == SCY_QD_MODE_RESPONSE) {
     if (!green_ready) SCY_TRY(build_green());
-    const double c = bcR_remote ? vL * t * (1.0 / fts) : 0.0;
-    const int wpb = 4;
-    chain_launch(qd_green_kernel, (Nz + wpb - 1) / wpb, 32 * wpb, 0, s, GL.as<double>(), g1.as<double>(),
-                 gs.as<double>(), c, 1.0 / fts, fp, var, f, slipVel.as<double>(), tauQSP.as<double>(),
-                 tauP.as<double>(), strength.as<double>(), bcL.as<double>(), flags.as<unsigned>(),
-                 fault_its.as<unsigned long long>());
-    SCY_LAUNCH_CHECK();
-    flags_known = 0;
-    last_t = t;
-    ++n_d_dt;
+    SCY_TRY(green_stage(t, var, Combo{}, nullptr, f));
     return SCY_OK;
   }
   SCY_TRY(solve_stage(t, var, nullptr, nullptr, [&]() -> int {
@@ -520,6 +575,32 @@ int QDContext::d_dt(double t, const double* var, double* f) {
   last_t = t;
   ++n_d_dt;
   return SCY_OK;
+}
+
+// d_dt in response mode at var + the terms of cb (then kept in k)
+int QDContext::green_stage(double t, const double* var, const Combo& cb, double* k, double* f) {
+  const double c = bcR_remote ? vL * t * (1.0 / fts) : 0.0;
+  chain_launch(qd_green_kernel, (Nz + kGreenWarps - 1) / kGreenWarps, 32 * kGreenWarps, 0, sbp.stream,
+               GL.as<double>(), g1.as<double>(), gs.as<double>(), c, 1.0 / fts, fp, var, cb, k, f,
+               slipVel.as<double>(), tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), bcL.as<double>(),
+               flags.as<unsigned>(), fault_its.as<unsigned long long>());
+  SCY_LAUNCH_CHECK();
+  flags_known = 0;
+  last_t = t;
+  ++n_d_dt;
+  return SCY_OK;
+}
+
+// One stage of an attempt: k = var + the terms of cb, f = d_dt(t, k)
+int QDContext::stage(double t, const Combo& cb, double* k, double* f) {
+  const double* var = rk[V_VAR].as<double>();
+  if (mode == SCY_QD_MODE_RESPONSE && !pl && green_ready && fp.state_law != SCY_LAW_FLASH) {
+    ++u_epoch;
+    return green_stage(t, var, cb, k, f);
+  }
+  chain_launch(rk_combine_kernel, (int)((nvar + 255) / 256), 256, 0, sbp.stream, k, var, cb, nvar);
+  SCY_LAUNCH_CHECK();
+  return d_dt(t, k, f);
 }
 
 // The elliptic solve of one d_dt (boundary data and rhs from the state, the
@@ -827,14 +908,22 @@ double QDContext::compute_step_size(double totErr) {
   return dt;
 }
 
-int QDContext::launch_error(const double* lo, const double* hi) {
-  cudaStream_t s = sbp.stream;
+KeyTable QDContext::key_table() const {
   KeyTable kt;
   for (int k = 0; k < 4; ++k) {
     kt.off[k] = key_off[k];
     kt.len[k] = key_len[k];
   }
-  chain_launch(rk_error_kernel, pl ? 4 : 2, 1024, 0, s, lo, hi, kt, flags.as<unsigned>(), errbuf.as<double>());
+  return kt;
+}
+
+int QDContext::launch_error(const double* lo, const double* hi) {
+  if (errors_ready) {  // came with the attempt's solutions
+    errors_ready = 0;
+    return SCY_OK;
+  }
+  chain_launch(rk_error_kernel, pl ? 4 : 2, 1024, 0, sbp.stream, lo, hi, key_table(), flags.as<unsigned>(),
+               errbuf.as<double>());
   SCY_LAUNCH_CHECK();
   return SCY_OK;
 }
@@ -880,30 +969,39 @@ static Combo combo(std::initializer_list<std::pair<const double*, double>> terms
 }
 
 
-int QDContext::attempt(double dt, double** lo, double** hi) {
+// The attempt's two solutions, and where the state is the fault's alone its
+// error sums in the same launch (a block per field, as rk_error_kernel)
+int QDContext::solutions(const Combo& cl, const Combo& ch) {
   cudaStream_t s = sbp.stream;
-  const long n = nvar;
-  const int tb = 256, gb = (int)((n + tb - 1) / tb);
-  double* var = rk[V_VAR].as<double>();
+  const double* var = rk[V_VAR].as<double>();
+  double *L = rk[V_LO].as<double>(), *H = rk[V_HI].as<double>();
+  if (!pl && nvar == key_len[SCY_KEY_PSI] + key_len[SCY_KEY_SLIP]) {
+    chain_launch(rk_finish_kernel, 2, 1024, 0, s, L, H, var, cl, ch, key_table(), flags.as<unsigned>(),
+                 errbuf.as<double>());
+    SCY_LAUNCH_CHECK();
+    errors_ready = 1;
+    return SCY_OK;
+  }
+  const int gb = (int)((nvar + 255) / 256);
+  chain_launch(rk_combine_kernel, gb, 256, 0, s, L, var, cl, nvar);
+  SCY_LAUNCH_CHECK();
+  chain_launch(rk_combine_kernel, gb, 256, 0, s, H, var, ch, nvar);
+  SCY_LAUNCH_CHECK();
+  return SCY_OK;
+}
+
+int QDContext::attempt(double dt, double** lo, double** hi) {
   double* f0 = rk[V_DVAR].as<double>();
   double* k = rk[V_K].as<double>();
-  double* L = rk[V_LO].as<double>();
-  double* H = rk[V_HI].as<double>();
   const double t = currT;
+  errors_ready = 0;
   if (ode.method == SCY_RK32) {
     double* fa = rk[V_F1].as<double>();
     double* fb = rk[V_F2].as<double>();
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, 0.5 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    SCY_TRY(d_dt(t + 0.5 * dt, k, fa));
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, -dt}, {fa, 2 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    SCY_TRY(d_dt(t + dt, k, fb));
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, L, var, combo({{f0, 0.5 * dt}, {fb, 0.5 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, H, var, combo({{f0, dt / 6.0}, {fa, 2 * dt / 3.0}, {fb, dt / 6.0}}),
-                 n);
-    SCY_LAUNCH_CHECK();
+    SCY_TRY(stage(t + 0.5 * dt, combo({{f0, 0.5 * dt}}), k, fa));
+    SCY_TRY(stage(t + dt, combo({{f0, -dt}, {fa, 2 * dt}}), k, fb));
+    SCY_TRY(solutions(combo({{f0, 0.5 * dt}, {fb, 0.5 * dt}}),
+                      combo({{f0, dt / 6.0}, {fa, 2 * dt / 3.0}, {fb, dt / 6.0}})));
   } else {
     using namespace rk43;
     double* f2 = rk[V_F2].as<double>();
@@ -911,32 +1009,17 @@ int QDContext::attempt(double dt, double** lo, double** hi) {
     double* f4 = rk[V_F4].as<double>();
     double* f5 = rk[V_F5].as<double>();
     double* f6 = rk[V_F6].as<double>();
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a21 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    SCY_TRY(d_dt(t + c2 * dt, k, f2));
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a31 * dt}, {f2, a32 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    SCY_TRY(d_dt(t + c3 * dt, k, f3));
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a41 * dt}, {f2, a42 * dt}, {f3, a43 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    SCY_TRY(d_dt(t + c4 * dt, k, f4));
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a51 * dt}, {f2, a52 * dt}, {f3, a53 * dt}, {f4,
-                 a54 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    SCY_TRY(d_dt(t + c5 * dt, k, f5));
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, k, var, combo({{f0, a61 * dt}, {f2, a62 * dt}, {f3, a63 * dt}, {f4,
-                 a64 * dt}, {f5, a65 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    SCY_TRY(d_dt(t + c6 * dt, k, f6));
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, L, var, combo({{f0, hb1 * dt}, {f3, hb3 * dt}, {f4, hb4 * dt}, {f5,
-                 hb5 * dt}, {f6, hb6 * dt}}), n);
-    SCY_LAUNCH_CHECK();
-    chain_launch(rk_combine_kernel, gb, tb, 0, s, H, var, combo({{f0, b1 * dt}, {f3, b3 * dt}, {f4, b4 * dt}, {f5,
-                 b5 * dt}, {f6, b6 * dt}}), n);
-    SCY_LAUNCH_CHECK();
+    SCY_TRY(stage(t + c2 * dt, combo({{f0, a21 * dt}}), k, f2));
+    SCY_TRY(stage(t + c3 * dt, combo({{f0, a31 * dt}, {f2, a32 * dt}}), k, f3));
+    SCY_TRY(stage(t + c4 * dt, combo({{f0, a41 * dt}, {f2, a42 * dt}, {f3, a43 * dt}}), k, f4));
+    SCY_TRY(stage(t + c5 * dt, combo({{f0, a51 * dt}, {f2, a52 * dt}, {f3, a53 * dt}, {f4, a54 * dt}}), k, f5));
+    SCY_TRY(stage(t + c6 * dt,
+                  combo({{f0, a61 * dt}, {f2, a62 * dt}, {f3, a63 * dt}, {f4, a64 * dt}, {f5, a65 * dt}}), k, f6));
+    SCY_TRY(solutions(combo({{f0, hb1 * dt}, {f3, hb3 * dt}, {f4, hb4 * dt}, {f5, hb5 * dt}, {f6, hb6 * dt}}),
+                      combo({{f0, b1 * dt}, {f3, b3 * dt}, {f4, b4 * dt}, {f5, b5 * dt}, {f6, b6 * dt}})));
   }
-  *lo = L;
-  *hi = H;
+  *lo = rk[V_LO].as<double>();
+  *hi = rk[V_HI].as<double>();
   return SCY_OK;
 }
 

@@ -35,6 +35,9 @@ constexpr double a61 = 647845179188. / 3216320057751., a62 = 73281519250. / 8382
 struct QDProblem;
 struct ThermalContext;
 
+struct Combo;     // a stage's state (qd.cu)
+struct KeyTable;  // the integrated fields' ranges
+
 struct QDContext {
   SbpContext sbp;
   int Ny = 0, Nz = 0;
@@ -154,6 +157,11 @@ struct QDContext {
   double compute_step_size(double totErr);
   int compute_error(const double* lo, const double* hi, double* err);
   int launch_error(const double* lo, const double* hi);
+  KeyTable key_table() const;
+  int errors_ready = 0;  // the last attempt's error sums are on their way (solutions())
+  int green_stage(double t, const double* var, const Combo& cb, double* k, double* f);
+  int stage(double t, const Combo& cb, double* k, double* f);
+  int solutions(const Combo& cl, const Combo& ch);
   int attempt_deferred(double dt, double** lo, double** hi, double* err, int* ok);
   int solve_stage(double t, const double* var, const double* gxy, const double* gxz,
                   const std::function<int()>& after);

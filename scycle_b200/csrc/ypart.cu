@@ -333,17 +333,20 @@ int YPart::build(const std::vector<double>& L, int Ny_, int Nz, int Nzp_, cudaSt
   nb = (Nzp + MB - 1) / MB;
   const size_t S = T * kRow + 2, blk = (size_t)P * MB * S;
   std::vector<double> Tb((size_t)nb * blk, 0.0), W((size_t)nb * 32 * MB, 0.0);
-  std::vector<double> col(T);
+  std::vector<double> col(T), Lj((size_t)Ny * 9);
   for (int j = 0; j < Nz; ++j) {
+    // the mode's factor in one piece: its entries are read up to nine times
+    for (size_t i = 0; i < Lj.size(); ++i) Lj[i] = L[i * Nz + j];
+    auto lj = [&](int i, int k) { return Lj[(size_t)i * 9 + k]; };
     const int jb = j / MB, md = j % MB;
     for (int sg = 0; sg < P; ++sg) {
       const int r0 = row0(sg), nr = rows(sg);
       double* c = &Tb[(size_t)jb * blk + (size_t)(sg * MB + md) * S + (size_t)(T - nr) * kRow];
       for (int r = 0; r < nr; ++r) {
         // off-diagonals to rows of this segment (those to earlier ones are in G)
-        for (int k = 0; k < 5; ++k) c[r * kRow + k] = r >= k ? at(r0 + r, k, j) : 0.0;
+        for (int k = 0; k < 5; ++k) c[r * kRow + k] = r >= k ? lj(r0 + r, k) : 0.0;
         if (const int wr = wide_row(sg, r); wr >= 0)
-          for (int k = 5; k <= 8 && k <= r; ++k) W[((size_t)jb * 32 + wr * 4 + k - 5) * MB + md] = at(r0 + r, k, j);
+          for (int k = 5; k <= 8 && k <= r; ++k) W[((size_t)jb * 32 + wr * 4 + k - 5) * MB + md] = lj(r0 + r, k);
       }
       // G: rows of this segment for a one in row r0 - 1 - d and no data
       if (sg > 0)
@@ -353,9 +356,9 @@ int YPart::build(const std::vector<double>& L, int Ny_, int Nz, int Nzp_, cudaSt
             for (int k = 1; k <= 8; ++k) {
               const int p = r - k;  // row of the segment; -1 - d is the incoming one
               const double v = p >= 0 ? col[p] : p == -1 - d ? 1.0 : 0.0;
-              if (v != 0.0) sum -= at(r0 + r, k, j) * v;
+              if (v != 0.0) sum -= lj(r0 + r, k) * v;
             }
-            col[r] = sum * at(r0 + r, 0, j);
+            col[r] = sum * lj(r0 + r, 0);
             c[r * kRow + 5 + d] = col[r];
           }
       // B: the same upwards for a one in row r0 + nr + d
@@ -367,9 +370,9 @@ int YPart::build(const std::vector<double>& L, int Ny_, int Nz, int Nzp_, cudaSt
               const int p = r + k;
               if (r0 + p >= Ny) break;
               const double v = p < nr ? col[p] : p == nr + d ? 1.0 : 0.0;
-              if (v != 0.0) sum -= at(r0 + p, k, j) * v;
+              if (v != 0.0) sum -= lj(r0 + p, k) * v;
             }
-            col[r] = sum * at(r0 + r, 0, j);
+            col[r] = sum * lj(r0 + r, 0);
             c[r * kRow + 9 + d] = col[r];
           }
     }

@@ -229,3 +229,27 @@ def test_response_mode_d_dt_matches_solve_mode(tmp_path):
         assert _rel(fb["slip"], fa["slip"], 1e-30) <= REL
         assert _rel(fb["psi"], fa["psi"], 1e-12) <= REL
         assert _rel(b.field("tauQSP"), a.field("tauQSP"), 1e-9) <= REL
+
+
+@pytest.mark.parametrize("Nz", [511, 512, 513, 1024])
+def test_response_mode_at_the_kernels_edges(tmp_path, Nz):
+    """Faults of as many nodes as the response kernel's warps hold ahead in
+    registers (512), one less and one more, and as many as its blocks hold in
+    shared memory (1024, also the most z lines that the solver's products
+    take): the stress against the matrix-free solve's, velocity and state rate with it
+    (both solves to 1e-13; tau / (a sN), about 40, times that, times the 10 by
+    which a residual may exceed its error, is 4e-11)."""
+    from scycle_b200.qd import QD
+    p = make_qd_problem(str(tmp_path), Ny=17, Nz=Nz, state_law="agingLaw", integrator="RK32",
+                        grid="constantGridSpacing")
+    P = build_qd_problem(open(p).read())
+    P["prestress"] = np.full(Nz, 27.0) + np.linspace(0, 0.5, Nz)
+    a, b = QD(P, solve_rtol=1e-13), QD(P, solve_rtol=1e-13)
+    b.set_mode("response")
+    rng = np.random.default_rng(Nz)
+    psi = P["psi"] + 1e-3 * rng.standard_normal(Nz)
+    slip = 0.05 * np.sin(np.linspace(0.0, 7.0, Nz)) ** 2
+    fa, fb = a.d_dt(5.0e8, psi, slip), b.d_dt(5.0e8, psi, slip)
+    assert _rel(fb["slip"], fa["slip"], 1e-30) <= REL
+    assert _nrel(fb["psi"], fa["psi"]) <= REL
+    assert _rel(b.field("tauQSP"), a.field("tauQSP"), 1e-9) <= REL
