@@ -99,6 +99,26 @@ def test_solve_matches_direct_solve(order, grid, precision, precond):
     assert _rel(u.cpu().numpy(), ref) <= 1e-9
 
 
+@pytest.mark.parametrize("Ny,Nz,precision", [
+    (45, 45, "fp64"), (46, 45, "fp64"), (17, 120, "mixed"), (33, 65, "fp64"), (129, 17, "fp64"), (89, 91, "mixed"),
+    (90, 95, "fp64")])
+def test_multigrid_solve_at_level_edges(Ny, Nz, precision):
+    """Multigrid on a varying shear modulus where the first level, or the
+    first coarse one, has just under and just over the 2048 nodes up to which
+    a cycle's levels run in one cluster launch, few rows or columns for its
+    eight blocks, and odd sizes.  The solve stops at 1e-12 of the rhs, the
+    error may be larger by the operator's spread: the tolerance of the other
+    solves against the direct one."""
+    import scipy.sparse.linalg as spla
+    dev, ora, rng = _case(4, "constantGridSpacing", Ny, Nz, seed=Ny)
+    rhs = ora.set_rhs(rng.standard_normal(Nz), rng.standard_normal(Nz), rng.standard_normal(Ny),
+                      rng.standard_normal(Ny))
+    ref = spla.spsolve(ora.A.tocsc(), rhs)
+    u, st = dev.solve(rhs, rtol=1e-12, max_its=400, precision=precision, precond="mg")
+    assert st.converged
+    assert _rel(u.cpu().numpy(), ref) <= 1e-9
+
+
 @pytest.mark.parametrize("rpt,grid,mu_kind", list(itertools.product(
     (1, 2, 4), ("constantGridSpacing", "variableGridSpacing"), ("constant", "one_column"))))
 def test_full_form_every_rows_per_thread(monkeypatch, rpt, grid, mu_kind):
