@@ -192,7 +192,7 @@ def oracle_errors(name, make, rtol=PARITY_RTOL, batch_precision=None):
 
 
 # ---------------------------------------------------------------------------
-ZT_DESC = ("ozk_gemm_kernel (z transforms of the preconditioner on the integer tensor cores: tcgen05 kind::i8 "
+ZT_DESC = ("ozk_gemm_kernel / ozk_gemm_pers_kernel (z transforms of the preconditioner on the integer tensor cores: tcgen05 kind::i8 "
            "digit-plane products, TMA-fed, tensor-memory accumulators; two per apply)")
 ZS_DESC = "ozk_split_kernel (digit planes of the z-transform operand, the row held in registers; two per apply)"
 BATCH_WORKLOAD = ("slip_var_401 ensemble: %d instances per GPU of the 401x401 stretched-grid slip-law workload "
@@ -289,18 +289,22 @@ def run_batched(args, dist, rank, world, local):
     # ncu captures of these kernels at 32 instances of the 401 x 401 workload
     # (profiles/batched_ensemble_kernels_401x401.md,
     # profiles/ozk_gemm_kernel_S5_12832x401x401.md,
-    # profiles/b_full_kernel_32x401x401.md); other sizes report none
+    # profiles/b_full_kernel_32x401x401.md,
+    # profiles/march_walks_2049x1537_and_32x401x401.md); other sizes report none
     sep = b.tuning(0)["operator_form"] != "cross"
+    corr = sep and args.batch_precision == "fp64"  # defect corrections instead of CG on this workload
     traffic = {"ysolve": 65362176.0, "ztransform": 28774656.0} if (args.batch == 32 and args.n == 401) else {}
     if args.batch == 32 and args.n == 401:
-        traffic.update({"matvec": 99618816.0, "residual": 98234880.0} if sep else
+        traffic.update({"matvec": 150265600.0 if corr else 99618816.0, "residual": 98234880.0} if sep else
                        {"matvec": 178643456.0, "residual": 187187968.0})
-    opk = "b_full_kernel<%d> (separable form: 1D coefficient tables, register window along y)" if sep else \
+    opk = "b_full_kernel<%d> (separable form: 1D coefficient tables, tiles or walks by warps)" if sep else \
         "b_cross_kernel<%d> (cross form: 33 coefficient planes)"
     kern = {}
     for nm, desc in (("ysolve", "b_ysolve_tma_kernel (banded Cholesky sweeps along y of the preconditioner)"),
-                     ("matvec", (opk % 1) + ", CG operator application, p update fused"),
-                     ("residual", (opk % 0) + ", initial residual of each stage solve"),
+                     ("matvec", (opk % 2) + ", defect correction u += z, r += A z" if corr else
+                      (opk % 1) + ", CG operator application, p update fused"),
+                     ("residual", (opk % 0) + (", residual once per accepted step" if corr else
+                                               ", initial residual of each stage solve")),
                      ("ztransform", ZT_DESC), ("zsplit", ZS_DESC)):
         pm, pl, pb = b.profile_collect(nm)
         if pl:
