@@ -684,15 +684,19 @@ scy_status scy_batch_set_sweep_test(scy_batch* b, int polls, int drop_first_copy
  * the cross form (33 coefficient planes) with 1, 2, 4 and 8 instances per
  * block and, when the operator is separable over every node, in the
  * separable form (1D coefficient tables) with 1, 2, 16 and 32 rows per thread,
- * the banded sweeps in six launch shapes (whole chains; chains per lane x warps per block:
- * 2 x 2, 1 x 4, 4 x 1 serving 8 instances per block, 1 x 2 and 2 x 1
- * serving 4, 1 x 1 serving 2) and the z-transform product in three shapes
- * (one CTA per tile, two CTAs per SM, persistent: one CTA per SM with two
- * accumulator sets) with 8-bit or bf16 digits (identical results), and keeps
+ * the banded sweeps in six launch shapes (whole chains, sweep_variant 0-5:
+ * chains per lane x warps per block 2 x 2, 1 x 4, 4 x 1 serving 8 instances
+ * per block, 1 x 2 and 2 x 1 serving 4, 1 x 1 serving 2; with the FP64
+ * preconditioner and fewer than 10,000 chains in segments, 6-11: 1 or 2
+ * instances a thread x 1, 2 or 4 groups a block) and the z-transform product
+ * in four shapes (one CTA per tile, two CTAs per SM, persistent: one CTA per
+ * SM with two accumulator sets, narrow tiles where the others leave SMs
+ * without one) with 8-bit or bf16 digits (identical results), and keeps
  * the fastest.  kpb / sweep_variant / ztransform get the choices (kpb: the
  * cross form's, see scy_batch_operator_form for the form in use; ztransform
- * bit 0: two CTAs per SM, bit 1: bf16 digits, bit 2: persistent), us (22
- * doubles, may be NULL) the timings in microseconds per launch (cross form
+ * bit 0: two CTAs per SM, bit 1: bf16 digits, bit 2: persistent, bit 3:
+ * narrow tiles), us (22 doubles, may be NULL) the timings in microseconds per
+ * launch (cross form
  * at kpb 1, 2, 4, 8; sweep shapes 0-5; product with 8-bit digits, one and
  * two CTAs per SM; with bf16 digits, one and two CTAs per SM; separable form
  * at 1 and 2 rows per thread with the compiler's register count, then with
