@@ -96,33 +96,66 @@ struct FDFaultArgs {
 
 constexpr int kFaultBlock = 128;
 
+// What the update of a fault node reads besides the new displacements: its
+// chain of roots is the longest of the step, so these are requested ahead of
+// the tile's stencil (a step of 801 x 801 @W@).
+struct FDNode {
+  double rho, alphay, a, b, sN, Dc, eta, slip0, slipPrev, slip, tau0, psi, psiPrev, V0, locked, prestress, mu, qy,
+      u0[BAND - HALF];
+};
+__device__ __forceinline__ FDNode fd_fault_load(const FDFaultArgs& A, int iz) {
+  const FaultParams& fp = A.fp;
+  FDNode n;
+  n.rho = A.rho_f[iz];
+  n.alphay = A.alphay[iz];
+  n.a = fp.a[iz];
+  n.b = fp.b[iz];
+  n.sN = fp.sN[iz];
+  n.Dc = fp.Dc[iz];
+  n.eta = fp.eta[iz];
+  n.slip0 = A.slip0[iz];
+  n.slipPrev = A.slipPrev[iz];
+  n.slip = A.slip[iz];
+  n.tau0 = A.tau0[iz];
+  n.psi = A.psi[iz];
+  n.psiPrev = A.psiPrev[iz];
+  n.V0 = A.slipVel[iz];
+  n.locked = fp.locked[iz];
+  n.prestress = fp.prestress[iz];
+  n.mu = A.mu0[iz];
+  n.qy = A.var_grid ? A.qy0[iz] : 1.0;
+#pragma unroll
+  for (int k = 0; k < BAND - HALF; ++k) n.u0[k] = k < A.Ny ? A.u0[(long)k * fp.Nz + iz] : 0.0;
+  return n;
+}
+
 // Fault_fd::d_dt for fault node iz by its four lanes together (fault_dev.cuh;
 // lane 0 stores) (fault.cpp:1436-1575), the fault-row
 // stress of uNext + u0, tauQS and tauP; returns eta V / tauQS.  d2u is the
 // node's Hinv Jinv A u; un(k) returns uNext at body row k (k = 1..4).
 template <class Rows>
-__device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, int iz, double d2u, const Rows& un_row,
+__device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, const FDNode& N, int iz, double d2u,
+                                                const Rows& un_row,
                                                 unsigned* bad_out) {
   const FaultParams& fp = A.fp;
-  const int Nz = fp.Nz;
   CycleDevState* st = A.st;
   const double dt = A.dt;
-  const double rho = A.rho_f[iz], alphay = A.alphay[iz];
-  const double a = fp.a[iz], sN = fp.sN[iz], eta = fp.eta[iz];
-  const double slip0 = A.slip0[iz];
-  const double uPrev = (A.slipPrev[iz] - slip0) * A.inv_fts;
-  double u = (A.slip[iz] - slip0) * A.inv_fts;
+  const double rho = N.rho, alphay = N.alphay;
+  const double a = N.a, sN = N.sN, eta = N.eta;
+  const double slip0 = N.slip0;
+  const double uPrev = (N.slipPrev - slip0) * A.inv_fts;
+  double u = (N.slip - slip0) * A.inv_fts;
   // setPhi (fault.cpp:1527-1575)
-  const double an = d2u + A.tau0[iz] / alphay;
+  const double an = d2u + N.tau0 / alphay;
   const double Phi = 2.0 / dt * (u - uPrev) + dt * an / rho;
   const double fricPen = dt / alphay / rho;
-  const double psi = A.psi[iz];
+  const double psi = N.psi;
   const bool out = (threadIdx.x & 3) == 0;
-  const double V0 = fabs(A.slipVel[iz]), E = exp(psi / a);
+  const double V0 = fabs(N.V0), E = exp(psi / a);
   __syncwarp(node_lanes());  // every lane has V0 before lane 0 overwrites it
   // ComputeVel_fd::computeVel (fault.cpp:1594-1644)
   double V;
-  const double lk = fp.locked[iz];
+  const double lk = N.locked;
   unsigned bad = 0;
   if (lk > 0.5) {
     V = 0.0;
@@ -153,16 +186,16 @@ __device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, int iz, do
     u = (2. * u + (an * dt * dt / rho) + (dt * alpha - 1.) * uPrev) / Ad;
   }
   // ComputeAging_fd / ComputeSlipLaw_fd (fault.cpp:1702-1745, :1802-1846)
-  const double psiPrev = A.psiPrev[iz];
+  const double psiPrev = N.psiPrev;
   double psiN;
   {
     int its = 0;
     bool ok = true;
     if (fp.state_law == 0) {
-      const ResidAgingFD R2{psiPrev, V, fp.b[iz], fp.f0, fp.v0, fp.Dc[iz], dt};
+      const ResidAgingFD R2{psiPrev, V, N.b, fp.f0, fp.v0, N.Dc, dt};
       psiN = bracketed_newton_f(R2, -2.0, 2.0, psi, fp.root_tol, fp.max_its, &its, &ok);
     } else {
-      const ResidSlipFD R2{psiPrev, V, a, fp.b[iz], fp.f0, fp.v0, fp.Dc[iz], dt};
+      const ResidSlipFD R2{psiPrev, V, a, N.b, fp.f0, fp.v0, N.Dc, dt};
       psiN = bracketed_newton_f(R2, -2.0, 2.0, psi, fp.root_tol, fp.max_its, &its, &ok);
     }
     if (out) atomicAdd(&st->its, (unsigned long long)its);
@@ -182,11 +215,11 @@ __device__ __forceinline__ double fd_fault_node(const FDFaultArgs& A, int iz, do
     const int k = j - HALF;
     if (k < A.Ny) {
       const double un = k == 0 ? u : un_row(k);
-      d += A.D0[j] * (un + 1.0 * A.u0[(long)k * Nz + iz]);
+      d += A.D0[j] * (un + 1.0 * N.u0[k]);
     }
   }
-  if (A.var_grid) d *= A.qy0[iz];
-  const double tq = A.mu0[iz] * d + 1.0 * fp.prestress[iz];
+  if (A.var_grid) d *= N.qy;
+  const double tq = N.mu * d + 1.0 * N.prestress;
   if (out) {
     A.tauQSP[iz] = tq;
     A.tauP[iz] = -1.0 * (eta * V) + tq;
@@ -241,7 +274,7 @@ __global__ void __launch_bounds__(kFaultBlock) fd_fault_kernel(FDFaultArgs A) {
   if (iz < Nz) {
     unsigned bad = 0;
     auto rows = [&](int k) { return A.uNext[(long)k * Nz + iz]; };
-    R = fd_fault_node(A, iz, A.d2u[iz], rows, &bad);
+    R = fd_fault_node(A, fd_fault_load(A, iz), iz, A.d2u[iz], rows, &bad);
     if (bad && (threadIdx.x & 3) == 0) atomicOr(&st->flags, bad);
   }
   __shared__ double sh[32];
@@ -253,10 +286,16 @@ __global__ void __launch_bounds__(kFaultBlock) fd_fault_kernel(FDFaultArgs A) {
   fd_switch_test(A, b, gridDim.x);
 }
 
+// The thread's node of a fault tile, four lanes a node
+__device__ __forceinline__ FDNode fd_tile_node(const FDFaultArgs& A, int z0) {
+  const int iz = z0 + (threadIdx.x >> 2);
+  return threadIdx.x < 4 * TZ && iz < A.fp.Nz ? fd_fault_load(A, iz) : FDNode{};
+}
+
 // The fault update of a fault tile's 32 columns (z0 on) from the rows it just
 // computed, and the switch test
-__device__ __forceinline__ void fd_fault_tile(const FDFaultArgs& A, int z0, const double* s_rows, const double* s_d2u,
-                                              unsigned nblocks) {
+__device__ __forceinline__ void fd_fault_tile(const FDFaultArgs& A, const FDNode& N, int z0, const double* s_rows,
+                                              const double* s_d2u, unsigned nblocks) {
   __shared__ double s_max[4];
   __syncthreads();
   if (threadIdx.x < 4 * TZ) {
@@ -265,7 +304,7 @@ __device__ __forceinline__ void fd_fault_tile(const FDFaultArgs& A, int z0, cons
     if (iz < A.fp.Nz) {
       unsigned bad = 0;
       auto rows = [&](int k) { return s_rows[k * TZ + col]; };
-      R = fd_fault_node(A, iz, s_d2u[col], rows, &bad);
+      R = fd_fault_node(A, N, iz, s_d2u[col], rows, &bad);
       if (bad && (threadIdx.x & 3) == 0) atomicOr(&A.st->flags, bad);
     }
     R = warp_max(R);
@@ -293,13 +332,13 @@ __global__ void __launch_bounds__(256) fd_step_kernel(LevelDev<double> L, LoadPl
   e.s_d2u = fault_tile ? s_d2u : nullptr;
   stencil_tile<double, LoadPlain<double>, EpiWave>(L, ld, e, nullptr, nullptr, nullptr);
   if (!fault_tile) return;
-  fd_fault_tile(A, blockIdx.x * TZ, s_rows, s_d2u, gridDim.x);
+  fd_fault_tile(A, fd_tile_node(A, blockIdx.x * TZ), blockIdx.x * TZ, s_rows, s_d2u, gridDim.x);
 }
 
 // The same with the operator in the full form: one block per 8 x 32 tile of
 // rows 0 .. 7 first (FAULT: with the fault update), the rest of the body in
 // walks by warps (march_part).  Bound by the fault tiles' chain of dependent
-// FP64 roots: a step of 61 x 61 takes 13.0 us, one of 801 x 801 15.4 (17.0
+// FP64 roots: a step of 61 x 61 takes about 13 us, one of 801 x 801 14.7 (17.0
 // with the body in block-staged tiles and 18.2 with, besides, the tiles'
 // maxima read one after the other).
 template <bool FAULT>
@@ -322,8 +361,10 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 2) fd_march_kernel(LevelDev<
       e.s_d2u = s_d2u;
     }
     auto row = [](int) {};
+    FDNode n;
+    if (FAULT) n = fd_tile_node(A, blockIdx.x * TZ);
     full_apply<double, 1>(L, ld, pre, out, row, sm, 0, blockIdx.x * TZ);
-    if (FAULT) fd_fault_tile(A, blockIdx.x * TZ, s_rows, s_d2u, nx);
+    if (FAULT) fd_fault_tile(A, n, blockIdx.x * TZ, s_rows, s_d2u, nx);
   } else {
     auto none = [](int, int) {};
     march_part<double>(L, p, blockIdx.x - nx, wv, ld, pre, out, none, sm + wv * kMarchSmem);
