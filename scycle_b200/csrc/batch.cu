@@ -680,9 +680,10 @@ __global__ void b_fault_kernel(LevelDev<double> L, const BatchInst* __restrict__
   const BatchInst& I = tab[k];
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (iz >= I.fp.Nz) return;
+  const FaultNode n = fault_node_load(I.fp, iz);
   const double sxy = I.c1 ? I.sxy[iz] : fault_row_sxy(L, I.u, iz);
-  fault_node_update(iz, sxy, I.fp, I.rk[in_slot][I.fp.psi_off + iz], I.rk[out_slot], I.slipVel, I.tauQSP, I.tauP, I.strength, I.flags,
-                    I.fault_its);
+  fault_node_update(iz, sxy, I.fp, n, I.rk[in_slot][I.fp.psi_off + iz], I.rk[out_slot], I.slipVel, I.tauQSP, I.tauP,
+                    I.strength, I.flags, I.fault_its);
 }
 
 // power law: strains, stresses, viscosity and viscous strain rates per node

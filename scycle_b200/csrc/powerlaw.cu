@@ -39,10 +39,11 @@ __global__ void pl_fault_kernel(const double* __restrict__ sxy, FaultParams fp, 
                                 double* __restrict__ f, double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                 double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                 unsigned long long* its_total) {
-  chain_enter();
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+  const FaultNode n = fault_node_load(fp, min(iz, fp.Nz - 1));
+  chain_enter();
   if (iz >= fp.Nz) return;
-  fault_node_update(iz, sxy[iz], fp, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags, its_total);
+  fault_node_update(iz, sxy[iz], fp, n, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags, its_total);
 }
 
 int pl_d_dt(QDContext& q, double t, const double* var, double* f) {

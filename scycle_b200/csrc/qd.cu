@@ -134,11 +134,12 @@ __global__ void qd_fault_kernel(LevelDev<double> L, const double* __restrict__ u
                                 double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                 double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                 unsigned long long* its_total) {
-  chain_enter();
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+  const FaultNode n = fault_node_load(fp, min(iz, fp.Nz - 1));
+  chain_enter();
   if (iz >= fp.Nz) return;
   const double sxy = fault_row_sxy(L, u, iz);
-  fault_node_update(iz, sxy, fp, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags, its_total);
+  fault_node_update(iz, sxy, fp, n, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags, its_total);
 }
 
 // Fault_qd::d_dt with the body's shear stress on the fault given by the
@@ -148,10 +149,12 @@ __global__ void qd_fault_given_tau_kernel(const double* __restrict__ tau_body, F
                                           double* __restrict__ slipVel, double* __restrict__ tauQSP,
                                           double* __restrict__ tauP, double* __restrict__ strength, unsigned* flags,
                                           unsigned long long* its_total) {
-  chain_enter();
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+  const FaultNode n = fault_node_load(fp, min(iz, fp.Nz - 1));
+  chain_enter();
   if (iz >= fp.Nz) return;
-  fault_node_update(iz, tau_body[iz], fp, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags, its_total);
+  fault_node_update(iz, tau_body[iz], fp, n, var[fp.psi_off + iz], f, slipVel, tauQSP, tauP, strength, flags,
+                    its_total);
 }
 
 int QDContext::fault_d_dt(const double* var, const double* tau_body, double* f) {
@@ -223,24 +226,25 @@ __global__ void __launch_bounds__(32 * kGreenWarps)
   double gl[kGreenPre];
 #pragma unroll
   for (int m = 0; m < kGreenPre; ++m) gl[m] = lane + 32 * m < Nz ? row[lane + 32 * m] : 0.0;
-  chain_enter();
   const int own = iz < Nz ? iz : 0;
+  const FaultNode n = fault_node_load(fp, own);
+  chain_enter();
   const double slip = combine(var, cb, fp.slip_off + own), psi = combine(var, cb, fp.psi_off + own);
   const double tau0 = c * g1[own] + gs[own];
   double acc = 0.0;
   for (int j0 = 0; j0 < Nz; j0 += kGreenCols) {
-    const int n = min(kGreenCols, Nz - j0);
+    const int nc = min(kGreenCols, Nz - j0);
     if (j0 > 0) __syncthreads();
 #pragma unroll 2
-    for (int j = threadIdx.x; j < n; j += 32 * kGreenWarps) sm[j] = combine(var, cb, fp.slip_off + j0 + j);
+    for (int j = threadIdx.x; j < nc; j += 32 * kGreenWarps) sm[j] = combine(var, cb, fp.slip_off + j0 + j);
     __syncthreads();
     int j = lane;
     if (j0 == 0) {
 #pragma unroll
       for (int m = 0; m < kGreenPre; ++m, j += 32)
-        if (j < n) acc += gl[m] * (sm[j] * inv_fts);
+        if (j < nc) acc += gl[m] * (sm[j] * inv_fts);
     }
-    for (; j < n; j += 32) acc += row[j0 + j] * (sm[j] * inv_fts);
+    for (; j < nc; j += 32) acc += row[j0 + j] * (sm[j] * inv_fts);
   }
   if (iz >= Nz) return;
   acc = warp_sum(acc);
@@ -253,7 +257,7 @@ __global__ void __launch_bounds__(32 * kGreenWarps)
       }
     }
     const double tau = acc + tau0;
-    fault_node_update(iz, tau, fp, psi, f, slipVel, tauQSP, tauP, strength, flags, its_total);
+    fault_node_update(iz, tau, fp, n, psi, f, slipVel, tauQSP, tauP, strength, flags, its_total);
   }
 }
 
