@@ -484,7 +484,10 @@ __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, c
   if constexpr (MODE == 0) {
     const double* u = tab[k].u;
     const double* rhs = tab[k].rhs;
-    const bool zero = sc[0] == 0.0;
+    // r = -rhs + A u; in a solve (first = 0), whose rhs kernel has just left
+    // |rhs|^2 in sc[0], zero where rhs = 0.  first = 1: outside of a solve,
+    // where sc[0] is that of some earlier stage, or of none
+    const bool zero = !first && sc[0] == 0.0;
     auto ld = [&](long node, int, int) { return u[node]; };
     auto pre = [&](long node, int, int) { return zero ? 0.0 : rhs[node]; };
     auto out = [&](long node, int, int, double Ax, double, double b) {
@@ -2058,7 +2061,8 @@ int BatchContext::run(long nsteps, scy_batch_stats* st) {
 
 // The carried residual of every instance whose displacement or rhs anything
 // but this batch's rounds has changed since the last run (a solve through
-// the instance's own handle, or a run that ended with an error).
+// the instance's own handle, or a run that ended with an error; before the
+// first run, the instance's own first rates).
 int BatchContext::refresh_residuals() {
   for (auto& G : groups) {
     BatchGroup& g = *G;
@@ -2066,7 +2070,7 @@ int BatchContext::refresh_residuals() {
     bool all = true;
     for (int k = 0; k < g.K; ++k) all = all && carried[g.base + k] == q(g.base + k).u_epoch;
     if (!all) {
-      launch_full<0, double>(g, g.full_shape, g.tab.as<BatchInst>(), g.ones.as<int>(), (const double*)nullptr, 0, 0,
+      launch_full<0, double>(g, g.full_shape, g.tab.as<BatchInst>(), g.ones.as<int>(), (const double*)nullptr, 1, 0,
                              0, 0);
       SCY_LAUNCH_CHECK();
       SCY_CUDA_TRY(cudaStreamSynchronize(g.stream));

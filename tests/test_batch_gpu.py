@@ -253,3 +253,35 @@ def test_batch_sweep_wait_timeout_is_reported_and_recoverable(tmp_path):
             assert _nrel(b.instance(i).field(f), ref.instance(i).field(f)) <= 1e-12, (i, f)
     b.close()
     ref.close()
+
+
+@pytest.mark.parametrize("detour", ["response", "solve"])
+@pytest.mark.parametrize("runs_before", [0, 1])
+def test_batch_residual_after_a_members_own_solve(tmp_path, detour, runs_before):
+    """An instance's own handle leaves another rhs behind than the one its
+    displacement solves (response mode: the build of the fault response), or
+    another displacement.  The batch's next run, its first one included, starts
+    from the residual of what is there: with the attempts of a batch without
+    the detour forced, the states are the same (both solve to SOLVE_RTOL)."""
+    paths = _le_paths(tmp_path)
+    ref = _batch(paths)
+    for i in range(ref.n):
+        ref.instance(i).record_attempts(True)
+    for _ in range(runs_before):
+        ref.run(2)
+    ref.run(1)
+    b = _batch(paths)
+    for i in range(b.n):
+        b.instance(i).force_attempts(ref.instance(i).attempts())
+    for _ in range(runs_before):
+        b.run(2)
+    for i in (0, 1):
+        q = b.instance(i)
+        psi, slip, t = q.field("psi"), q.field("slip"), q.integrate_steps(0).t
+        q.set_mode(detour)
+        q.d_dt(t, psi, slip if detour == "response" else slip + np.linspace(0.0, 1e-2, slip.size))
+        q.set_mode("solve")
+    b.run(1)
+    for i in range(b.n):
+        for nm in FIELDS:
+            assert _nrel(b.instance(i).field(nm), ref.instance(i).field(nm)) <= REL, (i, nm)
