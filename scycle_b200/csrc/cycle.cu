@@ -71,10 +71,18 @@ struct EpiWave {
   }
 };
 
+// Whether the phase ended with a step before this one.  A launch may set
+// st->stop itself while some of its blocks are still to start; these read a
+// number above their own step's and run.
+__device__ __forceinline__ bool fd_ended(const CycleDevState* st, int step) {
+  const int stop = *(volatile const int*)&st->stop;
+  return stop != 0 && stop <= step;
+}
+
 // The wave update where the operator has no full form: the two-stage tile.
 __global__ void __launch_bounds__(256) fd_wave_kernel(LevelDev<double> L, LoadPlain<double> ld, EpiWave ep,
-                                                      const CycleDevState* st) {
-  if (st->stop) return;
+                                                      const CycleDevState* st, int step) {
+  if (fd_ended(st, step)) return;
   stencil_tile<double, LoadPlain<double>, EpiWave>(L, ld, ep, nullptr, nullptr, nullptr);
 }
 
@@ -92,6 +100,7 @@ struct FDFaultArgs {
   double limit_fd, trigger_fd2qd;
   double* partials;  // >= gridDim.x
   CycleDevState* st;
+  int step;  // the step's number in its batch
 };
 
 constexpr int kFaultBlock = 128;
@@ -258,7 +267,7 @@ __device__ __forceinline__ void fd_switch_test(const FDFaultArgs& A, double bloc
     mx = m > mx ? m : mx;
     st->maxR = mx;
     if (!st->allowed && mx > A.limit_fd) st->allowed = 1;
-    if (st->allowed && mx < A.trigger_fd2qd) st->stop = 1;
+    if (st->allowed && mx < A.trigger_fd2qd) st->stop = A.step + 1;
     st->steps_done += 1;
     st->counter = 0u;
   }
@@ -268,7 +277,7 @@ __device__ __forceinline__ void fd_switch_test(const FDFaultArgs& A, double bloc
 // reference the fused step is tested against).
 __global__ void __launch_bounds__(kFaultBlock) fd_fault_kernel(FDFaultArgs A) {
   CycleDevState* st = A.st;
-  if (st->stop) return;
+  if (fd_ended(st, A.step)) return;
   const int Nz = A.fp.Nz;
   const int iz = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   double R = -INFINITY;
@@ -324,7 +333,7 @@ __device__ __forceinline__ void fd_fault_tile(const FDFaultArgs& A, const FDNode
 __global__ void __launch_bounds__(256) fd_step_kernel(LevelDev<double> L, LoadPlain<double> ld, EpiWave ep,
                                                       FDFaultArgs A) {
   CycleDevState* st = A.st;
-  if (st->stop) return;
+  if (fd_ended(st, A.step)) return;
   __shared__ double s_rows[5 * TZ];
   __shared__ double s_d2u[TZ];
   const bool fault_tile = blockIdx.y == 0;
@@ -345,7 +354,7 @@ __global__ void __launch_bounds__(256) fd_step_kernel(LevelDev<double> L, LoadPl
 template <bool FAULT>
 __global__ void __launch_bounds__(32 * kMarchWarps, 2) fd_march_kernel(LevelDev<double> L, LoadPlain<double> ld,
                                                                        EpiWave ep, FDFaultArgs A, MarchPlan p) {
-  if (A.st->stop) return;
+  if (fd_ended(A.st, A.step)) return;
   constexpr int NS = kMarchWarps * kMarchSmem > full_smem_values<1>() ? kMarchWarps * kMarchSmem : full_smem_values<1>();
   __shared__ double sm[NS];
   __shared__ double s_rows[5 * TZ];
@@ -687,7 +696,7 @@ int CycleContext::leave_fd() {
   return SCY_OK;
 }
 
-int CycleContext::fd_launch_step(int r, cudaStream_t s, int part) {
+int CycleContext::fd_launch_step(int r, cudaStream_t s, int part, int step) {
   const int prev = r % 3, cur = (r + 1) % 3, next = (r + 2) % 3;
   CycleDevState* st = dstate.as<CycleDevState>();
   const LevelDev<double>& L = fd_level.dev;
@@ -736,6 +745,7 @@ int CycleContext::fd_launch_step(int r, cudaStream_t s, int part) {
   A.trigger_fd2qd = trigger_fd2qd;
   A.partials = reinterpret_cast<double*>(dstate.as<char>() + sizeof(CycleDevState));
   A.st = st;
+  A.step = step;
   const LoadPlain<double> ld{u3[cur].as<double>()};
   const dim3 g = apply_grid(L);
   const MarchPlan mp = L.full ? march_plan(L, march_chunks(L), 1) : MarchPlan{};
@@ -751,7 +761,7 @@ int CycleContext::fd_launch_step(int r, cudaStream_t s, int part) {
     if (L.full)
       fd_march_kernel<false><<<mg, 32 * kMarchWarps, 0, s>>>(L, ld, ep, A, mp);
     else
-      fd_wave_kernel<<<g, 256, 0, s>>>(L, ld, ep, st);
+      fd_wave_kernel<<<g, 256, 0, s>>>(L, ld, ep, st, step);
     SCY_LAUNCH_CHECK();
   }
   if (part & FD_FAULT) {
@@ -808,7 +818,7 @@ int CycleContext::fd_batch_run(int K, int* n_done, int* stopped) {
     cudaGraph_t graph = nullptr;
     SCY_CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     int rc = SCY_OK;
-    for (int j = 0; j < K && rc == SCY_OK; ++j) rc = fd_launch_step(r0 + j, cs, fd_parts);
+    for (int j = 0; j < K && rc == SCY_OK; ++j) rc = fd_launch_step(r0 + j, cs, fd_parts, j);
     cudaError_t ce = cudaStreamEndCapture(cs, &graph);
     cudaStreamDestroy(cs);
     if (rc != SCY_OK) {
@@ -843,7 +853,7 @@ int CycleContext::fd_batch_run(int K, int* n_done, int* stopped) {
     return SCY_ERR_ROOT_NOCONV;
   }
   *n_done = h_state->steps_done;
-  *stopped = h_state->stop;
+  *stopped = h_state->stop != 0;
   return SCY_OK;
 }
 

@@ -9,8 +9,10 @@
 // runs Fault_fd::d_dt, the fault-row stress and the switch test
 // max(eta V / tauQS), whose last block decides on the device whether the
 // phase ends.  Steps are batched into CUDA graphs; a step after the switch
-// step finds the stop flag set and returns at once, so a batch never runs
-// past the switch.
+// step finds the switch step's number and returns at once, so a batch never
+// runs past the switch.  (The number, not a flag: the fault tiles of the fused
+// step finish ahead of body blocks that have not started yet, which still
+// belong to the switch step.)
 #pragma once
 #include <map>
 #include <utility>
@@ -23,7 +25,7 @@ namespace scy {
 // Device-side state of the fully dynamic phase (one instance).
 struct CycleDevState {
   unsigned counter;        // last-block detection in the fault launch
-  int stop;                // set by the step whose switch test fired
+  int stop;                // 1 + the number, within its batch, of the step whose switch test fired (0: none)
   int allowed;             // checkSwitchRegime's _allowed
   int steps_done;          // steps completed since the batch started
   double maxR;             // max(eta V / tauQS) of the last step
@@ -97,7 +99,7 @@ struct CycleContext {
   int enter_fd();                               // the rest of prepare_qd2fd
   int leave_fd();                               // prepare_fd2qd's data movement
   int fd_batch_run(int K, int* n_done, int* stopped);
-  int fd_launch_step(int r, cudaStream_t s, int part);  // FD_* bits
+  int fd_launch_step(int r, cudaStream_t s, int part, int step = 0);  // FD_* bits; step: its number in the batch
   int time_kernels(int reps, double* wave_us, double* fault_us, double* step_us);
   int fd_parts = FD_FUSED;  // what one graph step launches
   int current_u(double* dst);                   // material u of the phase (device)

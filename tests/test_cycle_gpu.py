@@ -242,3 +242,30 @@ def test_cycle_pid_restart_rule(tmp_path):
         st = c.run(1)
         assert st.step_count == 126 and st.phase == 0
         assert st.new_dt == pytest.approx(5 * st.dt, rel=1e-15)
+
+
+@pytest.mark.parametrize("ny,nz", [(377, 801), (801, 801)])
+def test_cycle_switch_step_is_whole_on_large_grids(tmp_path, ny, nz):
+    """The fault tiles of the fused step decide on the switch while blocks of
+    the same step that do not fit the GPU at once (296 do) are still to start:
+    these belong to the step.  Every phase ends with its first step here; its
+    fields are bitwise those of the two-launch form, where the body is stepped
+    ahead of the switch test."""
+    from scycle_b200.cycle import Cycle
+    path = make_qdfd_problem(str(tmp_path), Ny=ny, Nz=nz, guess_ss=0, extra={"trigger_fd2qd": "1e12", "initTime": "0"})
+    rng = np.random.default_rng(3)
+    y, z = np.linspace(0.0, 30.0, ny), np.linspace(0.0, 30.0, nz)
+    c = Cycle.from_in(path)
+    c.begin_from_in()
+    for _ in range(4):
+        u = 0.05 * np.outer(np.sin(0.3 * y + rng.random()), np.cos(0.2 * z + rng.random())).ravel()
+        now = dict(psi=0.6 + rng.normal(0.0, 1e-4, nz), slip=np.zeros(nz), u=u)
+        out = {}
+        for fused in (True, False):
+            c.set_fd_fused(fused)
+            c.set_fd_state(0.0, 0, True, now, now, np.zeros(u.size), now["slip"], np.full(nz, 26.5), np.full(nz, 1e-9))
+            st = c.run(1)
+            assert st.step_count == 1 and c.switches()[-1]["to"] == "qd"
+            out[fused] = {f: c.field(f) for f in FIELDS + ("u",)}
+        for f in out[True]:
+            assert np.array_equal(out[True][f], out[False][f]), f
