@@ -158,6 +158,7 @@ __global__ void qd_fault_given_tau_kernel(const double* __restrict__ tau_body, F
 }
 
 int QDContext::fault_d_dt(const double* var, const double* tau_body, double* f) {
+  flags_known = 0;
   const int tb = 64, gb = (4 * Nz + tb - 1) / tb;
   chain_launch(qd_fault_given_tau_kernel, gb, tb, 0, sbp.stream, tau_body, fp, var, f, slipVel.as<double>(),
                tauQSP.as<double>(), tauP.as<double>(), strength.as<double>(), flags.as<unsigned>(),

@@ -134,3 +134,26 @@ def test_adjoint_torch_binding_and_knots(tmp_path):
     assert abs(J.item() - J2) <= 1e-12 * J2
     for k, g in zip(knots, (ga, gb, gd)):
         assert np.allclose(k.grad.numpy(), Pm.numpy().T @ g, rtol=1e-12, atol=0)
+
+
+def test_fault_flags_after_a_failed_gradient(tmp_path):
+    """A gradient that ends with an error (targets that are not numbers: the
+    reverse solve's residual is not finite) leaves nothing behind that hides
+    the next call's own fault flags, and the next good call succeeds."""
+    from scycle_b200._lib import ScyError
+    from scycle_b200.adjoint import Adjoint
+    from scycle_b200.qd import QD
+    q = QD.from_in(_problem(tmp_path), solve_rtol=SOLVE_RTOL)
+    q.integrate_begin_from_in()
+    psi, slip, tau = q.field("psi"), q.field("slip"), np.full(q.Nz, 1.0)
+    good = q.fault_d_dt(psi, slip, tau)
+    adj = Adjoint(q, 2)
+    adj.set_steps(np.full(2, 1.0))
+    adj.set_targets(np.full((2, q.Ny), np.nan), np.zeros((2, q.Nz)))
+    with pytest.raises(ScyError, match="non-finite"):
+        adj.gradient()
+    with pytest.raises(ScyError, match="non-finite"):
+        q.fault_d_dt(np.full(q.Nz, np.nan), slip, tau)
+    again = q.fault_d_dt(psi, slip, tau)
+    for k in good:
+        assert np.allclose(again[k], good[k], rtol=1e-9)
