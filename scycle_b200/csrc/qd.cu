@@ -669,7 +669,12 @@ int QDContext::solve_stage(double t, const double* var, const double* gxy, const
     part.first = h_read;
     const bool more = !(std::sqrt(h_read[1]) <= tol || std::sqrt(h_read[5]) <= tol) || (h_read[0] == 0.0 && tol == 0.0);
     const unsigned before = hf[0];
-    SCY_TRY(sbp.solve(rhs.as<double>(), u.as<double>(), o, st, part));
+    if (const int failed = sbp.solve(rhs.as<double>(), u.as<double>(), o, st, part); failed != SCY_OK) {
+      // a solve that fails makes no fault update
+      SCY_CUDA_TRY(cudaMemsetAsync(flags.as<unsigned>() + 1, 0, sizeof(unsigned), s));
+      SCY_CUDA_TRY(cudaMemcpyAsync(slipVel.p, slipVel0.p, (size_t)Nz * 8, cudaMemcpyDeviceToDevice, s));
+      return failed;
+    }
     if (more) {
       SCY_CUDA_TRY(cudaMemsetAsync(flags.as<unsigned>() + 1, 0, sizeof(unsigned), s));
       SCY_CUDA_TRY(cudaMemcpyAsync(slipVel.p, slipVel0.p, (size_t)Nz * 8, cudaMemcpyDeviceToDevice, s));

@@ -253,3 +253,25 @@ def test_response_mode_at_the_kernels_edges(tmp_path, Nz):
     assert _rel(fb["slip"], fa["slip"], 1e-30) <= REL
     assert _nrel(fb["psi"], fa["psi"]) <= REL
     assert _rel(b.field("tauQSP"), a.field("tauQSP"), 1e-9) <= REL
+
+
+@pytest.mark.parametrize("its", [1, 2])
+def test_d_dt_whose_solve_fails_leaves_the_fault_alone(tmp_path, its):
+    """A solve that does not reach its tolerance, or whose residual is not
+    finite, ends d_dt with an error: the slip velocity (the next root find's
+    first guess) stays, and the next call's flags are its own."""
+    from scycle_b200._lib import ScyError
+    from scycle_b200.qd import QD
+    q = QD(_problem(tmp_path, n=33, grid="variableGridSpacing", prestress=26.0), solve_rtol=1e-13, solve_max_its=its)
+    psi, slip, tau = np.full(q.Nz, 0.6), np.linspace(0.0, 0.5, q.Nz), np.full(q.Nz, 1.0)
+    good = q.fault_d_dt(psi, slip, tau)
+    v = q.field("slipVel")
+    with pytest.raises(ScyError):
+        q.d_dt(1.0e9, psi, slip)
+    assert np.array_equal(q.field("slipVel"), v)
+    with pytest.raises(ScyError, match="non-finite"):
+        q.d_dt(1.0e9, psi, np.full(q.Nz, np.nan))
+    assert np.array_equal(q.field("slipVel"), v)
+    again = q.fault_d_dt(psi, slip, tau)
+    for k in good:
+        assert np.allclose(again[k], good[k], rtol=1e-9)
