@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(256, MINB) b_full_kernel(LevelDev<double> L, c
                                                      const Tz* __restrict__ zv, int first, int pi, int mixed,
                                                      int store_p, MarchPlan p) {
   chain_enter();
-  __shared__ double xs[RPT > 0 ? full_smem_values<RPT>() : kMarchWarps * kMarchSmem];
+  __shared__ __align__(16) double xs[RPT > 0 ? full_smem_values<RPT>() : kMarchWarps * kMarchSmem];
   __shared__ double cs[2][8 * RPT + 1][TZ];  // contributions by node of the tile
   const int k = blockIdx.z;
   if (!mask[k]) return;

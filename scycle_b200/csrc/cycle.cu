@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(32 * kMarchWarps, 2) fd_march_kernel(LevelDev<
                                                                        EpiWave ep, FDFaultArgs A, MarchPlan p) {
   if (fd_ended(A.st, A.step)) return;
   constexpr int NS = kMarchWarps * kMarchSmem > full_smem_values<1>() ? kMarchWarps * kMarchSmem : full_smem_values<1>();
-  __shared__ double sm[NS];
+  __shared__ __align__(16) double sm[NS];
   __shared__ double s_rows[5 * TZ];
   __shared__ double s_d2u[TZ];
   const int nx = p.nx, wv = threadIdx.x >> 5;

@@ -648,6 +648,9 @@ constexpr int kChunk = 4;                            // rows of a chunk
 constexpr int kMarchRows = kChunk * (TZ + 2 * HALF);  // shared values of an interior chunk's rows
 constexpr int kEdgeRows = kChunk * (TZ + 16);         // and of an edge chunk's
 constexpr int kMarchSmem = kEdgeRows + 2 * kChunk * 17;  // of one warp: the rows, then their y coefficients
+// the y coefficients are stored in pairs: a warp's part and its coefficients
+// start on pair boundaries of an array aligned to 16 bytes
+static_assert(kMarchSmem % 2 == 0 && kMarchRows % 2 == 0, "pairs of coefficients");
 
 template <typename T>
 struct Vec2;
@@ -907,7 +910,7 @@ template <typename T, class Loader, class Epi>
 __global__ void __launch_bounds__(32 * kMarchWarps, 2) march_kernel(LevelDev<T> L, Loader ld, Epi ep, MarchPlan p) {
   chain_enter();
   static_assert(!Epi::kReduce, "the warp form has no grid sum");
-  __shared__ T sm[kMarchWarps * kMarchSmem];
+  __shared__ __align__(16) T sm[kMarchWarps * kMarchSmem];
   auto pre = [&](long node, int iy, int iz) { return epi_pre(ep, node, iy, iz, 0); };
   auto out = [&](long node, int iy, int iz, T Ax, T xv, const auto& q) { epi_out(ep, node, iy, iz, Ax, xv, q); };
   auto none = [](int, int) {};
