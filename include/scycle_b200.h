@@ -687,7 +687,7 @@ scy_status scy_batch_set_sweep_test(scy_batch* b, int polls, int drop_first_copy
  * the banded sweeps in six launch shapes (whole chains, sweep_variant 0-5:
  * chains per lane x warps per block 2 x 2, 1 x 4, 4 x 1 serving 8 instances
  * per block, 1 x 2 and 2 x 1 serving 4, 1 x 1 serving 2; with the FP64
- * preconditioner and fewer than 10,000 chains in segments, 6-11: 1 or 2
+ * preconditioner and fewer than 4736 chains in segments, 6-11: 1 or 2
  * instances a thread x 1, 2 or 4 groups a block) and the z-transform product
  * in four shapes (one CTA per tile, two CTAs per SM, persistent: one CTA per
  * SM with two accumulator sets, narrow tiles where the others leave SMs

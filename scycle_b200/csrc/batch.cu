@@ -900,10 +900,14 @@ const int* BatchContext::d_acc(const BatchGroup& g) const { return d_copy(g) + n
 const int* BatchContext::d_run(const BatchGroup& g) const { return d_copy(g) + 2 * n; }
 
 // Whole chains instead of segments: one pass of whole chains takes the time of
-// one chain until they fill the GPU, segments a time that grows with the
-// instances.  Measured: 32 x 401 modes 72 us whole, 86 in segments; 3 x 301
-// 52 and 15; 7 x 97 26 and 9.
-static bool many_chains(int Nz, int K) { return (long)Nz * K >= 10000; }
+// one chain until the chains fill the lanes of a warp on every SM two or three
+// times over, segments a time that grows with the instances.  Measured, the
+// best shape of each, us whole and in segments: 401 rows 44 and 24 at 2406
+// chains, 46 and 42 at 4812, 46 and 58 at 7218, 71 and 67 at 9624, 72 and 86
+// at 12832; 301 rows 34 and 32 at 3010, 36 and 46 at 6020, 54 and 73 at 9933;
+// 201 rows 26 and 16 at 2412, 26 and 27 at 4824, 26 and 36 at 7236; 97 rows 15
+// and 11 at 3096, 17 and 20 at 6192, 24 and 28 at 9804.
+static bool many_chains(int Nz, int K) { return (long)Nz * K >= 32L * kNumSMs; }
 
 static bool same_operator(const SbpContext& a, const SbpContext& b) {
   const scy_grid_desc &x = a.desc, &y = b.desc;

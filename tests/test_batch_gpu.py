@@ -285,3 +285,23 @@ def test_batch_residual_after_a_members_own_solve(tmp_path, detour, runs_before)
     for i in range(b.n):
         for nm in FIELDS:
             assert _nrel(b.instance(i).field(nm), ref.instance(i).field(nm)) <= REL, (i, nm)
+
+
+def test_batch_sweeps_in_segments_up_to_a_warp_per_sm(tmp_path):
+    """The banded sweeps run in segments below 4736 chains (z modes times
+    instances) and whole from there on, where segments take longer; either way
+    an instance's steps are the same to the solve tolerance."""
+    paths = [_with_prestress(make_qd_problem(str(tmp_path / str(s)), Ny=17, Nz=257, seed=s), 257, 26.0 + 0.1 * s)
+             for s in range(19)]
+    few, many = _batch(paths[:18]), _batch(paths)
+    assert few.tuning()["sweep_variant"].startswith("segments")
+    assert "warp" in many.tuning()["sweep_variant"]
+    for i in range(few.n):
+        many.instance(i).record_attempts(True)
+    many.run(3)
+    for i in range(few.n):
+        few.instance(i).force_attempts(many.instance(i).attempts())
+    few.run(3)
+    for i in (0, 17):
+        for nm in FIELDS:
+            assert _nrel(few.instance(i).field(nm), many.instance(i).field(nm)) <= REL, (i, nm)
