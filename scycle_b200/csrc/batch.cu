@@ -993,8 +993,7 @@ int BatchContext::create(int n_inst, const char* const* paths, const scy_solve_o
   // members' own solves as well
   int base = 0;
   for (auto& m : members) {
-    SCY_TRY(q(base).sbp.ensure_fd(q(base).sbp.keeps_rounding(q(base).solve_opts.rtol) ||
-                                  many_chains(q(base).Nz, (int)m.size())));
+    SCY_TRY(q(base).sbp.ensure_fd());
     for (size_t k = 1; k < m.size(); ++k) q(base + (int)k).sbp.fd = q(base).sbp.fd;
     base += (int)m.size();
   }
@@ -1093,8 +1092,16 @@ int BatchContext::setup_group(int base, int K) {
   g.N = q0.N;
   // a steady-state guess changes the boundary types and back, which rebuilds
   // the members' operators: take the representative's current ones
-  SCY_TRY(q0.sbp.ensure_fd(many_chains(g.Nz, K)));
+  SCY_TRY(q0.sbp.ensure_fd());
   g.fd = q0.sbp.fd;
+  if (g.fd->ybanded && !fd_dense) {
+    if (precision != SCY_PREC_FP64)
+      SCY_TRY(g.fd->need_chains32(q0.sbp.stream));
+    else if (g.fd->yp.T > 0 && !many_chains(g.Nz, K))
+      SCY_TRY(g.fd->need_segments(q0.sbp.stream));
+    else
+      SCY_TRY(g.fd->need_chains(q0.sbp.stream));
+  }
   g.L = q0.sbp.fine->dev;
   const long KN = (long)g.K * g.N;
   // one group (one stream) of few nodes: a step of 7 x 129 x 97 takes 266 us
@@ -1206,8 +1213,10 @@ int BatchContext::setup_group(int base, int K) {
       SCY_TRY(tma_map_2d(&g.mLrow, g.fd->Lrow.p, d64, 8, g.Nz, (long)(g.Ny + 8) * 9, (long)Nzp * 8, YS_C, YS_R * 9));
     }
     SCY_TRY(tma_map_3d(&g.mT, g.t1p.p, d64, g.Nz, g.Ny, g.K, (long)Nzp * 8, (long)g.Ny * Nzp * 8, YS_C, YS_R, YS_B));
-    SCY_TRY(tma_map_2d(&g.mLcol32, g.fd->Lcol32.p, d32, 4, g.Nz, (long)g.Ny * 9, (long)Nzp * 4, YS_C, YS_R * 9));
-    SCY_TRY(tma_map_2d(&g.mLrow32, g.fd->Lrow32.p, d32, 4, g.Nz, (long)(g.Ny + 8) * 9, (long)Nzp * 4, YS_C, YS_R * 9));
+    if (g.fd->Lrow32.p) {
+      SCY_TRY(tma_map_2d(&g.mLcol32, g.fd->Lcol32.p, d32, 4, g.Nz, (long)g.Ny * 9, (long)Nzp * 4, YS_C, YS_R * 9));
+      SCY_TRY(tma_map_2d(&g.mLrow32, g.fd->Lrow32.p, d32, 4, g.Nz, (long)(g.Ny + 8) * 9, (long)Nzp * 4, YS_C, YS_R * 9));
+    }
     SCY_TRY(tma_map_3d(&g.mT32, g.t1pf.p, d32, g.Nz, g.Ny, g.K, (long)Nzp * 4, (long)g.Ny * Nzp * 4, YS_C, YS_R,
                        YS_B));
     SCY_TRY(tma_map_3d(&g.mT4, g.t1p.p, d64, g.Nz, g.Ny, g.K, (long)Nzp * 8, (long)g.Ny * Nzp * 8, YS_C, YS_R, 4));

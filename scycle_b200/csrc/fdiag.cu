@@ -285,33 +285,9 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
           }
       }
       if (spd) {
-        // padded row and column forms for the TMA-fed sweeps
         Nzp = (Nz + 3) / 4 * 4;
-        SCY_TRY(yp.build(Lbh, Ny, Nz, Nzp, s));
-        std::vector<double> Lr((size_t)(Ny + bw) * 9 * Nzp, 0.0), Lc((size_t)Ny * 9 * Nzp, 0.0);
-        // slot 1 holds the coupling to the row processed just before,
-        // divided by L_ii: L(i+1, i) / L_ii going up (row form), L(i, i-1) /
-        // L_ii going down (column form)
-        for (int i = 0; i < Ny + bw; ++i)
-          for (int k = 0; k < 9; ++k)
-            for (int j = 0; j < Nz; ++j) {
-              double v = Lbh[((size_t)i * 9 + k) * Nz + j];
-              if (k == 1)
-                v = i + 1 < Ny + bw ? Lbh[((size_t)(i + 1) * 9 + 1) * Nz + j] * Lbh[((size_t)i * 9) * Nz + j] : 0.0;
-              Lr[((size_t)i * 9 + k) * Nzp + j] = v;
-            }
-        for (int i = 0; i < Ny; ++i)
-          for (int j = 0; j < Nz; ++j) {
-            Lc[((size_t)i * 9) * Nzp + j] = Lbh[((size_t)i * 9) * Nz + j];
-            Lc[((size_t)i * 9 + 1) * Nzp + j] = Lbh[((size_t)i * 9 + 1) * Nz + j] * Lbh[((size_t)i * 9) * Nz + j];
-            for (int m = 2; m <= bw; ++m) Lc[((size_t)i * 9 + m) * Nzp + j] = Lbh[((size_t)(i + m) * 9 + m) * Nz + j];
-          }
-        if (want_chains || yp.T == 0) {
-          SCY_TRY(upload_as<double>(Lrow, Lr, s));
-          SCY_TRY(upload_as<double>(Lcol, Lc, s));
-        }
-        SCY_TRY(upload_as<float>(Lrow32, Lr, s));
-        SCY_TRY(upload_as<float>(Lcol32, Lc, s));
+        yp.plan(Lbh, Ny, Nz, Nzp);
+        SCY_TRY(upload_as<double>(Lf, Lbh, s));
         ybanded = 1;
       }
     }
@@ -343,13 +319,7 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
     }
     // tile maps of the TMA-fed sweeps over the one instance's transform
     const CUtensorMapDataType d64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64, d32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    if (Lrow.p) {
-      SCY_TRY(tma_map_2d(&mLcol, Lcol.p, d64, 8, Nz, (long)Ny * 9, (long)Nzp * 8, YS_C, YS_R * 9));
-      SCY_TRY(tma_map_2d(&mLrow, Lrow.p, d64, 8, Nz, (long)(Ny + 8) * 9, (long)Nzp * 8, YS_C, YS_R * 9));
-    }
     SCY_TRY(tma_map_3d(&mT, t1p.p, d64, Nz, Ny, 1, (long)Nzp * 8, (long)Ny * Nzp * 8, YS_C, YS_R, 2));
-    SCY_TRY(tma_map_2d(&mLcol32, Lcol32.p, d32, 4, Nz, (long)Ny * 9, (long)Nzp * 4, YS_C, YS_R * 9));
-    SCY_TRY(tma_map_2d(&mLrow32, Lrow32.p, d32, 4, Nz, (long)(Ny + 8) * 9, (long)Nzp * 4, YS_C, YS_R * 9));
     SCY_TRY(tma_map_3d(&mT32, t1pf.p, d32, Nz, Ny, 1, (long)Nzp * 4, (long)Ny * Nzp * 4, YS_C, YS_R, YS_B));
     SCY_CUDA_TRY(cudaFuncSetAttribute(b_ysolve_tma_kernel<double, 1, 1>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, ys_smem_bytes(8)));
@@ -368,13 +338,69 @@ int FDPrecond::build(const LevelHost& L, cudaStream_t s) {
   return SCY_OK;
 }
 
+namespace {
+// The padded row and column forms of the factors for the TMA-fed sweeps: slot
+// 1 holds the coupling to the row processed just before, divided by L_ii:
+// L(i+1, i) / L_ii going up (row form), L(i, i-1) / L_ii going down (column
+// form)
+template <typename T>
+__global__ void chain_tables_kernel(const double* __restrict__ L, int Ny, int Nz, int Nzp, T* __restrict__ Lr,
+                                    T* __restrict__ Lc) {
+  const int rows = Ny + 8;
+  const long n = (long)rows * 9 * Nzp;
+  for (long at = blockIdx.x * (long)blockDim.x + threadIdx.x; at < n; at += (long)gridDim.x * blockDim.x) {
+    const int j = (int)(at % Nzp), m = (int)(at / Nzp % 9), i = (int)(at / ((long)Nzp * 9));
+    auto l = [&](int row, int k) { return L[((long)row * 9 + k) * Nz + j]; };
+    double vr = 0.0, vc = 0.0;
+    if (j < Nz) {
+      vr = m != 1 ? l(i, m) : i + 1 < rows ? l(i + 1, 1) * l(i, 0) : 0.0;
+      if (i < Ny) vc = m == 0 ? l(i, 0) : m == 1 ? l(i, 1) * l(i, 0) : l(i + m, m);
+    }
+    Lr[at] = (T)vr;
+    if (i < Ny) Lc[at] = (T)vc;
+  }
+}
+
+template <typename T>
+int chain_tables(const DevBuf& Lf, int Ny, int Nz, int Nzp, DevBuf& Lrow, DevBuf& Lcol, CUtensorMap* mrow,
+                 CUtensorMap* mcol, CUtensorMapDataType type, cudaStream_t s) {
+  const long rows = (long)(Ny + 8) * 9, cols = (long)Ny * 9, e = sizeof(T);
+  DevBuf lr;  // Lrow once it is laid out
+  SCY_TRY(lr.alloc((size_t)(rows * Nzp * e)));
+  SCY_TRY(Lcol.alloc((size_t)(cols * Nzp * e)));
+  chain_tables_kernel<T><<<grid_for(rows * Nzp), 256, 0, s>>>(Lf.as<double>(), Ny, Nz, Nzp, lr.as<T>(), Lcol.as<T>());
+  SCY_LAUNCH_CHECK();
+  SCY_TRY(tma_map_2d(mcol, Lcol.p, type, (int)e, Nz, cols, Nzp * e, YS_C, YS_R * 9));
+  SCY_TRY(tma_map_2d(mrow, lr.p, type, (int)e, Nz, rows, Nzp * e, YS_C, YS_R * 9));
+  SCY_CUDA_TRY(cudaStreamSynchronize(s));
+  Lrow = std::move(lr);
+  return SCY_OK;
+}
+}  // namespace
+
+// The tables are laid out on the device (0.8 ms with their allocations at 401 x 401) and by the
+// form that asks for them: laid out on the host for every operator, the
+// segments' took 13 ms of the first solve there (89 ms, now 66) and the chains' 10,
+// whether or not a solve swept that way.
+int FDPrecond::need_segments(cudaStream_t s) { return yp.tab.p ? SCY_OK : yp.fill(Lf.as<double>(), s); }
+int FDPrecond::need_chains(cudaStream_t s) {
+  if (Lrow.p) return SCY_OK;
+  return chain_tables<double>(Lf, Ny, Nz, Nzp, Lrow, Lcol, &mLrow, &mLcol, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, s);
+}
+int FDPrecond::need_chains32(cudaStream_t s) {
+  if (Lrow32.p) return SCY_OK;
+  return chain_tables<float>(Lf, Ny, Nz, Nzp, Lrow32, Lcol32, &mLrow32, &mLcol32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, s);
+}
+
 int FDPrecond::apply(const double* r, double* z, cudaStream_t s, bool chains) {
   if (ybanded) {
     double* t = t1p.as<double>();
     const int shape = ozk_narrow_better(kPlanes64, Ny, Nz) ? 3 : 0;
+    const bool segments = yp.T > 0 && !chains;
+    SCY_TRY(segments ? need_segments(s) : need_chains(s));
     SCY_TRY(ozk_split(zx64, r, Nz, s));
     SCY_TRY(ozk_gemm(zx64, zw1_64, t, Nzp, Nz, s, nullptr, 1, 4u, shape));
-    if (yp.T > 0 && !chains) {
+    if (segments) {
       SCY_TRY(yp.solve(t, 1, 0, ys_status.as<unsigned>(), s, true));
     } else {
       // one chain a lane and one warp a block: fewest instructions a row
@@ -412,6 +438,7 @@ int FDPrecond::apply32(const double* r, float* z, cudaStream_t s) {
   if (ybanded) {
     float* t = t1pf.as<float>();
     const int shape = ozk_narrow_better(kPlanes32, Ny, Nz) ? 3 : 0;
+    SCY_TRY(need_chains32(s));
     SCY_TRY(ozk_split(zx32, r, Nz, s));
     SCY_TRY(ozk_gemm(zx32, zw1_32, t, Nzp, Nz, s, nullptr, 1, 4u, shape));
     chain_launch(b_ysolve_tma_kernel<float, YS_I, YS_W>, dim3((Nz + YS_C - 1) / YS_C, 1), 32 * YS_W, ys_smem_bytes(4),

@@ -26,7 +26,7 @@ namespace scy {
 // about 1900 rows, or off-diagonals outside its pattern); then the chains run
 // whole (ysolve.cuh).
 struct YPart {
-  int Ny = 0, Nzp = 0, T = 0, P = 0, MB = 0, base = 0, extra = 0, nb = 0;
+  int Ny = 0, Nz = 0, Nzp = 0, T = 0, P = 0, MB = 0, base = 0, extra = 0, nb = 0;
   DevBuf tab, wide;
   // instances a thread x groups a block; every shape gives the same results
   static constexpr int kShapes = 6;
@@ -34,7 +34,8 @@ struct YPart {
   bool fits(int shape) const;
   size_t smem_bytes(int shape) const;
   // L: the factors, value k of row i (1 / L_ii, then L(i, i - k)) and mode j at (i * 9 + k) * Nz + j
-  int build(const std::vector<double>& L, int Ny, int Nz, int Nzp, cudaStream_t s);
+  void plan(const std::vector<double>& L, int Ny, int Nz, int Nzp);
+  int fill(const double* L, cudaStream_t s);  // the tables, from the factors on the device
   int solve(double* t, int K, int shape, unsigned* status, cudaStream_t s, bool chain, int polls = 1 << 18, int drop = 0) const;
 };
 
@@ -48,9 +49,11 @@ struct FDPrecond {
   // Banded form of the y part (ybanded = 1 when the symmetric part of the y
   // line operator has half-bandwidth <= 8): after the z transform the
   // operator splits into one banded SPD system per z mode j,
-  // Ky + lz_j My, solved with its Cholesky factor L_j.  The factors are
-  // kept for the TMA-fed sweeps, rows padded to Nzp (a multiple of 4)
-  // values: row form [(i * 9 + m) * Nzp + j] = L_j(i, i - m) (Ny + 8
+  // Ky + lz_j My, solved with its Cholesky factor L_j.  The factors stay on
+  // the device (Lf: 1 / L_j(i, i) and L_j(i, i - m) at (i * 9 + m) * Nz + j, Ny
+  // + 8 rows), and the first call that sweeps in a form lays out that form's
+  // tables from them (need_*).  For the TMA-fed sweeps of whole chains, rows
+  // padded to Nzp (a multiple of 4) values: row form [(i * 9 + m) * Nzp + j] = L_j(i, i - m) (Ny + 8
   // rows), column form [(i * 9 + m) * Nzp + j] = L_j(i + m, i) (Ny rows)
   // for m = 2..8; slot m = 0 holds 1 / L_j(i, i) in both, slot 1 the
   // coupling to the row a sweep processes just before row i over L_j(i, i):
@@ -60,10 +63,10 @@ struct FDPrecond {
   int Nzp = 0;
   DevBuf Lrow, Lcol, Lrow32, Lcol32;
   YPart yp;  // the FP64 sweeps in segments
-  // set before build: keep the FP64 tables of the whole chains beside the
-  // segments' (there without a plan for segments)
-  int want_chains = 0;
-  bool has_chains() const { return !ybanded || Lrow.p; }
+  DevBuf Lf;
+  int need_segments(cudaStream_t s);  // yp's tables (yp.T > 0)
+  int need_chains(cudaStream_t s);    // Lrow, Lcol and their tile maps
+  int need_chains32(cudaStream_t s);  // Lrow32, Lcol32 and theirs
   // With the banded form, apply / apply32 run the z transforms on the
   // integer tensor cores (digit planes: kPlanes64 for apply, kPlanes32 for apply32) and the
   // TMA-fed sweeps of the batched ensemble (one instance) on the padded
@@ -75,7 +78,7 @@ struct FDPrecond {
   CUtensorMap mLcol, mLrow, mT, mLcol32, mLrow32, mT32;
   ~FDPrecond();
   int build(const LevelHost& L, cudaStream_t s);
-  // z = K_sep^-1 r (FP64); chains: sweep whole chains (has_chains)
+  // z = K_sep^-1 r (FP64); chains: sweep whole chains
   int apply(const double* r, double* z, cudaStream_t s, bool chains = false);
   // z = K_sep^-1 r with FP32 GEMMs (z in FP32)
   int apply32(const double* r, float* z, cudaStream_t s);

@@ -1464,10 +1464,9 @@ int SbpContext::correct(PC&& pc, const double* rhs, double* u, const scy_solve_o
   return finish_solve(rhs, u, o, tol, st);
 }
 
-int SbpContext::ensure_fd(bool chains) {
-  if (fd && fd->ready && (!chains || fd->has_chains())) return SCY_OK;
+int SbpContext::ensure_fd() {
+  if (fd && fd->ready) return SCY_OK;
   fd.reset(new FDPrecond());
-  fd->want_chains = chains;
   return fd->build(hosts[0], stream);
 }
 
@@ -1480,7 +1479,7 @@ int SbpContext::solve(const double* rhs, double* u, const scy_solve_opts& o, scy
                       const SolvePart& part) {
   const bool keeps = keeps_rounding(o.rtol);
   if (uses_fd(o)) {
-    SCY_TRY(ensure_fd(keeps));
+    SCY_TRY(ensure_fd());
     if (o.precision == SCY_PREC_MIXED) {
       float* z = cg_z32.as<float>();
       auto pc = [&](const double* r, float** zo) -> int {

@@ -185,7 +185,7 @@ struct SbpContext {
   DevBuf cross;  // cross-form planes of the fine level (built on first use)
   template <typename T>
   int ensure_mg(std::unique_ptr<Multigrid<T>>& mg);
-  int ensure_fd(bool chains);  // chains: with the tables of the whole sweep chains
+  int ensure_fd();
   template <typename Tz, class PC>
   int pcg(PC&& pc, const double* rhs, double* u, const scy_solve_opts& o, scy_solve_stats& st, const SolvePart& part);
   template <class PC>

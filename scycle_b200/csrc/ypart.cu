@@ -56,7 +56,7 @@ struct YPartArgs {
   unsigned* status;
   int polls, drop;
 };
-constexpr int kRow = 14, kMaxPad = 7;
+constexpr int kRow = 14, kMaxPad = 7, kMaxT = 48;
 
 template <int T, int I>
 __global__ void __launch_bounds__(384) ypart_kernel(const YPartArgs A) {
@@ -255,6 +255,55 @@ __global__ void __launch_bounds__(384) ypart_kernel(const YPartArgs A) {
   __syncthreads();
 }
 
+// The tables of mode j, segment sg (one thread each): the factor's entries
+// within the segment, its rows' answer G to the four rows before it and B to
+// the four rows after it.  L as YPart::plan takes it.
+__global__ void __launch_bounds__(128) ypart_fill_kernel(const double* __restrict__ L, int Nz, int Ny, int T, int P,
+                                                         int MB, int base, int extra, double* __restrict__ tab,
+                                                         double* __restrict__ wide) {
+  const int at = blockIdx.x * blockDim.x + threadIdx.x;
+  if (at >= P * Nz) return;
+  const int sg = at / Nz, j = at - sg * Nz, jb = j / MB, md = j % MB;
+  const int r0 = sg * base + min(sg, extra), nr = sg < extra ? base + 1 : base, S = T * kRow + 2;
+  auto lj = [&](int i, int k) { return L[((long)i * 9 + k) * Nz + j]; };
+  double* c = tab + ((long)jb * P * MB + sg * MB + md) * S + (T - nr) * kRow;
+  double* w = wide + (long)jb * 32 * MB + md;
+  double col[kMaxT];
+  for (int r = 0; r < nr; ++r) {
+    // off-diagonals to rows of this segment (those to earlier ones are in G)
+    for (int k = 0; k < 5; ++k) c[r * kRow + k] = r >= k ? lj(r0 + r, k) : 0.0;
+    const int wr = sg == 0 && r >= 5 && r <= 8 ? r - 5 : sg == P - 1 && r >= nr - 4 ? 4 + r - (nr - 4) : -1;
+    if (wr >= 0)
+      for (int k = 5; k <= 8 && k <= r; ++k) w[(wr * 4 + k - 5) * MB] = lj(r0 + r, k);
+  }
+  // G: rows of this segment for a one in row r0 - 1 - d and no data
+  if (sg > 0)
+    for (int d = 0; d < 4; ++d)
+      for (int r = 0; r < nr; ++r) {
+        double sum = 0.0;
+        for (int k = 1; k <= 8; ++k) {
+          const int p = r - k;  // row of the segment; -1 - d is the incoming one
+          const double v = p >= 0 ? col[p] : p == -1 - d ? 1.0 : 0.0;
+          if (v != 0.0) sum = __dsub_rn(sum, __dmul_rn(lj(r0 + r, k), v));
+        }
+        col[r] = __dmul_rn(sum, lj(r0 + r, 0));
+        c[r * kRow + 5 + d] = col[r];
+      }
+  // B: the same upwards for a one in row r0 + nr + d
+  if (sg < P - 1)
+    for (int d = 0; d < 4; ++d)
+      for (int r = nr - 1; r >= 0; --r) {
+        double sum = 0.0;
+        for (int k = 1; k <= 8 && r0 + r + k < Ny; ++k) {
+          const int p = r + k;
+          const double v = p < nr ? col[p] : p == nr + d ? 1.0 : 0.0;
+          if (v != 0.0) sum = __dsub_rn(sum, __dmul_rn(lj(r0 + p, k), v));
+        }
+        col[r] = __dmul_rn(sum, lj(r0 + r, 0));
+        c[r * kRow + 9 + d] = col[r];
+      }
+}
+
 int dev_smem_limit() { return 225 * 1024; }  // beside the static kilobyte
 
 template <int T, int I>
@@ -272,7 +321,7 @@ int launch_one(const YPartArgs& A, size_t smem, int nb, int NG, cudaStream_t s, 
   return SCY_OK;
 }
 
-constexpr int kT[] = {8, 12, 16, 20, 24, 28, 32, 40, 48};
+constexpr int kT[] = {8, 12, 16, 20, 24, 28, 32, 40, kMaxT};
 }  // namespace
 
 size_t YPart::smem_bytes(int shape) const {
@@ -284,8 +333,9 @@ bool YPart::fits(int shape) const {
          TP * kShapeNG[shape] <= 384 && 4 * MB * kShapeI[shape] <= TP;
 }
 
-int YPart::build(const std::vector<double>& L, int Ny_, int Nz, int Nzp_, cudaStream_t s) {
+void YPart::plan(const std::vector<double>& L, int Ny_, int Nz_, int Nzp_) {
   Ny = Ny_;
+  Nz = Nz_;
   Nzp = Nzp_;
   // Segments: a row costs about 120 cycles in its three passes and a carry
   // about 80 each way, so T near 1.15 sqrt(Ny); no segment below eight rows, so
@@ -310,7 +360,7 @@ int YPart::build(const std::vector<double>& L, int Ny_, int Nz, int Nzp_, cudaSt
     if (fits(0)) break;
   if (!T || MB < 1) {
     T = 0;
-    return SCY_OK;
+    return;
   }
   base = Ny / P;
   extra = Ny % P;
@@ -328,60 +378,23 @@ int YPart::build(const std::vector<double>& L, int Ny_, int Nz, int Nzp_, cudaSt
         for (int j = 0; j < Nz; ++j)
           if (at(row0(sg) + r, k, j) != 0.0 && (k > r || wide_row(sg, r) < 0)) {
             T = 0;
-            return SCY_OK;
+            return;
           }
   nb = (Nzp + MB - 1) / MB;
-  const size_t S = T * kRow + 2, blk = (size_t)P * MB * S;
-  std::vector<double> Tb((size_t)nb * blk, 0.0), W((size_t)nb * 32 * MB, 0.0);
-  std::vector<double> col(T), Lj((size_t)Ny * 9);
-  for (int j = 0; j < Nz; ++j) {
-    // the mode's factor in one piece: its entries are read up to nine times
-    for (size_t i = 0; i < Lj.size(); ++i) Lj[i] = L[i * Nz + j];
-    auto lj = [&](int i, int k) { return Lj[(size_t)i * 9 + k]; };
-    const int jb = j / MB, md = j % MB;
-    for (int sg = 0; sg < P; ++sg) {
-      const int r0 = row0(sg), nr = rows(sg);
-      double* c = &Tb[(size_t)jb * blk + (size_t)(sg * MB + md) * S + (size_t)(T - nr) * kRow];
-      for (int r = 0; r < nr; ++r) {
-        // off-diagonals to rows of this segment (those to earlier ones are in G)
-        for (int k = 0; k < 5; ++k) c[r * kRow + k] = r >= k ? lj(r0 + r, k) : 0.0;
-        if (const int wr = wide_row(sg, r); wr >= 0)
-          for (int k = 5; k <= 8 && k <= r; ++k) W[((size_t)jb * 32 + wr * 4 + k - 5) * MB + md] = lj(r0 + r, k);
-      }
-      // G: rows of this segment for a one in row r0 - 1 - d and no data
-      if (sg > 0)
-        for (int d = 0; d < 4; ++d)
-          for (int r = 0; r < nr; ++r) {
-            double sum = 0.0;
-            for (int k = 1; k <= 8; ++k) {
-              const int p = r - k;  // row of the segment; -1 - d is the incoming one
-              const double v = p >= 0 ? col[p] : p == -1 - d ? 1.0 : 0.0;
-              if (v != 0.0) sum -= lj(r0 + r, k) * v;
-            }
-            col[r] = sum * lj(r0 + r, 0);
-            c[r * kRow + 5 + d] = col[r];
-          }
-      // B: the same upwards for a one in row r0 + nr + d
-      if (sg < P - 1)
-        for (int d = 0; d < 4; ++d)
-          for (int r = nr - 1; r >= 0; --r) {
-            double sum = 0.0;
-            for (int k = 1; k <= 8; ++k) {
-              const int p = r + k;
-              if (r0 + p >= Ny) break;
-              const double v = p < nr ? col[p] : p == nr + d ? 1.0 : 0.0;
-              if (v != 0.0) sum -= lj(r0 + p, k) * v;
-            }
-            col[r] = sum * lj(r0 + r, 0);
-            c[r * kRow + 9 + d] = col[r];
-          }
-    }
-  }
-  SCY_TRY(tab.alloc(Tb.size() * 8));
-  SCY_TRY(wide.alloc(W.size() * 8));
-  SCY_CUDA_TRY(cudaMemcpyAsync(tab.p, Tb.data(), Tb.size() * 8, cudaMemcpyHostToDevice, s));
-  SCY_CUDA_TRY(cudaMemcpyAsync(wide.p, W.data(), W.size() * 8, cudaMemcpyHostToDevice, s));
+}
+
+int YPart::fill(const double* L, cudaStream_t s) {
+  const size_t S = T * kRow + 2, n = (size_t)nb * P * MB * S, nw = (size_t)nb * 32 * MB;
+  DevBuf t;  // tab once it is laid out
+  SCY_TRY(t.alloc(n * 8));
+  SCY_TRY(wide.alloc(nw * 8));
+  SCY_CUDA_TRY(cudaMemsetAsync(t.p, 0, n * 8, s));
+  SCY_CUDA_TRY(cudaMemsetAsync(wide.p, 0, nw * 8, s));
+  ypart_fill_kernel<<<(P * Nz + 127) / 128, 128, 0, s>>>(L, Nz, Ny, T, P, MB, base, extra, t.as<double>(),
+                                                         wide.as<double>());
+  SCY_LAUNCH_CHECK();
   SCY_CUDA_TRY(cudaStreamSynchronize(s));
+  tab = std::move(t);
   return SCY_OK;
 }
 
