@@ -115,7 +115,7 @@ static int upload_ints(DevBuf& buf, const std::vector<int>& v, cudaStream_t s) {
 }
 
 template <typename T>
-int LevelStore<T>::init(const LevelHost& h, cudaStream_t s) {
+int LevelStore<T>::init(const LevelHost& h, cudaStream_t s, const T* planes) {
   Ny = h.Ny;
   Nz = h.Nz;
   const DirTables* td[2] = {&h.ty, &h.tz};
@@ -320,7 +320,9 @@ int LevelStore<T>::init(const LevelHost& h, cudaStream_t s) {
       }
     }
   }
-  if (const long n = (long)Ny * Nz; !dev.full && n <= kCrossMaxNodes) {
+  if (planes) {
+    dev.cross = planes;
+  } else if (const long n = (long)Ny * Nz; !dev.full && n <= kCrossMaxNodes) {
     SCY_TRY(cross.alloc((size_t)n * 33 * sizeof(T)));
     chain_launch(cross_build_kernel<T>, grid_for(n), 256, 0, s, dev, cross.template as<T>());
     SCY_LAUNCH_CHECK();
@@ -708,13 +710,14 @@ static int red_blocks(long n) { return grid_for(n, 256, 1024); }
 
 // ------------------------------------------------------------------------
 template <typename T>
-int Multigrid<T>::init(const std::vector<LevelHost>& hosts, const std::vector<Transfer>& xfer, cudaStream_t s) {
+int Multigrid<T>::init(const std::vector<LevelHost>& hosts, const std::vector<Transfer>& xfer, cudaStream_t s,
+                       const T* planes0) {
   nlev = (int)hosts.size();
   lev.resize(nlev);
   work.resize(nlev);
   for (int l = 0; l < nlev; ++l) {
     lev[l].reset(new LevelStore<T>());
-    SCY_TRY(lev[l]->init(hosts[l], s));
+    SCY_TRY(lev[l]->init(hosts[l], s, l == 0 ? planes0 : nullptr));
     long n = (long)hosts[l].Ny * hosts[l].Nz;
     for (int k = 0; k < 5; ++k) SCY_TRY(work[l].v[k].alloc(n * sizeof(T)));
   }
@@ -1238,7 +1241,10 @@ template <typename T>
 int SbpContext::ensure_mg(std::unique_ptr<Multigrid<T>>& mg) {
   if (mg) return SCY_OK;
   mg.reset(new Multigrid<T>());
-  SCY_TRY(mg->init(hosts, xfer, stream));
+  // the finest level's planes are the operator's own (rebuilt together)
+  const T* planes0 = nullptr;
+  if constexpr (std::is_same<T, double>::value) planes0 = fine->dev.cross;
+  SCY_TRY(mg->init(hosts, xfer, stream, planes0));
   SCY_TRY(mg->setup_smoothers(hosts, red, scal.as<double>() + 8, stream));
   return SCY_OK;
 }

@@ -64,7 +64,8 @@ struct LevelStore {
   DevBuf cross;       // the cross form's coefficient planes (LevelDev::cross)
   DevBuf fullw[2];    // the full form's outer weights wy1 (Nz), wz1 (Ny) when the interior is not separable
   LevelDev<T> dev{};
-  int init(const LevelHost& h, cudaStream_t s);
+  // planes: the cross form's planes where another store of this level has them (and outlives this one)
+  int init(const LevelHost& h, cudaStream_t s, const T* planes = nullptr);
 };
 
 struct Transfer {
@@ -92,7 +93,7 @@ struct Multigrid {
   std::vector<std::vector<ChebCoef>> cheb;
   std::vector<double> lambda;
   DevBuf coarse_inv;
-  int init(const std::vector<LevelHost>& hosts, const std::vector<Transfer>& xfer, cudaStream_t s);
+  int init(const std::vector<LevelHost>& hosts, const std::vector<Transfer>& xfer, cudaStream_t s, const T* planes0);
   int setup_smoothers(const std::vector<LevelHost>& hosts, Reducer& red, double* dscal, cudaStream_t s);
   template <typename Tin>
   int vcycle(int l, const Tin* b_in, T** x_out, cudaStream_t s);
