@@ -7,8 +7,12 @@
 // control (:395-445, :846-898), including the reference's handling of the
 // 100-attempt cap and of a step that falls to the minimum size.
 #include <algorithm>
+#include <bitset>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <vector>
 
 #include "common.cuh"
 #include "fault_node.cuh"
@@ -321,6 +325,64 @@ struct KeyTable {
 // the fault flags, and the records of an attempt's enqueued solves
 enum { RB_FLAGS = 13, RB_SOLVE = 16, RB_SIZE = RB_SOLVE + 3 * 6 };
 
+// Pinned memory for the drivers' read-backs (QDContext::h_read): slots of
+// registered pages that the live drivers share; a page goes back when its last
+// driver does.  A driver's own cudaMallocHost took 1 to 3 ms (a 61 x 61 driver
+// 2.9 to 4.7 ms to create, 1.9 without it), a registered page takes 0.3 and a
+// slot of one nothing; a copy to pageable memory takes 2.6 us longer, each
+// attempt anew.
+class ReadSlots {
+  static constexpr size_t kSlot = 512, kPage = 64 << 10, kSlots = kPage / kSlot;
+  static_assert(RB_SIZE * sizeof(double) <= kSlot, "a slot holds what an attempt reads back");
+  struct Page {
+    char* p;
+    std::bitset<kSlots> used;
+  };
+  std::mutex m;
+  std::vector<Page> pages;
+
+ public:
+  double* take() {
+    std::lock_guard<std::mutex> lock(m);
+    for (Page& g : pages)
+      for (size_t i = 0; i < kSlots; ++i)
+        if (!g.used[i]) {
+          g.used[i] = true;
+          return reinterpret_cast<double*>(g.p + i * kSlot);
+        }
+    char* p = static_cast<char*>(std::aligned_alloc(4096, kPage));
+    if (!p) return nullptr;
+    std::memset(p, 0, kPage);
+    if (cudaHostRegister(p, kPage, cudaHostRegisterPortable) != cudaSuccess) {
+      cudaGetLastError();
+      std::free(p);
+      return nullptr;
+    }
+    pages.push_back(Page{p, {}});
+    pages.back().used[0] = true;
+    return reinterpret_cast<double*>(p);
+  }
+  void give(double* slot) {
+    std::lock_guard<std::mutex> lock(m);
+    char* at = reinterpret_cast<char*>(slot);
+    for (size_t k = 0; k < pages.size(); ++k) {
+      Page& g = pages[k];
+      if (at < g.p || at >= g.p + kPage) continue;
+      g.used[(size_t)(at - g.p) / kSlot] = false;
+      if (g.used.none()) {
+        cudaHostUnregister(g.p);
+        std::free(g.p);
+        pages.erase(pages.begin() + (long)k);
+      }
+      return;
+    }
+  }
+};
+ReadSlots& read_slots() {
+  static ReadSlots* s = new ReadSlots;  // drivers may outlive static objects
+  return *s;
+}
+
 // Block b's field with at(i, lo, hi) giving the two solutions at index i
 template <class At>
 __device__ __forceinline__ void error_sums(const KeyTable& kt, const unsigned* __restrict__ flags,
@@ -518,12 +580,16 @@ int QDContext::create(const scy_qd_desc& d, const scy_pl_desc* pld) {
   SCY_TRY(errbuf.alloc(RB_SIZE * 8));
   SCY_CUDA_TRY(cudaMemset(errbuf.p, 0, RB_SIZE * 8));
   SCY_TRY(slipVel0.alloc((size_t)Nz * 8));
-  SCY_CUDA_TRY(cudaMallocHost((void**)&h_read, RB_SIZE * 8));
+  h_read = read_slots().take();
+  if (!h_read) {
+    set_error("no pinned memory for a driver's read-backs");
+    return SCY_ERR_NOMEM;
+  }
   return SCY_OK;
 }
 
 QDContext::~QDContext() {
-  if (h_read) cudaFreeHost(h_read);
+  if (h_read) read_slots().give(h_read);
 }
 
 int QDContext::read_flags() {
