@@ -287,15 +287,17 @@ def run_batched(args, dist, rank, world, local):
         peak, peak_src = 6650.0, "fallback"
     # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of
     # ncu captures of these kernels at 32 instances of the 401 x 401 workload
-    # (profiles/batched_ensemble_kernels_401x401.md,
-    # profiles/ozk_gemm_kernel_S5_12832x401x401.md,
-    # profiles/b_full_kernel_32x401x401.md,
-    # profiles/march_walks_2049x1537_and_32x401x401.md); other sizes report none
+    # (profiles/solver_kernels_by_counters.md, caches as the kernels before left
+    # them; the forms of the CG path profiles/b_full_kernel_32x401x401.md and
+    # profiles/batched_ensemble_kernels_401x401.md); other sizes report none
     sep = b.tuning(0)["operator_form"] != "cross"
     corr = sep and args.batch_precision == "fp64"  # defect corrections instead of CG on this workload
-    traffic = {"ysolve": 65362176.0, "ztransform": 28774656.0} if (args.batch == 32 and args.n == 401) else {}
+    traffic = {}
     if args.batch == 32 and args.n == 401:
-        traffic.update({"matvec": 150265600.0 if corr else 99618816.0, "residual": 98234880.0} if sep else
+        traffic = {"ysolve": 37264128.0, "ztransform": 43820672.0, "zsplit": 45531648.0} if corr else \
+            {"ysolve": 65362176.0}
+        traffic.update({"matvec": 178510080.0, "residual": 140837632.0} if corr else
+                       {"matvec": 99618816.0, "residual": 98234880.0} if sep else
                        {"matvec": 178643456.0, "residual": 187187968.0})
     opk = "b_full_kernel<%d> (separable form: 1D coefficient tables, tiles or walks by warps)" if sep else \
         "b_cross_kernel<%d> (cross form: 33 coefficient planes)"
@@ -423,7 +425,8 @@ def run_c0(args):
     out = {"workload": C0_WORKLOAD, "steps": st.step_count, "stage_solves": st.d_dt_evals, "wall_s": wall,
            "sim_years": st.t / YEAR, "sim_years_per_hour": (st.t / YEAR) / (wall / 3600.0),
            "stage_solves_per_s": st.d_dt_evals / wall,
-           "oracle_error": oracle_errors("c0", lambda w: aging_const_101(w, seed=0))}
+           "oracle_error": oracle_errors("c0", lambda w: aging_const_101(w, seed=0)),
+           "oracle_error_at_timed_rtol": oracle_errors("c0", lambda w: aging_const_101(w, seed=0), args.rtol)}
     if not args.no_cpu_baseline:
         r = oracle_on_all_cores("c0", 10 ** 8, max_workers=1)
         out["cpu_oracle_one_core"] = {"wall_s": r["timed_s_max"], "stage_solves": r["stage_solves"],
@@ -783,8 +786,10 @@ def run_ours(args, dist, rank, world, local):
     head = batched if batched else single
     if batched:
         config = batch_config(args, world)
-        solver = ("FP64 CG preconditioned by fast diagonalisation (%s preconditioner; z transforms on the integer "
-                  "tensor cores, banded sweeps along y), device-verified rtol %g" % (args.batch_precision, args.rtol))
+        solver = ("FP64 %s by fast diagonalisation (%s preconditioner; z transforms on the integer "
+                  "tensor cores, banded sweeps along y), device-tested rtol %g"
+                  % ("defect correction" if args.batch_precision == "fp64" else "CG preconditioned",
+                     args.batch_precision, args.rtol))
         l2 = "not flushed: the ensemble's working set (about 20 MB per instance) exceeds the 126 MB L2"
     else:
         config = {"workload": WORKLOAD, "Ny": args.n, "Nz": args.n, "integrator": "RK32",

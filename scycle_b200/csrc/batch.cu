@@ -1385,8 +1385,8 @@ int BatchContext::autotune(BatchGroup& g) {
   g.full_shape = -1;
   if (g.L.full) {
     // defect correction where the preconditioner is near enough to the
-    // inverse; its launch moves u, so it is timed on a table whose u is a
-    // work vector
+    // inverse (for the power law too, see SbpContext::keep_rounding); its launch
+    // moves u, so it is timed on a table whose u is a work vector
     g.refine = precision == SCY_PREC_FP64 && q(g.base).sbp.near_inverse() && g.fd->ybanded && !fd_dense;
     DevBuf scratch;
     if (g.refine) {

@@ -7,9 +7,10 @@
 namespace scy {
 
 // A node's parameters, laid out by the host: a launch requests them ahead of
-// what it waits for (the kernel before, the node's stress).  Eight response
-// steps at 401 nodes take 592 us so and 640 with the loads in the update,
-// four solve steps at 101 x 101 775 and 787.
+// what it waits for (the kernel before, the node's stress).  In turn on one
+// GPU eight response steps at 401 nodes took 592 us so and 640 with the loads
+// in the update, four solve steps at 101 x 101 775 and 787 (600 to 617 and 760
+// to 780 over several GPUs).
 struct FaultNode {
   double prestress, a, b, sN, Dc, eta, locked;
 };

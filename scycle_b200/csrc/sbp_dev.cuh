@@ -1175,9 +1175,10 @@ inline void launch_apply(const LevelDev<T>& L, const Loader& ld, const Epi& ep, 
   const dim3 g = apply_grid(L);
   if constexpr (TakesMarch<Epi>::value) {
     // below, nearly all of the grid is edge, and the tiles are as fast or
-    // faster (a call at 61 x 61: 20.5 us in tiles, 21.5 in walks; 257 x 129:
-    // 21.2 and 21.6; 401 x 401: 23.6 and 22.8; 1201 x 1201: 34.7 and 31.9;
-    // 2049 x 1537: 45.0 and 40.9; 4097 x 3073: 107.8 and 94.1)
+    // faster (calls one after the other, at 61 x 61: 20.9 us in tiles, 21.7 in
+    // walks; 257 x 129: 21.3 and 22.0; 257 x 257: 21.6 and 21.9; 401 x 401:
+    // 23.1 and 22.6; 1201 x 1201: 34.1 and 31.1; 2049 x 1537: 44.4 and 40.4;
+    // 4097 x 3073: 107.4 and 93.6)
     if (L.full && (long)L.Ny * L.Nz >= 65536) {
       const MarchPlan p = march_plan(L, march_chunks(L));
       chain_launch(march_kernel<T, Loader, Epi>, p.blocks, 32 * kMarchWarps, 0, s, L, ld, ep, p);

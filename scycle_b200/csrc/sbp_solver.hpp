@@ -153,13 +153,16 @@ struct SbpContext {
            o.max_its >= kCorrectIts;
   }
   bool near_inverse() const { return separable && sep_misfit <= 0.25; }
-  // Solves that keep the arithmetic of plain CG with whole sweep chains: those of the
-  // power-law driver (keep_rounding: its viscous strain gVxz starts as a
-  // difference of displacements that agree to rounding, so its first digits
-  // are the solve's own rounding) and those asked for to near rounding, whose
-  // results are compared digit by digit with earlier runs (replays of
-  // recorded step sequences).  At 1e-13 the tolerance is a few hundred
-  // roundings of the residual.
+  // Solves that keep the arithmetic of plain CG with whole sweep chains: those
+  // asked for to near rounding and those of the single power-law driver
+  // (keep_rounding), whose results are compared digit by digit with earlier
+  // runs (replays of recorded step sequences; the viscous strain gVxz starts as
+  // a difference of displacements that agree to rounding, so its first digits
+  // are the solve's own rounding).  At 1e-13 the tolerance is a few hundred
+  // roundings of the residual.  It is no matter of accuracy: power-law batches
+  // solve by defect correction, and after 30 steps at 1e-12 on stretched grids
+  // their gVxz is 3e-12 to 5e-12 from the oracle's replay, the single driver's
+  // 7e-11 to 3e-10, a batch's by CG 1e-12 to 2e-11.
   int keep_rounding = 0;
   bool keeps_rounding(double rtol) const { return keep_rounding || rtol < 1e-13; }
   Reducer red;

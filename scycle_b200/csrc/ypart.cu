@@ -321,6 +321,8 @@ int launch_one(const YPartArgs& A, size_t smem, int nb, int NG, cudaStream_t s, 
   return SCY_OK;
 }
 
+// (rows a thread; from 24 on two instances a thread spill, 40 bytes there to 1300
+// at 48, and the autotuner times the forms with one beside them)
 constexpr int kT[] = {8, 12, 16, 20, 24, 28, 32, 40, kMaxT};
 }  // namespace
 
